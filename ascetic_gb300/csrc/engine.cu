@@ -136,10 +136,7 @@ struct RegionArgs {
     uint32_t in_resident;         // in_edges is device memory (a graph without a cap), else pinned host
     const uint32_t *in_heads;     // first in-edge of every vertex in HBM (a bit stream of in_ebits), or null
     const uint32_t *in_none;      // one bit per vertex without in-edges (never reached but as a source)
-    // standard PageRank pull, on-demand region: tiles copy their in-edge range
-    // through shared memory (see pr_vertices); edge_words bounds those reads
-    uint32_t stage_edges;
-    uint64_t edge_words;
+    uint64_t edge_words;          // words that may be read at edges (item passes of PageRank)
 };
 
 // True when this BFS iteration steps bottom-up: its input frontier (the
@@ -1088,15 +1085,8 @@ __device__ __forceinline__ void block_reduce2_atomic(double a, double b, double 
 #define ASC_PR_UNROLL 4
 #endif
 constexpr int kPrUnroll = ASC_PR_UNROLL;
-// Edge words a pull tile copies into shared memory per chunk (8 KB).
-#ifndef ASC_PR_STAGE_WORDS
-#define ASC_PR_STAGE_WORDS 2048
-#endif
-constexpr uint32_t kPrStageWords = ASC_PR_STAGE_WORDS;
-
 template <typename T>
 struct PrSmem {
-    alignas(16) uint32_t stage[kPrStageWords];
     uint32_t pref[kBlock + 1];
     uint32_t start[kBlock];
     uint32_t warp[kWarps + 1];
@@ -1104,95 +1094,6 @@ struct PrSmem {
     double red[2 * kWarps];
     uint32_t work;
 };
-
-// Sums the in-edge contributions of a standard-PageRank tile (consecutive
-// vertices, no long list, so their in-edges are one range [E0, E0 + total),
-// E0 = the first vertex's offset) with the range read through shared memory:
-// the CTA copies kPrStageWords edge words at a time with 16-byte loads, so
-// the host link serves runs of several KB per tile instead of one 128-byte
-// line per warp load, then every thread decodes its edges from shared memory
-// and gathers their contributions, kPrUnroll edges in flight. The summation
-// order is a fixed function of the range (same partials every pass).
-template <typename T>
-__device__ void pr_vertices_staged(const PrArgs<T> &p, uint32_t total, PrSmem<T> &sm) {
-    const RegionArgs &a = p.r;
-    const int lane = threadIdx.x & 31;
-    const uint32_t eb = a.ebits;
-    const uint64_t E0 = sm.start[0];
-    uint4 *st4 = reinterpret_cast<uint4 *>(sm.stage);
-    for (uint32_t c0 = 0; c0 < total;) {
-        // words [w_lo, w_end): edges [c0, c1) of the tile, w_lo 16-byte aligned
-        const uint64_t w_lo = (((E0 + c0) * eb) >> 5) & ~3ull;
-        const uint64_t cap_edges = (w_lo + kPrStageWords) * 32 / eb;  // edges ending in the chunk
-        const uint32_t c1 = (uint32_t)min((uint64_t)total, cap_edges - E0);
-        const uint64_t w_end = ((E0 + c1) * eb + 31) >> 5;
-        const uint32_t nq = (uint32_t)((w_end - w_lo + 3) >> 2);
-        for (uint32_t i = threadIdx.x; i < nq; i += kBlock) {
-            const uint64_t w = w_lo + 4ull * i;
-            uint4 q;
-            if (w + 4 <= a.edge_words) {
-                q = __ldg(reinterpret_cast<const uint4 *>(a.edges + w));
-            } else {  // the buffer's last words
-                q.x = w < a.edge_words ? __ldg(a.edges + w) : 0u;
-                q.y = w + 1 < a.edge_words ? __ldg(a.edges + w + 1) : 0u;
-                q.z = w + 2 < a.edge_words ? __ldg(a.edges + w + 2) : 0u;
-                q.w = 0u;
-            }
-            st4[i] = q;
-        }
-        __syncthreads();
-        const uint64_t bit0 = w_lo * 32;
-        for (uint32_t base = c0; base < c1; base += kPrUnroll * kBlock) {
-            T x[kPrUnroll];
-            int owner[kPrUnroll];
-            uint32_t srcv[kPrUnroll];
-#pragma unroll
-            for (int k = 0; k < kPrUnroll; k++) {
-                const uint32_t e = base + k * kBlock + threadIdx.x;
-                owner[k] = -1 - lane;  // distinct per invalid lane
-                srcv[k] = 0xffffffffu;
-                if (e < c1) {
-                    int lo = 0, hi = kBlock;
-                    while (hi - lo > 1) {
-                        int mid = (lo + hi) >> 1;
-                        if (sm.pref[mid] <= e) lo = mid;
-                        else hi = mid;
-                    }
-                    owner[k] = lo;
-                    const uint32_t bit = (uint32_t)((E0 + e) * eb - bit0);
-                    const uint32_t wi = bit >> 5, sh = bit & 31u;
-                    uint32_t v = sm.stage[wi] >> sh;
-                    if (eb < 32) {
-                        if (sh + eb > 32) v |= sm.stage[wi + 1] << (32 - sh);
-                        v &= (1u << eb) - 1u;
-                    }
-                    srcv[k] = v;
-                    if (ASC_BAD(srcv[k] >= a.V, 22, srcv[k])) {
-                        srcv[k] = 0xffffffffu;
-                        owner[k] = -1 - lane;
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kPrUnroll; k++) x[k] = srcv[k] != 0xffffffffu ? p.c_old[srcv[k]] : (T)0;
-#pragma unroll
-            for (int k = 0; k < kPrUnroll; k++) {
-                T xs = x[k];
-                const int ow = owner[k];
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    T y = __shfl_down_sync(kFull, xs, d);
-                    int oy = __shfl_down_sync(kFull, ow, d);
-                    if (lane + d < 32 && oy == ow) xs += y;
-                }
-                int oprev = __shfl_up_sync(kFull, ow, 1);
-                if (ow >= 0 && (lane == 0 || oprev != ow)) atomicAdd(&sm.sum[ow], PrAcc<T>::from(xs));
-            }
-        }
-        __syncthreads();  // the stage is rewritten by the next chunk
-        c0 = c1;
-    }
-}
 
 // Reference mode walks the active set like a traversal frontier (list, or
 // the bitmap in id order when dense) and a vertex that stays active sets its
@@ -1221,9 +1122,7 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
     // base + k * kBlock + thread): every source id is loaded, then every
     // contribution gathered, before any is summed, so a thread has kPrUnroll
     // reads in flight instead of one
-    const bool staged = !REF && a.stage_edges && !__syncthreads_or(valid && huge);
-    if (staged) pr_vertices_staged<T>(p, total, sm);
-    for (uint32_t base = 0; !staged && base < total; base += kPrUnroll * kBlock) {
+    for (uint32_t base = 0; base < total; base += kPrUnroll * kBlock) {
         T x[kPrUnroll];
         int owner[kPrUnroll];
         uint32_t srcv[kPrUnroll];
@@ -1317,62 +1216,7 @@ __device__ void pr_segment(const PrArgs<T> &p, uint64_t item, PrSmem<T> &sm) {
     const uint64_t e = min((uint64_t)e0, b + a.seg_len);
     const uint32_t n = (uint32_t)(e - b);
     T x = (T)0;  // this thread's edges in order, then a fixed warp tree
-    if (a.stage_edges) {
-        // the segment's range through shared memory, as a staged tile: thread
-        // t still adds edges t, t + kBlock, ... in order
-        const uint32_t eb = a.ebits;
-        uint4 *st4 = reinterpret_cast<uint4 *>(sm.stage);
-        for (uint32_t c0 = 0; c0 < n;) {
-            const uint64_t w_lo = (((b + c0) * eb) >> 5) & ~3ull;
-            const uint64_t cap_edges = (w_lo + kPrStageWords) * 32 / eb;
-            const uint32_t c1 = (uint32_t)min((uint64_t)n, cap_edges - b);
-            const uint64_t w_end = ((b + c1) * eb + 31) >> 5;
-            const uint32_t nq = (uint32_t)((w_end - w_lo + 3) >> 2);
-            for (uint32_t i = threadIdx.x; i < nq; i += kBlock) {
-                const uint64_t w = w_lo + 4ull * i;
-                uint4 q;
-                if (w + 4 <= a.edge_words) {
-                    q = __ldg(reinterpret_cast<const uint4 *>(a.edges + w));
-                } else {
-                    q.x = w < a.edge_words ? __ldg(a.edges + w) : 0u;
-                    q.y = w + 1 < a.edge_words ? __ldg(a.edges + w + 1) : 0u;
-                    q.z = w + 2 < a.edge_words ? __ldg(a.edges + w + 2) : 0u;
-                    q.w = 0u;
-                }
-                st4[i] = q;
-            }
-            __syncthreads();
-            const uint64_t bit0 = w_lo * 32;
-            const uint32_t first = c0 + ((threadIdx.x + kBlock - c0 % kBlock) % kBlock);
-            for (uint32_t j0 = first; j0 < c1; j0 += kPrUnroll * kBlock) {
-                uint32_t sv[kPrUnroll];
-#pragma unroll
-                for (int k = 0; k < kPrUnroll; k++) {
-                    const uint32_t j = j0 + k * kBlock;
-                    sv[k] = 0xffffffffu;
-                    if (j < c1) {
-                        const uint32_t bit = (uint32_t)((b + j) * eb - bit0);
-                        const uint32_t wi = bit >> 5, sh = bit & 31u;
-                        uint32_t v = sm.stage[wi] >> sh;
-                        if (eb < 32) {
-                            if (sh + eb > 32) v |= sm.stage[wi + 1] << (32 - sh);
-                            v &= (1u << eb) - 1u;
-                        }
-                        sv[k] = ASC_BAD(v >= a.V, 23, v) ? 0xffffffffu : v;
-                    }
-                }
-                T c[kPrUnroll];
-#pragma unroll
-                for (int k = 0; k < kPrUnroll; k++) c[k] = sv[k] != 0xffffffffu ? p.c_old[sv[k]] : (T)0;
-#pragma unroll
-                for (int k = 0; k < kPrUnroll; k++)
-                    if (sv[k] != 0xffffffffu) x += c[k];
-            }
-            __syncthreads();
-            c0 = c1;
-        }
-    }
-    for (uint32_t j0 = threadIdx.x; !a.stage_edges && j0 < n; j0 += kPrUnroll * kBlock) {
+    for (uint32_t j0 = threadIdx.x; j0 < n; j0 += kPrUnroll * kBlock) {
         // kPrUnroll loads in flight, added in edge order
         uint32_t sv[kPrUnroll];
 #pragma unroll
@@ -1536,6 +1380,330 @@ __global__ void pr_apply_segmented_kernel(PrArgs<T> p, const uint64_t *items_sta
     if (!REF) block_reduce2_atomic<T>(res, dang, p.acc, red);
 }
 
+// ------------------------------------------- edge-balanced PageRank passes --
+//
+// A standard pass reads every edge once, so its work is cut by position in the
+// merge of the rows (each counted at its end) and the edges, not by vertices:
+// item i covers merge positions [i*L, (i+1)*L), whatever the degrees, and is
+// the range of rows that end in it plus the range of its edges. A plan kernel
+// finds the items' first (row, edge) by binary search over the offsets, once
+// per workspace. Tiles of 256 vertices held from none to 131,000 edges (lists
+// of up to 512 each), every edge searched its owner in shared memory, and a
+// segmented 5-step shuffle sum ran per edge: 197 instructions per edge (ncu,
+// FP64 pull, 25.5 M edges), with 5 FP64 adds per edge on a pipe that takes 16
+// cycles per warp instruction.
+//
+// Here every row that ends in the item marks its last edge, a thread takes
+// kPrVt consecutive edges and closes a sum at each mark, and one segmented warp
+// scan joins the sums of rows that cross threads: one add per edge and no
+// search. Bound by the host link (30% resident: 2.29 of the 2.5 ms a pass takes
+// on RMAT scale 24, FP32; 172 of 215 us on 25.5 M edges, FP64).
+// Standard PageRank to 1e-9 before / after: FP32, RMAT scale 24, 101.0 / 73.5 ms
+// (its passes 3.26 / 2.53 ms); FP64, 1.5 M vertices of degree 17, 11.5 / 5.06 ms.
+// CTAs of 256 threads, 6 per SM: 73.5 and 5.06 ms; 128 threads, 12 per SM: 75.2
+// and 5.06 (8 per SM: 77.7, 5.10); 64 threads, 24 per SM: 104.3, 5.25. Shared
+// memory of more CTAs takes the L1 that holds the gathers in flight: 14 CTAs of
+// 128 threads measured 121.7 and 8.1 ms.
+#ifndef ASC_PR_ITEM_THREADS
+#define ASC_PR_ITEM_THREADS 256
+#endif
+#ifndef ASC_PR_ITEM_BLOCKS
+#define ASC_PR_ITEM_BLOCKS 6
+#endif
+constexpr int kPrThreads = ASC_PR_ITEM_THREADS;
+constexpr int kPrWarps = kPrThreads / 32;
+constexpr int kPrVt = 8;                          // edges per thread
+constexpr uint32_t kPrItem = kPrThreads * kPrVt;  // merge positions per item
+
+// First (row, edge) of every item; items[n] is the end. Region 0 is the rows
+// [0, S), region 1 the rows [S, V); each starts at an item boundary.
+__global__ void pr_plan_kernel(const uint32_t *ptr, uint32_t S, uint32_t V, uint32_t L, uint32_t n0, uint32_t n,
+                               uint2 *items) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+        if (i == n) {
+            items[i] = make_uint2(V, ptr[V]);
+            continue;
+        }
+        const uint32_t R0 = i < n0 ? 0 : S, R1 = i < n0 ? S : V;
+        const uint32_t E0 = ptr[R0];
+        const uint64_t d = (uint64_t)(i - (i < n0 ? 0 : n0)) * L;
+        // row r ends at merge position (its end - E0) + (r - R0): rows ending before d
+        uint32_t lo = 0, hi = R1 - R0;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if ((uint64_t)(ptr[R0 + mid + 1] - E0) + mid < d) lo = mid + 1;
+            else hi = mid;
+        }
+        items[i] = make_uint2(R0 + lo, E0 + (uint32_t)(d - lo));
+    }
+}
+
+// A range of items and where their edges are read.
+struct PrSlice {
+    const uint32_t *edges;   // indexed by global edge offset
+    uint64_t edge_words;     // words that may be read there
+    uint32_t begin, n;       // items [begin, begin + n)
+};
+
+template <typename T>
+struct PrItemArgs {
+    typedef typename PrAcc<T>::type Acc;
+    const uint2 *items;
+    PrSlice sl[2];           // static, on-demand
+    const uint32_t *ptr;
+    const uint32_t *outdeg;
+    double *rank;
+    const T *c_old;
+    T *c_new;
+    Acc *sum;                // sums of the rows cut by item boundaries (zero between passes)
+    double damping;
+    const double *dangling_prev;   // dangling mass of the previous pass
+    double *acc;             // [0] residual, [1] dangling of this pass
+    uint32_t *work;
+    uint32_t V, ebits;
+};
+
+template <typename T>
+struct PrItemSmem {
+    // the item's edge words, then its row sums: at most ne words and 2 (nr + 1)
+    // words with nr + ne <= kPrItem, plus alignment and one word read past the end
+    alignas(16) uint32_t pool[2 * kPrItem + 16];
+    uint16_t row_at[kPrItem];       // of an edge that ends a row: the row, from the item's first
+    uint32_t marks[2][kPrItem / 32];  // one bit per edge: it ends a row (this item's, the next one's)
+    double red[2 * kPrWarps];
+    double base;
+    uint32_t work[2];
+};
+
+// Copies the words holding edges [e0, e0 + ne) to smem with 16-byte loads (so
+// the host link serves runs of several KB); returns the bit of edge e0 there.
+__device__ __forceinline__ uint32_t pr_stage_words(const PrSlice &s, uint32_t e0, uint32_t ne, uint32_t eb,
+                                                   uint32_t *pool, uint32_t &nq) {
+    const uint64_t bit = (uint64_t)e0 * eb;
+    const uint64_t w_lo = (bit >> 5) & ~3ull;
+    nq = ne ? (uint32_t)(((((uint64_t)e0 + ne) * eb + 31) / 32 - w_lo + 3) >> 2) : 0;
+    for (uint32_t i = threadIdx.x; i < nq; i += kPrThreads) {
+        const uint64_t w = w_lo + 4ull * i;
+        uint4 q;
+        if (w + 4 <= s.edge_words) {
+            q = __ldg(reinterpret_cast<const uint4 *>(s.edges + w));
+        } else {  // the buffer's last words
+            q.x = w < s.edge_words ? __ldg(s.edges + w) : 0u;
+            q.y = w + 1 < s.edge_words ? __ldg(s.edges + w + 1) : 0u;
+            q.z = w + 2 < s.edge_words ? __ldg(s.edges + w + 2) : 0u;
+            q.w = 0u;
+        }
+        reinterpret_cast<uint4 *>(pool)[i] = q;
+    }
+    return (uint32_t)(bit - 32 * w_lo);
+}
+
+__device__ __forceinline__ uint32_t pr_staged_edge(const uint32_t *pool, uint32_t bit, uint32_t mask) {
+    return __funnelshift_r(pool[bit >> 5], pool[(bit >> 5) + 1], bit & 31u) & mask;
+}
+
+// Marks the rows that end in an item (r0 .. r0 + nr - 1, edges from e0) at
+// their last edges; rows without edges have none. Every thread calls it.
+template <typename T>
+__device__ __forceinline__ void pr_mark_rows(const uint32_t *ptr, uint32_t r0, uint32_t e0, uint32_t nr,
+                                             PrItemSmem<T> &sm, uint32_t *marks) {
+    for (uint32_t j = threadIdx.x; j < nr; j += kPrThreads) {
+        const uint32_t lo = max(ptr[r0 + j], e0), hi = ptr[r0 + j + 1];
+        if (hi > lo) {
+            const uint32_t x = hi - 1 - e0;
+            sm.row_at[x] = (uint16_t)j;
+            atomicOr(&marks[x >> 5], 1u << (x & 31));
+        }
+    }
+}
+
+// Item w of a launch over both slices: the on-demand and the static slice
+// alternate while both have items, so every SM overlaps host-link reads with
+// HBM reads.
+__device__ __forceinline__ uint32_t pr_slice_item(const PrSlice *sl, uint32_t w, bool &od) {
+    const uint32_t i0 = sl[0].n, i1 = sl[1].n, m = min(i0, i1);
+    uint32_t local;
+    if (w < 2 * m) {
+        od = (w & 1) == 0;
+        local = w >> 1;
+    } else {
+        od = i1 > i0;
+        local = m + (w - 2 * m);
+    }
+    return sl[od].begin + local;
+}
+
+// The update of one vertex from its sum (as pr_update's standard mode), with
+// the pass's constant part (1 - d) / V + d * dangling / V given.
+template <typename T>
+__device__ __forceinline__ void pr_std_row(const PrItemArgs<T> &p, uint32_t v, double s, double base, double &res,
+                                           double &dang) {
+    const uint32_t od = p.outdeg[v];
+    const double r = p.rank[v];
+    const double rn = base + p.damping * s;
+    res += fabs(rn - r);
+    p.rank[v] = rn;
+    T c = (T)0;
+    if (od) c = (T)(rn / (double)od);
+    else dang += rn;
+    p.c_new[v] = c;
+}
+
+// block_reduce2_atomic for the item kernels' blocks.
+__device__ __forceinline__ void pr_reduce2_atomic(double a, double b, double *out, double *s_buf) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        a += __shfl_down_sync(kFull, a, d);
+        b += __shfl_down_sync(kFull, b, d);
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) {
+        s_buf[2 * w] = a;
+        s_buf[2 * w + 1] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < kPrWarps; i++) {
+            a += s_buf[2 * i];
+            b += s_buf[2 * i + 1];
+        }
+        if (a != 0) atomicAdd(&out[0], a);
+        if (b != 0) atomicAdd(&out[1], b);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_kernel(PrItemArgs<T> p) {
+    typedef typename PrAcc<T>::type Acc;
+    __shared__ PrItemSmem<T> sm;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = p.sl[0].n + p.sl[1].n;
+    const uint32_t eb = p.ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    if (threadIdx.x < kPrItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        sm.work[0] = atomicAdd(p.work, 1u);
+        sm.base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
+    }
+    __syncthreads();
+    double res = 0, dang = 0;
+    for (int buf = 0;; buf ^= 1) {
+        const uint32_t w = sm.work[buf];
+        if (w >= total) break;
+        bool od;
+        const uint32_t it = pr_slice_item(p.sl, w, od);
+        const uint2 a = p.items[it], b = p.items[it + 1];
+        const uint32_t r0 = a.x, e0 = a.y, nr = b.x - a.x, ne = b.y - a.y;
+        uint32_t nq;
+        const uint32_t bit0 = pr_stage_words(p.sl[od], e0, ne, eb, sm.pool, nq);
+        Acc *sums = reinterpret_cast<Acc *>(sm.pool + 4 * nq + (nq ? 4 : 0));
+        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads) sums[j] = (Acc)0;
+        uint32_t *marks = sm.marks[buf];
+        pr_mark_rows<T>(p.ptr, r0, e0, nr, sm, marks);
+        if (threadIdx.x == 0) sm.work[buf ^ 1] = atomicAdd(p.work, 1u);
+        __syncthreads();
+        if (threadIdx.x < kPrItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
+        const uint32_t x0 = threadIdx.x * kPrVt, xw = x0 - lane * kPrVt;  // first edge of the thread, the warp
+        if (xw < ne) {
+            T c[kPrVt];
+#pragma unroll
+            for (int k = 0; k < kPrVt; k++) {
+                c[k] = (T)0;
+                if (x0 + k < ne) {
+                    const uint32_t v = pr_staged_edge(sm.pool, bit0 + (x0 + k) * eb, mask);
+                    if (!ASC_BAD(v >= p.V, 21, v)) c[k] = __ldg(p.c_old + v);
+                }
+            }
+            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kPrVt) - 1u);
+            // a thread's first sum may go on from earlier threads; later ones are its own
+            T part = (T)0, head = (T)0;
+#pragma unroll
+            for (int k = 0; k < kPrVt; k++) {
+                part += c[k];
+                if ((ends >> k) & 1u) {
+                    if (ends & ((1u << k) - 1u)) sums[sm.row_at[x0 + k]] = PrAcc<T>::from(part);
+                    else head = part;
+                    part = (T)0;
+                }
+            }
+            // open sums, scanned over the lanes: a lane with an end starts a new one
+            Acc tail = PrAcc<T>::from(part);
+            const unsigned ended = __ballot_sync(kFull, ends != 0);
+            // lanes since (and with) the last one that starts a sum
+            const uint32_t below = ended & (0xffffffffu >> (31 - lane));
+            const int run = below ? lane - (31 - __clz((int)below)) : lane + 1;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                if (!__any_sync(kFull, run >= d)) break;
+                const Acc y = __shfl_up_sync(kFull, tail, d);
+                if (run >= d && lane >= d) tail += y;
+            }
+            Acc before = __shfl_up_sync(kFull, tail, 1);
+            if (lane == 0) before = (Acc)0;
+            if (ends) {
+                const Acc h = PrAcc<T>::from(head) + before;
+                const uint32_t row = sm.row_at[x0 + __ffs((int)ends) - 1];
+                // the warp's first row may have begun in another warp
+                if (ended & ((1u << lane) - 1u)) sums[row] = h;
+                else atomicAdd(&sums[row], h);
+            }
+            // the warp's last open sum goes to the row that ends after it: the
+            // next mark, or the row that goes on past the item
+            const uint32_t xe = xw + 32 * kPrVt;
+            if (xe < ne || !((marks[(ne - 1) >> 5] >> ((ne - 1) & 31)) & 1u)) {
+                uint32_t row = nr;
+                for (uint32_t m0 = xe >> 5; m0 < kPrItem / 32; m0 += 32) {
+                    const uint32_t word = m0 + lane < kPrItem / 32 ? marks[m0 + lane] : 0u;
+                    const unsigned any = __ballot_sync(kFull, word != 0);
+                    if (any) {
+                        const int q = __ffs((int)any) - 1;
+                        const uint32_t bits = __shfl_sync(kFull, word, q);
+                        row = sm.row_at[32 * (m0 + q) + __ffs((int)bits) - 1];
+                        break;
+                    }
+                }
+                if (lane == 31) atomicAdd(&sums[row], tail);
+            }
+        }
+        __syncthreads();
+        // rows that end here are final, but for a first one that began in an
+        // earlier item; that one and the row that goes on past the item add to
+        // the global sums (pr_cut_rows_kernel applies them)
+        const bool cut = p.ptr[r0] < e0;
+        const bool goes_on = ne && !((marks[(ne - 1) >> 5] >> ((ne - 1) & 31)) & 1u);
+        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads) {
+            if (j == nr ? goes_on : (j == 0 && cut)) {
+                atomicAdd(&p.sum[r0 + j], sums[j]);
+            } else if (j < nr) {
+                pr_std_row<T>(p, r0 + j, PrAcc<T>::value(sums[j]), sm.base, res, dang);
+            }
+        }
+        __syncthreads();
+    }
+    pr_reduce2_atomic(res, dang, p.acc, sm.red);
+}
+
+// Applies the rows that were cut by an item boundary: the row at the start of
+// item i, when it began earlier and ends in item i.
+template <typename T>
+__global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n) {
+    __shared__ double red[2 * kWarps];
+    __shared__ double s_base;
+    if (threadIdx.x == 0)
+        s_base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
+    __syncthreads();
+    double res = 0, dang = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 a = p.items[i];
+        const uint32_t r_end = p.items[i + 1].x;
+        if (r_end > a.x && p.ptr[a.x] < a.y) {
+            const double s = PrAcc<T>::value(p.sum[a.x]);
+            p.sum[a.x] = 0;
+            pr_std_row<T>(p, a.x, s, s_base, res, dang);
+        }
+    }
+    block_reduce2_atomic<T>(res, dang, p.acc, red);
+}
+
 template <typename T>
 __global__ void pr_init_kernel(double *rank, T *c0, T *c1, typename PrAcc<T>::type *sum, const uint32_t *outdeg,
                                uint32_t V, double *dang) {
@@ -1684,6 +1852,27 @@ asc_status ensure_pr_buffers(asc_graph *g, size_t elem) {
     return ASC_OK;
 }
 
+// Work items of the edge-balanced PageRank passes (pr_plan_kernel), made once
+// per workspace.
+uint64_t pr_item_count(uint64_t rows, uint64_t edges) { return (rows + edges + kPrItem - 1) / kPrItem; }
+uint64_t pr_items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * (pr_item_count(V, E) + 2); }
+
+asc_status ensure_pr_items(asc_graph *g) {
+    Workspace *ws = g->ws;
+    if (ws->pr_items) return ASC_OK;
+    const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
+    const uint64_t n0 = pr_item_count(S, g->h_ptr[S]), n1 = pr_item_count(V - S, g->E - g->h_ptr[S]);
+    ASC_CUDA(cudaMalloc((void **)&ws->pr_items, sizeof(uint2) * (n0 + n1 + 1)));
+    ws->device_bytes += sizeof(uint2) * (n0 + n1 + 1);
+    ws->n_items_static = (uint32_t)n0;
+    ws->n_items = (uint32_t)(n0 + n1);
+    const uint64_t blocks = std::min<uint64_t>((n0 + n1) / kBlock + 1, (uint64_t)ws->num_sms * 8);
+    pr_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, kPrItem, ws->n_items_static,
+                                                               ws->n_items, ws->pr_items);
+    ASC_CUDA(cudaGetLastError());
+    return ASC_OK;
+}
+
 RegionArgs base_args(asc_graph *g, Workspace *ws, int parity_in) {
     RegionArgs a;
     memset(&a, 0, sizeof(a));
@@ -1740,14 +1929,6 @@ RegionArgs region_args(asc_graph *g, Workspace *ws, int parity_in, int region, b
     return a;
 }
 
-// Standard PageRank pulls the on-demand region's tiles through shared memory
-// (pr_vertices_staged) on single-word edge layouts; ASC_PR_TILE_STAGE=0 reads
-// every edge word with its own load instead (for comparison).
-bool pr_tile_stage(const asc_graph *g) {
-    const char *env = getenv("ASC_PR_TILE_STAGE");
-    return g->edge_words == 1 && !(env && env[0] == '0');
-}
-
 RegionArgs region_args(asc_graph *g, int parity_in, int region, bool dense) {
     return region_args(g, g->ws, parity_in, region, dense);
 }
@@ -1772,6 +1953,11 @@ uint32_t grid_for(const Workspace *ws, uint64_t work_items) {
 uint32_t bu_grid(const Workspace *ws, uint64_t nwords) {
     const uint64_t blocks = (nwords + kBuWords * (kBlock / 32) - 1) / (kBuWords * (kBlock / 32));
     return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)ws->num_sms * kBuMinBlocks));
+}
+
+// One wave of the item kernels' CTAs, or one per item.
+uint32_t item_grid(const Workspace *ws, uint64_t items) {
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ws->num_sms * ASC_PR_ITEM_BLOCKS));
 }
 
 uint32_t fill_grid(const Workspace *ws, uint64_t n) {
@@ -2307,7 +2493,7 @@ void free_ws_buffers(Workspace *ws) {
                     (void *)ws->queue[0],
                     (void *)ws->queue[1],
                     (void *)ws->segs[0], (void *)ws->segs[1], (void *)ws->ctl, (void *)ws->huge_list, ws->pr_rank,
-                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->in_ptr, (void *)ws->in_edges,
+                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->pr_items, (void *)ws->in_ptr, (void *)ws->in_edges,
                     (void *)ws->in_none})
         if (p) cudaFree(p);
     if (ws->h_ctl) cudaFreeHost(ws->h_ctl);
@@ -2832,22 +3018,21 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         seed_bits_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, 0, 1, nwords);
         build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, ws->bitmap[0], nwords);
         launches += 2;
-    } else if (ws->n_huge_total) {
-        seed_huge_segments_kernel<<<fill_grid(ws, ws->n_huge_total), kBlock, 0, s>>>(
-            sa, ws->huge_list, ws->n_huge_static, ws->n_huge_total);
-        launches++;
     }
     ASC_CUDA(cudaGetLastError());
-    ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
-    ASC_CUDA(cudaStreamSynchronize(s));
-    uint32_t cnt[CTL_BLOCK];
-    memcpy(cnt, ws->h_ctl, sizeof(cnt));
+    uint32_t cnt[CTL_BLOCK] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (REF) {
+        ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
+        ASC_CUDA(cudaStreamSynchronize(s));
+        memcpy(cnt, ws->h_ctl, sizeof(cnt));
+    }
 
     // standard PageRank on a graph with staging buffers: the on-demand edges are
     // copied in chunks every pass, overlapped with the kernels
     bool staged = false;
     if (!REF && !pt.on && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
     StagePlan *sp = staged ? ws->stage : nullptr;
+    if (!REF && !staged) ASC_TRY(ensure_pr_items(g));
 
     // REF: the active set alternates parity like a traversal frontier. STD:
     // every vertex every pass (dense ranges), fixed segment list in parity 0.
@@ -2899,13 +3084,48 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                 ASC_TRY(stage_release(sp, k, s));
                 launches++;
             }
+        } else if (!REF) {
+            // one launch for both regions; timed runs launch them apart
+            PrItemArgs<T> ia;
+            memset(&ia, 0, sizeof(ia));
+            ia.items = ws->pr_items;
+            ia.ptr = g->d_ptr;
+            ia.outdeg = g->d_outdeg;
+            ia.rank = rank;
+            ia.c_old = pa.c_old;
+            ia.c_new = pa.c_new;
+            ia.sum = pa.sum;
+            ia.damping = pa.damping;
+            ia.dangling_prev = pa.dangling_prev;
+            ia.acc = pa.acc;
+            ia.work = ws->ctl + CTL_BLOCK * po + 4;
+            ia.V = V;
+            ia.ebits = g->ebits;
+            const uint32_t first[3] = {0, ws->n_items_static, ws->n_items};
+            for (int region = pt.on ? 0 : 2; region < (pt.on ? 2 : 3); region++) {
+                for (int r = 0; r < 2; r++) {
+                    ia.sl[r].edges = r == 0 ? g->d_static : g->d_host_edges;
+                    ia.sl[r].edge_words = edge_store_words(g, r == 0 ? g->static_edges : g->E);
+                    ia.sl[r].begin = first[r];
+                    ia.sl[r].n = region == 2 || region == r ? first[r + 1] - first[r] : 0;
+                }
+                const uint32_t n = ia.sl[0].n + ia.sl[1].n;
+                if (!n) continue;
+                if (pt.on) ASC_CUDA(cudaMemsetAsync(ia.work, 0, 4, s));
+                ASC_TRY(pt.begin(region));
+                pt.record(s);
+                pr_pull_items_kernel<T><<<item_grid(ws, n), kPrThreads, 0, s>>>(ia);
+                pt.record(s);
+                launches++;
+            }
+            pr_cut_rows_kernel<T><<<fill_grid(ws, ws->n_items), kBlock, 0, s>>>(ia, ws->n_items);
+            launches++;
         } else if (!pt.on) {
             // one launch for both regions (the timed split below runs them apart)
             if (region_items[0] + region_items[1]) {
                 PrArgs<T> p0 = pa, p1 = pa;
                 p0.r = region_args(g, parity, 0, !REF);
                 p1.r = region_args(g, parity, 1, !REF);
-                p1.r.stage_edges = !REF && pr_tile_stage(g);
                 pr_pull_fused_kernel<T, REF>
                     <<<grid_for(ws, region_items[0] + region_items[1]), kBlock, 0, s>>>(p0, p1);
                 launches++;
@@ -2914,7 +3134,6 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             for (int region = 0; region < 2; region++) {
                 if (!region_items[region]) continue;
                 pa.r = region_args(g, parity, region, !REF);
-                pa.r.stage_edges = region == 1 && !REF && pr_tile_stage(g);
                 ASC_TRY(pt.begin(region));
                 pt.record(s);
                 pr_pull_kernel<T, REF><<<grid_for(ws, region_items[region]), kBlock, 0, s>>>(pa);
@@ -2922,7 +3141,7 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                 launches++;
             }
         }
-        const uint32_t nseg_items = REF ? cnt[2] + cnt[3] : ws->n_huge_total;
+        const uint32_t nseg_items = REF ? cnt[2] + cnt[3] : (staged ? ws->n_huge_total : 0);
         if (nseg_items) {
             pa.r = region_args(g, parity, 0, !REF);
             pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, nseg_items), kBlock, 0, s>>>(
@@ -2961,13 +3180,21 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     if (st) {
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
+        unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
+        if (!REF && !staged) {  // every pass reads every edge
+            const uint64_t se = g->h_ptr[g->static_vertices], passes = (uint64_t)it;
+            n[0] = passes * se;
+            n[1] = passes * (g->E - se);
+            n[2] = passes * g->static_vertices;
+            n[3] = passes * (V - g->static_vertices);
+        }
         st->iterations = it;
-        st->edges_processed = hs[0] + hs[1];
-        st->ondemand_edges = hs[1];
-        st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, hs[1]);
+        st->edges_processed = n[0] + n[1];
+        st->ondemand_edges = n[1];
+        st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, n[1]);
         st->staged_chunks = staged ? sp->chunks * (uint32_t)it : 0;
-        st->frontier_vertices = hs[2] + hs[3];
-        st->ondemand_vertices = hs[3];
+        st->frontier_vertices = n[2] + n[3];
+        st->ondemand_vertices = n[3];
         st->reached_vertices = V;
         st->reached_edges = g->E;
         st->residual = residual;
@@ -3755,6 +3982,7 @@ uint64_t workspace_bytes(asc_graph *g, bool pagerank) {
         b = 12 * V + 20 * (V / 32 + 2) + 4 * CTL_WORDS + 16 * segs + 4 * huge + 8 * 16;
     }
     if (pagerank && (!g->ws || !g->ws->pr_rank)) b += 4ull * 8 * V;
+    if (pagerank && (!g->ws || !g->ws->pr_items)) b += pr_items_bytes(V, E);
     // in-edge offsets of bottom-up BFS steps, allocated on the first BFS (with
     // the in-edges themselves when every out-edge is resident)
     if (!g->is_csc && t.bu_div && (!g->ws || !g->ws->in_ptr)) {
