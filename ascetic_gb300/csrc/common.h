@@ -68,6 +68,7 @@ struct Workspace {
     size_t pr_elem = 0;
     uint2 *pr_items = nullptr;       // first (row, edge) of each item of an edge-balanced pass
     uint32_t n_items_static = 0, n_items = 0;
+    unsigned long long *pr_hot = nullptr;  // scatter passes: most frequent destinations
     uint32_t *huge_list = nullptr;   // vertices with degree > huge_degree, static first
     uint32_t n_huge_static = 0, n_huge_total = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};

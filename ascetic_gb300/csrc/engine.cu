@@ -1414,6 +1414,14 @@ constexpr int kPrThreads = ASC_PR_ITEM_THREADS;
 constexpr int kPrWarps = kPrThreads / 32;
 constexpr int kPrVt = 8;                          // edges per thread
 constexpr uint32_t kPrItem = kPrThreads * kPrVt;  // merge positions per item
+// Scatter passes: slots for hot destinations and CTAs per SM (see pr_hot_slot).
+#ifndef ASC_PR_HOT
+#define ASC_PR_HOT 1024
+#endif
+#ifndef ASC_PR_SCATTER_BLOCKS
+#define ASC_PR_SCATTER_BLOCKS 4
+#endif
+constexpr uint32_t kPrHot = ASC_PR_HOT;
 
 // First (row, edge) of every item; items[n] is the end. Region 0 is the rows
 // [0, S), region 1 the rows [S, V); each starts at an item boundary.
@@ -1461,6 +1469,8 @@ struct PrItemArgs {
     double *acc;             // [0] residual, [1] dangling of this pass
     uint32_t *work;
     uint32_t V, ebits;
+    uint32_t wbits;          // scatter: weight bits below the destination in an edge word
+    const unsigned long long *hot;  // scatter: hot destinations by slot
 };
 
 template <typename T>
@@ -1517,6 +1527,23 @@ __device__ __forceinline__ void pr_mark_rows(const uint32_t *ptr, uint32_t r0, u
     }
 }
 
+// The row of the first mark at or after edge xe (a multiple of 32), or nr (the
+// row that goes on past the item) when there is none. The whole warp calls it.
+__device__ __forceinline__ uint32_t pr_next_row(const uint32_t *marks, const uint16_t *row_at, uint32_t xe,
+                                                uint32_t nr) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t m0 = xe >> 5; m0 < kPrItem / 32; m0 += 32) {
+        const uint32_t word = m0 + lane < kPrItem / 32 ? marks[m0 + lane] : 0u;
+        const unsigned any = __ballot_sync(kFull, word != 0);
+        if (any) {
+            const int q = __ffs((int)any) - 1;
+            const uint32_t bits = __shfl_sync(kFull, word, q);
+            return row_at[32 * (m0 + q) + __ffs((int)bits) - 1];
+        }
+    }
+    return nr;
+}
+
 // Item w of a launch over both slices: the on-demand and the static slice
 // alternate while both have items, so every SM overlaps host-link reads with
 // HBM reads.
@@ -1533,20 +1560,19 @@ __device__ __forceinline__ uint32_t pr_slice_item(const PrSlice *sl, uint32_t w,
     return sl[od].begin + local;
 }
 
-// The update of one vertex from its sum (as pr_update's standard mode), with
-// the pass's constant part (1 - d) / V + d * dangling / V given.
+// The standard update of one vertex from its sum, with the pass's constant part
+// (1 - d) / V + d * dangling / V given.
 template <typename T>
-__device__ __forceinline__ void pr_std_row(const PrItemArgs<T> &p, uint32_t v, double s, double base, double &res,
-                                           double &dang) {
-    const uint32_t od = p.outdeg[v];
-    const double r = p.rank[v];
-    const double rn = base + p.damping * s;
+__device__ __forceinline__ void pr_std_row(double *rank, T *c_new, uint32_t v, uint32_t od, double s, double damping,
+                                           double base, double &res, double &dang) {
+    const double r = rank[v];
+    const double rn = base + damping * s;
     res += fabs(rn - r);
-    p.rank[v] = rn;
+    rank[v] = rn;
     T c = (T)0;
     if (od) c = (T)(rn / (double)od);
     else dang += rn;
-    p.c_new[v] = c;
+    c_new[v] = c;
 }
 
 // block_reduce2_atomic for the item kernels' blocks.
@@ -1650,17 +1676,7 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
             // next mark, or the row that goes on past the item
             const uint32_t xe = xw + 32 * kPrVt;
             if (xe < ne || !((marks[(ne - 1) >> 5] >> ((ne - 1) & 31)) & 1u)) {
-                uint32_t row = nr;
-                for (uint32_t m0 = xe >> 5; m0 < kPrItem / 32; m0 += 32) {
-                    const uint32_t word = m0 + lane < kPrItem / 32 ? marks[m0 + lane] : 0u;
-                    const unsigned any = __ballot_sync(kFull, word != 0);
-                    if (any) {
-                        const int q = __ffs((int)any) - 1;
-                        const uint32_t bits = __shfl_sync(kFull, word, q);
-                        row = sm.row_at[32 * (m0 + q) + __ffs((int)bits) - 1];
-                        break;
-                    }
-                }
+                const uint32_t row = pr_next_row(marks, sm.row_at, xe, nr);
                 if (lane == 31) atomicAdd(&sums[row], tail);
             }
         }
@@ -1674,7 +1690,8 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
             if (j == nr ? goes_on : (j == 0 && cut)) {
                 atomicAdd(&p.sum[r0 + j], sums[j]);
             } else if (j < nr) {
-                pr_std_row<T>(p, r0 + j, PrAcc<T>::value(sums[j]), sm.base, res, dang);
+                pr_std_row<T>(p.rank, p.c_new, r0 + j, p.outdeg[r0 + j], PrAcc<T>::value(sums[j]), p.damping, sm.base,
+                              res, dang);
             }
         }
         __syncthreads();
@@ -1698,7 +1715,7 @@ __global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n) {
         if (r_end > a.x && p.ptr[a.x] < a.y) {
             const double s = PrAcc<T>::value(p.sum[a.x]);
             p.sum[a.x] = 0;
-            pr_std_row<T>(p, a.x, s, s_base, res, dang);
+            pr_std_row<T>(p.rank, p.c_new, a.x, p.outdeg[a.x], s, p.damping, s_base, res, dang);
         }
     }
     block_reduce2_atomic<T>(res, dang, p.acc, red);
@@ -1873,6 +1890,26 @@ asc_status ensure_pr_items(asc_graph *g) {
     return ASC_OK;
 }
 
+// A region's items and edges.
+PrSlice pr_slice(const asc_graph *g, int region) {
+    const Workspace *ws = g->ws;
+    PrSlice x;
+    x.edges = region == 0 ? g->d_static : g->d_host_edges;
+    x.edge_words = edge_store_words(g, region == 0 ? g->static_edges : g->E);
+    x.begin = region == 0 ? 0 : ws->n_items_static;
+    x.n = region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
+    return x;
+}
+
+// Edges (static, on-demand) and vertices (likewise) of passes that read every edge.
+void pr_pass_counts(const asc_graph *g, uint64_t passes, unsigned long long n[4]) {
+    const uint64_t se = g->h_ptr[g->static_vertices];
+    n[0] = passes * se;
+    n[1] = passes * (g->E - se);
+    n[2] = passes * g->static_vertices;
+    n[3] = passes * (g->V - g->static_vertices);
+}
+
 RegionArgs base_args(asc_graph *g, Workspace *ws, int parity_in) {
     RegionArgs a;
     memset(&a, 0, sizeof(a));
@@ -1956,8 +1993,8 @@ uint32_t bu_grid(const Workspace *ws, uint64_t nwords) {
 }
 
 // One wave of the item kernels' CTAs, or one per item.
-uint32_t item_grid(const Workspace *ws, uint64_t items) {
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ws->num_sms * ASC_PR_ITEM_BLOCKS));
+uint32_t item_grid(const Workspace *ws, uint64_t items, uint32_t ctas_per_sm = ASC_PR_ITEM_BLOCKS) {
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)ws->num_sms * ctas_per_sm));
 }
 
 uint32_t fill_grid(const Workspace *ws, uint64_t n) {
@@ -2493,7 +2530,7 @@ void free_ws_buffers(Workspace *ws) {
                     (void *)ws->queue[0],
                     (void *)ws->queue[1],
                     (void *)ws->segs[0], (void *)ws->segs[1], (void *)ws->ctl, (void *)ws->huge_list, ws->pr_rank,
-                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->pr_items, (void *)ws->in_ptr, (void *)ws->in_edges,
+                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->pr_items, (void *)ws->pr_hot, (void *)ws->in_ptr, (void *)ws->in_edges,
                     (void *)ws->in_none})
         if (p) cudaFree(p);
     if (ws->h_ctl) cudaFreeHost(ws->h_ctl);
@@ -3101,13 +3138,10 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             ia.work = ws->ctl + CTL_BLOCK * po + 4;
             ia.V = V;
             ia.ebits = g->ebits;
-            const uint32_t first[3] = {0, ws->n_items_static, ws->n_items};
             for (int region = pt.on ? 0 : 2; region < (pt.on ? 2 : 3); region++) {
                 for (int r = 0; r < 2; r++) {
-                    ia.sl[r].edges = r == 0 ? g->d_static : g->d_host_edges;
-                    ia.sl[r].edge_words = edge_store_words(g, r == 0 ? g->static_edges : g->E);
-                    ia.sl[r].begin = first[r];
-                    ia.sl[r].n = region == 2 || region == r ? first[r + 1] - first[r] : 0;
+                    ia.sl[r] = pr_slice(g, r);
+                    if (region != 2 && region != r) ia.sl[r].n = 0;
                 }
                 const uint32_t n = ia.sl[0].n + ia.sl[1].n;
                 if (!n) continue;
@@ -3181,13 +3215,7 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
         unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
-        if (!REF && !staged) {  // every pass reads every edge
-            const uint64_t se = g->h_ptr[g->static_vertices], passes = (uint64_t)it;
-            n[0] = passes * se;
-            n[1] = passes * (g->E - se);
-            n[2] = passes * g->static_vertices;
-            n[3] = passes * (V - g->static_vertices);
-        }
+        if (!REF && !staged) pr_pass_counts(g, (uint64_t)it, n);
         st->iterations = it;
         st->edges_processed = n[0] + n[1];
         st->ondemand_edges = n[1];
@@ -3982,7 +4010,7 @@ uint64_t workspace_bytes(asc_graph *g, bool pagerank) {
         b = 12 * V + 20 * (V / 32 + 2) + 4 * CTL_WORDS + 16 * segs + 4 * huge + 8 * 16;
     }
     if (pagerank && (!g->ws || !g->ws->pr_rank)) b += 4ull * 8 * V;
-    if (pagerank && (!g->ws || !g->ws->pr_items)) b += pr_items_bytes(V, E);
+    if (pagerank && (!g->ws || !g->ws->pr_items)) b += pr_items_bytes(V, E) + 8 * kPrHot;
     // in-edge offsets of bottom-up BFS steps, allocated on the first BFS (with
     // the in-edges themselves when every out-edge is resident)
     if (!g->is_csc && t.bu_div && (!g->ws || !g->ws->in_ptr)) {
@@ -4387,9 +4415,157 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_scatter_kernel(P
     }
 }
 
+// Destinations that most edges share, found once per workspace: kPrHot slots by
+// a hash of the id, each with the most frequent destination among a sample of
+// the edges (count << 32 | id; 0: empty). Their atomics meet in a few L2 slices:
+// on 1 M RMAT vertices the busiest slice took 451,000 of the pass's atomic
+// sectors against 128,000 on average, and set the pass's time (24 passes of 16 M
+// edges: 8.20 ms without the slots; 4.36 / 4.18 / 4.15 / 4.20 ms with 256 / 512 /
+// 1024 / 2048, the last two at 4 CTAs per SM, 4.29 with 1024 at 6; tiles of 256
+// vertices instead of items: 9.53 ms).
+constexpr uint32_t kPrHotSample = 16;   // every how many items are sampled
+__device__ __forceinline__ uint32_t pr_hot_slot(uint32_t v) { return (v * 2654435761u) >> (32 - __ffs(kPrHot) + 1); }
+
+template <typename T>
+__global__ void pr_hot_count_kernel(PrItemArgs<T> p, unsigned long long *count) {
+    const uint32_t mask = p.ebits >= 32 ? 0xffffffffu : (1u << p.ebits) - 1u;
+    const uint32_t total = p.sl[0].n + p.sl[1].n;
+    for (uint32_t it = blockIdx.x * kPrHotSample; it < total; it += gridDim.x * kPrHotSample) {
+        const PrSlice &sl = p.sl[it >= p.sl[0].n];
+        const uint32_t e0 = p.items[it].y, e1 = p.items[it + 1].y;
+        for (uint32_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+            const uint64_t bit = (uint64_t)e * p.ebits;
+            const uint64_t w = bit >> 5;
+            const uint32_t hi = w + 1 < sl.edge_words ? __ldg(sl.edges + w + 1) : 0u;
+            const uint32_t v = (__funnelshift_r(__ldg(sl.edges + w), hi, (uint32_t)bit & 31u) & mask) >> p.wbits;
+            if (!ASC_BAD(v >= p.V, 18, v)) atomicAdd(&count[v], 1ull);
+        }
+    }
+}
+
+// Puts the counts into the slots and clears them.
+__global__ void pr_hot_pick_kernel(unsigned long long *count, uint32_t V, unsigned long long *slots) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+        const unsigned long long n = count[v];
+        if (!n) continue;
+        count[v] = 0;
+        unsigned long long *s = slots + pr_hot_slot(v);
+        const unsigned long long x = (n << 32) | v;
+        if (*s < x) atomicMax(s, x);
+    }
+}
+
+// A CTA's sums of the hot destinations.
+template <typename T>
+struct PrHot;
+template <>
+struct PrHot<double> {
+    uint32_t key[kPrHot];
+    double acc[kPrHot];
+    __device__ __forceinline__ void clear(uint32_t i) { acc[i] = 0; }
+    __device__ __forceinline__ void add(uint32_t i, double x) { atomicAdd(&acc[i], x); }
+    __device__ __forceinline__ double get(uint32_t i) const { return acc[i]; }
+};
+template <>
+struct PrHot<float> {
+    uint32_t key[kPrHot];
+    uint32_t lo[kPrHot], hi[kPrHot];  // 64-bit fixed point as two 32-bit shared atomics with the carry between
+    __device__ __forceinline__ void clear(uint32_t i) { lo[i] = hi[i] = 0; }
+    __device__ __forceinline__ void add(uint32_t i, unsigned long long x) {
+        const uint32_t xl = (uint32_t)x, old = atomicAdd(&lo[i], xl);
+        const uint32_t xh = (uint32_t)(x >> 32) + (old + xl < xl ? 1u : 0u);
+        if (xh) atomicAdd(&hi[i], xh);
+    }
+    __device__ __forceinline__ unsigned long long get(uint32_t i) const {
+        return ((unsigned long long)hi[i] << 32) | lo[i];
+    }
+};
+
+// Edge-balanced scatter: items as in pr_pull_items_kernel, over out-edges. The
+// contributions of the item's rows are converted once into shared memory; a
+// thread adds its row's to the destinations of kPrVt consecutive edges, passing
+// to the next row at each mark. Hot destinations add up in shared memory and
+// reach the global sums once per CTA; the rest are atomics in L2, which bound
+// the pass. wbits > 0: edge words hold the weight below the destination; ebits
+// 64: {dst, weight}.
+template <typename T>
+__global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_items_kernel(PrItemArgs<T> p) {
+    typedef typename PrAcc<T>::type Acc;
+    __shared__ PrItemSmem<T> sm;
+    __shared__ PrHot<T> hot;
+    for (uint32_t i = threadIdx.x; i < kPrHot; i += kPrThreads) {
+        const unsigned long long x = p.hot[i];
+        hot.key[i] = x ? (uint32_t)x : 0xffffffffu;
+        hot.clear(i);
+    }
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = p.sl[0].n + p.sl[1].n;
+    const uint32_t eb = p.ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    if (threadIdx.x < kPrItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
+    if (threadIdx.x == 0) sm.work[0] = atomicAdd(p.work, 1u);
+    __syncthreads();
+    for (int buf = 0;; buf ^= 1) {
+        const uint32_t w = sm.work[buf];
+        if (w >= total) break;
+        bool od;
+        const uint32_t it = pr_slice_item(p.sl, w, od);
+        const uint2 a = p.items[it], b = p.items[it + 1];
+        const uint32_t r0 = a.x, e0 = a.y, nr = b.x - a.x, ne = b.y - a.y;
+        uint32_t nq;
+        const uint32_t bit0 = pr_stage_words(p.sl[od], e0, ne, eb, sm.pool, nq);
+        Acc *share = reinterpret_cast<Acc *>(sm.pool + 4 * nq + (nq ? 4 : 0));
+        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads)
+            share[j] = r0 + j < p.V ? PrAcc<T>::from(p.c_old[r0 + j]) : (Acc)0;
+        uint32_t *marks = sm.marks[buf];
+        pr_mark_rows<T>(p.ptr, r0, e0, nr, sm, marks);
+        if (threadIdx.x == 0) sm.work[buf ^ 1] = atomicAdd(p.work, 1u);
+        __syncthreads();
+        if (threadIdx.x < kPrItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
+        const uint32_t x0 = threadIdx.x * kPrVt, xw = x0 - lane * kPrVt;
+        if (xw < ne) {
+            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kPrVt) - 1u);
+            // the row that is open after this thread's edges: of the next mark in
+            // a later lane, in a later warp, or the one that goes on past the item
+            const unsigned ended = __ballot_sync(kFull, ends != 0);
+            const uint32_t first = ends ? sm.row_at[x0 + __ffs((int)ends) - 1] : nr;
+            const unsigned above = lane < 31 ? ended & (0xffffffffu << (lane + 1)) : 0u;
+            const uint32_t from_lane = __shfl_sync(kFull, first, above ? __ffs((int)above) - 1 : lane);
+            const uint32_t after = pr_next_row(marks, sm.row_at, xw + 32 * kPrVt, nr);
+            const uint32_t open = above ? from_lane : after;
+            Acc c = share[ends ? first : open];
+            uint32_t v[kPrVt];
+#pragma unroll
+            for (int k = 0; k < kPrVt; k++)
+                v[k] = x0 + k < ne ? pr_staged_edge(sm.pool, bit0 + (x0 + k) * eb, mask) >> p.wbits : 0u;
+#pragma unroll
+            for (int k = 0; k < kPrVt; k++) {
+                if (x0 + k < ne && !ASC_BAD(v[k] >= p.V, 18, v[k])) {
+                    const uint32_t h = pr_hot_slot(v[k]);
+                    if (hot.key[h] == v[k]) hot.add(h, c);
+                    else atomicAdd(&p.sum[v[k]], c);
+                }
+                if ((ends >> k) & 1u) {
+                    const uint32_t rest = ends >> k >> 1;
+                    c = share[rest ? sm.row_at[x0 + k + __ffs((int)rest)] : open];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < kPrHot; i += kPrThreads) {
+        const Acc x = hot.get(i);
+        if (x != (Acc)0) atomicAdd(&p.sum[hot.key[i]], x);
+    }
+}
+
 template <typename T, bool REF>
 __global__ void pr_push_apply_kernel(PushArgs<T> p, uint32_t V) {
     __shared__ double red[2 * kWarps];
+    __shared__ double s_base;
+    if (!REF) {
+        if (threadIdx.x == 0) s_base = (1.0 - p.damping) / (double)V + p.damping * (*p.dangling_prev) / (double)V;
+        __syncthreads();
+    }
     double res = 0, dang = 0;
     uint32_t nact = 0;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -4408,7 +4584,7 @@ __global__ void pr_push_apply_kernel(PushArgs<T> p, uint32_t V) {
             if (pr_update<T>(p.rank, p.c_old, p.c_new, v, od, s, true, 0.85, (double)V, nullptr, res, dang)) nact++;
             else atomicAnd(&p.active[v >> 5], ~bit);
         } else {
-            pr_update<T>(p.rank, p.c_old, p.c_new, v, od, s, false, p.damping, (double)V, p.dangling_prev, res, dang);
+            pr_std_row<T>(p.rank, p.c_new, v, od, s, p.damping, s_base, res, dang);
         }
     }
     if (REF) {
@@ -4464,17 +4640,41 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     pr_push_init_kernel<T><<<fill_grid(ws, V), kBlock, 0, s>>>(rank, c[0], c[1], (Acc *)ws->pr_sum, g->d_ptr, active,
                                                                V, acc + 2);
     launches++;
-    if (ws->n_huge_total) {
+    bool staged = false;
+    if (!REF && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
+    if (staged && ws->n_huge_total) {
         seed_huge_segments_kernel<<<fill_grid(ws, ws->n_huge_total), kBlock, 0, s>>>(
             base_args(g, 1), ws->huge_list, ws->n_huge_static, ws->n_huge_total);
         launches++;
     }
     ASC_CUDA(cudaGetLastError());
     const int max_it = p.max_iterations > 0 ? p.max_iterations : (REF ? 1000000 : 100);
-    const uint32_t grid = (uint32_t)(ws->num_sms * ws->tune.ctas_per_sm);
-    bool staged = false;
-    if (!REF && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
     StagePlan *sp = staged ? ws->stage : nullptr;
+    PrItemArgs<T> ia;
+    memset(&ia, 0, sizeof(ia));
+    if (!staged) {
+        ASC_TRY(ensure_pr_items(g));
+        ia.items = ws->pr_items;
+        ia.sl[0] = pr_slice(g, 0);
+        ia.sl[1] = pr_slice(g, 1);
+        ia.ptr = g->d_ptr;
+        ia.sum = (Acc *)ws->pr_sum;
+        ia.work = ws->ctl + CTL_BLOCK + 4;
+        ia.V = V;
+        ia.ebits = WORDS == 2 ? 64 : g->ebits;
+        ia.wbits = g->wbits;
+        if (!ws->pr_hot) {
+            ASC_CUDA(cudaMalloc((void **)&ws->pr_hot, 8 * kPrHot));
+            ws->device_bytes += 8 * kPrHot;
+            ASC_CUDA(cudaMemsetAsync(ws->pr_hot, 0, 8 * kPrHot, s));
+            pr_hot_count_kernel<T><<<item_grid(ws, ws->n_items / kPrHotSample + 1, 8), kBlock, 0, s>>>(
+                ia, (unsigned long long *)ws->pr_sum);
+            pr_hot_pick_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>((unsigned long long *)ws->pr_sum, V, ws->pr_hot);
+            launches += 2;
+            ASC_CUDA(cudaGetLastError());
+        }
+        ia.hot = ws->pr_hot;
+    }
     int it = 0;
     double residual = 0;
     for (;;) {
@@ -4515,7 +4715,9 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
                 launches++;
             }
         } else {
-            pr_scatter_kernel<T, WORDS><<<grid, kBlock, 0, s>>>(pa);
+            ia.c_old = pa.c_old;
+            pr_scatter_items_kernel<T>
+                <<<item_grid(ws, ws->n_items, ASC_PR_SCATTER_BLOCKS), kPrThreads, 0, s>>>(ia);
             launches++;
         }
         pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kBlock, 0, s>>>(pa, V);
@@ -4544,13 +4746,15 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     if (st) {
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
+        unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
+        if (!staged) pr_pass_counts(g, (uint64_t)it, n);
         st->iterations = it;
-        st->edges_processed = hs[0] + hs[1];
-        st->ondemand_edges = hs[1];
-        st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, hs[1]);
+        st->edges_processed = n[0] + n[1];
+        st->ondemand_edges = n[1];
+        st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, n[1]);
         st->staged_chunks = staged ? sp->chunks * (uint32_t)it : 0;
-        st->frontier_vertices = hs[2] + hs[3];
-        st->ondemand_vertices = hs[3];
+        st->frontier_vertices = n[2] + n[3];
+        st->ondemand_vertices = n[3];
         st->reached_vertices = V;
         st->reached_edges = g->E;
         st->residual = residual;

@@ -31,7 +31,7 @@ SHAPES = {
 }
 
 
-@pytest.mark.parametrize("layout", ["csc", "csr"])
+@pytest.mark.parametrize("layout", ["csc", "csr", "csr_w63", "csr_w99999"])
 @pytest.mark.parametrize("frac", [1.0, 0.4, 0.0])
 @pytest.mark.parametrize("shape", sorted(SHAPES))
 def test_items(shape, frac, layout):
@@ -40,7 +40,8 @@ def test_items(shape, frac, layout):
     ptr = np.zeros(V + 1, np.uint64)
     ptr[1:] = np.cumsum(deg)
     rng = np.random.RandomState(7)
-    other = rng.randint(0, V, E).astype(np.uint32)
+    # half of the entries name one of three vertices: hot destinations of a scatter
+    other = np.where(rng.rand(E) < 0.5, rng.randint(0, min(V, 3), E), rng.randint(0, V, E)).astype(np.uint32)
     rows = np.repeat(np.arange(V, dtype=np.uint32), deg)
     if layout == "csc":
         cptr, ccol = ptr, other
@@ -54,12 +55,15 @@ def test_items(shape, frac, layout):
     ref, _ = oracle.pr_ref(cptr, ccol, od)
     budget = A.make_budget(frac=frac, fragment_edges=16)
     kw = {"outdeg": od} if layout == "csc" else {}
-    with A.Graph.from_csr(ptr, other, budget=budget, **kw) as g:
+    edges = other
+    if "_w" in layout:  # packed with the destination, or beside it
+        edges = np.stack([other, rng.randint(1, int(layout[5:]) + 1, E).astype(np.uint32)], 1)
+    with A.Graph.from_csr(ptr, edges, budget=budget, **kw) as g:
         for prec in (A.F64, A.F32, A.F64):
             got, st = g.run("pr", params=A.make_params(pr_mode=A.PR_STD, precision=prec))
             err = np.abs(got.astype(np.float64) - exp) / exp
             assert err.max() <= TOL[prec], (prec, err.max())
             assert st["edges_processed"] == E * st["iterations"]
-            assert layout == "csr" or st["frontier_vertices"] == V * st["iterations"]
+            assert st["frontier_vertices"] == V * st["iterations"]
         got, _ = g.run("pr")
         assert np.abs(got - ref).max() <= 1e-6
