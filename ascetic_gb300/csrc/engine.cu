@@ -94,9 +94,10 @@ enum Alg { kBFS = 0, kSSSP = 1, kCC = 2 };
 // counts loop-body executions when the loop runs as a CUDA graph. Word 31 is
 // the SSSP near-far threshold, word 36 the minimum far distance of a pass.
 // Words 42-43 (u64): in-edges that bottom-up BFS steps read from host memory;
-// words 44-45 (u64): unreached vertices those steps examined.
+// words 44-45 (u64): unreached vertices those steps examined. Words 46-47 (u64):
+// in-edges of the vertices that a reference PageRank pass left active.
 enum { CTL_BLOCK = 8, CTL_STATS = 16, CTL_ITERS = 28, CTL_TIMEOUT = 29, CTL_BODIES = 30, CTL_THRESH = 31,
-       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_WORDS = 64 };
+       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_WORDS = 64 };
 
 struct RegionArgs {
     const uint32_t *ptr;
@@ -1172,6 +1173,8 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
     if (REF) {
         if (won) atomicOr(&a.bitmap[u >> 5], 1u << (u & 31));
         count_next(a, won, u, s_next);
+        const uint32_t e = __reduce_add_sync(kFull, won ? deg : 0u);
+        if (lane == 0 && e) atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)e);
     } else {
         block_reduce2_atomic<T>(res, dang, p.acc, sm.red);
     }
@@ -1369,7 +1372,10 @@ __global__ void pr_apply_segmented_kernel(PrArgs<T> p, const uint64_t *items_sta
         }
         if (REF) {
             // a long-list vertex that stays active joins the next bitmap
-            if (won) atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+            if (won) {
+                atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+                atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)(a.ptr[v + 1] - a.ptr[v]));
+            }
             const unsigned m0 = __ballot_sync(kFull, won && v < a.S), m1 = __ballot_sync(kFull, won && v >= a.S);
             if ((threadIdx.x & 31) == 0) {
                 if (m0) atomicAdd(&a.cnt_out[6], (uint32_t)__popc(m0));
@@ -1414,6 +1420,14 @@ constexpr int kPrThreads = ASC_PR_ITEM_THREADS;
 constexpr int kPrWarps = kPrThreads / 32;
 constexpr int kPrVt = 8;                          // edges per thread
 constexpr uint32_t kPrItem = kPrThreads * kPrVt;  // merge positions per item
+// A reference-mode pass runs over all items while the active vertices hold more
+// than 1 / kPrDenseDiv of the in-edges, else over their lists. 35 passes on RMAT
+// scale 20 (85% of the edges active on average), 30% resident: lists alone 11.15
+// ms; items above 1/2, 1/4, 1/8, 1/32 and always: 5.25, 5.38, 5.38, 5.47, 5.55.
+#ifndef ASC_PR_DENSE_DIV
+#define ASC_PR_DENSE_DIV 2
+#endif
+constexpr uint64_t kPrDenseDiv = ASC_PR_DENSE_DIV;
 // Scatter passes: slots for hot destinations and CTAs per SM (see pr_hot_slot).
 #ifndef ASC_PR_HOT
 #define ASC_PR_HOT 1024
@@ -1471,6 +1485,12 @@ struct PrItemArgs {
     uint32_t V, ebits;
     uint32_t wbits;          // scatter: weight bits below the destination in an edge word
     const unsigned long long *hot;  // scatter: hot destinations by slot
+    // reference mode: active vertices of this pass and the next one, their counts
+    // per region (cnt_out[6..7]) and the next one's in-edges
+    const uint32_t *bitmap_in;
+    uint32_t *bitmap, *cnt_out;
+    unsigned long long *active_edges;
+    uint32_t S;
 };
 
 template <typename T>
@@ -1598,7 +1618,50 @@ __device__ __forceinline__ void pr_reduce2_atomic(double a, double b, double *ou
     }
 }
 
-template <typename T>
+// What a thread of an item pass counts over the rows it applies.
+struct PrCounts {
+    double res = 0, dang = 0;         // standard mode
+    uint32_t n0 = 0, n1 = 0;          // reference mode: rows still active, per region,
+    unsigned long long edges = 0;     // and their in-edges
+};
+
+// Applies row v with sum s. Reference mode (prKernel_Opt, gpu_kernels.cuh:533-552)
+// leaves inactive vertices alone: both contribution arrays hold their last value.
+template <typename T, bool REF>
+__device__ __forceinline__ void pr_item_row(const PrItemArgs<T> &p, uint32_t v, double s, double base, PrCounts &n) {
+    if (!REF) {
+        pr_std_row<T>(p.rank, p.c_new, v, p.outdeg[v], s, p.damping, base, n.res, n.dang);
+        return;
+    }
+    const uint32_t bit = 1u << (v & 31);
+    if (!(p.bitmap_in[v >> 5] & bit)) return;
+    if (pr_update<T>(p.rank, p.c_old, p.c_new, v, p.outdeg[v], s, true, 0.85, 0.0, nullptr, n.res, n.dang)) {
+        atomicOr(&p.bitmap[v >> 5], bit);
+        if (v < p.S) n.n0++;
+        else n.n1++;
+        n.edges += p.ptr[v + 1] - p.ptr[v];
+    }
+}
+
+// Adds a block's counts to the pass's (whole warps call it).
+template <bool REF, typename T>
+__device__ __forceinline__ void pr_flush_counts(const PrItemArgs<T> &p, PrCounts n, double *s_buf) {
+    if (!REF) {
+        pr_reduce2_atomic(n.res, n.dang, p.acc, s_buf);
+        return;
+    }
+    n.n0 = __reduce_add_sync(kFull, n.n0);
+    n.n1 = __reduce_add_sync(kFull, n.n1);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) n.edges += __shfl_down_sync(kFull, n.edges, d);
+    if ((threadIdx.x & 31) == 0) {
+        if (n.n0) atomicAdd(&p.cnt_out[6], n.n0);
+        if (n.n1) atomicAdd(&p.cnt_out[7], n.n1);
+        if (n.edges) atomicAdd(p.active_edges, n.edges);
+    }
+}
+
+template <typename T, bool REF>
 __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_kernel(PrItemArgs<T> p) {
     typedef typename PrAcc<T>::type Acc;
     __shared__ PrItemSmem<T> sm;
@@ -1608,10 +1671,10 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
     if (threadIdx.x < kPrItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         sm.work[0] = atomicAdd(p.work, 1u);
-        sm.base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
+        if (!REF) sm.base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
     }
     __syncthreads();
-    double res = 0, dang = 0;
+    PrCounts n;
     for (int buf = 0;; buf ^= 1) {
         const uint32_t w = sm.work[buf];
         if (w >= total) break;
@@ -1690,35 +1753,34 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
             if (j == nr ? goes_on : (j == 0 && cut)) {
                 atomicAdd(&p.sum[r0 + j], sums[j]);
             } else if (j < nr) {
-                pr_std_row<T>(p.rank, p.c_new, r0 + j, p.outdeg[r0 + j], PrAcc<T>::value(sums[j]), p.damping, sm.base,
-                              res, dang);
+                pr_item_row<T, REF>(p, r0 + j, PrAcc<T>::value(sums[j]), sm.base, n);
             }
         }
         __syncthreads();
     }
-    pr_reduce2_atomic(res, dang, p.acc, sm.red);
+    pr_flush_counts<REF>(p, n, sm.red);
 }
 
 // Applies the rows that were cut by an item boundary: the row at the start of
-// item i, when it began earlier and ends in item i.
-template <typename T>
-__global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n) {
-    __shared__ double red[2 * kWarps];
+// item i, when it began earlier and ends in item i. Blocks of kPrThreads.
+template <typename T, bool REF>
+__global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n_items) {
+    __shared__ double red[2 * kPrWarps];
     __shared__ double s_base;
-    if (threadIdx.x == 0)
+    if (!REF && threadIdx.x == 0)
         s_base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
     __syncthreads();
-    double res = 0, dang = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    PrCounts n;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_items; i += gridDim.x * blockDim.x) {
         const uint2 a = p.items[i];
         const uint32_t r_end = p.items[i + 1].x;
         if (r_end > a.x && p.ptr[a.x] < a.y) {
             const double s = PrAcc<T>::value(p.sum[a.x]);
             p.sum[a.x] = 0;
-            pr_std_row<T>(p.rank, p.c_new, a.x, p.outdeg[a.x], s, p.damping, s_base, res, dang);
+            pr_item_row<T, REF>(p, a.x, s, s_base, n);
         }
     }
-    block_reduce2_atomic<T>(res, dang, p.acc, red);
+    pr_flush_counts<REF>(p, n, red);
 }
 
 template <typename T>
@@ -3053,23 +3115,20 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         // every vertex starts active: full bitmap, then lists/segments from it
         for (int i = 0; i < 2; i++) ASC_CUDA(cudaMemsetAsync(ws->bitmap[i], 0, 4 * (V / 32 + 2), s));
         seed_bits_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, 0, 1, nwords);
-        build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, ws->bitmap[0], nwords);
-        launches += 2;
+        launches++;
     }
     ASC_CUDA(cudaGetLastError());
-    uint32_t cnt[CTL_BLOCK] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (REF) {
-        ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
-        ASC_CUDA(cudaStreamSynchronize(s));
-        memcpy(cnt, ws->h_ctl, sizeof(cnt));
-    }
+    // reference mode: this pass's active vertices per region and their in-edges
+    uint32_t active[2] = {g->static_vertices, V - g->static_vertices};
+    uint64_t active_edges = g->E;
+    unsigned long long dense_counts[4] = {0, 0, 0, 0};  // of the passes over items
 
     // standard PageRank on a graph with staging buffers: the on-demand edges are
     // copied in chunks every pass, overlapped with the kernels
     bool staged = false;
     if (!REF && !pt.on && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
     StagePlan *sp = staged ? ws->stage : nullptr;
-    if (!REF && !staged) ASC_TRY(ensure_pr_items(g));
+    if (!staged) ASC_TRY(ensure_pr_items(g));
 
     // REF: the active set alternates parity like a traversal frontier. STD:
     // every vertex every pass (dense ranges), fixed segment list in parity 0.
@@ -3079,7 +3138,7 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     double residual = 0;
     double phase_ms[2] = {0, 0};
     for (;;) {
-        if (REF && !(cnt[6] | cnt[7])) break;
+        if (REF && !(active[0] | active[1])) break;
         if (it >= max_it) {
             if (REF) return fail(ASC_ERR_TIMEOUT, "reference PageRank still active after %d passes", it);
             break;
@@ -3087,8 +3146,12 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         const int cp = it & 1;
         const int po = 1 - parity;
         ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_BLOCK * po, 0, 4 * CTL_BLOCK, s));
-        if (REF) ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
-        if (!REF) ASC_CUDA(cudaMemsetAsync(acc + 2 * cp, 0, 16, s));
+        if (REF) {
+            ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
+            ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_ACTIVE, 0, 8, s));
+        } else {
+            ASC_CUDA(cudaMemsetAsync(acc + 2 * cp, 0, 16, s));
+        }
         PrArgs<T> pa;
         memset(&pa, 0, sizeof(pa));
         pa.outdeg = g->d_outdeg;
@@ -3099,13 +3162,6 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         pa.damping = REF ? 0.85 : p.damping;
         pa.acc = acc + 2 * cp;
         pa.dangling_prev = acc + 2 * (1 - cp) + 1;
-        uint64_t region_items[2];
-        for (int region = 0; region < 2; region++) {
-            const uint32_t range = region == 0 ? g->static_vertices : V - g->static_vertices;
-            const bool bitmap_mode = REF && ws->tune.dense_div && cnt[6 + region] > range / ws->tune.dense_div;
-            const uint32_t nvert = REF ? (bitmap_mode ? range : cnt[region]) : range;
-            region_items[region] = (uint64_t)cnt[2 + region] + (nvert + kBlock - 1) / kBlock;
-        }
         if (staged) {
             ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
             for (uint32_t k = 0; k < (uint32_t)sp->launches.size(); k++) {
@@ -3121,8 +3177,14 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                 ASC_TRY(stage_release(sp, k, s));
                 launches++;
             }
-        } else if (!REF) {
-            // one launch for both regions; timed runs launch them apart
+            if (ws->n_huge_total) {
+                pa.r = region_args(g, parity, 0, true);
+                pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, ws->n_huge_total), kBlock, 0, s>>>(
+                    pa, ws->segs[parity], ws->segs[parity] + ws->segcap_static, ws->huge_list, ws->n_huge_total);
+                launches++;
+            }
+        } else if (!REF || active_edges > g->E / kPrDenseDiv) {
+            // every row; one launch for both regions (timed runs launch them apart)
             PrItemArgs<T> ia;
             memset(&ia, 0, sizeof(ia));
             ia.items = ws->pr_items;
@@ -3138,6 +3200,11 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             ia.work = ws->ctl + CTL_BLOCK * po + 4;
             ia.V = V;
             ia.ebits = g->ebits;
+            ia.bitmap_in = ws->bitmap[parity];
+            ia.bitmap = ws->bitmap[po];
+            ia.cnt_out = ws->ctl + CTL_BLOCK * po;
+            ia.active_edges = (unsigned long long *)(ws->ctl + CTL_ACTIVE);
+            ia.S = g->static_vertices;
             for (int region = pt.on ? 0 : 2; region < (pt.on ? 2 : 3); region++) {
                 for (int r = 0; r < 2; r++) {
                     ia.sl[r] = pr_slice(g, r);
@@ -3148,55 +3215,60 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                 if (pt.on) ASC_CUDA(cudaMemsetAsync(ia.work, 0, 4, s));
                 ASC_TRY(pt.begin(region));
                 pt.record(s);
-                pr_pull_items_kernel<T><<<item_grid(ws, n), kPrThreads, 0, s>>>(ia);
+                pr_pull_items_kernel<T, REF><<<item_grid(ws, n), kPrThreads, 0, s>>>(ia);
                 pt.record(s);
                 launches++;
             }
-            pr_cut_rows_kernel<T><<<fill_grid(ws, ws->n_items), kBlock, 0, s>>>(ia, ws->n_items);
+            pr_cut_rows_kernel<T, REF><<<fill_grid(ws, ws->n_items), kPrThreads, 0, s>>>(ia, ws->n_items);
             launches++;
-        } else if (!pt.on) {
-            // one launch for both regions (the timed split below runs them apart)
-            if (region_items[0] + region_items[1]) {
+            unsigned long long n[4];
+            pr_pass_counts(g, 1, n);
+            dense_counts[0] += n[0];
+            dense_counts[1] += n[1];
+            dense_counts[2] += REF ? active[0] : n[2];
+            dense_counts[3] += REF ? active[1] : n[3];
+        } else {
+            // the active vertices' lists and segments, then one launch for both
+            // regions (timed runs launch them apart)
+            RegionArgs lists = region_args(g, po, 0, false);  // writes the lists of this parity
+            build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(lists, ws->bitmap[parity], nwords);
+            const uint32_t grid = (uint32_t)(ws->num_sms * ws->tune.ctas_per_sm);
+            launches++;
+            if (!pt.on) {
                 PrArgs<T> p0 = pa, p1 = pa;
                 p0.r = region_args(g, parity, 0, !REF);
                 p1.r = region_args(g, parity, 1, !REF);
-                pr_pull_fused_kernel<T, REF>
-                    <<<grid_for(ws, region_items[0] + region_items[1]), kBlock, 0, s>>>(p0, p1);
+                pr_pull_fused_kernel<T, REF><<<grid, kBlock, 0, s>>>(p0, p1);
                 launches++;
             }
-        } else {
-            for (int region = 0; region < 2; region++) {
-                if (!region_items[region]) continue;
+            for (int region = 0; pt.on && region < 2; region++) {
+                if (!active[region]) continue;
                 pa.r = region_args(g, parity, region, !REF);
                 ASC_TRY(pt.begin(region));
                 pt.record(s);
-                pr_pull_kernel<T, REF><<<grid_for(ws, region_items[region]), kBlock, 0, s>>>(pa);
+                pr_pull_kernel<T, REF><<<grid, kBlock, 0, s>>>(pa);
                 pt.record(s);
                 launches++;
             }
-        }
-        const uint32_t nseg_items = REF ? cnt[2] + cnt[3] : (staged ? ws->n_huge_total : 0);
-        if (nseg_items) {
-            pa.r = region_args(g, parity, 0, !REF);
-            pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, nseg_items), kBlock, 0, s>>>(
-                pa, ws->segs[parity], ws->segs[parity] + ws->segcap_static, ws->huge_list, ws->n_huge_total);
-            launches++;
-        }
-        if (REF) {
-            build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(region_args(g, parity, 0, false),
-                                                                            ws->bitmap[po], nwords);
-            launches++;
+            const uint64_t segs = ws->segcap_static + ws->segcap_ondemand;
+            if (segs) {
+                pa.r = region_args(g, parity, 0, !REF);
+                pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, segs), kBlock, 0, s>>>(
+                    pa, ws->segs[parity], ws->segs[parity] + ws->segcap_static, ws->huge_list, ws->n_huge_total);
+                launches++;
+            }
         }
         ASC_CUDA(cudaGetLastError());
-        if (REF)
-            ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl + CTL_BLOCK * po, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
+        if (REF) ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_WORDS, cudaMemcpyDeviceToHost, s));
         else ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, acc + 2 * cp, 16, cudaMemcpyDeviceToHost, s));
         ASC_CUDA(cudaStreamSynchronize(s));
         if (pt.on) ASC_TRY(pt.sum(phase_ms));
         it++;
         iteration_boundary();
         if (REF) {
-            memcpy(cnt, ws->h_ctl, sizeof(cnt));
+            active[0] = ws->h_ctl[CTL_BLOCK * po + 6];
+            active[1] = ws->h_ctl[CTL_BLOCK * po + 7];
+            memcpy(&active_edges, ws->h_ctl + CTL_ACTIVE, 8);
             parity = po;
         } else {
             memcpy(&residual, ws->h_ctl, 8);
@@ -3215,7 +3287,7 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
         unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
-        if (!REF && !staged) pr_pass_counts(g, (uint64_t)it, n);
+        for (int k = 0; k < 4; k++) n[k] += dense_counts[k];
         st->iterations = it;
         st->edges_processed = n[0] + n[1];
         st->ondemand_edges = n[1];
