@@ -69,8 +69,6 @@ struct Workspace {
     uint2 *pr_items = nullptr;       // first (row, edge) of each item of an edge-balanced pass
     uint32_t n_items_static = 0, n_items = 0;
     unsigned long long *pr_hot = nullptr;  // scatter passes: most frequent destinations
-    uint32_t *huge_list = nullptr;   // vertices with degree > huge_degree, static first
-    uint32_t n_huge_static = 0, n_huge_total = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> phase_events;
     struct BatchEngine *batch[2] = {nullptr, nullptr};  // asc_run_batch engines (BFS, SSSP)
@@ -129,9 +127,8 @@ struct asc_graph {
     // differ); the most recent few tunings are kept
     struct LongLists {
         uint32_t huge_degree = 0, segment_edges = 0;
-        std::vector<uint32_t> list, bits;  // long-list vertices; one bit per vertex (V/32+2 words)
+        std::vector<uint32_t> bits;  // one bit per vertex, set for the long lists (V/32+2 words)
         uint64_t seg_static = 0, seg_ondemand = 0;  // segments of the static / on-demand long lists
-        uint32_t n_static = 0;
     };
     std::vector<LongLists> long_lists;
     std::mutex long_lists_mu;

@@ -193,10 +193,6 @@ __device__ __forceinline__ uint32_t edge_word(const uint32_t *base, uint64_t idx
     return x & ((1u << ebits) - 1u);
 }
 
-// How a PageRank tile picks its vertices: from the active list, or every
-// vertex of a range (frontiers walked through their bitmap use chunks).
-enum TileMode { kList = 0, kRange = 1 };
-
 struct Smem {
     uint32_t pref[kBlock + 1];
     uint32_t start[kBlock];
@@ -1006,57 +1002,32 @@ struct PrAcc<float> {
     static __device__ __forceinline__ double value(unsigned long long a) { return __ull2double_rn(a) * 0x1p-62; }
 };
 
-template <typename T>
+// Arguments of the list-driven passes of reference PageRank.
 struct PrArgs {
-    typedef typename PrAcc<T>::type Acc;
     RegionArgs r;           // lists, segments, counts (pull over in-edges)
     const uint32_t *outdeg;
     double *rank;
-    const T *c_old;
-    T *c_new;
-    Acc *sum;               // partial sums of segmented vertices
-    double damping;
-    const double *dangling_prev;   // std mode: dangling mass of the previous pass
-    double *acc;            // std mode: [0] residual, [1] dangling of this pass
+    const double *c_old;
+    double *c_new;
+    double *sum;            // partial sums of segmented vertices
 };
 
-// The update of one vertex from its summed contributions s (FP64):
-// reference mode prKernel_Opt (gpu_kernels.cuh:533-552), standard mode
-// (1 - d) / V + d * (dangling mass / V + s) with the L1 residual and the
-// dangling mass of this pass accumulated in FP64.
-template <typename T>
-__device__ __forceinline__ bool pr_update(double *rank, const T *c_old, T *c_new, uint32_t v, uint32_t od, double s,
-                                          bool ref, double damping, double V, const double *dangling_prev,
-                                          double &res, double &dang) {
-    if (ref) {
-        const double r = rank[v];
-        const double t = fma(0.85, s, 0.15);
-        const double diff = t > r ? t - r : r - t;
-        if (diff > 0.001) {
-            rank[v] = t;
-            c_new[v] = od ? (T)(t / (double)od) : (T)0;
-            return true;
-        }
-        c_new[v] = c_old[v];
-        return false;
-    }
-    const double base = (1.0 - damping) / V + damping * (*dangling_prev) / V;
+// The reference update of an active vertex from its sum s (prKernel_Opt,
+// gpu_kernels.cuh:533-552): true while it stays active.
+__device__ __forceinline__ bool pr_ref_row(double *rank, const double *c_old, double *c_new, uint32_t v, uint32_t od,
+                                           double s) {
     const double r = rank[v];
-    const double rn = base + damping * s;
-    res += fabs(rn - r);
-    if (od == 0) dang += rn;
-    rank[v] = rn;
-    c_new[v] = od ? (T)(rn / (double)od) : (T)0;
+    const double t = fma(0.85, s, 0.15);
+    const double diff = t > r ? t - r : r - t;
+    if (diff > 0.001) {
+        rank[v] = t;
+        c_new[v] = od ? t / (double)od : 0.0;
+        return true;
+    }
+    c_new[v] = c_old[v];
     return false;
 }
 
-template <typename T, bool REF>
-__device__ __forceinline__ bool pr_apply(const PrArgs<T> &p, uint32_t v, double s, double &res, double &dang) {
-    return pr_update<T>(p.rank, p.c_old, p.c_new, v, p.outdeg[v], s, REF, p.damping, (double)p.r.V,
-                        p.dangling_prev, res, dang);
-}
-
-template <typename T>
 __device__ __forceinline__ void block_reduce2_atomic(double a, double b, double *out, double *s_buf) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -1086,22 +1057,18 @@ __device__ __forceinline__ void block_reduce2_atomic(double a, double b, double 
 #define ASC_PR_UNROLL 4
 #endif
 constexpr int kPrUnroll = ASC_PR_UNROLL;
-template <typename T>
 struct PrSmem {
     uint32_t pref[kBlock + 1];
     uint32_t start[kBlock];
     uint32_t warp[kWarps + 1];
-    typename PrAcc<T>::type sum[kBlock];
-    double red[2 * kWarps];
+    double sum[kBlock];
     uint32_t work;
 };
 
-// Reference mode walks the active set like a traversal frontier (list, or
-// the bitmap in id order when dense) and a vertex that stays active sets its
-// bit in the next bitmap; standard mode walks every vertex of the region.
-template <typename T, bool REF>
-__device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T> &sm, uint32_t *s_next) {
-    typedef typename PrAcc<T>::type Acc;
+// A tile of active vertices of a reference pass, which walks the active set
+// like a traversal frontier (list, or the bitmap in id order when dense); a
+// vertex that stays active sets its bit in the next bitmap.
+__device__ void pr_vertices(const PrArgs &p, bool valid, uint32_t u, PrSmem &sm, uint32_t *s_next) {
     const RegionArgs &a = p.r;
     uint32_t deg = 0, start = 0;
     bool huge = false;
@@ -1115,7 +1082,7 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
     uint32_t excl = block_excl_scan(deg, total, sm.warp);
     sm.pref[threadIdx.x] = excl;
     sm.start[threadIdx.x] = start;
-    sm.sum[threadIdx.x] = (Acc)0;
+    sm.sum[threadIdx.x] = 0;
     if (threadIdx.x == 0) sm.pref[kBlock] = total;
     const uint32_t nact = __syncthreads_count(valid && !huge);
     const int lane = threadIdx.x & 31;
@@ -1124,7 +1091,7 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
     // contribution gathered, before any is summed, so a thread has kPrUnroll
     // reads in flight instead of one
     for (uint32_t base = 0; base < total; base += kPrUnroll * kBlock) {
-        T x[kPrUnroll];
+        double x[kPrUnroll];
         int owner[kPrUnroll];
         uint32_t srcv[kPrUnroll];
 #pragma unroll
@@ -1148,36 +1115,30 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
             }
         }
 #pragma unroll
-        for (int k = 0; k < kPrUnroll; k++) x[k] = srcv[k] != 0xffffffffu ? p.c_old[srcv[k]] : (T)0;
+        for (int k = 0; k < kPrUnroll; k++) x[k] = srcv[k] != 0xffffffffu ? p.c_old[srcv[k]] : 0.0;
 #pragma unroll
         for (int k = 0; k < kPrUnroll; k++) {
             // segmented suffix sum over lanes with the same owner (owners
-            // ascend with the lane; a fixed shuffle tree, so the same edges
-            // give the same partial every pass)
-            T xs = x[k];
+            // ascend with the lane)
+            double xs = x[k];
             const int ow = owner[k];
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
-                T y = __shfl_down_sync(kFull, xs, d);
+                double y = __shfl_down_sync(kFull, xs, d);
                 int oy = __shfl_down_sync(kFull, ow, d);
                 if (lane + d < 32 && oy == ow) xs += y;
             }
             int oprev = __shfl_up_sync(kFull, ow, 1);
-            if (ow >= 0 && (lane == 0 || oprev != ow)) atomicAdd(&sm.sum[ow], PrAcc<T>::from(xs));
+            if (ow >= 0 && (lane == 0 || oprev != ow)) atomicAdd(&sm.sum[ow], xs);
         }
     }
     __syncthreads();
-    double res = 0, dang = 0;
-    bool won = false;
-    if (valid && !huge) won = pr_apply<T, REF>(p, u, PrAcc<T>::value(sm.sum[threadIdx.x]), res, dang);
-    if (REF) {
-        if (won) atomicOr(&a.bitmap[u >> 5], 1u << (u & 31));
-        count_next(a, won, u, s_next);
-        const uint32_t e = __reduce_add_sync(kFull, won ? deg : 0u);
-        if (lane == 0 && e) atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)e);
-    } else {
-        block_reduce2_atomic<T>(res, dang, p.acc, sm.red);
-    }
+    const bool won =
+        valid && !huge && pr_ref_row(p.rank, p.c_old, p.c_new, u, p.outdeg[u], sm.sum[threadIdx.x]);
+    if (won) atomicOr(&a.bitmap[u >> 5], 1u << (u & 31));
+    count_next(a, won, u, s_next);
+    const uint32_t e = __reduce_add_sync(kFull, won ? deg : 0u);
+    if (lane == 0 && e) atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)e);
     if (threadIdx.x == 0) {
         atomicAdd(&a.stats[a.region], (unsigned long long)total);
         atomicAdd(&a.stats[2 + a.region], (unsigned long long)nact);
@@ -1185,40 +1146,14 @@ __device__ void pr_vertices(const PrArgs<T> &p, bool valid, uint32_t u, PrSmem<T
     __syncthreads();
 }
 
-template <typename T, bool REF>
-__device__ __forceinline__ void pr_tile(const PrArgs<T> &p, uint32_t tile, uint32_t n_in, int mode, PrSmem<T> &sm,
-                                        uint32_t *s_next) {
-    const RegionArgs &a = p.r;
-    const uint32_t i = tile * kBlock + threadIdx.x;
-    bool valid;
-    uint32_t u = 0;
-    if (mode == kList) {
-        valid = i < n_in;
-        if (valid) u = a.q_in[i];
-    } else {
-        u = a.dense_begin + i;
-        valid = u < a.dense_end;
-    }
-    pr_vertices<T, REF>(p, valid, u, sm, s_next);
-}
-
-template <typename T, bool REF>
-__device__ void pr_bitmap_tile(const PrArgs<T> &p, uint32_t tile, PrSmem<T> &sm, uint32_t *s_next) {
-    const uint32_t u = (p.r.dense_begin & ~31u) + tile * kBlock + threadIdx.x;
-    const bool valid = (region_word(p.r, u & ~31u) >> (u & 31)) & 1u;
-    if (__syncthreads_or(valid)) pr_vertices<T, REF>(p, valid, u, sm, s_next);
-}
-
-template <typename T>
-__device__ void pr_segment(const PrArgs<T> &p, uint64_t item, PrSmem<T> &sm) {
-    typedef typename PrAcc<T>::type Acc;
+__device__ void pr_segment(const PrArgs &p, uint64_t item, PrSmem &sm) {
     const RegionArgs &a = p.r;
     const uint32_t u = (uint32_t)(item >> 32), k = (uint32_t)item;
     const uint32_t b0 = a.ptr[u], e0 = a.ptr[u + 1];
     const uint64_t b = (uint64_t)b0 + (uint64_t)k * a.seg_len;
     const uint64_t e = min((uint64_t)e0, b + a.seg_len);
     const uint32_t n = (uint32_t)(e - b);
-    T x = (T)0;  // this thread's edges in order, then a fixed warp tree
+    double x = 0;
     for (uint32_t j0 = threadIdx.x; j0 < n; j0 += kPrUnroll * kBlock) {
         // kPrUnroll loads in flight, added in edge order
         uint32_t sv[kPrUnroll];
@@ -1228,9 +1163,9 @@ __device__ void pr_segment(const PrArgs<T> &p, uint64_t item, PrSmem<T> &sm) {
             sv[k] = j < n ? edge_word(a.edges, b + j, a.ebits) : 0xffffffffu;
             if (sv[k] != 0xffffffffu && ASC_BAD(sv[k] >= a.V, 21, sv[k])) sv[k] = 0xffffffffu;
         }
-        T c[kPrUnroll];
+        double c[kPrUnroll];
 #pragma unroll
-        for (int k = 0; k < kPrUnroll; k++) c[k] = sv[k] != 0xffffffffu ? p.c_old[sv[k]] : (T)0;
+        for (int k = 0; k < kPrUnroll; k++) c[k] = sv[k] != 0xffffffffu ? p.c_old[sv[k]] : 0.0;
 #pragma unroll
         for (int k = 0; k < kPrUnroll; k++)
             if (sv[k] != 0xffffffffu) x += c[k];
@@ -1238,10 +1173,10 @@ __device__ void pr_segment(const PrArgs<T> &p, uint64_t item, PrSmem<T> &sm) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) x += __shfl_down_sync(kFull, x, d);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) sm.sum[w] = PrAcc<T>::from(x);
+    if (lane == 0) sm.sum[w] = x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        Acc s = (Acc)0;
+        double s = 0;
         for (int i = 0; i < kWarps; i++) s += sm.sum[i];
         atomicAdd(&p.sum[u], s);
         atomicAdd(&a.stats[a.region], (unsigned long long)n);
@@ -1250,72 +1185,40 @@ __device__ void pr_segment(const PrArgs<T> &p, uint64_t item, PrSmem<T> &sm) {
     __syncthreads();
 }
 
-template <typename T, bool REF>
-__global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_kernel(PrArgs<T> p) {
-    __shared__ PrSmem<T> sm;
-    __shared__ uint32_t s_next[2];
-    if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
+__device__ __forceinline__ void pr_list_item(const PrArgs &p, uint32_t w, uint32_t n_in, uint32_t nseg, bool bitmap,
+                                             PrSmem &sm, uint32_t *s_next) {
     const RegionArgs &a = p.r;
-    uint32_t n_in, nseg, total;
-    bool bitmap = false;
-    if (REF) {
-        region_items_bits(a, n_in, nseg, total, bitmap);
+    if (w < nseg) {
+        pr_segment(p, a.seg_in[w], sm);
+    } else if (bitmap) {
+        const uint32_t u = (a.dense_begin & ~31u) + (w - nseg) * kBlock + threadIdx.x;
+        const bool valid = (region_word(a, u & ~31u) >> (u & 31)) & 1u;
+        if (__syncthreads_or(valid)) pr_vertices(p, valid, u, sm, s_next);
     } else {
-        n_in = 0;
-        nseg = a.cnt_in[2 + a.region];
-        total = nseg + (a.dense_end - a.dense_begin + kBlock - 1) / kBlock;
-    }
-    for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(a.work, 1u);
-        __syncthreads();
-        const uint32_t w = sm.work;
-        __syncthreads();
-        if (w >= total) break;
-        if (w < nseg) pr_segment<T>(p, a.seg_in[w], sm);
-        else if (REF && bitmap) pr_bitmap_tile<T, REF>(p, w - nseg, sm, s_next);
-        else pr_tile<T, REF>(p, w - nseg, n_in, REF ? kList : kRange, sm, s_next);
-    }
-    if (REF) flush_next(a, s_next);
-}
-
-// Work items of one region for the pull pass (reference mode: its frontier;
-// standard mode: every vertex of the region, long lists as segments).
-template <bool REF>
-__device__ __forceinline__ void pr_items(const RegionArgs &a, uint32_t &n_in, uint32_t &nseg, uint32_t &total,
-                                         bool &bitmap) {
-    bitmap = false;
-    if (REF) {
-        region_items_bits(a, n_in, nseg, total, bitmap);
-    } else {
-        n_in = 0;
-        nseg = a.cnt_in[2 + a.region];
-        total = nseg + (a.dense_end - a.dense_begin + kBlock - 1) / kBlock;
+        const uint32_t i = (w - nseg) * kBlock + threadIdx.x;
+        pr_vertices(p, i < n_in, i < n_in ? a.q_in[i] : 0u, sm, s_next);
     }
 }
 
-template <typename T, bool REF>
-__device__ __forceinline__ void pr_item(const PrArgs<T> &p, uint32_t w, uint32_t n_in, uint32_t nseg, bool bitmap,
-                                        PrSmem<T> &sm, uint32_t *s_next) {
-    if (w < nseg) pr_segment<T>(p, p.r.seg_in[w], sm);
-    else if (REF && bitmap) pr_bitmap_tile<T, REF>(p, w - nseg, sm, s_next);
-    else pr_tile<T, REF>(p, w - nseg, n_in, REF ? kList : kRange, sm, s_next);
-}
-
-// Both regions of a pull pass in one launch, items alternating between the
-// on-demand and the static region while both have some (as the traversal's
+// Both regions of a list-driven pass in one launch, items alternating between
+// the on-demand and the static region while both have some (as the traversal's
 // fused expansion), so every SM overlaps host-link reads with HBM reads.
-template <typename T, bool REF>
-__global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_fused_kernel(PrArgs<T> p0, PrArgs<T> p1) {
-    __shared__ PrSmem<T> sm;
+// regions: bit 0 static, bit 1 on-demand.
+__global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_lists_kernel(PrArgs p0, PrArgs p1,
+                                                                                  uint32_t regions) {
+    __shared__ PrSmem sm;
     __shared__ uint32_t s_next[2];
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
     uint32_t n0, s0, i0, n1, s1, i1;
     bool b0, b1;
-    pr_items<REF>(p0.r, n0, s0, i0, b0);
-    pr_items<REF>(p1.r, n1, s1, i1, b1);
+    region_items_bits(p0.r, n0, s0, i0, b0);
+    region_items_bits(p1.r, n1, s1, i1, b1);
+    if (!(regions & 1u)) i0 = 0;
+    if (!(regions & 2u)) i1 = 0;
     const uint32_t m = min(i0, i1), total = i0 + i1;
+    uint32_t *work = (regions & 1u) ? p0.r.work : p1.r.work;
     for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(p0.r.work, 1u);
+        if (threadIdx.x == 0) sm.work = atomicAdd(work, 1u);
         __syncthreads();
         const uint32_t w = sm.work;
         __syncthreads();
@@ -1329,61 +1232,42 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_fused_kerne
             od = i1 > i0;
             local = m + (w - 2 * m);
         }
-        if (od) pr_item<T, REF>(p1, local, n1, s1, b1, sm, s_next);
-        else pr_item<T, REF>(p0, local, n0, s0, b0, sm, s_next);
+        if (od) pr_list_item(p1, local, n1, s1, b1, sm, s_next);
+        else pr_list_item(p0, local, n0, s0, b0, sm, s_next);
     }
-    if (REF) flush_next(p0.r, s_next);
+    flush_next(p0.r, s_next);
 }
 
-// Applies the segmented vertices once all their segments are summed. In
-// reference mode the list is this pass's segment items (k == 0 marks the
-// vertex); in standard mode it is the fixed list of long-list vertices.
-template <typename T, bool REF>
-__global__ void pr_apply_segmented_kernel(PrArgs<T> p, const uint64_t *items_static, const uint64_t *items_od,
-                                          const uint32_t *huge_list, uint32_t n_huge) {
-    __shared__ double red[2 * kWarps];
+// Applies the segmented vertices once all their segments are summed (this
+// pass's segment items; k == 0 marks the vertex).
+__global__ void pr_apply_segmented_kernel(PrArgs p, const uint64_t *items_static, const uint64_t *items_od) {
     const RegionArgs &a = p.r;
-    uint32_t n0 = 0, n1 = 0;
-    if (REF) {
-        n0 = a.cnt_in[2];
-        n1 = a.cnt_in[3];
-    }
-    const uint32_t n = REF ? n0 + n1 : n_huge;
+    const uint32_t n0 = a.cnt_in[2], n = n0 + a.cnt_in[3];
     const uint32_t stride = gridDim.x * blockDim.x;
-    double res = 0, dang = 0;
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
         const uint32_t i = base + threadIdx.x;
         bool won = false;
         uint32_t v = 0;
         if (i < n) {
-            bool go = true;
-            if (REF) {
-                uint64_t it = i < n0 ? items_static[i] : items_od[i - n0];
-                v = (uint32_t)(it >> 32);
-                go = (uint32_t)it == 0;
-            } else {
-                v = huge_list[i];
-            }
-            if (go) {
-                const double s = PrAcc<T>::value(p.sum[v]);
+            const uint64_t it = i < n0 ? items_static[i] : items_od[i - n0];
+            v = (uint32_t)(it >> 32);
+            if ((uint32_t)it == 0) {
+                const double s = p.sum[v];
                 p.sum[v] = 0;
-                won = pr_apply<T, REF>(p, v, s, res, dang);
+                won = pr_ref_row(p.rank, p.c_old, p.c_new, v, p.outdeg[v], s);
             }
         }
-        if (REF) {
-            // a long-list vertex that stays active joins the next bitmap
-            if (won) {
-                atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
-                atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)(a.ptr[v + 1] - a.ptr[v]));
-            }
-            const unsigned m0 = __ballot_sync(kFull, won && v < a.S), m1 = __ballot_sync(kFull, won && v >= a.S);
-            if ((threadIdx.x & 31) == 0) {
-                if (m0) atomicAdd(&a.cnt_out[6], (uint32_t)__popc(m0));
-                if (m1) atomicAdd(&a.cnt_out[7], (uint32_t)__popc(m1));
-            }
+        // a long-list vertex that stays active joins the next bitmap
+        if (won) {
+            atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+            atomicAdd(a.stats + (CTL_ACTIVE - CTL_STATS) / 2, (unsigned long long)(a.ptr[v + 1] - a.ptr[v]));
+        }
+        const unsigned m0 = __ballot_sync(kFull, won && v < a.S), m1 = __ballot_sync(kFull, won && v >= a.S);
+        if ((threadIdx.x & 31) == 0) {
+            if (m0) atomicAdd(&a.cnt_out[6], (uint32_t)__popc(m0));
+            if (m1) atomicAdd(&a.cnt_out[7], (uint32_t)__popc(m1));
         }
     }
-    if (!REF) block_reduce2_atomic<T>(res, dang, p.acc, red);
 }
 
 // ------------------------------------------- edge-balanced PageRank passes --
@@ -1635,7 +1519,7 @@ __device__ __forceinline__ void pr_item_row(const PrItemArgs<T> &p, uint32_t v, 
     }
     const uint32_t bit = 1u << (v & 31);
     if (!(p.bitmap_in[v >> 5] & bit)) return;
-    if (pr_update<T>(p.rank, p.c_old, p.c_new, v, p.outdeg[v], s, true, 0.85, 0.0, nullptr, n.res, n.dang)) {
+    if (pr_ref_row((double *)p.rank, (const double *)p.c_old, (double *)p.c_new, v, p.outdeg[v], s)) {
         atomicOr(&p.bitmap[v >> 5], bit);
         if (v < p.S) n.n0++;
         else n.n1++;
@@ -1803,7 +1687,7 @@ __global__ void pr_init_kernel(double *rank, T *c0, T *c1, typename PrAcc<T>::ty
             if (od == 0) d += r;
         }
     }
-    block_reduce2_atomic<T>(0.0, d, dang, red);
+    block_reduce2_atomic(0.0, d, dang, red);
 }
 
 // FP32 results: the FP64 ranks rounded to float (into the caller's device
@@ -1811,20 +1695,6 @@ __global__ void pr_init_kernel(double *rank, T *c0, T *c1, typename PrAcc<T>::ty
 __global__ void pr_rank_to_float_kernel(const double *rank, float *out, uint32_t V) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
         out[i] = (float)rank[i];
-}
-
-// Segment items of every long-list vertex (standard PageRank, fixed each pass).
-__global__ void seed_huge_segments_kernel(RegionArgs a, const uint32_t *huge_list, uint32_t n_static, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t v = huge_list[i];
-        const uint32_t deg = a.ptr[v + 1] - a.ptr[v];
-        const uint32_t nseg = (deg + a.seg_len - 1) / a.seg_len;
-        const bool od = i >= n_static;
-        const uint32_t base = atomicAdd(&a.cnt_out[2 + od], nseg);
-        if (ASC_BAD((uint64_t)base + nseg > (od ? a.segcap_ondemand : a.segcap_static), 20, base)) continue;
-        uint64_t *dst = a.seg_out + (od ? a.segcap_static : 0) + base;
-        for (uint32_t k = 0; k < nseg; k++) dst[k] = ((uint64_t)v << 32) | k;
-    }
 }
 
 // --------------------------------------------------------------- host -------
@@ -1856,25 +1726,21 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         cache.emplace_back();
         hit = cache.end() - 1;
         asc_graph::LongLists &ll = *hit;
+        ll.bits.assign(V / 32 + 2, 0);
         for (uint64_t v = 0; v < V; v++) {
             uint32_t d = g->h_ptr[v + 1] - g->h_ptr[v];
             if (d > t.huge_degree) {
                 uint64_t ns = (d + t.segment_edges - 1) / t.segment_edges;
-                if (v < S) { ll.seg_static += ns; ll.n_static++; }
-                else ll.seg_ondemand += ns;
-                ll.list.push_back((uint32_t)v);
+                (v < S ? ll.seg_static : ll.seg_ondemand) += ns;
+                ll.bits[v >> 5] |= 1u << (v & 31);
             }
         }
-        ll.bits.assign(V / 32 + 2, 0);
-        for (uint32_t v : ll.list) ll.bits[v >> 5] |= 1u << (v & 31);
         ll.huge_degree = t.huge_degree;
         ll.segment_edges = t.segment_edges;
     }
     const asc_graph::LongLists &ll = *hit;
-    const std::vector<uint32_t> &huge = ll.list, &hbits = ll.bits;
+    const std::vector<uint32_t> &hbits = ll.bits;
     const uint64_t cs = ll.seg_static, co = ll.seg_ondemand;
-    ws->n_huge_static = ll.n_static;
-    ws->n_huge_total = (uint32_t)huge.size();
     ws->segcap_static = cs;
     ws->segcap_ondemand = co;
     uint64_t bytes = 0;
@@ -1895,9 +1761,6 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         ASC_TRY(dalloc((void **)&ws->segs[i], 8 * (cs + co)));
     }
     ASC_TRY(dalloc((void **)&ws->ctl, 4 * CTL_WORDS));
-    ASC_TRY(dalloc((void **)&ws->huge_list, 4 * huge.size()));
-    if (!huge.empty())
-        ASC_CUDA(cudaMemcpy(ws->huge_list, huge.data(), 4 * huge.size(), cudaMemcpyHostToDevice));
     ASC_CUDA(cudaHostAlloc((void **)&ws->h_ctl, 4 * CTL_WORDS, cudaHostAllocDefault));
     for (auto &e : ws->ev) ASC_CUDA(cudaEventCreate(&e));
     ws->device_bytes = bytes;
@@ -1933,20 +1796,24 @@ asc_status ensure_pr_buffers(asc_graph *g, size_t elem) {
 
 // Work items of the edge-balanced PageRank passes (pr_plan_kernel), made once
 // per workspace.
-uint64_t pr_item_count(uint64_t rows, uint64_t edges) { return (rows + edges + kPrItem - 1) / kPrItem; }
-uint64_t pr_items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * (pr_item_count(V, E) + 2); }
+uint64_t pr_items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * ((V + E + kPrItem - 1) / kPrItem + 2); }
 
 asc_status ensure_pr_items(asc_graph *g) {
     Workspace *ws = g->ws;
     if (ws->pr_items) return ASC_OK;
     const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
-    const uint64_t n0 = pr_item_count(S, g->h_ptr[S]), n1 = pr_item_count(V - S, g->E - g->h_ptr[S]);
+    // shorter items where a staging buffer is smaller than one (its words, and
+    // up to 3 on either side to start and end on 16 bytes)
+    const uint64_t bits = g->edge_words == 2 ? 64 : g->ebits;
+    uint64_t L = kPrItem;
+    while (g->stage_words && L > 32 && (L * bits + 31) / 32 + 8 > g->stage_words) L /= 2;
+    const uint64_t n0 = (S + (uint64_t)g->h_ptr[S] + L - 1) / L, n1 = (V - S + g->E - g->h_ptr[S] + L - 1) / L;
     ASC_CUDA(cudaMalloc((void **)&ws->pr_items, sizeof(uint2) * (n0 + n1 + 1)));
     ws->device_bytes += sizeof(uint2) * (n0 + n1 + 1);
     ws->n_items_static = (uint32_t)n0;
     ws->n_items = (uint32_t)(n0 + n1);
     const uint64_t blocks = std::min<uint64_t>((n0 + n1) / kBlock + 1, (uint64_t)ws->num_sms * 8);
-    pr_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, kPrItem, ws->n_items_static,
+    pr_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, (uint32_t)L, ws->n_items_static,
                                                                ws->n_items, ws->pr_items);
     ASC_CUDA(cudaGetLastError());
     return ASC_OK;
@@ -2231,40 +2098,22 @@ asc_status build_loop_graph(asc_graph *g, asc_algo algo, uint32_t cap) {
 // region is copied each pass in chunks by the copy engine, on a stream of its
 // own, into the two device buffers (chunk k into buffer k % 2), while the
 // kernels consume the chunk before it; the copy of chunk k + 2 waits only for
-// the launch that read chunk k. Chunks end at vertex boundaries, except inside
-// a long list (more than huge_degree edges, summed by segments), which is cut
-// at segment boundaries; a chunk's tile range holds the vertices that start in
-// it, so every vertex is summed exactly once. The static region is cut into as
-// many slices by edges, and launch k runs static slice k with chunk k in one
-// grid (items interleaved), so every launch mixes HBM-bound gathers with the
-// staged chunk and the copies never wait for the static work. The reference
-// moves its gathered partitions into its staging area one at a time with
-// synchronous copies before each partition kernel (CalculateOpt.cu:161-178).
-struct StagePiece {
-    uint32_t v_lo = 0, v_hi = 0;  // tile range: the vertices that start in this piece
-    uint64_t e_lo = 0, e_hi = 0;  // its edges [e_lo, e_hi)
-    std::vector<uint64_t> segs;   // segment items (v << 32 | k) of long lists, in order
-};
-
+// the launch that read chunk k. A chunk is a run of items (pr_plan_kernel), so
+// long lists are cut between chunks as between items. The static items are cut
+// into as many slices, and launch k runs static slice k with chunk k in one
+// grid, so every launch mixes HBM-bound gathers with the staged chunk and the
+// copies never wait for the static work. The reference moves its gathered
+// partitions into its staging area one at a time with synchronous copies before
+// each partition kernel (CalculateOpt.cu:161-178).
 struct StageLaunch {
-    uint32_t s_lo = 0, s_hi = 0;  // static slice tile range
-    uint32_t c_lo = 0, c_hi = 0;  // chunk tile range
-    uint64_t w_lo = 0, w_n = 0;   // u32 words the chunk's copy moves (0: no chunk)
-    uint64_t seg_s = 0, seg_c = 0;  // offsets of the slice's and the chunk's segment items
-    uint32_t nseg_s = 0, nseg_c = 0;
-    // work items of the launch: segments plus tiles of kBlock vertices
-    uint64_t items() const {
-        return (uint64_t)nseg_s + nseg_c + (s_hi - s_lo + kBlock - 1) / kBlock + (c_hi - c_lo + kBlock - 1) / kBlock;
-    }
+    uint32_t s_begin = 0, s_n = 0;  // static items
+    uint32_t c_begin = 0, c_n = 0;  // the chunk's items
+    uint64_t w_lo = 0, w_n = 0;     // u32 words the chunk's copy moves, from a 16-byte boundary
 };
 
 struct StagePlan {
-    uint32_t huge = 0, seg_len = 0;  // the tuning the plan was made for
-    uint32_t chunks = 0;             // launches [0, chunks) carry a chunk
-    std::vector<StageLaunch> launches;
+    std::vector<StageLaunch> launches;  // one per chunk
     uint64_t copy_bytes = 0;         // moved per pass
-    uint64_t *d_segs = nullptr;      // every launch's segment items
-    uint32_t *d_cnt = nullptr;       // per launch, 8 words: [2] slice segments, [3] chunk segments
     uint32_t *d_work = nullptr;      // per launch work cursor
     cudaStream_t copy = nullptr;
     cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr};
@@ -2273,8 +2122,7 @@ struct StagePlan {
 void destroy_stage_plan(StagePlan *sp) {
     if (!sp) return;
     if (sp->copy) cudaStreamSynchronize(sp->copy);
-    for (void *q : {(void *)sp->d_segs, (void *)sp->d_cnt, (void *)sp->d_work})
-        if (q) cudaFree(q);
+    if (sp->d_work) cudaFree(sp->d_work);
     for (int i = 0; i < 2; i++) {
         if (sp->copied[i]) cudaEventDestroy(sp->copied[i]);
         if (sp->consumed[i]) cudaEventDestroy(sp->consumed[i]);
@@ -2299,140 +2147,60 @@ void edge_words_of(const asc_graph *g, uint64_t e_lo, uint64_t e_hi, uint64_t &w
     }
 }
 
-// Cuts vertices [v0, v1) into pieces whose edges satisfy fits(e_lo, e_hi).
-// False when a single short list or segment does not fit by itself.
-template <typename Fits>
-bool plan_pieces(const uint32_t *ptr, uint32_t v0, uint32_t v1, uint32_t huge, uint32_t seg_len, Fits fits,
-                 std::vector<StagePiece> &out) {
-    StagePiece cur;
-    cur.v_lo = v0;
-    cur.e_lo = cur.e_hi = ptr[v0];
-    auto close = [&](uint32_t v_hi, uint64_t next_e) {
-        cur.v_hi = v_hi;
-        out.push_back(std::move(cur));
-        cur = StagePiece();
-        cur.v_lo = v_hi;
-        cur.e_lo = cur.e_hi = next_e;
-    };
-    for (uint32_t v = v0; v < v1; v++) {
-        const uint64_t b = ptr[v], e = ptr[v + 1];
-        if (e - b <= huge) {
-            if (!fits(cur.e_lo, e)) {
-                if (cur.e_hi == cur.e_lo) return false;
-                close(v, b);
-                if (!fits(cur.e_lo, e)) return false;
-            }
-            cur.e_hi = e;
-            continue;
-        }
-        const uint64_t nseg = (e - b + seg_len - 1) / seg_len;
-        for (uint64_t k = 0; k < nseg; k++) {
-            const uint64_t sb = b + k * seg_len, se = std::min<uint64_t>(e, sb + seg_len);
-            if (!fits(cur.e_lo, se)) {
-                if (cur.e_hi == cur.e_lo) return false;
-                // v belongs to the piece holding its first segment
-                close(k == 0 ? v : v + 1, sb);
-                if (!fits(cur.e_lo, se)) return false;
-            }
-            cur.segs.push_back(((uint64_t)v << 32) | k);
-            cur.e_hi = se;
-        }
-    }
-    cur.v_hi = v1;
-    out.push_back(std::move(cur));
-    return true;
+// The words [w_lo, w_lo + w_n) of the edge array that a copy of edges
+// [e_lo, e_hi) moves so that it starts and ends on 16 bytes (or at the end).
+void staged_words(const asc_graph *g, uint64_t e_lo, uint64_t e_hi, uint64_t &w_lo, uint64_t &w_n) {
+    edge_words_of(g, e_lo, e_hi, w_lo, w_n);
+    if (!w_n) return;
+    const uint64_t end = std::min<uint64_t>(edge_store_words(g, g->E), (w_lo + w_n + 3) & ~3ull);
+    w_lo &= ~3ull;
+    w_n = end - w_lo;
 }
 
-// The chunk plan for the graph's current tuning; *ok false (and no plan) when
-// a long-list segment or a short list does not fit a staging buffer.
+// The chunks of the graph's on-demand items; *ok false (and no plan) when a
+// single item does not fit a staging buffer.
 asc_status ensure_stage_plan(asc_graph *g, bool *ok) {
     Workspace *ws = g->ws;
     *ok = false;
     if (!g->stage_words || g->static_edges >= g->E) return ASC_OK;
-    const uint32_t huge = ws->tune.huge_degree, seg_len = ws->tune.segment_edges;
-    if (ws->stage && ws->stage->huge == huge && ws->stage->seg_len == seg_len) {
+    if (ws->stage) {
         *ok = true;
         return ASC_OK;
     }
-    destroy_stage_plan(ws->stage);
-    ws->stage = nullptr;
-    const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
-    std::vector<StagePiece> chunks, slices;
-    const uint64_t cap_words = g->stage_words;
-    if (!plan_pieces(g->h_ptr, S, V, huge, seg_len,
-                     [&](uint64_t lo, uint64_t hi) {
-                         uint64_t w0, wn;
-                         edge_words_of(g, lo, hi, w0, wn);
-                         return wn <= cap_words;
-                     },
-                     chunks))
-        return ASC_OK;
-    // every chunk read stays inside its copy: the short lists of its tile range
-    // and its segments lie in its edges, which fit a buffer; the tile ranges
-    // cover [S, V) once
-    for (size_t k = 0; k < chunks.size(); k++) {
-        const StagePiece &c = chunks[k];
-        uint64_t w0, wn;
-        edge_words_of(g, c.e_lo, c.e_hi, w0, wn);
-        bool good = wn <= cap_words && c.v_lo == (k ? chunks[k - 1].v_hi : S) && c.v_hi >= c.v_lo;
-        for (uint32_t v = c.v_lo; good && v < c.v_hi; v++) {
-            const uint64_t b = g->h_ptr[v], e = g->h_ptr[v + 1];
-            if (e - b <= huge) good = b >= c.e_lo && e <= c.e_hi;
+    ASC_TRY(ensure_pr_items(g));
+    const uint32_t ns = ws->n_items_static, n = ws->n_items;
+    std::vector<uint2> items(n + 1);
+    ASC_CUDA(cudaMemcpyAsync(items.data(), ws->pr_items, sizeof(uint2) * items.size(), cudaMemcpyDeviceToHost,
+                             g->stream));
+    ASC_CUDA(cudaStreamSynchronize(g->stream));
+    StagePlan plan;
+    for (uint32_t i = ns; i < n;) {
+        StageLaunch x;
+        x.c_begin = i;
+        uint64_t w_lo, w_n;
+        for (; i < n; i++) {
+            staged_words(g, items[x.c_begin].y, items[i + 1].y, w_lo, w_n);
+            if (w_n > g->stage_words) break;
+            x.w_lo = w_lo;
+            x.w_n = w_n;
         }
-        for (uint64_t it : c.segs) {
-            const uint32_t v = (uint32_t)(it >> 32), j = (uint32_t)it;
-            const uint64_t b = (uint64_t)g->h_ptr[v] + (uint64_t)j * seg_len;
-            good = good && b >= c.e_lo && std::min<uint64_t>(g->h_ptr[v + 1], b + seg_len) <= c.e_hi;
-        }
-        if (!good) return fail(ASC_ERR_INVALID, "internal: staging chunk %zu does not cover its reads", k);
+        x.c_n = i - x.c_begin;
+        if (!x.c_n) return ASC_OK;
+        plan.copy_bytes += 4 * x.w_n;
+        plan.launches.push_back(x);
     }
-    if (chunks.back().v_hi != V) return fail(ASC_ERR_INVALID, "internal: staging chunks do not cover the region");
-    const uint64_t static_edges = g->h_ptr[S];
-    if (S > 0) {
-        const uint64_t cap = std::max<uint64_t>({(static_edges + chunks.size() - 1) / chunks.size(),
-                                                 (uint64_t)huge + 1, (uint64_t)seg_len});
-        plan_pieces(g->h_ptr, 0, S, huge, seg_len, [&](uint64_t lo, uint64_t hi) { return hi - lo <= cap; },
-                    slices);
+    const uint64_t L = plan.launches.size();
+    for (uint64_t k = 0; k < L; k++) {
+        StageLaunch &x = plan.launches[k];
+        x.s_begin = (uint32_t)(k * ns / L);
+        x.s_n = (uint32_t)((k + 1) * ns / L) - x.s_begin;
     }
-    StagePlan *sp = new StagePlan();
-    sp->huge = huge;
-    sp->seg_len = seg_len;
-    sp->chunks = (uint32_t)chunks.size();
-    const size_t L = std::max(chunks.size(), slices.size());
-    std::vector<uint64_t> segs;
-    std::vector<uint32_t> cnt(8 * L, 0);
-    sp->launches.resize(L);
-    for (size_t k = 0; k < L; k++) {
-        StageLaunch &x = sp->launches[k];
-        if (k < slices.size()) {
-            x.s_lo = slices[k].v_lo;
-            x.s_hi = slices[k].v_hi;
-            x.seg_s = segs.size();
-            x.nseg_s = (uint32_t)slices[k].segs.size();
-            cnt[8 * k + 2] = x.nseg_s;
-            segs.insert(segs.end(), slices[k].segs.begin(), slices[k].segs.end());
-        }
-        if (k < chunks.size()) {
-            x.c_lo = chunks[k].v_lo;
-            x.c_hi = chunks[k].v_hi;
-            edge_words_of(g, chunks[k].e_lo, chunks[k].e_hi, x.w_lo, x.w_n);
-            sp->copy_bytes += 4 * x.w_n;
-            x.seg_c = segs.size();
-            x.nseg_c = (uint32_t)chunks[k].segs.size();
-            cnt[8 * k + 3] = x.nseg_c;
-            segs.insert(segs.end(), chunks[k].segs.begin(), chunks[k].segs.end());
-        }
-    }
+    StagePlan *sp = new StagePlan(plan);
     asc_status st = ASC_OK;
     auto cu = [&](cudaError_t e, const char *what) {
         if (e != cudaSuccess && st == ASC_OK) st = cuda_fail(e, what, __FILE__, __LINE__);
     };
-    cu(cudaMalloc(&sp->d_segs, 8 * std::max<size_t>(1, segs.size())), "cudaMalloc(stage segments)");
-    cu(cudaMalloc(&sp->d_cnt, 4 * cnt.size()), "cudaMalloc(stage counts)");
     cu(cudaMalloc(&sp->d_work, 4 * L), "cudaMalloc(stage cursors)");
-    if (st == ASC_OK && !segs.empty())
-        cu(cudaMemcpy(sp->d_segs, segs.data(), 8 * segs.size(), cudaMemcpyHostToDevice), "cudaMemcpy(segments)");
-    if (st == ASC_OK) cu(cudaMemcpy(sp->d_cnt, cnt.data(), 4 * cnt.size(), cudaMemcpyHostToDevice), "cudaMemcpy");
     if (st == ASC_OK) cu(cudaStreamCreateWithFlags(&sp->copy, cudaStreamNonBlocking), "cudaStreamCreate");
     for (int i = 0; i < 2 && st == ASC_OK; i++) {
         cu(cudaEventCreateWithFlags(&sp->copied[i], cudaEventDisableTiming), "cudaEventCreate");
@@ -2452,8 +2220,13 @@ asc_status ensure_stage_plan(asc_graph *g, bool *ok) {
 // partitions of one staging buffer, cut at vertex boundaries only; each
 // iteration copies every partition that holds a frontier vertex, whole, and
 // expands that partition's frontier vertices from the copy.
+struct Partition {
+    uint32_t v_lo = 0, v_hi = 0;  // vertices
+    uint64_t w_lo = 0, w_n = 0;   // u32 words of their lists
+};
+
 struct PartPlan {
-    std::vector<StageLaunch> parts;  // c_lo / c_hi (tile range), w_lo / w_n (copy)
+    std::vector<Partition> parts;
     uint32_t *d_ranges = nullptr;    // per partition: tile range
     uint32_t *d_flags = nullptr;     // per partition: holds a frontier vertex this iteration
     uint32_t *h_flags = nullptr;     // page-locked mirror
@@ -2483,30 +2256,34 @@ asc_status ensure_part_plan(asc_graph *g) {
     if (!g->stage_words)
         return fail(ASC_ERR_INVALID, "the partition-copy engine needs staging buffers (asc_budget.stage_bytes)");
     const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
-    std::vector<StagePiece> parts;
+    std::vector<Partition> parts(1);
     const uint64_t cap = g->stage_words;
-    if (!plan_pieces(g->h_ptr, S, V, 0xffffffffu, 1u << 30,
-                     [&](uint64_t lo, uint64_t hi) {
-                         uint64_t w0, wn;
-                         edge_words_of(g, lo, hi, w0, wn);
-                         return wn <= cap;
-                     },
-                     parts))
-        return fail(ASC_ERR_BUDGET, "an adjacency list is longer than a partition (%llu words)",
-                    (unsigned long long)cap);
+    parts[0].v_lo = parts[0].v_hi = S;
+    for (uint32_t v = S; v < V; v++) {
+        uint64_t w_lo, w_n;
+        edge_words_of(g, g->h_ptr[parts.back().v_lo], g->h_ptr[v + 1], w_lo, w_n);
+        if (w_n > cap) {
+            Partition next;
+            next.v_lo = v;
+            edge_words_of(g, g->h_ptr[v], g->h_ptr[v + 1], w_lo, w_n);
+            if (w_n > cap)
+                return fail(ASC_ERR_BUDGET, "an adjacency list is longer than a partition (%llu words)",
+                            (unsigned long long)cap);
+            parts.push_back(next);
+        }
+        parts.back().v_hi = v + 1;
+        parts.back().w_lo = w_lo;
+        parts.back().w_n = w_n;
+    }
     PartPlan *pp = new PartPlan();
     const size_t n = parts.size();
     std::vector<uint32_t> ranges(2 * n), cnt(8 * n, 0);
-    pp->parts.resize(n);
     for (size_t k = 0; k < n; k++) {
-        StageLaunch &x = pp->parts[k];
-        x.c_lo = parts[k].v_lo;
-        x.c_hi = parts[k].v_hi;
-        edge_words_of(g, parts[k].e_lo, parts[k].e_hi, x.w_lo, x.w_n);
-        ranges[2 * k] = x.c_lo;
-        ranges[2 * k + 1] = x.c_hi;
+        ranges[2 * k] = parts[k].v_lo;
+        ranges[2 * k + 1] = parts[k].v_hi;
         cnt[8 * k + 7] = 1;  // with dense_div at its maximum: walk the range in id order
     }
+    pp->parts = std::move(parts);
     asc_status st = ASC_OK;
     auto cu = [&](cudaError_t e, const char *what) {
         if (e != cudaSuccess && st == ASC_OK) st = cuda_fail(e, what, __FILE__, __LINE__);
@@ -2549,39 +2326,32 @@ __global__ void part_active_kernel(const uint32_t *bitmap_in, const uint32_t *ra
     }
 }
 
-// Launch k's chunk: its copy on the copy stream once the launch that last read
-// the same buffer is done, and the compute stream s waits for it. Returns the
-// device address that the chunk's edge offsets index (the buffer less the
-// chunk's first word), or the static prefix when launch k has no chunk.
-const uint32_t *stage_chunk(asc_graph *g, StagePlan *sp, uint32_t k, cudaStream_t s, asc_status *st) {
+// Launch k's slices: static items in place and the chunk, whose copy goes to the
+// copy stream once the launch that last read the same buffer is done; the
+// compute stream s waits for it.
+asc_status stage_chunk(asc_graph *g, StagePlan *sp, uint32_t k, cudaStream_t s, PrSlice sl[2]) {
     const StageLaunch &x = sp->launches[k];
-    *st = ASC_OK;
-    if (!x.w_n) return g->d_static;
-    const int b = k & 1;
-    cudaError_t e = cudaStreamWaitEvent(sp->copy, sp->consumed[b], 0);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(g->d_stage[b], g->h_edges + x.w_lo, 4 * x.w_n, cudaMemcpyHostToDevice, sp->copy);
-    if (e == cudaSuccess) e = cudaEventRecord(sp->copied[b], sp->copy);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, sp->copied[b], 0);
-    if (e != cudaSuccess) *st = cuda_fail(e, "staged chunk copy", __FILE__, __LINE__);
-    return (const uint32_t *)((uintptr_t)g->d_stage[b] - 4 * (uintptr_t)x.w_lo);
+    sl[0] = pr_slice(g, 0);
+    sl[0].begin = x.s_begin;
+    sl[0].n = x.s_n;
+    sl[1].begin = x.c_begin;
+    sl[1].n = x.c_n;
+    sl[1].edges = g->d_stage[k & 1];
+    sl[1].edge_words = 0;
+    if (!x.w_n) return ASC_OK;  // rows without edges
+    ASC_CUDA(cudaStreamWaitEvent(sp->copy, sp->consumed[k & 1], 0));
+    ASC_CUDA(cudaMemcpyAsync(g->d_stage[k & 1], g->h_edges + x.w_lo, 4 * x.w_n, cudaMemcpyHostToDevice, sp->copy));
+    ASC_CUDA(cudaEventRecord(sp->copied[k & 1], sp->copy));
+    ASC_CUDA(cudaStreamWaitEvent(s, sp->copied[k & 1], 0));
+    // indexed by global edge offset: the buffer less the chunk's first word
+    sl[1].edges = (const uint32_t *)((uintptr_t)g->d_stage[k & 1] - 4 * (uintptr_t)x.w_lo);
+    sl[1].edge_words = x.w_lo + x.w_n;
+    return ASC_OK;
 }
 
 asc_status stage_release(StagePlan *sp, uint32_t k, cudaStream_t s) {
     if (sp->launches[k].w_n) ASC_CUDA(cudaEventRecord(sp->consumed[k & 1], s));
     return ASC_OK;
-}
-
-// Region arguments of launch k: the static slice (region 0) or the chunk
-// (region 1) with its tile range, segment items, counts and cursor.
-void stage_region(const StagePlan *sp, uint32_t k, int region, const uint32_t *edges, RegionArgs &a) {
-    const StageLaunch &x = sp->launches[k];
-    a.dense_begin = region == 0 ? x.s_lo : x.c_lo;
-    a.dense_end = region == 0 ? x.s_hi : x.c_hi;
-    a.seg_in = sp->d_segs + (region == 0 ? x.seg_s : x.seg_c);
-    a.cnt_in = sp->d_cnt + 8 * k;
-    a.work = sp->d_work + k;
-    if (region == 1) a.edges = edges;
 }
 
 void free_ws_buffers(Workspace *ws) {
@@ -2591,7 +2361,7 @@ void free_ws_buffers(Workspace *ws) {
                     (void *)ws->bitmap[1],
                     (void *)ws->queue[0],
                     (void *)ws->queue[1],
-                    (void *)ws->segs[0], (void *)ws->segs[1], (void *)ws->ctl, (void *)ws->huge_list, ws->pr_rank,
+                    (void *)ws->segs[0], (void *)ws->segs[1], (void *)ws->ctl, ws->pr_rank,
                     ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->pr_items, (void *)ws->pr_hot, (void *)ws->in_ptr, (void *)ws->in_edges,
                     (void *)ws->in_none})
         if (p) cudaFree(p);
@@ -2918,7 +2688,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             }
             for (uint32_t k = 0; cnt[7] && k < np; k++) {
                 if (!pp->h_flags[k]) continue;
-                const StageLaunch &x = pp->parts[k];
+                const Partition &x = pp->parts[k];
                 const int b = part_copies & 1;
                 ASC_CUDA(cudaStreamWaitEvent(pp->copy, pp->consumed[b], 0));
                 ASC_CUDA(cudaMemcpyAsync(g->d_stage[b], g->h_edges + x.w_lo, 4 * x.w_n, cudaMemcpyHostToDevice,
@@ -2928,13 +2698,13 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
                 RegionArgs a = region_args(g, parity, 1, false);
                 attach_far(g, algo, a);
                 a.edges = (const uint32_t *)((uintptr_t)g->d_stage[b] - 4 * (uintptr_t)x.w_lo);
-                a.dense_begin = x.c_lo;
-                a.dense_end = x.c_hi;
+                a.dense_begin = x.v_lo;
+                a.dense_end = x.v_hi;
                 a.cnt_in = pp->d_cnt + 8ull * k;  // id-order walk of the range, no segments
                 a.dense_div = 0xffffffffu;
                 a.huge = 0xffffffffu;             // long lists too are expanded from the copy
                 a.work = pp->d_work + k;
-                expand(g, a, grid_for(ws, (x.c_hi - (x.c_lo & ~31u) + kBlock - 1) / kBlock));
+                expand(g, a, grid_for(ws, (x.v_hi - (x.v_lo & ~31u) + kBlock - 1) / kBlock));
                 ASC_CUDA(cudaEventRecord(pp->consumed[b], s));
                 launches++;
                 part_copies++;
@@ -3121,14 +2891,14 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     // reference mode: this pass's active vertices per region and their in-edges
     uint32_t active[2] = {g->static_vertices, V - g->static_vertices};
     uint64_t active_edges = g->E;
-    unsigned long long dense_counts[4] = {0, 0, 0, 0};  // of the passes over items
+    unsigned long long item_counts[4] = {0, 0, 0, 0};  // of the passes over items
 
     // standard PageRank on a graph with staging buffers: the on-demand edges are
     // copied in chunks every pass, overlapped with the kernels
     bool staged = false;
     if (!REF && !pt.on && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
     StagePlan *sp = staged ? ws->stage : nullptr;
-    if (!staged) ASC_TRY(ensure_pr_items(g));
+    ASC_TRY(ensure_pr_items(g));
 
     // REF: the active set alternates parity like a traversal frontier. STD:
     // every vertex every pass (dense ranges), fixed segment list in parity 0.
@@ -3152,51 +2922,20 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         } else {
             ASC_CUDA(cudaMemsetAsync(acc + 2 * cp, 0, 16, s));
         }
-        PrArgs<T> pa;
-        memset(&pa, 0, sizeof(pa));
-        pa.outdeg = g->d_outdeg;
-        pa.rank = rank;
-        pa.c_old = c[cp];
-        pa.c_new = c[1 - cp];
-        pa.sum = (Acc *)ws->pr_sum;
-        pa.damping = REF ? 0.85 : p.damping;
-        pa.acc = acc + 2 * cp;
-        pa.dangling_prev = acc + 2 * (1 - cp) + 1;
-        if (staged) {
-            ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
-            for (uint32_t k = 0; k < (uint32_t)sp->launches.size(); k++) {
-                asc_status cs;
-                const uint32_t *chunk_edges = stage_chunk(g, sp, k, s, &cs);
-                ASC_TRY(cs);
-                PrArgs<T> p0 = pa, p1 = pa;
-                p0.r = region_args(g, parity, 0, true);
-                p1.r = region_args(g, parity, 1, true);
-                stage_region(sp, k, 0, chunk_edges, p0.r);
-                stage_region(sp, k, 1, chunk_edges, p1.r);
-                pr_pull_fused_kernel<T, REF><<<grid_for(ws, sp->launches[k].items()), kBlock, 0, s>>>(p0, p1);
-                ASC_TRY(stage_release(sp, k, s));
-                launches++;
-            }
-            if (ws->n_huge_total) {
-                pa.r = region_args(g, parity, 0, true);
-                pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, ws->n_huge_total), kBlock, 0, s>>>(
-                    pa, ws->segs[parity], ws->segs[parity] + ws->segcap_static, ws->huge_list, ws->n_huge_total);
-                launches++;
-            }
-        } else if (!REF || active_edges > g->E / kPrDenseDiv) {
-            // every row; one launch for both regions (timed runs launch them apart)
+        if (!REF || active_edges > g->E / kPrDenseDiv) {
+            // every row
             PrItemArgs<T> ia;
             memset(&ia, 0, sizeof(ia));
             ia.items = ws->pr_items;
             ia.ptr = g->d_ptr;
             ia.outdeg = g->d_outdeg;
             ia.rank = rank;
-            ia.c_old = pa.c_old;
-            ia.c_new = pa.c_new;
-            ia.sum = pa.sum;
-            ia.damping = pa.damping;
-            ia.dangling_prev = pa.dangling_prev;
-            ia.acc = pa.acc;
+            ia.c_old = c[cp];
+            ia.c_new = c[1 - cp];
+            ia.sum = (Acc *)ws->pr_sum;
+            ia.damping = p.damping;
+            ia.acc = acc + 2 * cp;
+            ia.dangling_prev = acc + 2 * (1 - cp) + 1;
             ia.work = ws->ctl + CTL_BLOCK * po + 4;
             ia.V = V;
             ia.ebits = g->ebits;
@@ -3205,56 +2944,66 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             ia.cnt_out = ws->ctl + CTL_BLOCK * po;
             ia.active_edges = (unsigned long long *)(ws->ctl + CTL_ACTIVE);
             ia.S = g->static_vertices;
-            for (int region = pt.on ? 0 : 2; region < (pt.on ? 2 : 3); region++) {
-                for (int r = 0; r < 2; r++) {
-                    ia.sl[r] = pr_slice(g, r);
-                    if (region != 2 && region != r) ia.sl[r].n = 0;
+            if (staged) ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
+            // one launch for both regions; one per chunk when staged; timed runs
+            // launch the regions apart
+            const uint32_t runs = staged ? (uint32_t)sp->launches.size() : pt.on ? 2 : 1;
+            for (uint32_t k = 0; k < runs; k++) {
+                if (staged) {
+                    ASC_TRY(stage_chunk(g, sp, k, s, ia.sl));
+                    ia.work = sp->d_work + k;
+                } else {
+                    for (uint32_t r = 0; r < 2; r++) {
+                        ia.sl[r] = pr_slice(g, (int)r);
+                        if (pt.on && r != k) ia.sl[r].n = 0;
+                    }
                 }
                 const uint32_t n = ia.sl[0].n + ia.sl[1].n;
                 if (!n) continue;
-                if (pt.on) ASC_CUDA(cudaMemsetAsync(ia.work, 0, 4, s));
-                ASC_TRY(pt.begin(region));
+                if (pt.on && !staged) ASC_CUDA(cudaMemsetAsync(ia.work, 0, 4, s));
+                ASC_TRY(pt.begin((int)k));
                 pt.record(s);
                 pr_pull_items_kernel<T, REF><<<item_grid(ws, n), kPrThreads, 0, s>>>(ia);
                 pt.record(s);
+                if (staged) ASC_TRY(stage_release(sp, k, s));
                 launches++;
             }
             pr_cut_rows_kernel<T, REF><<<fill_grid(ws, ws->n_items), kPrThreads, 0, s>>>(ia, ws->n_items);
             launches++;
             unsigned long long n[4];
             pr_pass_counts(g, 1, n);
-            dense_counts[0] += n[0];
-            dense_counts[1] += n[1];
-            dense_counts[2] += REF ? active[0] : n[2];
-            dense_counts[3] += REF ? active[1] : n[3];
+            item_counts[0] += n[0];
+            item_counts[1] += n[1];
+            item_counts[2] += REF ? active[0] : n[2];
+            item_counts[3] += REF ? active[1] : n[3];
         } else {
             // the active vertices' lists and segments, then one launch for both
             // regions (timed runs launch them apart)
             RegionArgs lists = region_args(g, po, 0, false);  // writes the lists of this parity
             build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(lists, ws->bitmap[parity], nwords);
-            const uint32_t grid = (uint32_t)(ws->num_sms * ws->tune.ctas_per_sm);
             launches++;
-            if (!pt.on) {
-                PrArgs<T> p0 = pa, p1 = pa;
-                p0.r = region_args(g, parity, 0, !REF);
-                p1.r = region_args(g, parity, 1, !REF);
-                pr_pull_fused_kernel<T, REF><<<grid, kBlock, 0, s>>>(p0, p1);
-                launches++;
+            PrArgs pr[2];
+            for (int r = 0; r < 2; r++) {
+                pr[r].r = region_args(g, parity, r, false);
+                pr[r].outdeg = g->d_outdeg;
+                pr[r].rank = rank;
+                pr[r].c_old = (const double *)c[cp];
+                pr[r].c_new = (double *)c[1 - cp];
+                pr[r].sum = (double *)ws->pr_sum;
             }
-            for (int region = 0; pt.on && region < 2; region++) {
-                if (!active[region]) continue;
-                pa.r = region_args(g, parity, region, !REF);
-                ASC_TRY(pt.begin(region));
+            for (uint32_t k = 0; k < (pt.on ? 2u : 1u); k++) {
+                if (pt.on && !active[k]) continue;
+                ASC_TRY(pt.begin((int)k));
                 pt.record(s);
-                pr_pull_kernel<T, REF><<<grid, kBlock, 0, s>>>(pa);
+                pr_pull_lists_kernel<<<(uint32_t)(ws->num_sms * ws->tune.ctas_per_sm), kBlock, 0, s>>>(
+                    pr[0], pr[1], pt.on ? 1u << k : 3u);
                 pt.record(s);
                 launches++;
             }
             const uint64_t segs = ws->segcap_static + ws->segcap_ondemand;
             if (segs) {
-                pa.r = region_args(g, parity, 0, !REF);
-                pr_apply_segmented_kernel<T, REF><<<fill_grid(ws, segs), kBlock, 0, s>>>(
-                    pa, ws->segs[parity], ws->segs[parity] + ws->segcap_static, ws->huge_list, ws->n_huge_total);
+                pr_apply_segmented_kernel<<<fill_grid(ws, segs), kBlock, 0, s>>>(
+                    pr[0], ws->segs[parity], ws->segs[parity] + ws->segcap_static);
                 launches++;
             }
         }
@@ -3287,12 +3036,12 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
         unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
-        for (int k = 0; k < 4; k++) n[k] += dense_counts[k];
+        for (int k = 0; k < 4; k++) n[k] += item_counts[k];
         st->iterations = it;
         st->edges_processed = n[0] + n[1];
         st->ondemand_edges = n[1];
         st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, n[1]);
-        st->staged_chunks = staged ? sp->chunks * (uint32_t)it : 0;
+        st->staged_chunks = staged ? (uint32_t)(sp->launches.size() * it) : 0;
         st->frontier_vertices = n[2] + n[3];
         st->ondemand_vertices = n[3];
         st->reached_vertices = V;
@@ -4353,10 +4102,10 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
 // the standard ones are the same as the pull kernels'.
 namespace {
 
+// Arguments of the update after a scatter.
 template <typename T>
 struct PushArgs {
     typedef typename PrAcc<T>::type Acc;
-    RegionArgs r0, r1;         // dense ranges and the fixed segment list
     const uint32_t *ptr;
     double *rank;
     const T *c_old;
@@ -4367,125 +4116,7 @@ struct PushArgs {
     double damping;
     const double *dangling_prev;
     double *acc;
-    uint32_t *work;
 };
-
-template <typename T>
-struct PushSmem {
-    uint32_t pref[kBlock + 1];
-    uint32_t start[kBlock];
-    typename PrAcc<T>::type c[kBlock];   // each tile vertex's contribution, as added
-    uint32_t warp[kWarps + 1];
-    uint32_t work;
-};
-
-template <typename T, int WORDS>
-__device__ void push_tile(const PushArgs<T> &p, const RegionArgs &a, uint32_t tile, PushSmem<T> &sm) {
-    typedef typename PrAcc<T>::type Acc;
-    const uint32_t u = a.dense_begin + tile * kBlock + threadIdx.x;
-    uint32_t deg = 0, start = 0;
-    Acc c = (Acc)0;
-    if (u < a.dense_end) {
-        start = a.ptr[u];
-        deg = a.ptr[u + 1] - start;
-        if (deg > a.huge) deg = 0;
-        c = PrAcc<T>::from(p.c_old[u]);
-    }
-    uint32_t total;
-    const uint32_t excl = block_excl_scan(deg, total, sm.warp);
-    sm.pref[threadIdx.x] = excl;
-    sm.start[threadIdx.x] = start;
-    sm.c[threadIdx.x] = c;
-    if (threadIdx.x == 0) sm.pref[kBlock] = total;
-    __syncthreads();
-    for (uint32_t base = 0; base < total; base += kUnroll * kBlock) {
-        uint32_t v[kUnroll];
-        Acc ck[kUnroll];
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++) {
-            const uint32_t e = base + k * kBlock + threadIdx.x;
-            v[k] = 0xffffffffu;
-            ck[k] = (Acc)0;
-            if (e < total) {
-                int lo = 0, hi = kBlock;
-                while (hi - lo > 1) {
-                    int mid = (lo + hi) >> 1;
-                    if (sm.pref[mid] <= e) lo = mid;
-                    else hi = mid;
-                }
-                const uint64_t idx = (uint64_t)sm.start[lo] + (e - sm.pref[lo]);
-                v[k] = WORDS == 2 ? __ldg(a.edges + 2 * idx) : edge_word(a.edges, idx, a.ebits) >> a.wbits;
-                ck[k] = sm.c[lo];
-                if (ASC_BAD(v[k] >= a.V, 18, v[k])) v[k] = 0xffffffffu;
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++)
-            if (v[k] != 0xffffffffu) atomicAdd(&p.sum[v[k]], ck[k]);
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(&a.stats[a.region], (unsigned long long)total);
-        atomicAdd(&a.stats[2 + a.region], (unsigned long long)min((uint32_t)kBlock, a.dense_end - a.dense_begin -
-                                                                                       tile * kBlock));
-    }
-    __syncthreads();
-}
-
-template <typename T, int WORDS>
-__device__ void push_segment(const PushArgs<T> &p, const RegionArgs &a, uint64_t item) {
-    const uint32_t u = (uint32_t)(item >> 32), k0 = (uint32_t)item;
-    if (ASC_BAD(u >= a.V, 19, u)) return;
-    const uint64_t b = (uint64_t)a.ptr[u] + (uint64_t)k0 * a.seg_len;
-    const uint64_t e = min((uint64_t)a.ptr[u + 1], b + a.seg_len);
-    const uint32_t n = (uint32_t)(e - b);
-    const typename PrAcc<T>::type c = PrAcc<T>::from(p.c_old[u]);
-    for (uint32_t base = 0; base < n; base += kUnroll * kBlock) {
-        uint32_t v[kUnroll];
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++) {
-            const uint32_t j = base + k * kBlock + threadIdx.x;
-            v[k] = j < n ? (WORDS == 2 ? __ldg(a.edges + 2 * (b + j)) : edge_word(a.edges, b + j, a.ebits) >> a.wbits)
-                         : 0xffffffffu;
-            if (v[k] != 0xffffffffu && ASC_BAD(v[k] >= a.V, 18, v[k])) v[k] = 0xffffffffu;
-        }
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++)
-            if (v[k] != 0xffffffffu) atomicAdd(&p.sum[v[k]], c);
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(&a.stats[a.region], (unsigned long long)n);
-        if (k0 == 0) atomicAdd(&a.stats[2 + a.region], 1ull);
-    }
-}
-
-template <typename T, int WORDS>
-__global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_scatter_kernel(PushArgs<T> p) {
-    __shared__ PushSmem<T> sm;
-    const uint32_t s0 = p.r0.cnt_in[2], s1 = p.r1.cnt_in[3];
-    const uint32_t t0 = s0 + (p.r0.dense_end - p.r0.dense_begin + kBlock - 1) / kBlock;
-    const uint32_t t1 = s1 + (p.r1.dense_end - p.r1.dense_begin + kBlock - 1) / kBlock;
-    const uint32_t mm = min(t0, t1), total = t0 + t1;
-    for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(p.work, 1u);
-        __syncthreads();
-        const uint32_t w = sm.work;
-        __syncthreads();
-        if (w >= total) break;
-        bool od;
-        uint32_t local;
-        if (w < 2 * mm) {
-            od = (w & 1) == 0;
-            local = w >> 1;
-        } else {
-            od = t1 > t0;
-            local = mm + (w - 2 * mm);
-        }
-        const RegionArgs &a = od ? p.r1 : p.r0;
-        const uint32_t s = od ? s1 : s0;
-        if (local < s) push_segment<T, WORDS>(p, a, a.seg_in[local]);
-        else push_tile<T, WORDS>(p, a, local - s, sm);
-    }
-}
 
 // Destinations that most edges share, found once per workspace: kPrHot slots by
 // a hash of the id, each with the most frequent destination among a sample of
@@ -4653,7 +4284,7 @@ __global__ void pr_push_apply_kernel(PushArgs<T> p, uint32_t V) {
                 p.c_new[v] = p.c_old[v];
                 continue;
             }
-            if (pr_update<T>(p.rank, p.c_old, p.c_new, v, od, s, true, 0.85, (double)V, nullptr, res, dang)) nact++;
+            if (pr_ref_row((double *)p.rank, (const double *)p.c_old, (double *)p.c_new, v, od, s)) nact++;
             else atomicAnd(&p.active[v >> 5], ~bit);
         } else {
             pr_std_row<T>(p.rank, p.c_new, v, od, s, p.damping, s_base, res, dang);
@@ -4664,7 +4295,7 @@ __global__ void pr_push_apply_kernel(PushArgs<T> p, uint32_t V) {
         for (int d = 16; d > 0; d >>= 1) nact += __shfl_down_sync(kFull, nact, d);
         if ((threadIdx.x & 31) == 0 && nact) atomicAdd(p.active_count, nact);
     } else {
-        block_reduce2_atomic<T>(res, dang, p.acc, red);
+        block_reduce2_atomic(res, dang, p.acc, red);
     }
 }
 
@@ -4688,7 +4319,7 @@ __global__ void pr_push_init_kernel(double *rank, T *c0, T *c1, typename PrAcc<T
         }
         if (i < (V + 31) / 32) active[i] = 0xffffffffu;
     }
-    block_reduce2_atomic<T>(0.0, d, acc_pair, red);
+    block_reduce2_atomic(0.0, d, acc_pair, red);
 }
 
 }  // namespace
@@ -4714,39 +4345,32 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     launches++;
     bool staged = false;
     if (!REF && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
-    if (staged && ws->n_huge_total) {
-        seed_huge_segments_kernel<<<fill_grid(ws, ws->n_huge_total), kBlock, 0, s>>>(
-            base_args(g, 1), ws->huge_list, ws->n_huge_static, ws->n_huge_total);
-        launches++;
-    }
     ASC_CUDA(cudaGetLastError());
     const int max_it = p.max_iterations > 0 ? p.max_iterations : (REF ? 1000000 : 100);
     StagePlan *sp = staged ? ws->stage : nullptr;
     PrItemArgs<T> ia;
     memset(&ia, 0, sizeof(ia));
-    if (!staged) {
-        ASC_TRY(ensure_pr_items(g));
-        ia.items = ws->pr_items;
-        ia.sl[0] = pr_slice(g, 0);
-        ia.sl[1] = pr_slice(g, 1);
-        ia.ptr = g->d_ptr;
-        ia.sum = (Acc *)ws->pr_sum;
-        ia.work = ws->ctl + CTL_BLOCK + 4;
-        ia.V = V;
-        ia.ebits = WORDS == 2 ? 64 : g->ebits;
-        ia.wbits = g->wbits;
-        if (!ws->pr_hot) {
-            ASC_CUDA(cudaMalloc((void **)&ws->pr_hot, 8 * kPrHot));
-            ws->device_bytes += 8 * kPrHot;
-            ASC_CUDA(cudaMemsetAsync(ws->pr_hot, 0, 8 * kPrHot, s));
-            pr_hot_count_kernel<T><<<item_grid(ws, ws->n_items / kPrHotSample + 1, 8), kBlock, 0, s>>>(
-                ia, (unsigned long long *)ws->pr_sum);
-            pr_hot_pick_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>((unsigned long long *)ws->pr_sum, V, ws->pr_hot);
-            launches += 2;
-            ASC_CUDA(cudaGetLastError());
-        }
-        ia.hot = ws->pr_hot;
+    ASC_TRY(ensure_pr_items(g));
+    ia.items = ws->pr_items;
+    ia.sl[0] = pr_slice(g, 0);
+    ia.sl[1] = pr_slice(g, 1);
+    ia.ptr = g->d_ptr;
+    ia.sum = (Acc *)ws->pr_sum;
+    ia.work = ws->ctl + CTL_BLOCK + 4;
+    ia.V = V;
+    ia.ebits = WORDS == 2 ? 64 : g->ebits;
+    ia.wbits = g->wbits;
+    if (!ws->pr_hot) {
+        ASC_CUDA(cudaMalloc((void **)&ws->pr_hot, 8 * kPrHot));
+        ws->device_bytes += 8 * kPrHot;
+        ASC_CUDA(cudaMemsetAsync(ws->pr_hot, 0, 8 * kPrHot, s));
+        pr_hot_count_kernel<T><<<item_grid(ws, ws->n_items / kPrHotSample + 1, 8), kBlock, 0, s>>>(
+            ia, (unsigned long long *)ws->pr_sum);
+        pr_hot_pick_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>((unsigned long long *)ws->pr_sum, V, ws->pr_hot);
+        launches += 2;
+        ASC_CUDA(cudaGetLastError());
     }
+    ia.hot = ws->pr_hot;
     int it = 0;
     double residual = 0;
     for (;;) {
@@ -4759,9 +4383,6 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
         ASC_CUDA(cudaMemsetAsync(REF ? (void *)active_count : (void *)(acc + 2 * cp), 0, REF ? 4 : 16, s));
         PushArgs<T> pa;
         memset(&pa, 0, sizeof(pa));
-        pa.r0 = region_args(g, 0, 0, true);
-        pa.r1 = region_args(g, 0, 1, true);
-        pa.work = ws->ctl + CTL_BLOCK + 4;
         pa.ptr = g->d_ptr;
         pa.rank = rank;
         pa.c_old = c[cp];
@@ -4772,24 +4393,16 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
         pa.damping = REF ? 0.85 : p.damping;
         pa.acc = acc + 2 * cp;
         pa.dangling_prev = acc + 2 * (1 - cp) + 1;
-        if (staged) {
-            ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
-            for (uint32_t k = 0; k < (uint32_t)sp->launches.size(); k++) {
-                asc_status cs;
-                const uint32_t *chunk_edges = stage_chunk(g, sp, k, s, &cs);
-                ASC_TRY(cs);
-                PushArgs<T> pk = pa;
-                stage_region(sp, k, 0, chunk_edges, pk.r0);
-                stage_region(sp, k, 1, chunk_edges, pk.r1);
-                pk.work = sp->d_work + k;
-                pr_scatter_kernel<T, WORDS><<<grid_for(ws, sp->launches[k].items()), kBlock, 0, s>>>(pk);
-                ASC_TRY(stage_release(sp, k, s));
-                launches++;
+        ia.c_old = pa.c_old;
+        if (staged) ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
+        for (uint32_t k = 0; k < (staged ? (uint32_t)sp->launches.size() : 1u); k++) {
+            if (staged) {
+                ASC_TRY(stage_chunk(g, sp, k, s, ia.sl));
+                ia.work = sp->d_work + k;
             }
-        } else {
-            ia.c_old = pa.c_old;
-            pr_scatter_items_kernel<T>
-                <<<item_grid(ws, ws->n_items, ASC_PR_SCATTER_BLOCKS), kPrThreads, 0, s>>>(ia);
+            pr_scatter_items_kernel<T><<<item_grid(ws, ia.sl[0].n + ia.sl[1].n, ASC_PR_SCATTER_BLOCKS), kPrThreads, 0,
+                                         s>>>(ia);
+            if (staged) ASC_TRY(stage_release(sp, k, s));
             launches++;
         }
         pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kBlock, 0, s>>>(pa, V);
@@ -4818,13 +4431,13 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     if (st) {
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
-        unsigned long long n[4] = {hs[0], hs[1], hs[2], hs[3]};
-        if (!staged) pr_pass_counts(g, (uint64_t)it, n);
+        unsigned long long n[4];
+        pr_pass_counts(g, (uint64_t)it, n);
         st->iterations = it;
         st->edges_processed = n[0] + n[1];
         st->ondemand_edges = n[1];
         st->ondemand_bytes = staged ? sp->copy_bytes * (uint64_t)it : edge_store_bytes(g, n[1]);
-        st->staged_chunks = staged ? sp->chunks * (uint32_t)it : 0;
+        st->staged_chunks = staged ? (uint32_t)(sp->launches.size() * it) : 0;
         st->frontier_vertices = n[2] + n[3];
         st->ondemand_vertices = n[3];
         st->reached_vertices = V;
