@@ -71,6 +71,7 @@ struct Workspace {
     unsigned long long *pr_hot = nullptr;  // scatter passes: most frequent destinations
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> phase_events;
+    cudaEvent_t pass_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // ends of PageRank passes
     struct BatchEngine *batch[2] = {nullptr, nullptr};  // asc_run_batch engines (BFS, SSSP)
     cudaGraphExec_t loop_exec[3] = {nullptr, nullptr, nullptr};  // BFS, SSSP, CC iteration loops
     uint32_t loop_cap[3] = {0, 0, 0};

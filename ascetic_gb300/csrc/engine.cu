@@ -95,9 +95,12 @@ enum Alg { kBFS = 0, kSSSP = 1, kCC = 2 };
 // the SSSP near-far threshold, word 36 the minimum far distance of a pass.
 // Words 42-43 (u64): in-edges that bottom-up BFS steps read from host memory;
 // words 44-45 (u64): unreached vertices those steps examined. Words 46-47 (u64):
-// in-edges of the vertices that a reference PageRank pass left active.
+// in-edges of the vertices that a reference PageRank pass left active; words
+// 48-59: three residual and dangling-mass pairs (FP64) of PageRank passes, word
+// 60 the ticket of the blocks that end a pass.
 enum { CTL_BLOCK = 8, CTL_STATS = 16, CTL_ITERS = 28, CTL_TIMEOUT = 29, CTL_BODIES = 30, CTL_THRESH = 31,
-       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_WORDS = 64 };
+       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_ACC = 48,
+       CTL_TICKET = 60, CTL_WORDS = 64 };
 
 struct RegionArgs {
     const uint32_t *ptr;
@@ -1369,12 +1372,19 @@ struct PrItemArgs {
     uint32_t V, ebits;
     uint32_t wbits;          // scatter: weight bits below the destination in an edge word
     const unsigned long long *hot;  // scatter: hot destinations by slot
+    const uint32_t *active_prev;    // scatter, reference mode: vertices the previous pass left active
     // reference mode: active vertices of this pass and the next one, their counts
     // per region (cnt_out[6..7]) and the next one's in-edges
     const uint32_t *bitmap_in;
-    uint32_t *bitmap, *cnt_out;
+    uint32_t *bitmap, *cnt_in, *cnt_out;
     unsigned long long *active_edges;
     uint32_t S;
+    // how a pass ends (see pr_pass_over)
+    const double *res_prev;  // residual of the previous pass (null: first pass)
+    double tolerance;
+    double *acc_next;        // cleared for the next pass
+    uint32_t *ticket;
+    unsigned long long *report;  // host: residual, or active vertices (2) and in-edges
 };
 
 template <typename T>
@@ -1502,6 +1512,39 @@ __device__ __forceinline__ void pr_reduce2_atomic(double a, double b, double *ou
     }
 }
 
+// The host reads how a pass ended one pass late, so that the next one is
+// already in flight: a pass that follows the last one changes nothing.
+template <bool REF, typename T>
+__device__ __forceinline__ bool pr_pass_over(const PrItemArgs<T> &p) {
+    if (REF) return !(p.cnt_in[6] | p.cnt_in[7]);
+    return p.res_prev && *p.res_prev < p.tolerance;
+}
+
+// Run by every block of the kernel that ends a pass: the last one reports to the
+// host and clears what the next pass counts in.
+template <bool REF, typename T>
+__device__ __forceinline__ void pr_end_pass(const PrItemArgs<T> &p) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(p.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last || threadIdx.x) return;
+    __threadfence();
+    volatile unsigned long long *r = p.report;
+    if (REF) {
+        volatile uint32_t *c = p.cnt_out;
+        r[0] = ((unsigned long long)c[7] << 32) | c[6];
+        r[1] = *(volatile unsigned long long *)p.active_edges;
+        *p.active_edges = 0;
+    } else {
+        r[0] = *(volatile unsigned long long *)p.acc;
+        p.acc_next[0] = p.acc_next[1] = 0;
+    }
+    for (int i = 0; i < CTL_BLOCK; i++) p.cnt_in[i] = 0;  // the next pass's output counts and cursor
+    *p.ticket = 0;
+}
+
 // What a thread of an item pass counts over the rows it applies.
 struct PrCounts {
     double res = 0, dang = 0;         // standard mode
@@ -1548,6 +1591,7 @@ __device__ __forceinline__ void pr_flush_counts(const PrItemArgs<T> &p, PrCounts
 template <typename T, bool REF>
 __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_kernel(PrItemArgs<T> p) {
     typedef typename PrAcc<T>::type Acc;
+    if (pr_pass_over<REF>(p)) return;
     __shared__ PrItemSmem<T> sm;
     const int lane = threadIdx.x & 31;
     const uint32_t total = p.sl[0].n + p.sl[1].n;
@@ -1646,9 +1690,11 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
 }
 
 // Applies the rows that were cut by an item boundary: the row at the start of
-// item i, when it began earlier and ends in item i. Blocks of kPrThreads.
+// item i, when it began earlier and ends in item i. Ends the pass. Blocks of
+// kPrThreads.
 template <typename T, bool REF>
 __global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n_items) {
+    if (pr_pass_over<REF>(p)) return;
     __shared__ double red[2 * kPrWarps];
     __shared__ double s_base;
     if (!REF && threadIdx.x == 0)
@@ -1665,6 +1711,13 @@ __global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n_items) {
         }
     }
     pr_flush_counts<REF>(p, n, red);
+    pr_end_pass<REF>(p);
+}
+
+// Ends a list-driven reference pass.
+template <typename T>
+__global__ void pr_end_pass_kernel(PrItemArgs<T> p) {
+    pr_end_pass<true>(p);
 }
 
 template <typename T>
@@ -1817,6 +1870,34 @@ asc_status ensure_pr_items(asc_graph *g) {
                                                                ws->n_items, ws->pr_items);
     ASC_CUDA(cudaGetLastError());
     return ASC_OK;
+}
+
+// How PageRank passes report to the host: pass k writes two words of page-locked
+// memory (kPassSlots slots) and an event says when. At most two passes are in
+// flight; one at a time where the caller watches iterations.
+constexpr int kPassSlots = 4;
+unsigned long long *pass_slot(Workspace *ws, int k) {
+    return (unsigned long long *)ws->h_ctl + 2 * (k % kPassSlots);
+}
+asc_status ensure_pass_events(Workspace *ws) {
+    for (auto &e : ws->pass_ev)
+        if (!e) ASC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return ASC_OK;
+}
+// The waits of pass k's end and the standard-mode fields of its arguments: the
+// residual and dangling-mass pairs of three consecutive passes.
+template <typename T>
+void set_pass(Workspace *ws, const asc_params &p, int k, PrItemArgs<T> &a) {
+    double *acc = (double *)(ws->ctl + CTL_ACC);
+    a.acc = acc + 2 * (k % 3);
+    a.acc_next = acc + 2 * ((k + 1) % 3);
+    const double *prev = acc + 2 * ((k + 2) % 3);
+    a.dangling_prev = prev + 1;
+    a.res_prev = k ? prev : nullptr;
+    a.tolerance = p.tolerance;
+    a.damping = p.damping;
+    a.ticket = ws->ctl + CTL_TICKET;
+    a.report = pass_slot(ws, k);
 }
 
 // A region's items and edges.
@@ -2375,6 +2456,8 @@ void free_ws_buffers(Workspace *ws) {
     for (auto e : ws->ev)
         if (e) cudaEventDestroy(e);
     for (auto e : ws->phase_events) cudaEventDestroy(e);
+    for (auto e : ws->pass_ev)
+        if (e) cudaEventDestroy(e);
     destroy_stage_plan(ws->stage);
     ws->stage = nullptr;
     destroy_part_plan(ws->part);
@@ -2868,16 +2951,14 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     uint32_t launches = 0;
     PhaseTimer pt(ws, (p.flags & ASC_RUN_PHASE_TIMING) != 0);
     typedef typename PrAcc<T>::type Acc;
-    // FP64 accumulators per pass parity q: acc[2q] residual, acc[2q+1] dangling mass
-    double *acc = (double *)(ws->ctl + CTL_PR);
     double *rank = (double *)ws->pr_rank;
     T *c[2] = {(T *)ws->pr_contrib[0], (T *)ws->pr_contrib[1]};
 
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
     ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
-    // the start vector's dangling mass goes to the parity-1 pair, which pass 0 reads
+    // the start vector's dangling mass goes to the pair before pass 0's
     pr_init_kernel<T><<<fill_grid(ws, V), kBlock, 0, s>>>(rank, c[0], c[1], (Acc *)ws->pr_sum, g->d_outdeg, V,
-                                                          acc + 2);
+                                                          (double *)(ws->ctl + CTL_ACC) + 4);
     launches++;
     RegionArgs sa = base_args(g, 1);  // seeds land in parity 0
     const uint32_t nwords = V / 32 + 1;
@@ -2900,29 +2981,59 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     StagePlan *sp = staged ? ws->stage : nullptr;
     ASC_TRY(ensure_pr_items(g));
 
-    // REF: the active set alternates parity like a traversal frontier. STD:
-    // every vertex every pass (dense ranges), fixed segment list in parity 0.
-    int parity = 0;
-    int it = 0;
+    // REF: the active set alternates parity like a traversal frontier.
+    ASC_TRY(ensure_pass_events(ws));
+    const int depth = pt.on || staged || t_iteration_hook.fn ? 1 : 2;
+    int it = 0, launched = 0;  // passes that ended, that were launched
+    bool over_items[kPassSlots];  // a pass in flight runs over items, not lists
     const int max_it = p.max_iterations > 0 ? p.max_iterations : (REF ? 1000000 : 100);
     double residual = 0;
     double phase_ms[2] = {0, 0};
+    bool over = false;
+    auto wait_pass = [&]() -> asc_status {  // for the oldest pass in flight
+        ASC_CUDA(cudaEventSynchronize(ws->pass_ev[it % kPassSlots]));
+        if (over_items[it % kPassSlots]) {
+            unsigned long long n[4];
+            pr_pass_counts(g, 1, n);
+            item_counts[0] += n[0];
+            item_counts[1] += n[1];
+            item_counts[2] += REF ? active[0] : n[2];
+            item_counts[3] += REF ? active[1] : n[3];
+        }
+        const unsigned long long *r = pass_slot(ws, it);
+        if (REF) {
+            active[0] = (uint32_t)r[0];
+            active[1] = (uint32_t)(r[0] >> 32);
+            active_edges = r[1];
+            over = !(active[0] | active[1]);
+        } else {
+            memcpy(&residual, r, 8);
+            over = residual < p.tolerance;
+        }
+        if (pt.on) ASC_TRY(pt.sum(phase_ms));
+        it++;
+        iteration_boundary();
+        return ASC_OK;
+    };
     for (;;) {
-        if (REF && !(active[0] | active[1])) break;
-        if (it >= max_it) {
+        if (launched - it >= depth || (launched > it && launched >= max_it)) ASC_TRY(wait_pass());
+        if (over) break;  // a pass launched after the last one changes nothing
+        if (launched >= max_it) {
+            if (launched > it) continue;
             if (REF) return fail(ASC_ERR_TIMEOUT, "reference PageRank still active after %d passes", it);
             break;
         }
-        const int cp = it & 1;
-        const int po = 1 - parity;
-        ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_BLOCK * po, 0, 4 * CTL_BLOCK, s));
-        if (REF) {
-            ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
-            ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_ACTIVE, 0, 8, s));
-        } else {
-            ASC_CUDA(cudaMemsetAsync(acc + 2 * cp, 0, 16, s));
+        // reference mode: lists are made from this pass's own counts; items serve
+        // any, so their rule may look at those of the pass before
+        if (REF && active_edges <= g->E / kPrDenseDiv && launched > it) {
+            ASC_TRY(wait_pass());
+            if (over) break;
         }
-        if (!REF || active_edges > g->E / kPrDenseDiv) {
+        const int cp = launched & 1;
+        const int parity = cp, po = 1 - cp;
+        if (REF) ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
+        over_items[launched % kPassSlots] = !REF || active_edges > g->E / kPrDenseDiv;
+        if (over_items[launched % kPassSlots]) {
             // every row
             PrItemArgs<T> ia;
             memset(&ia, 0, sizeof(ia));
@@ -2933,14 +3044,13 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             ia.c_old = c[cp];
             ia.c_new = c[1 - cp];
             ia.sum = (Acc *)ws->pr_sum;
-            ia.damping = p.damping;
-            ia.acc = acc + 2 * cp;
-            ia.dangling_prev = acc + 2 * (1 - cp) + 1;
+            set_pass(ws, p, launched, ia);
             ia.work = ws->ctl + CTL_BLOCK * po + 4;
             ia.V = V;
             ia.ebits = g->ebits;
             ia.bitmap_in = ws->bitmap[parity];
             ia.bitmap = ws->bitmap[po];
+            ia.cnt_in = ws->ctl + CTL_BLOCK * parity;
             ia.cnt_out = ws->ctl + CTL_BLOCK * po;
             ia.active_edges = (unsigned long long *)(ws->ctl + CTL_ACTIVE);
             ia.S = g->static_vertices;
@@ -2970,12 +3080,6 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             }
             pr_cut_rows_kernel<T, REF><<<fill_grid(ws, ws->n_items), kPrThreads, 0, s>>>(ia, ws->n_items);
             launches++;
-            unsigned long long n[4];
-            pr_pass_counts(g, 1, n);
-            item_counts[0] += n[0];
-            item_counts[1] += n[1];
-            item_counts[2] += REF ? active[0] : n[2];
-            item_counts[3] += REF ? active[1] : n[3];
         } else {
             // the active vertices' lists and segments, then one launch for both
             // regions (timed runs launch them apart)
@@ -3006,23 +3110,18 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                     pr[0], ws->segs[parity], ws->segs[parity] + ws->segcap_static);
                 launches++;
             }
+            PrItemArgs<T> ia;
+            memset(&ia, 0, sizeof(ia));
+            set_pass(ws, p, launched, ia);
+            ia.cnt_in = ws->ctl + CTL_BLOCK * parity;
+            ia.cnt_out = ws->ctl + CTL_BLOCK * po;
+            ia.active_edges = (unsigned long long *)(ws->ctl + CTL_ACTIVE);
+            pr_end_pass_kernel<T><<<1, 32, 0, s>>>(ia);
+            launches++;
         }
         ASC_CUDA(cudaGetLastError());
-        if (REF) ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_WORDS, cudaMemcpyDeviceToHost, s));
-        else ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, acc + 2 * cp, 16, cudaMemcpyDeviceToHost, s));
-        ASC_CUDA(cudaStreamSynchronize(s));
-        if (pt.on) ASC_TRY(pt.sum(phase_ms));
-        it++;
-        iteration_boundary();
-        if (REF) {
-            active[0] = ws->h_ctl[CTL_BLOCK * po + 6];
-            active[1] = ws->h_ctl[CTL_BLOCK * po + 7];
-            memcpy(&active_edges, ws->h_ctl + CTL_ACTIVE, 8);
-            parity = po;
-        } else {
-            memcpy(&residual, ws->h_ctl, 8);
-            if (residual < p.tolerance) break;
-        }
+        ASC_CUDA(cudaEventRecord(ws->pass_ev[launched % kPassSlots], s));
+        launched++;
     }
     ASC_CUDA(cudaEventRecord(ws->ev[1], s));
     if (out && !(p.flags & ASC_RUN_NO_OUTPUT)) {
@@ -4102,22 +4201,6 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
 // the standard ones are the same as the pull kernels'.
 namespace {
 
-// Arguments of the update after a scatter.
-template <typename T>
-struct PushArgs {
-    typedef typename PrAcc<T>::type Acc;
-    const uint32_t *ptr;
-    double *rank;
-    const T *c_old;
-    T *c_new;
-    Acc *sum;
-    uint32_t *active;          // reference mode: one bit per still-active vertex
-    uint32_t *active_count;
-    double damping;
-    const double *dangling_prev;
-    double *acc;
-};
-
 // Destinations that most edges share, found once per workspace: kPrHot slots by
 // a hash of the id, each with the most frequent destination among a sample of
 // the edges (count << 32 | id; 0: empty). Their atomics meet in a few L2 slices:
@@ -4194,6 +4277,7 @@ struct PrHot<float> {
 template <typename T>
 __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_items_kernel(PrItemArgs<T> p) {
     typedef typename PrAcc<T>::type Acc;
+    if (p.active_prev ? !*p.active_prev : pr_pass_over<false>(p)) return;
     __shared__ PrItemSmem<T> sm;
     __shared__ PrHot<T> hot;
     for (uint32_t i = threadIdx.x; i < kPrHot; i += kPrThreads) {
@@ -4261,42 +4345,56 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_
     }
 }
 
+// The update of every vertex after a scatter; ends the pass. Reference mode:
+// active holds one bit per vertex that is still active, active_count this
+// pass's and active_next the next one's number of them.
 template <typename T, bool REF>
-__global__ void pr_push_apply_kernel(PushArgs<T> p, uint32_t V) {
-    __shared__ double red[2 * kWarps];
+__global__ void __launch_bounds__(kPrThreads) pr_push_apply_kernel(PrItemArgs<T> p, uint32_t *active,
+                                                                   uint32_t *active_count, uint32_t *active_next) {
+    if (p.active_prev ? !*p.active_prev : pr_pass_over<false>(p)) return;
+    __shared__ double red[2 * kPrWarps];
     __shared__ double s_base;
+    const uint32_t V = p.V;
     if (!REF) {
         if (threadIdx.x == 0) s_base = (1.0 - p.damping) / (double)V + p.damping * (*p.dangling_prev) / (double)V;
         __syncthreads();
     }
     double res = 0, dang = 0;
     uint32_t nact = 0;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < V; base += stride) {
-        const uint32_t v = base + threadIdx.x;
-        if (v >= V) continue;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
         const double s = PrAcc<T>::value(p.sum[v]);
         p.sum[v] = 0;
         const uint32_t od = p.ptr[v + 1] - p.ptr[v];
         if (REF) {
             const uint32_t bit = 1u << (v & 31);
-            if (!(p.active[v >> 5] & bit)) {
+            if (!(active[v >> 5] & bit)) {
                 p.c_new[v] = p.c_old[v];
                 continue;
             }
             if (pr_ref_row((double *)p.rank, (const double *)p.c_old, (double *)p.c_new, v, od, s)) nact++;
-            else atomicAnd(&p.active[v >> 5], ~bit);
+            else atomicAnd(&active[v >> 5], ~bit);
         } else {
             pr_std_row<T>(p.rank, p.c_new, v, od, s, p.damping, s_base, res, dang);
         }
     }
-    if (REF) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) nact += __shfl_down_sync(kFull, nact, d);
-        if ((threadIdx.x & 31) == 0 && nact) atomicAdd(p.active_count, nact);
-    } else {
-        block_reduce2_atomic(res, dang, p.acc, red);
+    if (!REF) {
+        pr_reduce2_atomic(res, dang, p.acc, red);
+        pr_end_pass<false>(p);
+        return;
     }
+    nact = __reduce_add_sync(kFull, nact);
+    if ((threadIdx.x & 31) == 0 && nact) atomicAdd(active_count, nact);
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(p.ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last || threadIdx.x) return;
+    __threadfence();
+    *(volatile unsigned long long *)p.report = *(volatile uint32_t *)active_count;
+    *active_next = 0;
+    *p.work = 0;
+    *p.ticket = 0;
 }
 
 template <typename T>
@@ -4331,8 +4429,6 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     const uint32_t V = (uint32_t)g->V;
     cudaStream_t s = g->stream;
     uint32_t launches = 0;
-    double *acc = (double *)(ws->ctl + CTL_PR);   // residual/dangling pairs by pass parity
-    uint32_t *active_count = ws->ctl + CTL_PR + 8;  // word 40
     typedef typename PrAcc<T>::type Acc;
     double *rank = (double *)ws->pr_rank;
     T *c[2] = {(T *)ws->pr_contrib[0], (T *)ws->pr_contrib[1]};
@@ -4341,7 +4437,7 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
     ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
     pr_push_init_kernel<T><<<fill_grid(ws, V), kBlock, 0, s>>>(rank, c[0], c[1], (Acc *)ws->pr_sum, g->d_ptr, active,
-                                                               V, acc + 2);
+                                                               V, (double *)(ws->ctl + CTL_ACC) + 4);
     launches++;
     bool staged = false;
     if (!REF && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
@@ -4356,6 +4452,8 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     ia.sl[1] = pr_slice(g, 1);
     ia.ptr = g->d_ptr;
     ia.sum = (Acc *)ws->pr_sum;
+    ia.rank = rank;
+    ia.cnt_in = ws->ctl + CTL_BLOCK;
     ia.work = ws->ctl + CTL_BLOCK + 4;
     ia.V = V;
     ia.ebits = WORDS == 2 ? 64 : g->ebits;
@@ -4371,29 +4469,32 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
         ASC_CUDA(cudaGetLastError());
     }
     ia.hot = ws->pr_hot;
-    int it = 0;
+    ASC_TRY(ensure_pass_events(ws));
+    const int depth = staged || t_iteration_hook.fn ? 1 : 2;
+    int it = 0, launched = 0;  // passes that ended, that were launched
     double residual = 0;
+    bool over = false;
     for (;;) {
-        if (it >= max_it) {
+        if (launched - it >= depth || (launched > it && launched >= max_it)) {
+            ASC_CUDA(cudaEventSynchronize(ws->pass_ev[it % kPassSlots]));
+            const unsigned long long *r = pass_slot(ws, it);
+            memcpy(&residual, r, 8);
+            over = REF ? r[0] == 0 : residual < p.tolerance;
+            if (REF) residual = 0;
+            it++;
+            iteration_boundary();
+        }
+        if (over) break;  // a pass launched after the last one changes nothing
+        if (launched >= max_it) {
+            if (launched > it) continue;
             if (REF) return fail(ASC_ERR_TIMEOUT, "reference PageRank still active after %d passes", it);
             break;
         }
-        const int cp = it & 1;
-        ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_BLOCK, 0, 4 * CTL_BLOCK, s));  // work cursors (block 1)
-        ASC_CUDA(cudaMemsetAsync(REF ? (void *)active_count : (void *)(acc + 2 * cp), 0, REF ? 4 : 16, s));
-        PushArgs<T> pa;
-        memset(&pa, 0, sizeof(pa));
-        pa.ptr = g->d_ptr;
-        pa.rank = rank;
-        pa.c_old = c[cp];
-        pa.c_new = c[1 - cp];
-        pa.sum = (Acc *)ws->pr_sum;
-        pa.active = active;
-        pa.active_count = active_count;
-        pa.damping = REF ? 0.85 : p.damping;
-        pa.acc = acc + 2 * cp;
-        pa.dangling_prev = acc + 2 * (1 - cp) + 1;
-        ia.c_old = pa.c_old;
+        ia.c_old = c[launched & 1];
+        ia.c_new = c[1 - (launched & 1)];
+        set_pass(ws, p, launched, ia);
+        uint32_t *counts = ws->ctl + CTL_PR;  // reference mode: active vertices after three consecutive passes
+        ia.active_prev = REF && launched ? counts + (launched + 2) % 3 : nullptr;
         if (staged) ASC_CUDA(cudaMemsetAsync(sp->d_work, 0, 4 * sp->launches.size(), s));
         for (uint32_t k = 0; k < (staged ? (uint32_t)sp->launches.size() : 1u); k++) {
             if (staged) {
@@ -4405,20 +4506,12 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
             if (staged) ASC_TRY(stage_release(sp, k, s));
             launches++;
         }
-        pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kBlock, 0, s>>>(pa, V);
+        pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kPrThreads, 0, s>>>(ia, active, counts + launched % 3,
+                                                                              counts + (launched + 1) % 3);
         launches++;
         ASC_CUDA(cudaGetLastError());
-        ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, REF ? (void *)active_count : (void *)(acc + 2 * cp), REF ? 4 : 16,
-                                 cudaMemcpyDeviceToHost, s));
-        ASC_CUDA(cudaStreamSynchronize(s));
-        it++;
-        iteration_boundary();
-        if (REF) {
-            if (ws->h_ctl[0] == 0) break;
-        } else {
-            memcpy(&residual, ws->h_ctl, 8);
-            if (residual < p.tolerance) break;
-        }
+        ASC_CUDA(cudaEventRecord(ws->pass_ev[launched % kPassSlots], s));
+        launched++;
     }
     ASC_CUDA(cudaEventRecord(ws->ev[1], s));
     if (out && !(p.flags & ASC_RUN_NO_OUTPUT)) {
@@ -4426,11 +4519,9 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
         launches += sizeof(T) == 4;
     }
     ASC_CUDA(cudaEventRecord(ws->ev[2], s));
-    ASC_CUDA(cudaMemcpyAsync(ws->h_ctl + CTL_STATS, ws->ctl + CTL_STATS, 8 * 4, cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
     if (st) {
         memset(st, 0, sizeof(*st));
-        const unsigned long long *hs = (const unsigned long long *)(ws->h_ctl + CTL_STATS);
         unsigned long long n[4];
         pr_pass_counts(g, (uint64_t)it, n);
         st->iterations = it;
