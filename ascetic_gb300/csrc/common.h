@@ -66,15 +66,14 @@ struct Workspace {
     void *pr_contrib[2] = {nullptr, nullptr};
     void *pr_sum = nullptr;          // segment partial sums [V]
     size_t pr_elem = 0;
-    uint2 *pr_items = nullptr;       // first (row, edge) of each item of an edge-balanced pass
+    uint2 *items = nullptr;          // first (row, edge) of each merge item
     uint32_t n_items_static = 0, n_items = 0;
     unsigned long long *pr_hot = nullptr;  // scatter passes: most frequent destinations
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> phase_events;
     cudaEvent_t pass_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // ends of PageRank passes
+    int loop_per_sm[3] = {0, 0, 0};  // resident CTAs per SM of the persistent loop (BFS, SSSP, CC)
     struct BatchEngine *batch[2] = {nullptr, nullptr};  // asc_run_batch engines (BFS, SSSP)
-    cudaGraphExec_t loop_exec[3] = {nullptr, nullptr, nullptr};  // BFS, SSSP, CC iteration loops
-    uint32_t loop_cap[3] = {0, 0, 0};
     Tuning tune;
     int num_sms = 0;
     uint64_t device_bytes = 0;

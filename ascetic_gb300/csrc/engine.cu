@@ -90,17 +90,18 @@ enum Alg { kBFS = 0, kSSSP = 1, kCC = 2 };
 // Stats at word 16 (u64): edges static, edges on-demand, frontier vertices
 // static, frontier vertices on-demand, reached vertices, reached edges. PageRank FP64 accumulators at word 32:
 // residual[2], dangling[2].
-// Word 28 counts iterations, word 29 flags an iteration cap hit and word 30
-// counts loop-body executions when the loop runs as a CUDA graph. Word 31 is
-// the SSSP near-far threshold, word 36 the minimum far distance of a pass.
+// Word 28 counts iterations and word 29 flags an iteration cap hit when the
+// loop runs on the device. Word 31 is the SSSP near-far threshold, words 36-39
+// the minimum far distance of a pass.
 // Words 42-43 (u64): in-edges that bottom-up BFS steps read from host memory;
 // words 44-45 (u64): unreached vertices those steps examined. Words 46-47 (u64):
 // in-edges of the vertices that a reference PageRank pass left active; words
 // 48-59: three residual and dangling-mass pairs (FP64) of PageRank passes, word
-// 60 the ticket of the blocks that end a pass.
-enum { CTL_BLOCK = 8, CTL_STATS = 16, CTL_ITERS = 28, CTL_TIMEOUT = 29, CTL_BODIES = 30, CTL_THRESH = 31,
+// 60 the ticket of the blocks that end a pass. Word 61 counts the arrivals at a
+// grid barrier; word 29 is 2 when one ran out of time.
+enum { CTL_BLOCK = 8, CTL_STATS = 16, CTL_ITERS = 28, CTL_TIMEOUT = 29, CTL_THRESH = 31,
        CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_ACC = 48,
-       CTL_TICKET = 60, CTL_WORDS = 64 };
+       CTL_TICKET = 60, CTL_BARRIER = 61, CTL_WORDS = 64 };
 
 struct RegionArgs {
     const uint32_t *ptr;
@@ -140,7 +141,11 @@ struct RegionArgs {
     uint32_t in_resident;         // in_edges is device memory (a graph without a cap), else pinned host
     const uint32_t *in_heads;     // first in-edge of every vertex in HBM (a bit stream of in_ebits), or null
     const uint32_t *in_none;      // one bit per vertex without in-edges (never reached but as a source)
-    uint64_t edge_words;          // words that may be read at edges (item passes of PageRank)
+    // merge items of the region (null: a region walked in id order is cut into
+    // tiles of kBlock vertices and segments), and the words that may be read at edges
+    const uint2 *items;
+    uint32_t item_begin, item_n;
+    uint64_t edge_words;
 };
 
 // True when this BFS iteration steps bottom-up: its input frontier (the
@@ -230,6 +235,68 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t &total,
     return s_warp[w] + incl - x;
 }
 
+// Merge items: a region's rows (each counted at its end) and edges in their
+// merged order, cut every kItem positions. An item is the rows that end in it
+// and the edges at its positions, so items hold equal work whatever the
+// degrees; long lists span several. Passes and iterations that read most of a
+// region run over its items, a CTA per item and kVt consecutive edges per thread.
+// Both ways measured on the second iteration of a symmetrised RMAT graph of 6 M
+// vertices (180 M edges, 355 MB of them over the host link): tiles of 256
+// vertices, an owner search per edge and 4-byte reads 2.22 ms (160 GB/s over the
+// link), items 1.77 (200 of the 211 a copy reaches).
+constexpr int kVt = 8;
+constexpr uint32_t kItem = kBlock * kVt;
+
+// First (row, edge) of every item; items[n] is the end. Region 0 is the rows
+// [0, S), region 1 the rows [S, V); each starts at an item boundary.
+__global__ void merge_plan_kernel(const uint32_t *ptr, uint32_t S, uint32_t V, uint32_t L, uint32_t n0, uint32_t n,
+                               uint2 *items) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+        if (i == n) {
+            items[i] = make_uint2(V, ptr[V]);
+            continue;
+        }
+        const uint32_t R0 = i < n0 ? 0 : S, R1 = i < n0 ? S : V;
+        const uint32_t E0 = ptr[R0];
+        const uint64_t d = (uint64_t)(i - (i < n0 ? 0 : n0)) * L;
+        // row r ends at merge position (its end - E0) + (r - R0): rows ending before d
+        uint32_t lo = 0, hi = R1 - R0;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if ((uint64_t)(ptr[R0 + mid + 1] - E0) + mid < d) lo = mid + 1;
+            else hi = mid;
+        }
+        items[i] = make_uint2(R0 + lo, E0 + (uint32_t)(d - lo));
+    }
+}
+
+// Words [w, w + 4) of an edge array of edge_words words, w a multiple of 4.
+__device__ __forceinline__ uint4 load_words16(const uint32_t *edges, uint64_t edge_words, uint64_t w) {
+    if (w + 4 <= edge_words) return __ldg(reinterpret_cast<const uint4 *>(edges + w));
+    uint4 q;  // the buffer's last words
+    q.x = w < edge_words ? __ldg(edges + w) : 0u;
+    q.y = w + 1 < edge_words ? __ldg(edges + w + 1) : 0u;
+    q.z = w + 2 < edge_words ? __ldg(edges + w + 2) : 0u;
+    q.w = 0u;
+    return q;
+}
+
+// Copies the words holding edges [e0, e0 + ne) to smem with 16-byte loads (so
+// the host link serves runs of several KB); returns the bit of edge e0 there.
+__device__ __forceinline__ uint32_t stage_words(const uint32_t *edges, uint64_t edge_words, uint32_t e0, uint32_t ne, uint32_t eb,
+                                                   uint32_t *pool, uint32_t &nq) {
+    const uint64_t bit = (uint64_t)e0 * eb;
+    const uint64_t w_lo = (bit >> 5) & ~3ull;
+    nq = ne ? (uint32_t)(((((uint64_t)e0 + ne) * eb + 31) / 32 - w_lo + 3) >> 2) : 0;
+    for (uint32_t i = threadIdx.x; i < nq; i += kBlock)
+        reinterpret_cast<uint4 *>(pool)[i] = load_words16(edges, edge_words, w_lo + 4ull * i);
+    return (uint32_t)(bit - 32 * w_lo);
+}
+
+__device__ __forceinline__ uint32_t staged_word(const uint32_t *pool, uint32_t bit, uint32_t mask) {
+    return __funnelshift_r(pool[bit >> 5], pool[(bit >> 5) + 1], bit & 31u) & mask;
+}
+
 template <int ALG, int WORDS>
 __device__ __forceinline__ void load_edge(const RegionArgs &a, uint32_t vu, uint64_t idx, uint32_t &v, uint32_t &nv) {
     if (WORDS == 2) {
@@ -276,7 +343,7 @@ __device__ __forceinline__ uint32_t probe(const RegionArgs &a, uint32_t v) {
 // set a bit. Otherwise the returned old bit decides, and counts are exact.
 constexpr bool kClaimRed = ASC_CLAIM_RED != 0;
 template <int ALG>
-__device__ __forceinline__ bool lower(const RegionArgs &a, uint32_t v, uint32_t nv, uint32_t cur) {
+__device__ __forceinline__ bool lower(const RegionArgs &a, uint32_t v, uint32_t nv, uint32_t cur, uint32_t thresh) {
     const uint32_t bit = 1u << (v & 31);
     if (ALG == kBFS) {
         if (nv == 0xffffffffu || (cur & bit)) return false;
@@ -288,9 +355,11 @@ __device__ __forceinline__ bool lower(const RegionArgs &a, uint32_t v, uint32_t 
     }
     if (nv >= cur) return false;
     if (ALG == kSSSP && a.far_bits) {
-        uint32_t old = atomicMin(&a.val[v], nv);
-        if (nv >= old) return false;
-        if (nv >= *a.thresh) {
+        // fire-and-forget, as below: a vertex lowered below the threshold by
+        // another thread meanwhile may stay in the far set and is then expanded
+        // once more when it is promoted
+        atomicMin(&a.val[v], nv);
+        if (nv >= thresh) {
             atomicOr(&a.far_bits[v >> 5], bit);  // waits until the threshold reaches it
             return false;
         }
@@ -322,7 +391,8 @@ constexpr int kUnroll = ASC_EXPAND_UNROLL;
 // thread has none): a block scan of their degrees lays the edges out as one
 // range, which all threads walk kUnroll edges at a time.
 template <int ALG, int WORDS>
-__device__ void expand_vertices(const RegionArgs &a, bool act, uint32_t u, Smem &sm, uint32_t *s_next) {
+__device__ void expand_vertices(const RegionArgs &a, bool act, uint32_t u, Smem &sm, uint32_t *s_next,
+                                uint32_t thresh) {
     uint32_t deg = 0, start = 0, vu = 0;
     if (act && ASC_BAD(u >= a.V, 1, u)) act = false;
     if (act) {
@@ -370,7 +440,7 @@ __device__ void expand_vertices(const RegionArgs &a, bool act, uint32_t u, Smem 
 #pragma unroll
         for (int k = 0; k < kUnroll; k++) cur[k] = nv[k] != 0xffffffffu ? probe<ALG>(a, v[k]) : 0;
 #pragma unroll
-        for (int k = 0; k < kUnroll; k++) count_next(a, lower<ALG>(a, v[k], nv[k], cur[k]), v[k], s_next);
+        for (int k = 0; k < kUnroll; k++) count_next(a, lower<ALG>(a, v[k], nv[k], cur[k], thresh), v[k], s_next);
     }
     if (threadIdx.x == 0) {
         atomicAdd(&a.stats[a.region], (unsigned long long)total);
@@ -395,7 +465,7 @@ __device__ __forceinline__ uint32_t region_word(const RegionArgs &a, uint32_t u0
 // vertex costs one bitmap read per warp).
 template <int ALG, int WORDS>
 __device__ __forceinline__ void expand_tile(const RegionArgs &a, uint32_t tile, uint32_t n_in, bool bitmap, Smem &sm,
-                                            uint32_t *s_next) {
+                                            uint32_t *s_next, uint32_t thresh) {
     bool act;
     uint32_t u;
     if (bitmap) {
@@ -407,11 +477,11 @@ __device__ __forceinline__ void expand_tile(const RegionArgs &a, uint32_t tile, 
         act = i < n_in;
         u = act ? a.q_in[i] : 0;
     }
-    expand_vertices<ALG, WORDS>(a, act, u, sm, s_next);
+    expand_vertices<ALG, WORDS>(a, act, u, sm, s_next, thresh);
 }
 
 template <int ALG, int WORDS>
-__device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_next) {
+__device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_next, uint32_t thresh) {
     const uint32_t u = (uint32_t)(item >> 32), k0 = (uint32_t)item;
     if (ASC_BAD(u >= a.V, 3, u)) return;
     const uint32_t b0 = a.ptr[u], e0 = a.ptr[u + 1];
@@ -438,7 +508,7 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 #pragma unroll
         for (int k = 0; k < kUnroll; k++) cur[k] = nv[k] != 0xffffffffu ? probe<ALG>(a, v[k]) : 0;
 #pragma unroll
-        for (int k = 0; k < kUnroll; k++) count_next(a, lower<ALG>(a, v[k], nv[k], cur[k]), v[k], s_next);
+        for (int k = 0; k < kUnroll; k++) count_next(a, lower<ALG>(a, v[k], nv[k], cur[k], thresh), v[k], s_next);
     }
     if (threadIdx.x == 0) {
         atomicAdd(&a.stats[a.region], (unsigned long long)n);
@@ -451,7 +521,8 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 // region whose frontier holds more than 1/dense_div of its vertices is walked
 // in id order through its bitmap (its list was not built), kBlock ids per
 // item, so the lists of neighbouring active vertices are read as one
-// contiguous run; otherwise through its list, kBlock entries per item.
+// contiguous run; otherwise through its list, kBlock entries per item. With
+// merge items, the id-order walk runs over those alone.
 __device__ __forceinline__ void region_items_bits(const RegionArgs &a, uint32_t &n_in, uint32_t &nseg,
                                                   uint32_t &items, bool &bitmap) {
     const uint32_t range = a.dense_end - a.dense_begin;
@@ -461,13 +532,169 @@ __device__ __forceinline__ void region_items_bits(const RegionArgs &a, uint32_t 
     n_in = bitmap ? 0 : a.cnt_in[a.region];
     const uint32_t nvert = bitmap ? a.dense_end - (a.dense_begin & ~31u) : n_in;
     items = nseg + (nvert + kBlock - 1) / kBlock;
+    if (bitmap && a.items) {
+        nseg = 0;
+        items = a.item_n;
+    }
+}
+
+// A region's merge item: the edges of its active rows, staged in shared memory
+// by 16-byte chunks that hold any (so the host link serves long runs and only
+// what is active), then kVt consecutive edges per thread.
+template <int WORDS>
+struct ItemSmem {
+    // the staged words, then one value per row: at most ne (2 ne) words and nr + 1
+    // with nr + ne <= kItem, plus alignment and one word read past the end
+    alignas(16) uint32_t pool[(WORDS == 2 ? 2 : 1) * kItem + 24];
+    uint16_t row_at[kItem];         // of an active row's first edge here: the row, from the item's first
+    uint32_t starts[kItem / 32];    // one bit per edge: an active row starts here
+    uint32_t active[kItem / 32];    // one bit per edge: it belongs to an active row
+};
+
+// The row of the last start before edge xw (a multiple of 32), when there is
+// one. The whole warp calls it.
+__device__ __forceinline__ uint32_t row_before(const uint32_t *starts, const uint16_t *row_at, uint32_t xw) {
+    const int lane = threadIdx.x & 31;
+    for (int m0 = (int)(xw >> 5) - 32; m0 > -32; m0 -= 32) {
+        const uint32_t word = m0 + lane >= 0 ? starts[m0 + lane] : 0u;
+        const unsigned any = __ballot_sync(kFull, word != 0);
+        if (any) {
+            const int q = 31 - __clz((int)any);
+            const uint32_t bits = __shfl_sync(kFull, word, q);
+            return row_at[32 * (m0 + q) + 31 - __clz((int)bits)];
+        }
+    }
+    return 0;
 }
 
 template <int ALG, int WORDS>
+__device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WORDS> &sm, uint32_t *s_next,
+                                  uint32_t thresh) {
+    const uint2 i0 = a.items[it], i1 = a.items[it + 1];
+    const uint32_t r0 = i0.x, e0 = i0.y, nr = i1.x - i0.x, ne = i1.y - i0.y;
+    const int lane = threadIdx.x & 31;
+    const uint32_t eb = WORDS == 2 ? 64 : WORDS == 1 ? 32 : a.ebits;
+    const uint64_t bit = (uint64_t)e0 * eb, w_lo = (bit >> 5) & ~3ull;
+    const uint32_t bit0 = (uint32_t)(bit - 32 * w_lo), nq = (bit0 + ne * eb + 127) >> 7;
+    uint32_t *value = sm.pool + 4 * nq + 4;
+    if (threadIdx.x < kItem / 32) sm.starts[threadIdx.x] = sm.active[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t edges = 0, verts = 0;
+    for (uint32_t j = threadIdx.x; j <= nr; j += kBlock) {
+        const uint32_t u = r0 + j;
+        if (u >= a.dense_end || !((a.bitmap_in[u >> 5] >> (u & 31)) & 1u)) continue;
+        const uint32_t b = a.ptr[u], e = a.ptr[u + 1];
+        const uint32_t lo = b > e0 ? b - e0 : 0, hi = min(e - e0, ne);
+        verts += j < nr;  // a vertex counts where its row ends
+        if (lo >= hi) continue;
+        edges += hi - lo;
+        value[j] = a.val[u];
+        sm.row_at[lo] = (uint16_t)j;
+        atomicOr(&sm.starts[lo >> 5], 1u << (lo & 31));
+        for (uint32_t w = lo >> 5; w <= (hi - 1) >> 5; w++) {
+            uint32_t m = 0xffffffffu;
+            if (w == lo >> 5) m &= 0xffffffffu << (lo & 31);
+            if (w == (hi - 1) >> 5) m &= 0xffffffffu >> (31 - ((hi - 1) & 31));
+            atomicOr(&sm.active[w], m);
+        }
+        if (a.frag) count_fragments(a.frag, (uint64_t)e0 + lo, hi - lo);
+    }
+    const bool any = __syncthreads_or(edges != 0);
+    edges = __reduce_add_sync(kFull, edges);
+    verts = __reduce_add_sync(kFull, verts);
+    if (lane == 0 && edges) atomicAdd(&s_next[2 + a.region], edges);
+    if (lane == 0 && verts) atomicAdd(&s_next[4 + a.region], verts);
+    if (!any) return;
+    for (uint32_t i = threadIdx.x; i < nq; i += kBlock) {
+        // edges with a bit in this chunk
+        const uint32_t c0 = 128 * i;
+        const uint32_t x0 = c0 > bit0 ? (c0 - bit0) / eb : 0, x1 = min(ne - 1, (c0 + 127 - bit0) / eb);
+        uint32_t need = 0;
+        for (uint32_t w = x0 >> 5; w <= x1 >> 5; w++) {
+            uint32_t m = sm.active[w];
+            if (w == x0 >> 5) m &= 0xffffffffu << (x0 & 31);
+            if (w == x1 >> 5) m &= 0xffffffffu >> (31 - (x1 & 31));
+            need |= m;
+        }
+        if (need) reinterpret_cast<uint4 *>(sm.pool)[i] = load_words16(a.edges, a.edge_words, w_lo + 4ull * i);
+    }
+    __syncthreads();
+    const uint32_t x0 = threadIdx.x * kVt, xw = x0 - lane * kVt;  // first edge of the thread, the warp
+    uint32_t n0 = 0, n1 = 0;
+    if (xw < ne) {
+        const uint32_t act = (sm.active[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
+        const uint32_t st = (sm.starts[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
+        if (__any_sync(kFull, act != 0)) {
+            // the row open at the thread's first edge: of the last start in an
+            // earlier lane, or in an earlier warp
+            const unsigned began = __ballot_sync(kFull, st != 0);
+            const uint32_t last = st ? sm.row_at[x0 + 31 - __clz((int)st)] : 0u;
+            const unsigned below = began & ((1u << lane) - 1u);
+            const uint32_t from_lane = __shfl_sync(kFull, last, below ? 31 - __clz((int)below) : lane);
+            const uint32_t before = row_before(sm.starts, sm.row_at, xw);
+            uint32_t row = below ? from_lane : before;
+            uint32_t vu = (act & 1u) ? value[(st & 1u) ? (uint32_t)sm.row_at[x0] : row] : 0u;
+            constexpr uint32_t kMask = 0xffffffffu;
+            const uint32_t mask = eb >= 32 ? kMask : (1u << eb) - 1u;
+#pragma unroll
+            for (int k0 = 0; k0 < kVt; k0 += kUnroll) {
+                uint32_t v[kUnroll], nv[kUnroll], cur[kUnroll];
+#pragma unroll
+                for (int k = 0; k < kUnroll; k++) {
+                    v[k] = 0;
+                    nv[k] = 0xffffffffu;  // never lower than a value: no update
+                    if ((act >> (k0 + k)) & 1u) {
+                        if (k0 + k > 0 && ((st >> (k0 + k)) & 1u)) vu = value[sm.row_at[x0 + k0 + k]];
+                        const uint32_t at = bit0 + (x0 + k0 + k) * eb;
+                        if (WORDS == 2) {
+                            v[k] = sm.pool[at >> 5];
+                            nv[k] = ALG == kSSSP ? vu + sm.pool[(at >> 5) + 1] : (ALG == kBFS ? vu + 1 : vu);
+                        } else {
+                            const uint32_t e = WORDS == 1 ? sm.pool[at >> 5] : staged_word(sm.pool, at, mask);
+                            v[k] = e >> a.wbits;
+                            nv[k] = ALG == kBFS ? vu + 1
+                                                : (ALG == kSSSP ? vu + (e & ((1u << a.wbits) - 1u)) : vu);
+                        }
+                        if (ASC_BAD(v[k] >= a.V, 2, v[k])) {
+                            v[k] = 0;
+                            nv[k] = 0xffffffffu;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < kUnroll; k++) cur[k] = nv[k] != 0xffffffffu ? probe<ALG>(a, v[k]) : 0;
+#pragma unroll
+                for (int k = 0; k < kUnroll; k++) {
+                    const bool won = lower<ALG>(a, v[k], nv[k], cur[k], thresh);
+                    n0 += won && v[k] < a.S;
+                    n1 += won && v[k] >= a.S;
+                }
+            }
+        }
+    }
+    n0 = __reduce_add_sync(kFull, n0);
+    n1 = __reduce_add_sync(kFull, n1);
+    if (lane == 0 && n0) atomicAdd(&s_next[0], n0);
+    if (lane == 0 && n1) atomicAdd(&s_next[1], n1);
+    __syncthreads();
+}
+
+// Shared memory of an expansion: a tile's or a merge item's.
+template <int WORDS>
+union ExpandSmem {
+    Smem tile;
+    ItemSmem<WORDS> item;
+};
+// Shared counters of an expansion: next-frontier vertices per region, then the
+// edges and the vertices that merge items expanded.
+constexpr int kNextWords = 6;
+
+template <int ALG, int WORDS>
 __device__ __forceinline__ void expand_item(const RegionArgs &a, uint32_t w, uint32_t n_in, uint32_t nseg,
-                                            bool bitmap, Smem &sm, uint32_t *s_next) {
-    if (w < nseg) expand_segment<ALG, WORDS>(a, a.seg_in[w], s_next);
-    else expand_tile<ALG, WORDS>(a, w - nseg, n_in, bitmap, sm, s_next);
+                                            bool bitmap, ExpandSmem<WORDS> &sm, uint32_t *s_next, uint32_t thresh) {
+    if (w < nseg) expand_segment<ALG, WORDS>(a, a.seg_in[w], s_next, thresh);
+    else if (bitmap && a.items) expand_merge_item<ALG, WORDS>(a, a.item_begin + w, sm.item, s_next, thresh);
+    else expand_tile<ALG, WORDS>(a, w - nseg, n_in, bitmap, sm.tile, s_next, thresh);
 }
 
 __device__ __forceinline__ void flush_next(const RegionArgs &a, uint32_t *s_next) {
@@ -478,24 +705,32 @@ __device__ __forceinline__ void flush_next(const RegionArgs &a, uint32_t *s_next
     }
 }
 
+// The same with what merge items counted.
+__device__ __forceinline__ void flush_expansion(const RegionArgs &a, uint32_t *s_next) {
+    flush_next(a, s_next);
+    if (threadIdx.x < 4 && s_next[2 + threadIdx.x])
+        atomicAdd(&a.stats[threadIdx.x], (unsigned long long)s_next[2 + threadIdx.x]);
+}
+
 template <int ALG, int WORDS>
 __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_kernel(RegionArgs a) {
     if (ALG == kBFS && bottom_up_step(a)) return;
-    __shared__ Smem sm;
-    __shared__ uint32_t s_next[2];
-    if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
+    __shared__ ExpandSmem<WORDS> sm;
+    __shared__ uint32_t s_next[kNextWords], s_work;
+    if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     uint32_t n_in, nseg, total;
     bool bitmap;
     region_items_bits(a, n_in, nseg, total, bitmap);
+    const uint32_t thresh = ALG == kSSSP && a.far_bits ? *a.thresh : 0u;
     for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(a.work, 1u);
+        if (threadIdx.x == 0) s_work = atomicAdd(a.work, 1u);
         __syncthreads();
-        const uint32_t w = sm.work;
+        const uint32_t w = s_work;
         __syncthreads();
         if (w >= total) break;
-        expand_item<ALG, WORDS>(a, w, n_in, nseg, bitmap, sm, s_next);
+        expand_item<ALG, WORDS>(a, w, n_in, nseg, bitmap, sm, s_next, thresh);
     }
-    flush_next(a, s_next);
+    flush_expansion(a, s_next);
 }
 
 // Both regions in one launch. Work items alternate between the on-demand and
@@ -507,23 +742,20 @@ struct FusedArgs {
     uint32_t *work;
 };
 
+// A CTA's first item is its own number; later ones come from the cursor, which
+// starts behind them.
 template <int ALG, int WORDS>
-__global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_kernel(FusedArgs x) {
-    if (ALG == kBFS && bottom_up_step(x.r0)) return;
-    __shared__ Smem sm;
-    __shared__ uint32_t s_next[2];
-    if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
+__device__ __forceinline__ void expand_regions(const FusedArgs &x, uint32_t thresh, ExpandSmem<WORDS> &sm,
+                                               uint32_t *s_next) {
+    __shared__ uint32_t s_work;
     uint32_t n0, s0, i0, n1, s1, i1;
     bool m0, m1;
     region_items_bits(x.r0, n0, s0, i0, m0);
     region_items_bits(x.r1, n1, s1, i1, m1);
     const uint32_t m = min(i0, i1), total = i0 + i1;
-    for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(x.work, 1u);
-        __syncthreads();
-        const uint32_t w = sm.work;
-        __syncthreads();
-        if (w >= total) break;
+    if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t w = blockIdx.x; w < total;) {
         bool od;
         uint32_t local;
         if (w < 2 * m) {
@@ -533,10 +765,22 @@ __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_ke
             od = i1 > i0;
             local = m + (w - 2 * m);
         }
-        if (od) expand_item<ALG, WORDS>(x.r1, local, n1, s1, m1, sm, s_next);
-        else expand_item<ALG, WORDS>(x.r0, local, n0, s0, m0, sm, s_next);
+        if (threadIdx.x == 0) s_work = gridDim.x + atomicAdd(x.work, 1u);
+        if (od) expand_item<ALG, WORDS>(x.r1, local, n1, s1, m1, sm, s_next, thresh);
+        else expand_item<ALG, WORDS>(x.r0, local, n0, s0, m0, sm, s_next, thresh);
+        __syncthreads();
+        w = s_work;
+        __syncthreads();
     }
-    flush_next(x.r0, s_next);
+    flush_expansion(x.r0, s_next);
+}
+
+template <int ALG, int WORDS>
+__global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_kernel(FusedArgs x) {
+    if (ALG == kBFS && bottom_up_step(x.r0)) return;
+    __shared__ ExpandSmem<WORDS> sm;
+    __shared__ uint32_t s_next[kNextWords];
+    expand_regions<ALG, WORDS>(x, ALG == kSSSP && x.r0.far_bits ? *x.r0.thresh : 0u, sm, s_next);
 }
 
 // Bottom-up BFS step (direction-optimizing BFS): every vertex not yet reached
@@ -572,12 +816,13 @@ constexpr int kBuWords = ASC_BU_WORDS;
 #endif
 constexpr int kBuMinBlocks = ASC_BU_MIN_BLOCKS;
 
-__global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionArgs a, uint32_t nwords) {
-    if (!bottom_up_step(a)) return;
-    __shared__ uint32_t s_next[2];
-    __shared__ unsigned long long s_scanned, s_examined;
+struct BuSmem {
+    unsigned long long scanned, examined;
+};
+
+__device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nwords, BuSmem &bs, uint32_t *s_next) {
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
-    if (threadIdx.x == 0) s_scanned = s_examined = 0;
+    if (threadIdx.x == 0) bs.scanned = bs.examined = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kBlock / 32);
@@ -667,17 +912,24 @@ __global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionA
         scanned += __shfl_down_sync(kFull, scanned, d);
         examined += __shfl_down_sync(kFull, examined, d);
     }
-    if (lane == 0 && scanned) atomicAdd(&s_scanned, scanned);
-    if (lane == 0 && examined) atomicAdd(&s_examined, examined);
+    if (lane == 0 && scanned) atomicAdd(&bs.scanned, scanned);
+    if (lane == 0 && examined) atomicAdd(&bs.examined, examined);
     flush_next(a, s_next);
-    if (threadIdx.x == 0 && s_examined)
-        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_VERTS - CTL_STATS) / 2), s_examined);
+    if (threadIdx.x == 0 && bs.examined)
+        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_VERTS - CTL_STATS) / 2), bs.examined);
     // in-edges are read in place from host memory (resident only on a graph
     // without a cap): the run's on-demand edges and its bottom-up edges
-    if (threadIdx.x == 0 && s_scanned) {
-        atomicAdd(&a.stats[a.in_resident ? 0 : 1], s_scanned);
-        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_EDGES - CTL_STATS) / 2), s_scanned);
+    if (threadIdx.x == 0 && bs.scanned) {
+        atomicAdd(&a.stats[a.in_resident ? 0 : 1], bs.scanned);
+        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_EDGES - CTL_STATS) / 2), bs.scanned);
     }
+}
+
+__global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionArgs a, uint32_t nwords) {
+    if (!bottom_up_step(a)) return;
+    __shared__ uint32_t s_next[2];
+    __shared__ BuSmem bs;
+    bottom_up_words(a, nwords, bs, s_next);
 }
 
 // Gather-and-copy comparison engine: expands on-demand edges that host
@@ -718,7 +970,7 @@ __global__ void __launch_bounds__(kBlock) expand_staged_kernel(StagedArgs x) {
                 }
             }
             const uint32_t cur = nv != 0xffffffffu ? probe<ALG>(a, v) : 0;
-            count_next(a, lower<ALG>(a, v, nv, cur), v, s_next);
+            count_next(a, lower<ALG>(a, v, nv, cur, a.far_bits ? *a.thresh : 0u), v, s_next);
         }
         if (lane == 0) {
             atomicAdd(&a.stats[1], (unsigned long long)len);
@@ -733,7 +985,7 @@ __global__ void __launch_bounds__(kBlock) expand_staged_kernel(StagedArgs x) {
 // their region's list only when that region will be walked as a list (warp
 // scan of the per-word counts, one atomic per warp). cnt_out[6..7] hold the
 // region bit counts the expansion flushed; cnt_out[0..3] receive the lists.
-__global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, uint32_t nwords) {
+__device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32_t *next_bits, uint32_t nwords) {
     const int lane = threadIdx.x & 31;
     const uint32_t range0 = a.S, range1 = a.V - a.S;
     const bool list0 = !(a.dense_div && a.cnt_out[6] > range0 / a.dense_div);
@@ -746,7 +998,16 @@ __global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, u
             word = next_bits[w];
             hw = word & a.huge_bits[w];
         }
-        // long lists: one thread per vertex appends its segments (rare)
+        // region split of this word: bits of vertices below S are static
+        uint32_t smask;
+        const uint32_t v0 = 32 * w;
+        if (v0 + 32 <= a.S) smask = 0xffffffffu;
+        else if (v0 >= a.S) smask = 0;
+        else smask = (1u << (a.S - v0)) - 1u;
+        // long lists: one thread per vertex appends its segments (rare); merge
+        // items need none
+        if (a.items && !list0) hw &= ~smask;
+        if (a.items && !list1) hw &= smask;
         while (hw) {
             const int b = __ffs(hw) - 1;
             hw &= hw - 1;
@@ -760,12 +1021,6 @@ __global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, u
             for (uint32_t k = 0; k < nseg; k++) dst[k] = ((uint64_t)v << 32) | k;
         }
         if (w < nwords) word &= ~a.huge_bits[w];
-        // region split of this word: bits of vertices below S are static
-        uint32_t smask;
-        const uint32_t v0 = 32 * w;
-        if (v0 + 32 <= a.S) smask = 0xffffffffu;
-        else if (v0 >= a.S) smask = 0;
-        else smask = (1u << (a.S - v0)) - 1u;
         const uint32_t w0 = list0 ? (word & smask) : 0, w1 = list1 ? (word & ~smask) : 0;
         const uint32_t c0 = __popc(w0), c1 = __popc(w1);
         uint32_t i0 = c0, i1 = c1;
@@ -800,6 +1055,10 @@ __global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, u
             b1++;
         }
     }
+}
+
+__global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, uint32_t nwords) {
+    build_frontier(a, next_bits, nwords);
 }
 
 // SSSP near-far, step 1: when the pass left the near frontier empty, the
@@ -889,24 +1148,6 @@ __global__ void seed_bits_kernel(RegionArgs a, uint32_t src, uint32_t all, uint3
     }
 }
 
-// End of one CUDA-graph loop body (two iterations: parity 0 then parity 1).
-// Block 1 holds what the first half produced (the second half's input),
-// block 0 what the second half produced. Keeps looping while block 0 is
-// non-empty, counts the iterations that had input, and stops at the cap.
-__global__ void loop_cond_kernel(cudaGraphConditionalHandle h, uint32_t *ctl, uint32_t cap) {
-    const uint32_t *b0 = ctl, *b1 = ctl + CTL_BLOCK;
-    const bool second = (b1[6] | b1[7]) != 0;
-    bool more = (b0[6] | b0[7]) != 0;
-    const uint32_t it = ctl[CTL_ITERS] + 1 + (second ? 1 : 0);
-    ctl[CTL_ITERS] = it;
-    ctl[CTL_BODIES] += 1;
-    if (more && it >= cap) {
-        ctl[CTL_TIMEOUT] = 1;
-        more = false;
-    }
-    cudaGraphSetConditional(h, more ? 1u : 0u);
-}
-
 template <int ALG>
 __global__ void init_values_kernel(uint32_t *val, uint32_t V, uint32_t src) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
@@ -914,7 +1155,8 @@ __global__ void init_values_kernel(uint32_t *val, uint32_t V, uint32_t src) {
 }
 
 // Reached vertices and the sum of their out-degrees (TEPS numerator).
-__global__ void reached_kernel(const uint32_t *val, const uint32_t *ptr, uint32_t V, unsigned long long *out) {
+__device__ __forceinline__ void reached_values(const uint32_t *val, const uint32_t *ptr, uint32_t V,
+                                               unsigned long long *out) {
     unsigned long long cnt = 0, edges = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x)
         if (val[i] < V + 1) {
@@ -932,6 +1174,10 @@ __global__ void reached_kernel(const uint32_t *val, const uint32_t *ptr, uint32_
     }
 }
 
+__global__ void reached_kernel(const uint32_t *val, const uint32_t *ptr, uint32_t V, unsigned long long *out) {
+    reached_values(val, ptr, V, out);
+}
+
 // BFS: reached vertices are the reached-vertex bitmap's bits (no level read).
 // A warp takes kReachedWords consecutive 32-vertex words at a time, lane =
 // vertex: all of their bitmap words and then all the offsets of their reached
@@ -939,8 +1185,8 @@ __global__ void reached_kernel(const uint32_t *val, const uint32_t *ptr, uint32_
 // independent loads in flight instead of a chain per word.
 constexpr int kReachedWords = 4;
 
-__global__ void reached_bits_kernel(const uint32_t *visited, const uint32_t *ptr, uint32_t V, uint32_t nwords,
-                                    unsigned long long *out) {
+__device__ __forceinline__ void reached_bits(const uint32_t *visited, const uint32_t *ptr, uint32_t V,
+                                             uint32_t nwords, unsigned long long *out) {
     unsigned long long cnt = 0, edges = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
@@ -969,6 +1215,232 @@ __global__ void reached_bits_kernel(const uint32_t *visited, const uint32_t *ptr
         atomicAdd(&out[0], cnt);
         atomicAdd(&out[1], edges);
     }
+}
+
+__global__ void reached_bits_kernel(const uint32_t *visited, const uint32_t *ptr, uint32_t V, uint32_t nwords,
+                                    unsigned long long *out) {
+    reached_bits(visited, ptr, V, nwords, out);
+}
+
+// ------------------------------------------------------- persistent loop -----
+//
+// A whole traversal in one cooperative launch: set-up, every iteration
+// (expansion or bottom-up step, then the next frontier's lists) and the reached
+// counts, with a barrier over the grid between phases. An iteration as separate
+// launches was five graph nodes, two of them clears, around a few microseconds
+// of work when the frontier is small: BFS on 1,001 vertices, 5 iterations, 111 us
+// as a CUDA graph of launches and 48 so; RMAT scale 24, 9 iterations, 706 and 651.
+// CTAs per SM (registers 48 / 40 / 32 / 32): connected components of 6 M vertices
+// 3.60 / 3.61 / 3.65 / 3.64 ms at 5 / 6 / 7 / 8, SSSP on RMAT scale 23 2.95 /
+// 2.94 / 2.98 / 2.98, BFS on scale 24 685 / 651 / 658 / 658 us.
+#ifndef ASC_TRAV_BLOCKS
+#define ASC_TRAV_BLOCKS 6
+#endif
+struct LoopArgs {
+    FusedArgs x0, x1;       // arguments of an iteration by the parity of its input frontier
+    uint32_t *ctl;
+    uint32_t *report;       // host: the control block at the end
+    uint32_t nwords;
+    uint32_t src;           // the first frontier's vertex,
+    uint32_t all;           // or every vertex
+    uint32_t cap;           // iterations
+    uint32_t thresh;        // near-far: the first threshold
+    uint32_t delta;         // near-far: step of the next one beyond the smallest far value
+    uint32_t count_reached;
+};
+
+// Polls of a grid barrier (a read of L2 and a short sleep each) before it gives
+// up: tens of seconds, far above any phase.
+constexpr uint32_t kBarrierPolls = 1u << 25;
+
+// Barrier over the grid: arrivals count up from zero for the whole launch.
+// False when the other CTAs did not arrive in time.
+__device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target) {
+    __shared__ uint32_t s_ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(ctl + CTL_BARRIER, 1u);
+        uint32_t now, polls = 0;
+        for (;;) {
+            // relaxed: an acquire would empty the L1 that the SM's other CTAs still work in
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(ctl + CTL_BARRIER) : "memory");
+            if ((int32_t)(now - target) >= 0 || ++polls > kBarrierPolls) break;
+            if (polls > 16) __nanosleep(64);
+        }
+        s_ok = (int32_t)(now - target) >= 0;
+        if (!s_ok) atomicExch(ctl + CTL_TIMEOUT, 2u);
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Values, bitmaps and the first frontier (parity 0) with its list.
+template <int ALG>
+__device__ __forceinline__ void loop_setup(const LoopArgs &x) {
+    const RegionArgs &a = x.x1.r0;  // writes parity 0
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    const uint32_t V = a.V;
+    for (uint32_t i = 4 * t; i < V; i += 4 * stride) {
+        uint4 q;
+        q.x = ALG == kCC ? i : V + 1;
+        q.y = ALG == kCC ? i + 1 : V + 1;
+        q.z = ALG == kCC ? i + 2 : V + 1;
+        q.w = ALG == kCC ? i + 3 : V + 1;
+        if (ALG != kCC) {
+            if (x.src == i) q.x = 1;
+            if (x.src == i + 1) q.y = 1;
+            if (x.src == i + 2) q.z = 1;
+            if (x.src == i + 3) q.w = 1;
+        }
+        if (i + 4 <= V) {
+            *reinterpret_cast<uint4 *>(a.val + i) = q;
+        } else {
+            a.val[i] = q.x;
+            if (i + 1 < V) a.val[i + 1] = q.y;
+            if (i + 2 < V) a.val[i + 2] = q.z;
+        }
+    }
+    for (uint32_t w = t; w < V / 32 + 2; w += stride) {
+        uint32_t m = 0;
+        if (x.all) m = 32 * w + 32 <= V ? 0xffffffffu : (32 * w < V ? (1u << (V - 32 * w)) - 1u : 0u);
+        else if (w == x.src >> 5) m = 1u << (x.src & 31);
+        a.bitmap[w] = m;
+        x.x0.r0.bitmap[w] = 0;
+        if (ALG == kBFS) a.visited[w] = m;
+        if (ALG == kSSSP && a.far_bits) a.far_bits[w] = 0;
+    }
+    if (blockIdx.x == 0 && x.all) {
+        if (threadIdx.x == 0) {
+            a.cnt_out[6] = a.S;
+            a.cnt_out[7] = V - a.S;
+        }
+    } else if (blockIdx.x == 0) {
+        const uint32_t deg = a.ptr[x.src + 1] - a.ptr[x.src], od = x.src >= a.S;
+        const uint32_t nseg = deg > a.huge ? (deg + a.seg_len - 1) / a.seg_len : 0;
+        for (uint32_t k = threadIdx.x; k < nseg; k += blockDim.x)
+            a.seg_out[(od ? a.segcap_static : 0) + k] = ((uint64_t)x.src << 32) | k;
+        if (threadIdx.x == 0) {
+            a.cnt_out[6 + od] = 1;
+            a.cnt_out[2 + od] = nseg;
+            a.cnt_out[od] = nseg ? 0 : 1;
+            if (!nseg) a.q_out[od ? a.S : 0] = x.src;
+        }
+    }
+}
+
+// Near-far: the far vertices below thresh join the frontier in bits (counts at
+// cnt), the smallest value of those that stay goes to *minfar.
+__device__ __forceinline__ void promote_far(const RegionArgs &a, uint32_t *bits, uint32_t *cnt, uint32_t nwords,
+                                            uint32_t thresh, uint32_t *minfar) {
+    uint32_t n0 = 0, n1 = 0, least = 0xffffffffu;
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
+        const uint32_t word = a.far_bits[w];
+        uint32_t x = word, promo = 0;
+        while (x) {
+            const int b = __ffs(x) - 1;
+            x &= x - 1;
+            const uint32_t val = a.val[32 * w + b];
+            if (val < thresh) promo |= 1u << b;
+            else least = min(least, val);
+        }
+        if (!promo) continue;
+        a.far_bits[w] = word & ~promo;
+        bits[w] |= promo;
+        const uint32_t v0 = 32 * w;
+        const uint32_t smask = v0 + 32 <= a.S ? 0xffffffffu : (v0 >= a.S ? 0 : (1u << (a.S - v0)) - 1u);
+        n0 += __popc(promo & smask);
+        n1 += __popc(promo & ~smask);
+    }
+    n0 = __reduce_add_sync(kFull, n0);
+    n1 = __reduce_add_sync(kFull, n1);
+    least = __reduce_min_sync(kFull, least);
+    if ((threadIdx.x & 31) == 0) {
+        if (n0) atomicAdd(&cnt[6], n0);
+        if (n1) atomicAdd(&cnt[7], n1);
+        if (least != 0xffffffffu) atomicMin(minfar, least);
+    }
+}
+
+struct LoopState {
+    uint32_t target = 0;      // of the grid barrier
+    uint32_t it = 0;
+    uint32_t thresh = 0;
+    uint32_t promotions = 0;
+};
+
+enum LoopNext { kLoopGo, kLoopEnd, kLoopStuck };
+
+// One iteration from the frontier that x reads; y's arguments write that
+// frontier's lists (the other parity).
+template <int ALG, int WORDS>
+__device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const FusedArgs &x, const FusedArgs &y,
+                                                   LoopState &st, ExpandSmem<WORDS> &sm, BuSmem &bs, uint32_t *s_next) {
+    const RegionArgs &a = x.r0;
+    volatile const uint32_t *cin = a.cnt_in;
+    if (!(cin[6] | cin[7])) {
+        if (ALG != kSSSP || !a.far_bits) return kLoopEnd;
+        // the near frontier is empty: the threshold moves on. Four slots for the
+        // smallest far value: this one's was cleared two promotions ago
+        for (;;) {
+            uint32_t *slot = l.ctl + CTL_MINFAR + (st.promotions & 3);
+            if (blockIdx.x == 0 && threadIdx.x == 0) l.ctl[CTL_MINFAR + ((st.promotions + 2) & 3)] = 0xffffffffu;
+            promote_far(a, y.r0.bitmap, y.r0.cnt_out, l.nwords, st.thresh, slot);
+            st.promotions++;
+            if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+            if (cin[6] | cin[7]) break;
+            const uint32_t least = *(volatile uint32_t *)slot;
+            if (least == 0xffffffffu) return kLoopEnd;
+            st.thresh = least > 0xffffffffu - l.delta ? 0xffffffffu : least + l.delta;
+        }
+        build_frontier(y.r0, y.r0.bitmap, l.nwords);
+        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+    }
+    if (st.it >= l.cap) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) l.ctl[CTL_TIMEOUT] = 1;
+        return kLoopEnd;
+    }
+    st.it++;
+    if (ALG == kBFS && bottom_up_step(a)) bottom_up_words(a, l.nwords, bs, s_next);
+    else expand_regions<ALG, WORDS>(x, st.thresh, sm, s_next);
+    if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+    build_frontier(a, a.bitmap, l.nwords);
+    // the input frontier's bitmap and counts are the next output's
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < l.nwords; w += gridDim.x * blockDim.x)
+        y.r0.bitmap[w] = 0;
+    if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
+    return grid_barrier(l.ctl, st.target) ? kLoopGo : kLoopStuck;
+}
+
+template <int ALG, int WORDS>
+__global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const __grid_constant__ LoopArgs l) {
+    __shared__ ExpandSmem<WORDS> sm;
+    __shared__ BuSmem bs;
+    __shared__ uint32_t s_next[kNextWords];
+    LoopState st;
+    st.thresh = l.thresh;
+    loop_setup<ALG>(l);
+    if (!grid_barrier(l.ctl, st.target)) return;
+    if (l.all) {
+        build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords);
+        if (!grid_barrier(l.ctl, st.target)) return;
+    }
+    for (;;) {
+        LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, bs, s_next);
+        if (n == kLoopGo) n = loop_iteration<ALG, WORDS>(l, l.x1, l.x0, st, sm, bs, s_next);
+        if (n == kLoopStuck) return;
+        if (n == kLoopEnd) break;
+    }
+    unsigned long long *out = (unsigned long long *)(l.ctl + CTL_STATS) + 4;
+    if (l.count_reached) {
+        if (ALG == kBFS) reached_bits(l.x0.r0.visited, l.x0.r0.ptr, l.x0.r0.V, l.nwords, out);
+        else reached_values(l.x0.r0.val, l.x0.r0.ptr, l.x0.r0.V, out);
+    }
+    if (!grid_barrier(l.ctl, st.target)) return;
+    if (blockIdx.x == 0 && threadIdx.x < CTL_WORDS)
+        l.report[threadIdx.x] = threadIdx.x == CTL_ITERS ? st.it : ((volatile uint32_t *)l.ctl)[threadIdx.x];
 }
 
 // ------------------------------------------------------------- PageRank -----
@@ -1275,19 +1747,14 @@ __global__ void pr_apply_segmented_kernel(PrArgs p, const uint64_t *items_static
 
 // ------------------------------------------- edge-balanced PageRank passes --
 //
-// A standard pass reads every edge once, so its work is cut by position in the
-// merge of the rows (each counted at its end) and the edges, not by vertices:
-// item i covers merge positions [i*L, (i+1)*L), whatever the degrees, and is
-// the range of rows that end in it plus the range of its edges. A plan kernel
-// finds the items' first (row, edge) by binary search over the offsets, once
-// per workspace. Tiles of 256 vertices held from none to 131,000 edges (lists
-// of up to 512 each), every edge searched its owner in shared memory, and a
-// segmented 5-step shuffle sum ran per edge: 197 instructions per edge (ncu,
-// FP64 pull, 25.5 M edges), with 5 FP64 adds per edge on a pipe that takes 16
-// cycles per warp instruction.
+// A standard pass runs over the merge items (kItem positions each). Tiles of 256
+// vertices held from none to 131,000 edges (lists of up to 512 each), every edge
+// searched its owner in shared memory, and a segmented 5-step shuffle sum ran
+// per edge: 197 instructions per edge (ncu, FP64 pull, 25.5 M edges), with 5 FP64
+// adds per edge on a pipe that takes 16 cycles per warp instruction.
 //
 // Here every row that ends in the item marks its last edge, a thread takes
-// kPrVt consecutive edges and closes a sum at each mark, and one segmented warp
+// kVt consecutive edges and closes a sum at each mark, and one segmented warp
 // scan joins the sums of rows that cross threads: one add per edge and no
 // search. Bound by the host link (30% resident: 2.29 of the 2.5 ms a pass takes
 // on RMAT scale 24, FP32; 172 of 215 us on 25.5 M edges, FP64).
@@ -1297,16 +1764,9 @@ __global__ void pr_apply_segmented_kernel(PrArgs p, const uint64_t *items_static
 // and 5.06 (8 per SM: 77.7, 5.10); 64 threads, 24 per SM: 104.3, 5.25. Shared
 // memory of more CTAs takes the L1 that holds the gathers in flight: 14 CTAs of
 // 128 threads measured 121.7 and 8.1 ms.
-#ifndef ASC_PR_ITEM_THREADS
-#define ASC_PR_ITEM_THREADS 256
-#endif
 #ifndef ASC_PR_ITEM_BLOCKS
 #define ASC_PR_ITEM_BLOCKS 6
 #endif
-constexpr int kPrThreads = ASC_PR_ITEM_THREADS;
-constexpr int kPrWarps = kPrThreads / 32;
-constexpr int kPrVt = 8;                          // edges per thread
-constexpr uint32_t kPrItem = kPrThreads * kPrVt;  // merge positions per item
 // A reference-mode pass runs over all items while the active vertices hold more
 // than 1 / kPrDenseDiv of the in-edges, else over their lists. 35 passes on RMAT
 // scale 20 (85% of the edges active on average), 30% resident: lists alone 11.15
@@ -1323,29 +1783,6 @@ constexpr uint64_t kPrDenseDiv = ASC_PR_DENSE_DIV;
 #define ASC_PR_SCATTER_BLOCKS 4
 #endif
 constexpr uint32_t kPrHot = ASC_PR_HOT;
-
-// First (row, edge) of every item; items[n] is the end. Region 0 is the rows
-// [0, S), region 1 the rows [S, V); each starts at an item boundary.
-__global__ void pr_plan_kernel(const uint32_t *ptr, uint32_t S, uint32_t V, uint32_t L, uint32_t n0, uint32_t n,
-                               uint2 *items) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-        if (i == n) {
-            items[i] = make_uint2(V, ptr[V]);
-            continue;
-        }
-        const uint32_t R0 = i < n0 ? 0 : S, R1 = i < n0 ? S : V;
-        const uint32_t E0 = ptr[R0];
-        const uint64_t d = (uint64_t)(i - (i < n0 ? 0 : n0)) * L;
-        // row r ends at merge position (its end - E0) + (r - R0): rows ending before d
-        uint32_t lo = 0, hi = R1 - R0;
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            if ((uint64_t)(ptr[R0 + mid + 1] - E0) + mid < d) lo = mid + 1;
-            else hi = mid;
-        }
-        items[i] = make_uint2(R0 + lo, E0 + (uint32_t)(d - lo));
-    }
-}
 
 // A range of items and where their edges are read.
 struct PrSlice {
@@ -1390,48 +1827,21 @@ struct PrItemArgs {
 template <typename T>
 struct PrItemSmem {
     // the item's edge words, then its row sums: at most ne words and 2 (nr + 1)
-    // words with nr + ne <= kPrItem, plus alignment and one word read past the end
-    alignas(16) uint32_t pool[2 * kPrItem + 16];
-    uint16_t row_at[kPrItem];       // of an edge that ends a row: the row, from the item's first
-    uint32_t marks[2][kPrItem / 32];  // one bit per edge: it ends a row (this item's, the next one's)
-    double red[2 * kPrWarps];
+    // words with nr + ne <= kItem, plus alignment and one word read past the end
+    alignas(16) uint32_t pool[2 * kItem + 16];
+    uint16_t row_at[kItem];       // of an edge that ends a row: the row, from the item's first
+    uint32_t marks[2][kItem / 32];  // one bit per edge: it ends a row (this item's, the next one's)
+    double red[2 * kWarps];
     double base;
     uint32_t work[2];
 };
-
-// Copies the words holding edges [e0, e0 + ne) to smem with 16-byte loads (so
-// the host link serves runs of several KB); returns the bit of edge e0 there.
-__device__ __forceinline__ uint32_t pr_stage_words(const PrSlice &s, uint32_t e0, uint32_t ne, uint32_t eb,
-                                                   uint32_t *pool, uint32_t &nq) {
-    const uint64_t bit = (uint64_t)e0 * eb;
-    const uint64_t w_lo = (bit >> 5) & ~3ull;
-    nq = ne ? (uint32_t)(((((uint64_t)e0 + ne) * eb + 31) / 32 - w_lo + 3) >> 2) : 0;
-    for (uint32_t i = threadIdx.x; i < nq; i += kPrThreads) {
-        const uint64_t w = w_lo + 4ull * i;
-        uint4 q;
-        if (w + 4 <= s.edge_words) {
-            q = __ldg(reinterpret_cast<const uint4 *>(s.edges + w));
-        } else {  // the buffer's last words
-            q.x = w < s.edge_words ? __ldg(s.edges + w) : 0u;
-            q.y = w + 1 < s.edge_words ? __ldg(s.edges + w + 1) : 0u;
-            q.z = w + 2 < s.edge_words ? __ldg(s.edges + w + 2) : 0u;
-            q.w = 0u;
-        }
-        reinterpret_cast<uint4 *>(pool)[i] = q;
-    }
-    return (uint32_t)(bit - 32 * w_lo);
-}
-
-__device__ __forceinline__ uint32_t pr_staged_edge(const uint32_t *pool, uint32_t bit, uint32_t mask) {
-    return __funnelshift_r(pool[bit >> 5], pool[(bit >> 5) + 1], bit & 31u) & mask;
-}
 
 // Marks the rows that end in an item (r0 .. r0 + nr - 1, edges from e0) at
 // their last edges; rows without edges have none. Every thread calls it.
 template <typename T>
 __device__ __forceinline__ void pr_mark_rows(const uint32_t *ptr, uint32_t r0, uint32_t e0, uint32_t nr,
                                              PrItemSmem<T> &sm, uint32_t *marks) {
-    for (uint32_t j = threadIdx.x; j < nr; j += kPrThreads) {
+    for (uint32_t j = threadIdx.x; j < nr; j += kBlock) {
         const uint32_t lo = max(ptr[r0 + j], e0), hi = ptr[r0 + j + 1];
         if (hi > lo) {
             const uint32_t x = hi - 1 - e0;
@@ -1446,8 +1856,8 @@ __device__ __forceinline__ void pr_mark_rows(const uint32_t *ptr, uint32_t r0, u
 __device__ __forceinline__ uint32_t pr_next_row(const uint32_t *marks, const uint16_t *row_at, uint32_t xe,
                                                 uint32_t nr) {
     const int lane = threadIdx.x & 31;
-    for (uint32_t m0 = xe >> 5; m0 < kPrItem / 32; m0 += 32) {
-        const uint32_t word = m0 + lane < kPrItem / 32 ? marks[m0 + lane] : 0u;
+    for (uint32_t m0 = xe >> 5; m0 < kItem / 32; m0 += 32) {
+        const uint32_t word = m0 + lane < kItem / 32 ? marks[m0 + lane] : 0u;
         const unsigned any = __ballot_sync(kFull, word != 0);
         if (any) {
             const int q = __ffs((int)any) - 1;
@@ -1487,29 +1897,6 @@ __device__ __forceinline__ void pr_std_row(double *rank, T *c_new, uint32_t v, u
     if (od) c = (T)(rn / (double)od);
     else dang += rn;
     c_new[v] = c;
-}
-
-// block_reduce2_atomic for the item kernels' blocks.
-__device__ __forceinline__ void pr_reduce2_atomic(double a, double b, double *out, double *s_buf) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        a += __shfl_down_sync(kFull, a, d);
-        b += __shfl_down_sync(kFull, b, d);
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) {
-        s_buf[2 * w] = a;
-        s_buf[2 * w + 1] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < kPrWarps; i++) {
-            a += s_buf[2 * i];
-            b += s_buf[2 * i + 1];
-        }
-        if (a != 0) atomicAdd(&out[0], a);
-        if (b != 0) atomicAdd(&out[1], b);
-    }
 }
 
 // The host reads how a pass ended one pass late, so that the next one is
@@ -1574,7 +1961,7 @@ __device__ __forceinline__ void pr_item_row(const PrItemArgs<T> &p, uint32_t v, 
 template <bool REF, typename T>
 __device__ __forceinline__ void pr_flush_counts(const PrItemArgs<T> &p, PrCounts n, double *s_buf) {
     if (!REF) {
-        pr_reduce2_atomic(n.res, n.dang, p.acc, s_buf);
+        block_reduce2_atomic(n.res, n.dang, p.acc, s_buf);
         return;
     }
     n.n0 = __reduce_add_sync(kFull, n.n0);
@@ -1589,14 +1976,14 @@ __device__ __forceinline__ void pr_flush_counts(const PrItemArgs<T> &p, PrCounts
 }
 
 template <typename T, bool REF>
-__global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_kernel(PrItemArgs<T> p) {
+__global__ void __launch_bounds__(kBlock, ASC_PR_ITEM_BLOCKS) pr_pull_items_kernel(PrItemArgs<T> p) {
     typedef typename PrAcc<T>::type Acc;
     if (pr_pass_over<REF>(p)) return;
     __shared__ PrItemSmem<T> sm;
     const int lane = threadIdx.x & 31;
     const uint32_t total = p.sl[0].n + p.sl[1].n;
     const uint32_t eb = p.ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
-    if (threadIdx.x < kPrItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
+    if (threadIdx.x < kItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         sm.work[0] = atomicAdd(p.work, 1u);
         if (!REF) sm.base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
@@ -1611,30 +1998,30 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
         const uint2 a = p.items[it], b = p.items[it + 1];
         const uint32_t r0 = a.x, e0 = a.y, nr = b.x - a.x, ne = b.y - a.y;
         uint32_t nq;
-        const uint32_t bit0 = pr_stage_words(p.sl[od], e0, ne, eb, sm.pool, nq);
+        const uint32_t bit0 = stage_words(p.sl[od].edges, p.sl[od].edge_words, e0, ne, eb, sm.pool, nq);
         Acc *sums = reinterpret_cast<Acc *>(sm.pool + 4 * nq + (nq ? 4 : 0));
-        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads) sums[j] = (Acc)0;
+        for (uint32_t j = threadIdx.x; j <= nr; j += kBlock) sums[j] = (Acc)0;
         uint32_t *marks = sm.marks[buf];
         pr_mark_rows<T>(p.ptr, r0, e0, nr, sm, marks);
         if (threadIdx.x == 0) sm.work[buf ^ 1] = atomicAdd(p.work, 1u);
         __syncthreads();
-        if (threadIdx.x < kPrItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
-        const uint32_t x0 = threadIdx.x * kPrVt, xw = x0 - lane * kPrVt;  // first edge of the thread, the warp
+        if (threadIdx.x < kItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
+        const uint32_t x0 = threadIdx.x * kVt, xw = x0 - lane * kVt;  // first edge of the thread, the warp
         if (xw < ne) {
-            T c[kPrVt];
+            T c[kVt];
 #pragma unroll
-            for (int k = 0; k < kPrVt; k++) {
+            for (int k = 0; k < kVt; k++) {
                 c[k] = (T)0;
                 if (x0 + k < ne) {
-                    const uint32_t v = pr_staged_edge(sm.pool, bit0 + (x0 + k) * eb, mask);
+                    const uint32_t v = staged_word(sm.pool, bit0 + (x0 + k) * eb, mask);
                     if (!ASC_BAD(v >= p.V, 21, v)) c[k] = __ldg(p.c_old + v);
                 }
             }
-            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kPrVt) - 1u);
+            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
             // a thread's first sum may go on from earlier threads; later ones are its own
             T part = (T)0, head = (T)0;
 #pragma unroll
-            for (int k = 0; k < kPrVt; k++) {
+            for (int k = 0; k < kVt; k++) {
                 part += c[k];
                 if ((ends >> k) & 1u) {
                     if (ends & ((1u << k) - 1u)) sums[sm.row_at[x0 + k]] = PrAcc<T>::from(part);
@@ -1665,7 +2052,7 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
             }
             // the warp's last open sum goes to the row that ends after it: the
             // next mark, or the row that goes on past the item
-            const uint32_t xe = xw + 32 * kPrVt;
+            const uint32_t xe = xw + 32 * kVt;
             if (xe < ne || !((marks[(ne - 1) >> 5] >> ((ne - 1) & 31)) & 1u)) {
                 const uint32_t row = pr_next_row(marks, sm.row_at, xe, nr);
                 if (lane == 31) atomicAdd(&sums[row], tail);
@@ -1677,7 +2064,7 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
         // the global sums (pr_cut_rows_kernel applies them)
         const bool cut = p.ptr[r0] < e0;
         const bool goes_on = ne && !((marks[(ne - 1) >> 5] >> ((ne - 1) & 31)) & 1u);
-        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads) {
+        for (uint32_t j = threadIdx.x; j <= nr; j += kBlock) {
             if (j == nr ? goes_on : (j == 0 && cut)) {
                 atomicAdd(&p.sum[r0 + j], sums[j]);
             } else if (j < nr) {
@@ -1691,11 +2078,11 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_ITEM_BLOCKS) pr_pull_items_
 
 // Applies the rows that were cut by an item boundary: the row at the start of
 // item i, when it began earlier and ends in item i. Ends the pass. Blocks of
-// kPrThreads.
+// kBlock.
 template <typename T, bool REF>
 __global__ void pr_cut_rows_kernel(PrItemArgs<T> p, uint32_t n_items) {
     if (pr_pass_over<REF>(p)) return;
-    __shared__ double red[2 * kPrWarps];
+    __shared__ double red[2 * kWarps];
     __shared__ double s_base;
     if (!REF && threadIdx.x == 0)
         s_base = (1.0 - p.damping) / (double)p.V + p.damping * (*p.dangling_prev) / (double)p.V;
@@ -1847,27 +2234,26 @@ asc_status ensure_pr_buffers(asc_graph *g, size_t elem) {
     return ASC_OK;
 }
 
-// Work items of the edge-balanced PageRank passes (pr_plan_kernel), made once
-// per workspace.
-uint64_t pr_items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * ((V + E + kPrItem - 1) / kPrItem + 2); }
+// A graph's merge items, made once per workspace.
+uint64_t items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * ((V + E + kItem - 1) / kItem + 2); }
 
-asc_status ensure_pr_items(asc_graph *g) {
+asc_status ensure_items(asc_graph *g) {
     Workspace *ws = g->ws;
-    if (ws->pr_items) return ASC_OK;
+    if (ws->items) return ASC_OK;
     const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
     // shorter items where a staging buffer is smaller than one (its words, and
     // up to 3 on either side to start and end on 16 bytes)
     const uint64_t bits = g->edge_words == 2 ? 64 : g->ebits;
-    uint64_t L = kPrItem;
+    uint64_t L = kItem;
     while (g->stage_words && L > 32 && (L * bits + 31) / 32 + 8 > g->stage_words) L /= 2;
     const uint64_t n0 = (S + (uint64_t)g->h_ptr[S] + L - 1) / L, n1 = (V - S + g->E - g->h_ptr[S] + L - 1) / L;
-    ASC_CUDA(cudaMalloc((void **)&ws->pr_items, sizeof(uint2) * (n0 + n1 + 1)));
+    ASC_CUDA(cudaMalloc((void **)&ws->items, sizeof(uint2) * (n0 + n1 + 1)));
     ws->device_bytes += sizeof(uint2) * (n0 + n1 + 1);
     ws->n_items_static = (uint32_t)n0;
     ws->n_items = (uint32_t)(n0 + n1);
     const uint64_t blocks = std::min<uint64_t>((n0 + n1) / kBlock + 1, (uint64_t)ws->num_sms * 8);
-    pr_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, (uint32_t)L, ws->n_items_static,
-                                                               ws->n_items, ws->pr_items);
+    merge_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, (uint32_t)L, ws->n_items_static,
+                                                                  ws->n_items, ws->items);
     ASC_CUDA(cudaGetLastError());
     return ASC_OK;
 }
@@ -1984,6 +2370,13 @@ RegionArgs region_args(asc_graph *g, int parity_in, int region, bool dense) {
 // the far set.
 bool near_far(asc_graph *g, asc_algo algo) { return algo == ASC_SSSP && g->ws->tune.delta != 0; }
 
+void attach_items(const asc_graph *g, RegionArgs &a) {
+    const Workspace *ws = g->ws;
+    a.items = ws->items;
+    a.item_begin = a.region == 0 ? 0 : ws->n_items_static;
+    a.item_n = a.region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
+}
+
 void attach_far(asc_graph *g, asc_algo algo, RegionArgs &a) {
     if (near_far(g, algo)) {
         a.far_bits = g->ws->far_bits;
@@ -2095,78 +2488,32 @@ struct PhaseTimer {
     }
 };
 
-// Builds the iteration loop of one algorithm as a CUDA graph: a conditional
-// WHILE node whose body runs two iterations (parity 0 then 1; an iteration
-// with an empty input costs only empty launches) and loop_cond_kernel. The
-// kernels read their frontier sizes from the control block, so nothing
-// returns to the host between iterations.
-asc_status build_loop_graph(asc_graph *g, asc_algo algo, uint32_t cap) {
+// The kernel and grid of a traversal's persistent loop.
+typedef void (*TraverseFn)(LoopArgs);
+TraverseFn pick_traverse(asc_algo algo, int layout) {
+    if (algo == ASC_BFS)
+        return layout == 2 ? traverse_kernel<kBFS, 2> : layout == kBitsLayout ? traverse_kernel<kBFS, kBitsLayout>
+                                                                               : traverse_kernel<kBFS, 1>;
+    if (algo == ASC_CC)
+        return layout == 2 ? traverse_kernel<kCC, 2> : layout == kBitsLayout ? traverse_kernel<kCC, kBitsLayout>
+                                                                              : traverse_kernel<kCC, 1>;
+    return layout == 2 ? traverse_kernel<kSSSP, 2> : layout == kBitsLayout ? traverse_kernel<kSSSP, kBitsLayout>
+                                                                            : traverse_kernel<kSSSP, 1>;
+}
+
+#ifndef ASC_LOOP_EDGES
+#define ASC_LOOP_EDGES 4096
+#endif
+// CTAs of the persistent loop: all that stay resident, or one per
+// ASC_LOOP_EDGES edges of a small graph (fewer arrivals per barrier): a two-
+// iteration BFS on 1 M edges took 63 / 58 / 33 / 29 / 28 us at 512 / 1024 / 2048 /
+// 4096 / 8192.
+asc_status loop_grid(asc_graph *g, asc_algo algo, TraverseFn fn, uint32_t *grid) {
     Workspace *ws = g->ws;
-    const int slot = algo == ASC_BFS ? 0 : (algo == ASC_SSSP ? 1 : 2);
-    if (ws->loop_exec[slot] && ws->loop_cap[slot] == cap) return ASC_OK;
-    if (ws->loop_exec[slot]) {
-        cudaGraphExecDestroy(ws->loop_exec[slot]);
-        ws->loop_exec[slot] = nullptr;
-    }
-    FusedFn fused = pick_fused(algo, edge_layout(g));
-    const uint32_t V = (uint32_t)g->V;
-    const uint32_t grid = (uint32_t)(ws->num_sms * ws->tune.ctas_per_sm);
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaStream_t cs = nullptr;
-    asc_status st = ASC_OK;
-    auto chk = [&](cudaError_t e, const char *what) {
-        if (e != cudaSuccess && st == ASC_OK) st = cuda_fail(e, what, __FILE__, __LINE__);
-        return st == ASC_OK;
-    };
-    cudaGraphConditionalHandle handle;
-    cudaGraphNodeParams cp = {};
-    cudaGraphNode_t node;
-    if (chk(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "stream") &&
-        chk(cudaGraphCreate(&graph, 0), "cudaGraphCreate") &&
-        chk(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault), "handle")) {
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        if (chk(cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &cp), "cudaGraphAddNode")) {
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            if (chk(cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
-                    "capture")) {
-                for (int parity = 0; parity < 2; parity++) {
-                    const int po = 1 - parity;
-                    cudaMemsetAsync(ws->ctl + CTL_BLOCK * po, 0, 4 * CTL_BLOCK, cs);
-                    cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), cs);
-                    FusedArgs x;
-                    x.r0 = region_args(g, parity, 0, false);
-                    x.r1 = region_args(g, parity, 1, false);
-                    attach_far(g, algo, x.r0);
-                    attach_far(g, algo, x.r1);
-                    x.work = x.r0.cnt_out + 4;
-                    if (near_far(g, algo)) cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 4, cs);
-                    fused(cs, x, grid);
-                    if (algo == ASC_BFS && x.r0.in_ptr)
-                        bottom_up_kernel<<<bu_grid(ws, V / 32 + 1), kBlock, 0, cs>>>(x.r0, V / 32 + 1);
-                    if (near_far(g, algo)) launch_far(g, cs, x.r0);
-                    build_frontier_kernel<<<fill_grid(ws, V / 32 + 1), kBlock, 0, cs>>>(x.r0, ws->bitmap[po],
-                                                                                        V / 32 + 1);
-                }
-                loop_cond_kernel<<<1, 1, 0, cs>>>(handle, ws->ctl, cap);
-                cudaGraph_t out = nullptr;
-                chk(cudaStreamEndCapture(cs, &out), "end capture");
-            }
-        }
-    }
-    if (st == ASC_OK) chk(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
-    if (graph) cudaGraphDestroy(graph);
-    if (cs) cudaStreamDestroy(cs);
-    if (st != ASC_OK) {
-        if (exec) cudaGraphExecDestroy(exec);
-        cudaGetLastError();
-        return st;
-    }
-    ws->loop_exec[slot] = exec;
-    ws->loop_cap[slot] = cap;
+    int &per_sm = ws->loop_per_sm[algo];
+    if (!per_sm) ASC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0));
+    const uint64_t resident = (uint64_t)ws->num_sms * std::max(1, std::min(per_sm, (int)ws->tune.ctas_per_sm));
+    *grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(resident, (g->E + g->V) / ASC_LOOP_EDGES + 1));
     return ASC_OK;
 }
 
@@ -2179,7 +2526,7 @@ asc_status build_loop_graph(asc_graph *g, asc_algo algo, uint32_t cap) {
 // region is copied each pass in chunks by the copy engine, on a stream of its
 // own, into the two device buffers (chunk k into buffer k % 2), while the
 // kernels consume the chunk before it; the copy of chunk k + 2 waits only for
-// the launch that read chunk k. A chunk is a run of items (pr_plan_kernel), so
+// the launch that read chunk k. A chunk is a run of items (merge_plan_kernel), so
 // long lists are cut between chunks as between items. The static items are cut
 // into as many slices, and launch k runs static slice k with chunk k in one
 // grid, so every launch mixes HBM-bound gathers with the staged chunk and the
@@ -2248,10 +2595,10 @@ asc_status ensure_stage_plan(asc_graph *g, bool *ok) {
         *ok = true;
         return ASC_OK;
     }
-    ASC_TRY(ensure_pr_items(g));
+    ASC_TRY(ensure_items(g));
     const uint32_t ns = ws->n_items_static, n = ws->n_items;
     std::vector<uint2> items(n + 1);
-    ASC_CUDA(cudaMemcpyAsync(items.data(), ws->pr_items, sizeof(uint2) * items.size(), cudaMemcpyDeviceToHost,
+    ASC_CUDA(cudaMemcpyAsync(items.data(), ws->items, sizeof(uint2) * items.size(), cudaMemcpyDeviceToHost,
                              g->stream));
     ASC_CUDA(cudaStreamSynchronize(g->stream));
     StagePlan plan;
@@ -2443,7 +2790,7 @@ void free_ws_buffers(Workspace *ws) {
                     (void *)ws->queue[0],
                     (void *)ws->queue[1],
                     (void *)ws->segs[0], (void *)ws->segs[1], (void *)ws->ctl, ws->pr_rank,
-                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->pr_items, (void *)ws->pr_hot, (void *)ws->in_ptr, (void *)ws->in_edges,
+                    ws->pr_contrib[0], ws->pr_contrib[1], ws->pr_sum, (void *)ws->items, (void *)ws->pr_hot, (void *)ws->in_ptr, (void *)ws->in_edges,
                     (void *)ws->in_none})
         if (p) cudaFree(p);
     if (ws->h_ctl) cudaFreeHost(ws->h_ctl);
@@ -2451,8 +2798,6 @@ void free_ws_buffers(Workspace *ws) {
         if (p) cudaFree(p);
     for (void *p : {(void *)ws->h_stage, (void *)ws->h_items, (void *)ws->h_list, (void *)ws->h_segs})
         if (p) cudaFreeHost(p);
-    for (auto &e : ws->loop_exec)
-        if (e) cudaGraphExecDestroy(e);
     for (auto e : ws->ev)
         if (e) cudaEventDestroy(e);
     for (auto e : ws->phase_events) cudaEventDestroy(e);
@@ -2648,10 +2993,6 @@ asc_status ensure_in_ptr(asc_graph *g) {
         ASC_CUDA(cudaMemcpy(ws->in_edges, g->h_in_edges, 4 * words, cudaMemcpyHostToDevice));
         ws->device_bytes += 4 * words;
     }
-    if (ws->loop_exec[0]) {  // the BFS loop was captured without bottom-up steps
-        cudaGraphExecDestroy(ws->loop_exec[0]);
-        ws->loop_exec[0] = nullptr;
-    }
     return ASC_OK;
 }
 
@@ -2663,7 +3004,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     const bool all = algo == ASC_CC;
     uint32_t launches = 0;
     PhaseTimer pt(ws, (p.flags & ASC_RUN_PHASE_TIMING) != 0);
-    // bottom-up steps: BFS on a CSR graph, in the CUDA-graph loop or the host
+    // bottom-up steps: BFS on a CSR graph, in the persistent loop or the host
     // loop (the per-region timing, fragment counting and gather-and-copy runs
     // measure the top-down expansion alone)
     ws->bu_active = algo == ASC_BFS && ws->tune.bu_div && !g->is_csc &&
@@ -2672,49 +3013,81 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     ExpandFn expand = pick_expand(algo, edge_layout(g));
     FusedFn fused = pick_fused(algo, edge_layout(g));
 
-    ASC_CUDA(cudaEventRecord(ws->ev[0], s));
-    ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
-    for (int i = 0; i < 2; i++) ASC_CUDA(cudaMemsetAsync(ws->bitmap[i], 0, 4 * (V / 32 + 2), s));
-    ASC_CUDA(cudaMemsetAsync(ws->visited, 0, 4 * (V / 32 + 2), s));
-    const uint32_t ig = fill_grid(ws, V);
-    if (algo == ASC_CC) init_values_kernel<kCC><<<ig, kBlock, 0, s>>>(ws->val, V, 0);
-    else if (algo == ASC_BFS) init_values_kernel<kBFS><<<ig, kBlock, 0, s>>>(ws->val, V, source);
-    else init_values_kernel<kSSSP><<<ig, kBlock, 0, s>>>(ws->val, V, source);
-    if (near_far(g, algo)) {
-        ASC_CUDA(cudaMemsetAsync(ws->far_bits, 0, 4 * (V / 32 + 2), s));
-        ASC_CUDA(cudaStreamSynchronize(s));  // the staging word below is host memory
-        ws->h_ctl[CTL_THRESH] = 1 + ws->tune.delta;
-        ASC_CUDA(cudaMemcpyAsync(ws->ctl + CTL_THRESH, ws->h_ctl + CTL_THRESH, 4, cudaMemcpyHostToDevice, s));
-    }
-    // the seeded frontier lands in parity 0 (as the output of a virtual pass from parity 1)
-    RegionArgs sa = base_args(g, 1);
-    const uint32_t nwords = V / 32 + 1;
-    seed_bits_kernel<<<all ? fill_grid(ws, nwords) : 1, kBlock, 0, s>>>(sa, source, all ? 1 : 0, nwords);
-    build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, ws->bitmap[0], nwords);
-    launches += 3;
-    ASC_CUDA(cudaGetLastError());
     const int64_t cap = p.max_iterations > 0 ? p.max_iterations : (int64_t)4 * V + 64;
-    // fragment counting runs the host-driven loop: the captured graph loop is
-    // built without counters
     const bool gather = (p.flags & ASC_RUN_GATHER_COPY) != 0;
     if (gather) ASC_TRY(ensure_gather_buffers(g));
     const bool part = !gather && (p.flags & ASC_RUN_PARTITION_COPY) != 0;
     if (part) ASC_TRY(ensure_part_plan(g));
+    // regions walked in id order go by merge items, but for the partition copies,
+    // which walk vertex ranges
+    if (!part) ASC_TRY(ensure_items(g));
+    auto args_of = [&](int parity_in, int region) {
+        RegionArgs a = region_args(g, parity_in, region, false);
+        if (!part) attach_items(g, a);
+        attach_far(g, algo, a);
+        return a;
+    };
     uint64_t part_bytes = 0;
     uint32_t part_copies = 0;
-    const bool use_graph = !(p.flags & (ASC_RUN_PHASE_TIMING | ASC_RUN_HOST_LOOP | ASC_RUN_FRAGMENT_COUNTS |
-                                        ASC_RUN_GATHER_COPY | ASC_RUN_PARTITION_COPY));
+    const bool device_loop = !(p.flags & (ASC_RUN_PHASE_TIMING | ASC_RUN_HOST_LOOP | ASC_RUN_FRAGMENT_COUNTS |
+                                          ASC_RUN_GATHER_COPY | ASC_RUN_PARTITION_COPY));
     int iters = 0;
     double phase_ms[3] = {0, 0, 0};  // static top-down, on-demand top-down, bottom-up
-    if (use_graph) {
-        const uint32_t gcap = (uint32_t)std::min<int64_t>(cap, 0x7fffffff);
-        ASC_TRY(build_loop_graph(g, algo, gcap));
-        const int slot = algo == ASC_BFS ? 0 : (algo == ASC_SSSP ? 1 : 2);
-        ASC_CUDA(cudaGraphLaunch(ws->loop_exec[slot], s));
+    const uint32_t nwords = V / 32 + 1;
+    // SSSP re-expands, and bottom-up steps reach vertices without expanding
+    // them, so reached vertices are counted at the end; a top-down BFS expands
+    // every reached vertex exactly once: its expansion counts are the reached ones
+    const bool count_reached = algo == ASC_SSSP || (algo == ASC_BFS && ws->bu_active);
+    ASC_CUDA(cudaEventRecord(ws->ev[0], s));
+    ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
+    if (device_loop) {
+        LoopArgs l;
+        memset(&l, 0, sizeof(l));
+        for (int parity = 0; parity < 2; parity++) {
+            FusedArgs &x = parity ? l.x1 : l.x0;
+            x.r0 = args_of(parity, 0);
+            x.r1 = args_of(parity, 1);
+            x.work = x.r0.cnt_out + 4;
+        }
+        l.ctl = ws->ctl;
+        l.report = ws->h_ctl;
+        l.nwords = nwords;
+        l.src = source;
+        l.all = all ? 1 : 0;
+        l.cap = (uint32_t)std::min<int64_t>(cap, 0x7fffffff);
+        l.thresh = 1 + ws->tune.delta;
+        l.delta = ws->tune.delta;
+        l.count_reached = count_reached ? 1 : 0;
+        if (near_far(g, algo)) ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 16, s));
+        const TraverseFn fn = pick_traverse(algo, edge_layout(g));
+        uint32_t grid;
+        ASC_TRY(loop_grid(g, algo, fn, &grid));
+        ws->h_ctl[CTL_TIMEOUT] = 2;  // stays when a barrier ran out of time and nothing is reported
+        void *args[] = {&l};
+        ASC_CUDA(cudaLaunchCooperativeKernel((const void *)fn, dim3(grid), dim3(kBlock), args, 0, s));
         launches += 1;
+    } else {
+        for (int i = 0; i < 2; i++) ASC_CUDA(cudaMemsetAsync(ws->bitmap[i], 0, 4 * (V / 32 + 2), s));
+        ASC_CUDA(cudaMemsetAsync(ws->visited, 0, 4 * (V / 32 + 2), s));
+        const uint32_t ig = fill_grid(ws, V);
+        if (algo == ASC_CC) init_values_kernel<kCC><<<ig, kBlock, 0, s>>>(ws->val, V, 0);
+        else if (algo == ASC_BFS) init_values_kernel<kBFS><<<ig, kBlock, 0, s>>>(ws->val, V, source);
+        else init_values_kernel<kSSSP><<<ig, kBlock, 0, s>>>(ws->val, V, source);
+        if (near_far(g, algo)) {
+            ASC_CUDA(cudaMemsetAsync(ws->far_bits, 0, 4 * (V / 32 + 2), s));
+            ASC_CUDA(cudaStreamSynchronize(s));  // the staging word below is host memory
+            ws->h_ctl[CTL_THRESH] = 1 + ws->tune.delta;
+            ASC_CUDA(cudaMemcpyAsync(ws->ctl + CTL_THRESH, ws->h_ctl + CTL_THRESH, 4, cudaMemcpyHostToDevice, s));
+        }
+        // the seeded frontier lands in parity 0 (as the output of a virtual pass from parity 1)
+        RegionArgs sa = args_of(1, 0);
+        seed_bits_kernel<<<all ? fill_grid(ws, nwords) : 1, kBlock, 0, s>>>(sa, source, all ? 1 : 0, nwords);
+        build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, ws->bitmap[0], nwords);
+        launches += 3;
+        ASC_CUDA(cudaGetLastError());
     }
     uint32_t cnt[CTL_BLOCK] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (!use_graph) {
+    if (!device_loop) {
         ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
         ASC_CUDA(cudaStreamSynchronize(s));
         memcpy(cnt, ws->h_ctl, sizeof(cnt));
@@ -2724,6 +3097,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     auto region_work = [&](int region) -> uint64_t {
         const uint32_t range = region == 0 ? g->static_vertices : V - g->static_vertices;
         const bool bitmap_mode = div && cnt[6 + region] > range / div;
+        if (bitmap_mode && !part) return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
         return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + kBlock - 1) / kBlock;
     };
     while (cnt[6] | cnt[7]) {
@@ -2742,8 +3116,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             ASC_CUDA(cudaEventRecord(ws->ev[3], s));
             const uint64_t items0 = region_work(0);
             if (items0) {
-                RegionArgs a = region_args(g, parity, 0, false);
-                attach_far(g, algo, a);
+                RegionArgs a = args_of(parity, 0);
                 expand(g, a, grid_for(ws, items0));
                 launches++;
             }
@@ -2754,8 +3127,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             // the copy (partition j of this run into buffer j % 2)
             const uint64_t items0 = region_work(0);
             if (items0) {
-                RegionArgs a = region_args(g, parity, 0, false);
-                attach_far(g, algo, a);
+                RegionArgs a = args_of(parity, 0);
                 expand(g, a, grid_for(ws, items0));
                 launches++;
             }
@@ -2778,8 +3150,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
                                          pp->copy));
                 ASC_CUDA(cudaEventRecord(pp->copied[b], pp->copy));
                 ASC_CUDA(cudaStreamWaitEvent(s, pp->copied[b], 0));
-                RegionArgs a = region_args(g, parity, 1, false);
-                attach_far(g, algo, a);
+                RegionArgs a = args_of(parity, 1);
                 a.edges = (const uint32_t *)((uintptr_t)g->d_stage[b] - 4 * (uintptr_t)x.w_lo);
                 a.dense_begin = x.v_lo;
                 a.dense_end = x.v_hi;
@@ -2795,7 +3166,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             }
         } else if (pt.on && ws->bu_active && ws->in_ptr && ((uint64_t)cnt[6] + cnt[7]) * ws->tune.bu_div > V) {
             // diagnostic: a bottom-up step, timed on its own
-            RegionArgs a = region_args(g, parity, 0, false);
+            RegionArgs a = args_of(parity, 0);
             ASC_TRY(pt.begin(2));
             pt.record(s);
             bottom_up_kernel<<<bu_grid(ws, nwords), kBlock, 0, s>>>(a, nwords);
@@ -2807,8 +3178,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             for (int region = 0; region < 2; region++) {
                 const uint64_t items = region_work(region);
                 if (!items) continue;
-                RegionArgs a = region_args(g, parity, region, false);
-                attach_far(g, algo, a);
+                RegionArgs a = args_of(parity, region);
                 ASC_TRY(pt.begin(region));
                 pt.record(s);
                 expand(g, a, grid_for(ws, items));
@@ -2818,10 +3188,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         } else {
             const uint64_t items = region_work(0) + region_work(1);
             FusedArgs x;
-            x.r0 = region_args(g, parity, 0, false);
-            x.r1 = region_args(g, parity, 1, false);
-            attach_far(g, algo, x.r0);
-            attach_far(g, algo, x.r1);
+            x.r0 = args_of(parity, 0);
+            x.r1 = args_of(parity, 1);
             x.work = x.r0.cnt_out + 4;
             if (near_far(g, algo)) ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 4, s));
             fused(s, x, grid_for(ws, items));
@@ -2832,8 +3200,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             }
         }
         {
-            RegionArgs out_args = region_args(g, parity, 0, false);
-            attach_far(g, algo, out_args);
+            RegionArgs out_args = args_of(parity, 0);
             if (near_far(g, algo)) {
                 launch_far(g, s, out_args);
                 launches += 2;
@@ -2849,12 +3216,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         parity = po;
         iteration_boundary();
     }
-    // a top-down BFS expands every reached vertex exactly once, so its
-    // expansion counts already are the reached vertices and edges; SSSP
-    // re-expands, and bottom-up steps reach vertices without expanding them,
-    // so count them
-    const bool count_reached = algo == ASC_SSSP || (algo == ASC_BFS && ws->bu_active);
-    if (count_reached) {
+    if (count_reached && !device_loop) {
         if (algo == ASC_BFS)
             reached_bits_kernel<<<fill_grid(ws, 32ull * nwords), kBlock, 0, s>>>(
                 ws->visited, g->d_ptr, V, nwords, (unsigned long long *)(ws->ctl + CTL_STATS) + 4);
@@ -2871,15 +3233,11 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
                                  s));
     }
     ASC_CUDA(cudaEventRecord(ws->ev[2], s));
-    ASC_CUDA(cudaMemcpyAsync(ws->h_ctl + CTL_STATS, ws->ctl + CTL_STATS, 4 * (CTL_BODIES + 1 - CTL_STATS),
-                             cudaMemcpyDeviceToHost, s));
-    ASC_CUDA(cudaMemcpyAsync(ws->h_ctl + CTL_BU_EDGES, ws->ctl + CTL_BU_EDGES, 16, cudaMemcpyDeviceToHost, s));
+    if (!device_loop) ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_WORDS, cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
-    if (use_graph) {
+    if (device_loop) {
+        if (ws->h_ctl[CTL_TIMEOUT] == 2) return fail(ASC_ERR_TIMEOUT, "a grid barrier ran out of time");
         iters = (int)ws->h_ctl[CTL_ITERS];
-        // per body: two expansions, two builds (and two near-far pairs, or two
-        // bottom-up kernels), the loop test
-        launches += (near_far(g, algo) ? 9 : (algo == ASC_BFS && ws->bu_active ? 7 : 5)) * ws->h_ctl[CTL_BODIES] - 1;
         if (ws->h_ctl[CTL_TIMEOUT]) return fail(ASC_ERR_TIMEOUT, "no fixpoint after %d iterations", iters);
     }
     if (st) {
@@ -2979,13 +3337,13 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
     bool staged = false;
     if (!REF && !pt.on && !(p.flags & ASC_RUN_NO_STAGING)) ASC_TRY(ensure_stage_plan(g, &staged));
     StagePlan *sp = staged ? ws->stage : nullptr;
-    ASC_TRY(ensure_pr_items(g));
+    ASC_TRY(ensure_items(g));
 
     // REF: the active set alternates parity like a traversal frontier.
     ASC_TRY(ensure_pass_events(ws));
     const int depth = pt.on || staged || t_iteration_hook.fn ? 1 : 2;
     int it = 0, launched = 0;  // passes that ended, that were launched
-    bool over_items[kPassSlots];  // a pass in flight runs over items, not lists
+    bool over_items[kPassSlots] = {};  // a pass in flight runs over items, not lists
     const int max_it = p.max_iterations > 0 ? p.max_iterations : (REF ? 1000000 : 100);
     double residual = 0;
     double phase_ms[2] = {0, 0};
@@ -3037,7 +3395,7 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
             // every row
             PrItemArgs<T> ia;
             memset(&ia, 0, sizeof(ia));
-            ia.items = ws->pr_items;
+            ia.items = ws->items;
             ia.ptr = g->d_ptr;
             ia.outdeg = g->d_outdeg;
             ia.rank = rank;
@@ -3073,12 +3431,12 @@ static asc_status pagerank_impl(asc_graph *g, const asc_params &p, void *out, as
                 if (pt.on && !staged) ASC_CUDA(cudaMemsetAsync(ia.work, 0, 4, s));
                 ASC_TRY(pt.begin((int)k));
                 pt.record(s);
-                pr_pull_items_kernel<T, REF><<<item_grid(ws, n), kPrThreads, 0, s>>>(ia);
+                pr_pull_items_kernel<T, REF><<<item_grid(ws, n), kBlock, 0, s>>>(ia);
                 pt.record(s);
                 if (staged) ASC_TRY(stage_release(sp, k, s));
                 launches++;
             }
-            pr_cut_rows_kernel<T, REF><<<fill_grid(ws, ws->n_items), kPrThreads, 0, s>>>(ia, ws->n_items);
+            pr_cut_rows_kernel<T, REF><<<fill_grid(ws, ws->n_items), kBlock, 0, s>>>(ia, ws->n_items);
             launches++;
         } else {
             // the active vertices' lists and segments, then one launch for both
@@ -3930,7 +4288,8 @@ uint64_t workspace_bytes(asc_graph *g, bool pagerank) {
         b = 12 * V + 20 * (V / 32 + 2) + 4 * CTL_WORDS + 16 * segs + 4 * huge + 8 * 16;
     }
     if (pagerank && (!g->ws || !g->ws->pr_rank)) b += 4ull * 8 * V;
-    if (pagerank && (!g->ws || !g->ws->pr_items)) b += pr_items_bytes(V, E) + 8 * kPrHot;
+    if (!g->ws || !g->ws->items) b += items_bytes(V, E);
+    if (pagerank && (!g->ws || !g->ws->pr_hot)) b += 8 * kPrHot;
     // in-edge offsets of bottom-up BFS steps, allocated on the first BFS (with
     // the in-edges themselves when every out-edge is resident)
     if (!g->is_csc && t.bu_div && (!g->ws || !g->ws->in_ptr)) {
@@ -4269,18 +4628,18 @@ struct PrHot<float> {
 
 // Edge-balanced scatter: items as in pr_pull_items_kernel, over out-edges. The
 // contributions of the item's rows are converted once into shared memory; a
-// thread adds its row's to the destinations of kPrVt consecutive edges, passing
+// thread adds its row's to the destinations of kVt consecutive edges, passing
 // to the next row at each mark. Hot destinations add up in shared memory and
 // reach the global sums once per CTA; the rest are atomics in L2, which bound
 // the pass. wbits > 0: edge words hold the weight below the destination; ebits
 // 64: {dst, weight}.
 template <typename T>
-__global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_items_kernel(PrItemArgs<T> p) {
+__global__ void __launch_bounds__(kBlock, ASC_PR_SCATTER_BLOCKS) pr_scatter_items_kernel(PrItemArgs<T> p) {
     typedef typename PrAcc<T>::type Acc;
     if (p.active_prev ? !*p.active_prev : pr_pass_over<false>(p)) return;
     __shared__ PrItemSmem<T> sm;
     __shared__ PrHot<T> hot;
-    for (uint32_t i = threadIdx.x; i < kPrHot; i += kPrThreads) {
+    for (uint32_t i = threadIdx.x; i < kPrHot; i += kBlock) {
         const unsigned long long x = p.hot[i];
         hot.key[i] = x ? (uint32_t)x : 0xffffffffu;
         hot.clear(i);
@@ -4288,7 +4647,7 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_
     const int lane = threadIdx.x & 31;
     const uint32_t total = p.sl[0].n + p.sl[1].n;
     const uint32_t eb = p.ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
-    if (threadIdx.x < kPrItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
+    if (threadIdx.x < kItem / 32) sm.marks[0][threadIdx.x] = sm.marks[1][threadIdx.x] = 0;
     if (threadIdx.x == 0) sm.work[0] = atomicAdd(p.work, 1u);
     __syncthreads();
     for (int buf = 0;; buf ^= 1) {
@@ -4299,33 +4658,33 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_
         const uint2 a = p.items[it], b = p.items[it + 1];
         const uint32_t r0 = a.x, e0 = a.y, nr = b.x - a.x, ne = b.y - a.y;
         uint32_t nq;
-        const uint32_t bit0 = pr_stage_words(p.sl[od], e0, ne, eb, sm.pool, nq);
+        const uint32_t bit0 = stage_words(p.sl[od].edges, p.sl[od].edge_words, e0, ne, eb, sm.pool, nq);
         Acc *share = reinterpret_cast<Acc *>(sm.pool + 4 * nq + (nq ? 4 : 0));
-        for (uint32_t j = threadIdx.x; j <= nr; j += kPrThreads)
+        for (uint32_t j = threadIdx.x; j <= nr; j += kBlock)
             share[j] = r0 + j < p.V ? PrAcc<T>::from(p.c_old[r0 + j]) : (Acc)0;
         uint32_t *marks = sm.marks[buf];
         pr_mark_rows<T>(p.ptr, r0, e0, nr, sm, marks);
         if (threadIdx.x == 0) sm.work[buf ^ 1] = atomicAdd(p.work, 1u);
         __syncthreads();
-        if (threadIdx.x < kPrItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
-        const uint32_t x0 = threadIdx.x * kPrVt, xw = x0 - lane * kPrVt;
+        if (threadIdx.x < kItem / 32) sm.marks[buf ^ 1][threadIdx.x] = 0;
+        const uint32_t x0 = threadIdx.x * kVt, xw = x0 - lane * kVt;
         if (xw < ne) {
-            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kPrVt) - 1u);
+            const uint32_t ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
             // the row that is open after this thread's edges: of the next mark in
             // a later lane, in a later warp, or the one that goes on past the item
             const unsigned ended = __ballot_sync(kFull, ends != 0);
             const uint32_t first = ends ? sm.row_at[x0 + __ffs((int)ends) - 1] : nr;
             const unsigned above = lane < 31 ? ended & (0xffffffffu << (lane + 1)) : 0u;
             const uint32_t from_lane = __shfl_sync(kFull, first, above ? __ffs((int)above) - 1 : lane);
-            const uint32_t after = pr_next_row(marks, sm.row_at, xw + 32 * kPrVt, nr);
+            const uint32_t after = pr_next_row(marks, sm.row_at, xw + 32 * kVt, nr);
             const uint32_t open = above ? from_lane : after;
             Acc c = share[ends ? first : open];
-            uint32_t v[kPrVt];
+            uint32_t v[kVt];
 #pragma unroll
-            for (int k = 0; k < kPrVt; k++)
-                v[k] = x0 + k < ne ? pr_staged_edge(sm.pool, bit0 + (x0 + k) * eb, mask) >> p.wbits : 0u;
+            for (int k = 0; k < kVt; k++)
+                v[k] = x0 + k < ne ? staged_word(sm.pool, bit0 + (x0 + k) * eb, mask) >> p.wbits : 0u;
 #pragma unroll
-            for (int k = 0; k < kPrVt; k++) {
+            for (int k = 0; k < kVt; k++) {
                 if (x0 + k < ne && !ASC_BAD(v[k] >= p.V, 18, v[k])) {
                     const uint32_t h = pr_hot_slot(v[k]);
                     if (hot.key[h] == v[k]) hot.add(h, c);
@@ -4339,7 +4698,7 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_
         }
         __syncthreads();
     }
-    for (uint32_t i = threadIdx.x; i < kPrHot; i += kPrThreads) {
+    for (uint32_t i = threadIdx.x; i < kPrHot; i += kBlock) {
         const Acc x = hot.get(i);
         if (x != (Acc)0) atomicAdd(&p.sum[hot.key[i]], x);
     }
@@ -4349,10 +4708,10 @@ __global__ void __launch_bounds__(kPrThreads, ASC_PR_SCATTER_BLOCKS) pr_scatter_
 // active holds one bit per vertex that is still active, active_count this
 // pass's and active_next the next one's number of them.
 template <typename T, bool REF>
-__global__ void __launch_bounds__(kPrThreads) pr_push_apply_kernel(PrItemArgs<T> p, uint32_t *active,
+__global__ void __launch_bounds__(kBlock) pr_push_apply_kernel(PrItemArgs<T> p, uint32_t *active,
                                                                    uint32_t *active_count, uint32_t *active_next) {
     if (p.active_prev ? !*p.active_prev : pr_pass_over<false>(p)) return;
-    __shared__ double red[2 * kPrWarps];
+    __shared__ double red[2 * kWarps];
     __shared__ double s_base;
     const uint32_t V = p.V;
     if (!REF) {
@@ -4378,7 +4737,7 @@ __global__ void __launch_bounds__(kPrThreads) pr_push_apply_kernel(PrItemArgs<T>
         }
     }
     if (!REF) {
-        pr_reduce2_atomic(res, dang, p.acc, red);
+        block_reduce2_atomic(res, dang, p.acc, red);
         pr_end_pass<false>(p);
         return;
     }
@@ -4446,8 +4805,8 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
     StagePlan *sp = staged ? ws->stage : nullptr;
     PrItemArgs<T> ia;
     memset(&ia, 0, sizeof(ia));
-    ASC_TRY(ensure_pr_items(g));
-    ia.items = ws->pr_items;
+    ASC_TRY(ensure_items(g));
+    ia.items = ws->items;
     ia.sl[0] = pr_slice(g, 0);
     ia.sl[1] = pr_slice(g, 1);
     ia.ptr = g->d_ptr;
@@ -4501,12 +4860,12 @@ static asc_status pagerank_push_impl(asc_graph *g, const asc_params &p, void *ou
                 ASC_TRY(stage_chunk(g, sp, k, s, ia.sl));
                 ia.work = sp->d_work + k;
             }
-            pr_scatter_items_kernel<T><<<item_grid(ws, ia.sl[0].n + ia.sl[1].n, ASC_PR_SCATTER_BLOCKS), kPrThreads, 0,
+            pr_scatter_items_kernel<T><<<item_grid(ws, ia.sl[0].n + ia.sl[1].n, ASC_PR_SCATTER_BLOCKS), kBlock, 0,
                                          s>>>(ia);
             if (staged) ASC_TRY(stage_release(sp, k, s));
             launches++;
         }
-        pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kPrThreads, 0, s>>>(ia, active, counts + launched % 3,
+        pr_push_apply_kernel<T, REF><<<fill_grid(ws, V), kBlock, 0, s>>>(ia, active, counts + launched % 3,
                                                                               counts + (launched + 1) % 3);
         launches++;
         ASC_CUDA(cudaGetLastError());
