@@ -96,11 +96,12 @@ enum Alg { kBFS = 0, kSSSP = 1, kCC = 2 };
 // Words 42-43 (u64): in-edges that bottom-up BFS steps read from host memory;
 // words 44-45 (u64): unreached vertices those steps examined. Words 46-47 (u64):
 // in-edges of the vertices that a reference PageRank pass left active; words
+// 48-55: vertices that a near-far promotion moved (two regions, four slots);
 // 48-59: three residual and dangling-mass pairs (FP64) of PageRank passes, word
 // 60 the ticket of the blocks that end a pass. Word 61 counts the arrivals at a
 // grid barrier; word 29 is 2 when one ran out of time.
 enum { CTL_BLOCK = 8, CTL_STATS = 16, CTL_ITERS = 28, CTL_TIMEOUT = 29, CTL_THRESH = 31,
-       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_ACC = 48,
+       CTL_PR = 32, CTL_MINFAR = 36, CTL_BU_EDGES = 42, CTL_BU_VERTS = 44, CTL_ACTIVE = 46, CTL_PROMOTED = 48, CTL_ACC = 48,
        CTL_TICKET = 60, CTL_BARRIER = 61, CTL_WORDS = 64 };
 
 struct RegionArgs {
@@ -983,13 +984,15 @@ __global__ void __launch_bounds__(kBlock) expand_staged_kernel(StagedArgs x) {
 // Builds the next frontier from its bitmap (one thread per 32-vertex word):
 // vertices with long lists become segment items; the others are appended to
 // their region's list only when that region will be walked as a list (warp
-// scan of the per-word counts, one atomic per warp). cnt_out[6..7] hold the
-// region bit counts the expansion flushed; cnt_out[0..3] receive the lists.
-__device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32_t *next_bits, uint32_t nwords) {
+// scan of the per-word counts, one atomic per warp). bits0 and bits1 are the
+// region bit counts (cnt_out[6..7], which the expansion flushed); cnt_out[0..3]
+// receive the lists.
+__device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32_t *next_bits, uint32_t nwords,
+                                               uint32_t bits0, uint32_t bits1) {
     const int lane = threadIdx.x & 31;
     const uint32_t range0 = a.S, range1 = a.V - a.S;
-    const bool list0 = !(a.dense_div && a.cnt_out[6] > range0 / a.dense_div);
-    const bool list1 = !(a.dense_div && a.cnt_out[7] > range1 / a.dense_div);
+    const bool list0 = !(a.dense_div && bits0 > range0 / a.dense_div);
+    const bool list1 = !(a.dense_div && bits1 > range1 / a.dense_div);
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t base = blockIdx.x * blockDim.x; base < nwords; base += stride) {
         const uint32_t w = base + threadIdx.x;
@@ -1058,7 +1061,7 @@ __device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32
 }
 
 __global__ void build_frontier_kernel(RegionArgs a, const uint32_t *next_bits, uint32_t nwords) {
-    build_frontier(a, next_bits, nwords);
+    build_frontier(a, next_bits, nwords, a.cnt_out[6], a.cnt_out[7]);
 }
 
 // SSSP near-far, step 1: when the pass left the near frontier empty, the
@@ -1331,9 +1334,10 @@ __device__ __forceinline__ void loop_setup(const LoopArgs &x) {
     }
 }
 
-// Near-far: the far vertices below thresh join the frontier in bits (counts at
-// cnt), the smallest value of those that stay goes to *minfar.
-__device__ __forceinline__ void promote_far(const RegionArgs &a, uint32_t *bits, uint32_t *cnt, uint32_t nwords,
+// Near-far: the far vertices below thresh join the frontier in bits (their
+// numbers per region are added to moved[0..1]), the smallest value of those that
+// stay goes to *minfar.
+__device__ __forceinline__ void promote_far(const RegionArgs &a, uint32_t *bits, uint32_t *moved, uint32_t nwords,
                                             uint32_t thresh, uint32_t *minfar) {
     uint32_t n0 = 0, n1 = 0, least = 0xffffffffu;
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) {
@@ -1358,8 +1362,8 @@ __device__ __forceinline__ void promote_far(const RegionArgs &a, uint32_t *bits,
     n1 = __reduce_add_sync(kFull, n1);
     least = __reduce_min_sync(kFull, least);
     if ((threadIdx.x & 31) == 0) {
-        if (n0) atomicAdd(&cnt[6], n0);
-        if (n1) atomicAdd(&cnt[7], n1);
+        if (n0) atomicAdd(&moved[0], n0);
+        if (n1) atomicAdd(&moved[1], n1);
         if (least != 0xffffffffu) atomicMin(minfar, least);
     }
 }
@@ -1382,20 +1386,31 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
     volatile const uint32_t *cin = a.cnt_in;
     if (!(cin[6] | cin[7])) {
         if (ALG != kSSSP || !a.far_bits) return kLoopEnd;
-        // the near frontier is empty: the threshold moves on. Four slots for the
-        // smallest far value: this one's was cleared two promotions ago
+        // The near frontier is empty: the threshold moves on. Every promotion
+        // counts in a slot of its own (of four; the one after next is cleared), and
+        // the frontier's counts are set only once every thread has read them as zero.
+        uint32_t n0, n1;
         for (;;) {
-            uint32_t *slot = l.ctl + CTL_MINFAR + (st.promotions & 3);
-            if (blockIdx.x == 0 && threadIdx.x == 0) l.ctl[CTL_MINFAR + ((st.promotions + 2) & 3)] = 0xffffffffu;
-            promote_far(a, y.r0.bitmap, y.r0.cnt_out, l.nwords, st.thresh, slot);
-            st.promotions++;
+            const uint32_t k = st.promotions++ & 3, clear = (k + 2) & 3;
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                l.ctl[CTL_MINFAR + clear] = 0xffffffffu;
+                l.ctl[CTL_PROMOTED + 2 * clear] = l.ctl[CTL_PROMOTED + 2 * clear + 1] = 0;
+            }
+            promote_far(a, y.r0.bitmap, l.ctl + CTL_PROMOTED + 2 * k, l.nwords, st.thresh, l.ctl + CTL_MINFAR + k);
             if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
-            if (cin[6] | cin[7]) break;
-            const uint32_t least = *(volatile uint32_t *)slot;
+            volatile const uint32_t *moved = l.ctl + CTL_PROMOTED + 2 * k;
+            n0 = moved[0];
+            n1 = moved[1];
+            if (n0 | n1) break;
+            const uint32_t least = *(volatile uint32_t *)(l.ctl + CTL_MINFAR + k);
             if (least == 0xffffffffu) return kLoopEnd;
             st.thresh = least > 0xffffffffu - l.delta ? 0xffffffffu : least + l.delta;
         }
-        build_frontier(y.r0, y.r0.bitmap, l.nwords);
+        build_frontier(y.r0, y.r0.bitmap, l.nwords, n0, n1);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            y.r0.cnt_out[6] = n0;
+            y.r0.cnt_out[7] = n1;
+        }
         if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
     }
     if (st.it >= l.cap) {
@@ -1406,7 +1421,7 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
     if (ALG == kBFS && bottom_up_step(a)) bottom_up_words(a, l.nwords, bs, s_next);
     else expand_regions<ALG, WORDS>(x, st.thresh, sm, s_next);
     if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
-    build_frontier(a, a.bitmap, l.nwords);
+    build_frontier(a, a.bitmap, l.nwords, a.cnt_out[6], a.cnt_out[7]);
     // the input frontier's bitmap and counts are the next output's
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < l.nwords; w += gridDim.x * blockDim.x)
         y.r0.bitmap[w] = 0;
@@ -1424,7 +1439,7 @@ __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const
     loop_setup<ALG>(l);
     if (!grid_barrier(l.ctl, st.target)) return;
     if (l.all) {
-        build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords);
+        build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords, l.x1.r0.cnt_out[6], l.x1.r0.cnt_out[7]);
         if (!grid_barrier(l.ctl, st.target)) return;
     }
     for (;;) {
@@ -3018,6 +3033,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     if (gather) ASC_TRY(ensure_gather_buffers(g));
     const bool part = !gather && (p.flags & ASC_RUN_PARTITION_COPY) != 0;
     if (part) ASC_TRY(ensure_part_plan(g));
+    const bool device_loop = !(p.flags & (ASC_RUN_PHASE_TIMING | ASC_RUN_HOST_LOOP | ASC_RUN_FRAGMENT_COUNTS |
+                                          ASC_RUN_GATHER_COPY | ASC_RUN_PARTITION_COPY));
     // regions walked in id order go by merge items, but for the partition copies,
     // which walk vertex ranges
     if (!part) ASC_TRY(ensure_items(g));
@@ -3029,8 +3046,6 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     };
     uint64_t part_bytes = 0;
     uint32_t part_copies = 0;
-    const bool device_loop = !(p.flags & (ASC_RUN_PHASE_TIMING | ASC_RUN_HOST_LOOP | ASC_RUN_FRAGMENT_COUNTS |
-                                          ASC_RUN_GATHER_COPY | ASC_RUN_PARTITION_COPY));
     int iters = 0;
     double phase_ms[3] = {0, 0, 0};  // static top-down, on-demand top-down, bottom-up
     const uint32_t nwords = V / 32 + 1;
