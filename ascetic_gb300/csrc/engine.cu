@@ -1250,7 +1250,11 @@ struct LoopArgs {
     uint32_t thresh;        // near-far: the first threshold
     uint32_t delta;         // near-far: step of the next one beyond the smallest far value
     uint32_t count_reached;
+    uint32_t first_label;   // connected components: src's label is spread first, the rest follow
+    uint32_t first_cap;     // after at most this many iterations
 };
+
+constexpr uint32_t kFirstLabelIterations = 32;
 
 // Polls of a grid barrier (a read of L2 and a short sleep each) before it gives
 // up: tens of seconds, far above any phase.
@@ -1368,6 +1372,31 @@ __device__ __forceinline__ void promote_far(const RegionArgs &a, uint32_t *bits,
     }
 }
 
+// Connected components, once the first label is spread: every other vertex with
+// out-edges that kept its own id joins the frontier in bits (their numbers per
+// region are added to moved[0..1]).
+__device__ __forceinline__ void seed_unlabelled(const RegionArgs &a, uint32_t *bits, uint32_t src, uint32_t *moved) {
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * kWarps;
+    uint32_t n0 = 0, n1 = 0;
+    for (uint32_t w = blockIdx.x * kWarps + (threadIdx.x >> 5); 32 * w < a.V; w += warps) {
+        const uint32_t v = 32 * w + lane;
+        const bool join = v < a.V && v != src && a.val[v] == v && a.ptr[v + 1] != a.ptr[v];
+        const uint32_t word = __ballot_sync(kFull, join) | bits[w];
+        if (lane == 0 && word) {
+            bits[w] = word;
+            const uint32_t smask = 32 * w + 32 <= a.S ? 0xffffffffu : (32 * w >= a.S ? 0 : (1u << (a.S - 32 * w)) - 1u);
+            n0 += __popc(word & smask);
+            n1 += __popc(word & ~smask);
+        }
+    }
+    if (lane == 0 && n0) atomicAdd(&moved[0], n0);
+    if (lane == 0 && n1) atomicAdd(&moved[1], n1);
+}
+
+__global__ void seed_unlabelled_kernel(RegionArgs a, uint32_t *bits, uint32_t src, uint32_t *moved) {
+    seed_unlabelled(a, bits, src, moved);
+}
+
 struct LoopState {
     uint32_t target = 0;      // of the grid barrier
     uint32_t it = 0;
@@ -1384,6 +1413,23 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
                                                    LoopState &st, ExpandSmem<WORDS> &sm, BuSmem &bs, uint32_t *s_next) {
     const RegionArgs &a = x.r0;
     volatile const uint32_t *cin = a.cnt_in;
+    if (ALG == kCC && l.first_label && !st.promotions && (!(cin[6] | cin[7]) || st.it >= l.first_cap)) {
+        // the frontier of the remaining labels, in place of an empty one or beside
+        // what the first label still has to reach
+        st.promotions = 1;
+        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;  // every thread has read the counts
+        if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
+        seed_unlabelled(a, y.r0.bitmap, l.src, l.ctl + CTL_PROMOTED);
+        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+        volatile const uint32_t *moved = l.ctl + CTL_PROMOTED;
+        const uint32_t n0 = moved[0], n1 = moved[1];
+        build_frontier(y.r0, y.r0.bitmap, l.nwords, n0, n1);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            y.r0.cnt_out[6] = n0;
+            y.r0.cnt_out[7] = n1;
+        }
+        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+    }
     if (!(cin[6] | cin[7])) {
         if (ALG != kSSSP || !a.far_bits) return kLoopEnd;
         // The near frontier is empty: the threshold moves on. Every promotion
@@ -3053,6 +3099,20 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     // them, so reached vertices are counted at the end; a top-down BFS expands
     // every reached vertex exactly once: its expansion counts are the reached ones
     const bool count_reached = algo == ASC_SSSP || (algo == ASC_BFS && ws->bu_active);
+    // Connected components without an iteration cap of the caller's: the label of
+    // the smallest id with out-edges first. Nothing smaller reaches what it
+    // reaches, so those labels are final and each of its lists is read once; with
+    // every vertex in the first frontier, nearly all lists are read again when the
+    // giant component's label arrives (6 M vertices symmetrised, 180 M edges: 2.39
+    // ms against 3.61). A label that spreads slowly (a long path) is joined by the
+    // rest after kFirstLabelIterations. The timed, counting and comparison runs
+    // start from every vertex.
+    const bool first_label = all && p.max_iterations <= 0 && g->E &&
+                             !(p.flags & (ASC_RUN_PHASE_TIMING | ASC_RUN_FRAGMENT_COUNTS | ASC_RUN_GATHER_COPY |
+                                          ASC_RUN_PARTITION_COPY));
+    const uint32_t first =
+        first_label ? (uint32_t)(std::upper_bound(g->h_ptr, g->h_ptr + V + 1, 0u) - g->h_ptr) - 1 : source;
+    bool rest_waits = first_label && !device_loop;  // the other labels have not started
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
     ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
     if (device_loop) {
@@ -3067,8 +3127,10 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         l.ctl = ws->ctl;
         l.report = ws->h_ctl;
         l.nwords = nwords;
-        l.src = source;
-        l.all = all ? 1 : 0;
+        l.src = first;
+        l.all = all && !first_label ? 1 : 0;
+        l.first_label = first_label ? 1 : 0;
+        l.first_cap = kFirstLabelIterations;
         l.cap = (uint32_t)std::min<int64_t>(cap, 0x7fffffff);
         l.thresh = 1 + ws->tune.delta;
         l.delta = ws->tune.delta;
@@ -3096,7 +3158,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         }
         // the seeded frontier lands in parity 0 (as the output of a virtual pass from parity 1)
         RegionArgs sa = args_of(1, 0);
-        seed_bits_kernel<<<all ? fill_grid(ws, nwords) : 1, kBlock, 0, s>>>(sa, source, all ? 1 : 0, nwords);
+        const bool seed_all = all && !first_label;
+        seed_bits_kernel<<<seed_all ? fill_grid(ws, nwords) : 1, kBlock, 0, s>>>(sa, first, seed_all ? 1 : 0, nwords);
         build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(sa, ws->bitmap[0], nwords);
         launches += 3;
         ASC_CUDA(cudaGetLastError());
@@ -3115,7 +3178,20 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         if (bitmap_mode && !part) return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
         return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + kBlock - 1) / kBlock;
     };
-    while (cnt[6] | cnt[7]) {
+    while ((cnt[6] | cnt[7]) || rest_waits) {
+        if (rest_waits && (!(cnt[6] | cnt[7]) || iters >= (int)kFirstLabelIterations)) {
+            rest_waits = false;
+            RegionArgs a = args_of(1 - parity, 0);  // writes this parity's lists
+            ASC_CUDA(cudaMemsetAsync(a.cnt_out, 0, 4 * CTL_BLOCK, s));
+            seed_unlabelled_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>(a, a.bitmap, first, a.cnt_out + 6);
+            build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(a, a.bitmap, nwords);
+            launches += 2;
+            ASC_CUDA(cudaGetLastError());
+            ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, a.cnt_out, 4 * CTL_BLOCK, cudaMemcpyDeviceToHost, s));
+            ASC_CUDA(cudaStreamSynchronize(s));
+            memcpy(cnt, ws->h_ctl, sizeof(cnt));
+            continue;
+        }
         if (iters >= cap) return fail(ASC_ERR_TIMEOUT, "no fixpoint after %d iterations", iters);
         iters++;
         const int po = 1 - parity;
