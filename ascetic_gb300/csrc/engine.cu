@@ -32,6 +32,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <chrono>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -541,12 +542,13 @@ __device__ __forceinline__ void region_items_bits(const RegionArgs &a, uint32_t 
 
 // A region's merge item: the edges of its active rows, staged in shared memory
 // by 16-byte chunks that hold any (so the host link serves long runs and only
-// what is active), then kVt consecutive edges per thread.
-template <int WORDS>
+// what is active), then kVt consecutive edges per thread. Val is what an active
+// row carries to its edges.
+template <int WORDS, typename Val>
 struct ItemSmem {
-    // the staged words, then one value per row: at most ne (2 ne) words and nr + 1
-    // with nr + ne <= kItem, plus alignment and one word read past the end
-    alignas(16) uint32_t pool[(WORDS == 2 ? 2 : 1) * kItem + 24];
+    // the staged words, then one Val per row: at most ne (2 ne) words and nr + 1
+    // Vals with nr + ne <= kItem, plus alignment and one word read past the end
+    alignas(16) uint32_t pool[(WORDS == 2 || sizeof(Val) == 8 ? 2 : 1) * kItem + 24];
     uint16_t row_at[kItem];         // of an active row's first edge here: the row, from the item's first
     uint32_t starts[kItem / 32];    // one bit per edge: an active row starts here
     uint32_t active[kItem / 32];    // one bit per edge: it belongs to an active row
@@ -568,16 +570,21 @@ __device__ __forceinline__ uint32_t row_before(const uint32_t *starts, const uin
     return 0;
 }
 
-template <int ALG, int WORDS>
-__device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WORDS> &sm, uint32_t *s_next,
-                                  uint32_t thresh) {
+// Stages item it; false when it holds no active edge. loads(u) is row u's Val;
+// counts (shared) receive the edges and vertices. The block calls it together.
+template <int WORDS, typename Val, typename Load>
+__device__ __forceinline__ bool stage_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WORDS, Val> &sm, Load load,
+                                                 uint32_t *n_edges, uint32_t *n_verts, uint32_t &ne_out,
+                                                 uint32_t &bit0_out, Val *&value) {
     const uint2 i0 = a.items[it], i1 = a.items[it + 1];
     const uint32_t r0 = i0.x, e0 = i0.y, nr = i1.x - i0.x, ne = i1.y - i0.y;
     const int lane = threadIdx.x & 31;
     const uint32_t eb = WORDS == 2 ? 64 : WORDS == 1 ? 32 : a.ebits;
     const uint64_t bit = (uint64_t)e0 * eb, w_lo = (bit >> 5) & ~3ull;
     const uint32_t bit0 = (uint32_t)(bit - 32 * w_lo), nq = (bit0 + ne * eb + 127) >> 7;
-    uint32_t *value = sm.pool + 4 * nq + 4;
+    value = reinterpret_cast<Val *>(sm.pool + 4 * nq + 4);
+    ne_out = ne;
+    bit0_out = bit0;
     if (threadIdx.x < kItem / 32) sm.starts[threadIdx.x] = sm.active[threadIdx.x] = 0;
     __syncthreads();
     uint32_t edges = 0, verts = 0;
@@ -589,7 +596,7 @@ __device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WOR
         verts += j < nr;  // a vertex counts where its row ends
         if (lo >= hi) continue;
         edges += hi - lo;
-        value[j] = a.val[u];
+        value[j] = load(u);
         sm.row_at[lo] = (uint16_t)j;
         atomicOr(&sm.starts[lo >> 5], 1u << (lo & 31));
         for (uint32_t w = lo >> 5; w <= (hi - 1) >> 5; w++) {
@@ -603,9 +610,9 @@ __device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WOR
     const bool any = __syncthreads_or(edges != 0);
     edges = __reduce_add_sync(kFull, edges);
     verts = __reduce_add_sync(kFull, verts);
-    if (lane == 0 && edges) atomicAdd(&s_next[2 + a.region], edges);
-    if (lane == 0 && verts) atomicAdd(&s_next[4 + a.region], verts);
-    if (!any) return;
+    if (lane == 0 && edges) atomicAdd(n_edges, edges);
+    if (lane == 0 && verts) atomicAdd(n_verts, verts);
+    if (!any) return false;
     for (uint32_t i = threadIdx.x; i < nq; i += kBlock) {
         // edges with a bit in this chunk
         const uint32_t c0 = 128 * i;
@@ -620,63 +627,82 @@ __device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WOR
         if (need) reinterpret_cast<uint4 *>(sm.pool)[i] = load_words16(a.edges, a.edge_words, w_lo + 4ull * i);
     }
     __syncthreads();
-    const uint32_t x0 = threadIdx.x * kVt, xw = x0 - lane * kVt;  // first edge of the thread, the warp
-    uint32_t n0 = 0, n1 = 0;
-    if (xw < ne) {
-        const uint32_t act = (sm.active[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
-        const uint32_t st = (sm.starts[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
-        if (__any_sync(kFull, act != 0)) {
-            // the row open at the thread's first edge: of the last start in an
-            // earlier lane, or in an earlier warp
-            const unsigned began = __ballot_sync(kFull, st != 0);
-            const uint32_t last = st ? sm.row_at[x0 + 31 - __clz((int)st)] : 0u;
-            const unsigned below = began & ((1u << lane) - 1u);
-            const uint32_t from_lane = __shfl_sync(kFull, last, below ? 31 - __clz((int)below) : lane);
-            const uint32_t before = row_before(sm.starts, sm.row_at, xw);
-            uint32_t row = below ? from_lane : before;
-            uint32_t vu = (act & 1u) ? value[(st & 1u) ? (uint32_t)sm.row_at[x0] : row] : 0u;
-            constexpr uint32_t kMask = 0xffffffffu;
-            const uint32_t mask = eb >= 32 ? kMask : (1u << eb) - 1u;
+    return true;
+}
+
+// A thread's kVt edges of a staged item: which are active, where rows start, and
+// the Val of the row open at the first one (when that is active). False for the
+// whole warp when it has none.
+template <int WORDS, typename Val>
+__device__ __forceinline__ bool merge_item_edges(const ItemSmem<WORDS, Val> &sm, const Val *value, uint32_t ne,
+                                                 uint32_t x0, uint32_t &act, uint32_t &st, Val &open) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t xw = x0 - lane * kVt;  // the warp's first edge
+    if (xw >= ne) return false;
+    act = (sm.active[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
+    st = (sm.starts[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
+    if (!__any_sync(kFull, act != 0)) return false;
+    // of the last start in an earlier lane, or in an earlier warp
+    const unsigned began = __ballot_sync(kFull, st != 0);
+    const uint32_t last = st ? sm.row_at[x0 + 31 - __clz((int)st)] : 0u;
+    const unsigned below = began & ((1u << lane) - 1u);
+    const uint32_t from_lane = __shfl_sync(kFull, last, below ? 31 - __clz((int)below) : lane);
+    const uint32_t before = row_before(sm.starts, sm.row_at, xw);
+    const uint32_t row = (st & 1u) ? (uint32_t)sm.row_at[x0] : below ? from_lane : before;
+    open = (act & 1u) ? value[row] : (Val)0;
+    return true;
+}
+
+template <int ALG, int WORDS>
+__device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WORDS, uint32_t> &sm, uint32_t *s_next,
+                                  uint32_t thresh) {
+    uint32_t ne, bit0, *value;
+    if (!stage_merge_item(a, it, sm, [&](uint32_t u) { return a.val[u]; }, &s_next[2 + a.region],
+                          &s_next[4 + a.region], ne, bit0, value))
+        return;
+    const uint32_t eb = WORDS == 2 ? 64 : WORDS == 1 ? 32 : a.ebits;
+    const uint32_t mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    const uint32_t x0 = threadIdx.x * kVt;
+    uint32_t n0 = 0, n1 = 0, act, st, vu;
+    if (merge_item_edges(sm, value, ne, x0, act, st, vu)) {
 #pragma unroll
-            for (int k0 = 0; k0 < kVt; k0 += kUnroll) {
-                uint32_t v[kUnroll], nv[kUnroll], cur[kUnroll];
+        for (int k0 = 0; k0 < kVt; k0 += kUnroll) {
+            uint32_t v[kUnroll], nv[kUnroll], cur[kUnroll];
 #pragma unroll
-                for (int k = 0; k < kUnroll; k++) {
-                    v[k] = 0;
-                    nv[k] = 0xffffffffu;  // never lower than a value: no update
-                    if ((act >> (k0 + k)) & 1u) {
-                        if (k0 + k > 0 && ((st >> (k0 + k)) & 1u)) vu = value[sm.row_at[x0 + k0 + k]];
-                        const uint32_t at = bit0 + (x0 + k0 + k) * eb;
-                        if (WORDS == 2) {
-                            v[k] = sm.pool[at >> 5];
-                            nv[k] = ALG == kSSSP ? vu + sm.pool[(at >> 5) + 1] : (ALG == kBFS ? vu + 1 : vu);
-                        } else {
-                            const uint32_t e = WORDS == 1 ? sm.pool[at >> 5] : staged_word(sm.pool, at, mask);
-                            v[k] = e >> a.wbits;
-                            nv[k] = ALG == kBFS ? vu + 1
-                                                : (ALG == kSSSP ? vu + (e & ((1u << a.wbits) - 1u)) : vu);
-                        }
-                        if (ASC_BAD(v[k] >= a.V, 2, v[k])) {
-                            v[k] = 0;
-                            nv[k] = 0xffffffffu;
-                        }
+            for (int k = 0; k < kUnroll; k++) {
+                v[k] = 0;
+                nv[k] = 0xffffffffu;  // never lower than a value: no update
+                if ((act >> (k0 + k)) & 1u) {
+                    if (k0 + k > 0 && ((st >> (k0 + k)) & 1u)) vu = value[sm.row_at[x0 + k0 + k]];
+                    const uint32_t at = bit0 + (x0 + k0 + k) * eb;
+                    if (WORDS == 2) {
+                        v[k] = sm.pool[at >> 5];
+                        nv[k] = ALG == kSSSP ? vu + sm.pool[(at >> 5) + 1] : (ALG == kBFS ? vu + 1 : vu);
+                    } else {
+                        const uint32_t e = WORDS == 1 ? sm.pool[at >> 5] : staged_word(sm.pool, at, mask);
+                        v[k] = e >> a.wbits;
+                        nv[k] = ALG == kBFS ? vu + 1 : (ALG == kSSSP ? vu + (e & ((1u << a.wbits) - 1u)) : vu);
+                    }
+                    if (ASC_BAD(v[k] >= a.V, 2, v[k])) {
+                        v[k] = 0;
+                        nv[k] = 0xffffffffu;
                     }
                 }
+            }
 #pragma unroll
-                for (int k = 0; k < kUnroll; k++) cur[k] = nv[k] != 0xffffffffu ? probe<ALG>(a, v[k]) : 0;
+            for (int k = 0; k < kUnroll; k++) cur[k] = nv[k] != 0xffffffffu ? probe<ALG>(a, v[k]) : 0;
 #pragma unroll
-                for (int k = 0; k < kUnroll; k++) {
-                    const bool won = lower<ALG>(a, v[k], nv[k], cur[k], thresh);
-                    n0 += won && v[k] < a.S;
-                    n1 += won && v[k] >= a.S;
-                }
+            for (int k = 0; k < kUnroll; k++) {
+                const bool won = lower<ALG>(a, v[k], nv[k], cur[k], thresh);
+                n0 += won && v[k] < a.S;
+                n1 += won && v[k] >= a.S;
             }
         }
     }
     n0 = __reduce_add_sync(kFull, n0);
     n1 = __reduce_add_sync(kFull, n1);
-    if (lane == 0 && n0) atomicAdd(&s_next[0], n0);
-    if (lane == 0 && n1) atomicAdd(&s_next[1], n1);
+    if ((threadIdx.x & 31) == 0 && n0) atomicAdd(&s_next[0], n0);
+    if ((threadIdx.x & 31) == 0 && n1) atomicAdd(&s_next[1], n1);
     __syncthreads();
 }
 
@@ -684,7 +710,7 @@ __device__ void expand_merge_item(const RegionArgs &a, uint32_t it, ItemSmem<WOR
 template <int WORDS>
 union ExpandSmem {
     Smem tile;
-    ItemSmem<WORDS> item;
+    ItemSmem<WORDS, uint32_t> item;
 };
 // Shared counters of an expansion: next-frontier vertices per region, then the
 // edges and the vertices that merge items expanded.
@@ -2298,8 +2324,7 @@ asc_status ensure_pr_buffers(asc_graph *g, size_t elem) {
 // A graph's merge items, made once per workspace.
 uint64_t items_bytes(uint64_t V, uint64_t E) { return sizeof(uint2) * ((V + E + kItem - 1) / kItem + 2); }
 
-asc_status ensure_items(asc_graph *g) {
-    Workspace *ws = g->ws;
+asc_status ensure_items(asc_graph *g, Workspace *ws, cudaStream_t s) {
     if (ws->items) return ASC_OK;
     const uint32_t V = (uint32_t)g->V, S = g->static_vertices;
     // shorter items where a staging buffer is smaller than one (its words, and
@@ -2313,11 +2338,13 @@ asc_status ensure_items(asc_graph *g) {
     ws->n_items_static = (uint32_t)n0;
     ws->n_items = (uint32_t)(n0 + n1);
     const uint64_t blocks = std::min<uint64_t>((n0 + n1) / kBlock + 1, (uint64_t)ws->num_sms * 8);
-    merge_plan_kernel<<<(uint32_t)blocks, kBlock, 0, g->stream>>>(g->d_ptr, S, V, (uint32_t)L, ws->n_items_static,
-                                                                  ws->n_items, ws->items);
+    merge_plan_kernel<<<(uint32_t)blocks, kBlock, 0, s>>>(g->d_ptr, S, V, (uint32_t)L, ws->n_items_static, ws->n_items,
+                                                          ws->items);
     ASC_CUDA(cudaGetLastError());
     return ASC_OK;
 }
+
+asc_status ensure_items(asc_graph *g) { return ensure_items(g, g->ws, g->stream); }
 
 // How PageRank passes report to the host: pass k writes two words of page-locked
 // memory (kPassSlots slots) and an event says when. At most two passes are in
@@ -2431,8 +2458,7 @@ RegionArgs region_args(asc_graph *g, int parity_in, int region, bool dense) {
 // the far set.
 bool near_far(asc_graph *g, asc_algo algo) { return algo == ASC_SSSP && g->ws->tune.delta != 0; }
 
-void attach_items(const asc_graph *g, RegionArgs &a) {
-    const Workspace *ws = g->ws;
+void attach_items(const Workspace *ws, RegionArgs &a) {
     a.items = ws->items;
     a.item_begin = a.region == 0 ? 0 : ws->n_items_static;
     a.item_n = a.region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
@@ -3086,7 +3112,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     if (!part) ASC_TRY(ensure_items(g));
     auto args_of = [&](int parity_in, int region) {
         RegionArgs a = region_args(g, parity_in, region, false);
-        if (!part) attach_items(g, a);
+        if (!part) attach_items(ws, a);
         attach_far(g, algo, a);
         return a;
     };
@@ -3631,7 +3657,8 @@ struct BatchEngine {
     bool sssp = false;
     uint32_t stride = 64;             // SSSP distance row length (sources per row)
     Workspace ws;                     // own frontier lists, bitmaps, counters
-    unsigned long long *visit = nullptr, *front = nullptr, *next = nullptr;
+    unsigned long long *front = nullptr;
+    ulonglong2 *masks = nullptr;      // per vertex: visited (BFS) and next masks, one 16-byte load
     uint32_t *touched = nullptr;      // bitmap of vertices whose next mask went non-zero
     uint32_t *dist = nullptr;         // SSSP [V][stride]
     uint32_t *plane[64] = {nullptr};  // BFS per-slot level planes [V]
@@ -3639,6 +3666,11 @@ struct BatchEngine {
     int32_t *d_lvl_off = nullptr;     // per-slot level offset (level = iteration + offset)
     int32_t lvl_off[64] = {0};
     uint32_t *staging = nullptr;      // SSSP column gather [V]
+    // asc_run_batch copies finished rows out while later iterations run: two
+    // streams, each with 8 gathered SSSP columns, made on first use
+    cudaStream_t out_stream[2] = {nullptr, nullptr};
+    uint32_t *out_rows[2] = {nullptr, nullptr};
+    cudaEvent_t out_ready = nullptr;  // the iteration that finished the rows
     cudaStream_t stream = nullptr;
     int parity = 0;
     uint32_t it = 0;                  // iterations run so far
@@ -3652,9 +3684,9 @@ enum { CTL_ALIVE = 34 };  // u64 (words 34-35): OR of the new frontier masks of 
 
 struct MsArgs {
     RegionArgs r0, r1;            // frontier lists/segments/bitmaps of both regions (val unused)
-    unsigned long long *visit;    // BFS: sources that reached v
     unsigned long long *front;    // sources for which v is in the current frontier
-    unsigned long long *next;     // sources that reached v in this iteration (atomicOr)
+    ulonglong2 *masks;            // per vertex: x sources that reached it (BFS), y those that reached it
+                                  // in this iteration (atomicOr)
     uint32_t *touched;            // bitmap: v's next mask went non-zero this iteration
     uint32_t *work;
     uint32_t *dist;               // SSSP: [V][64]
@@ -3669,25 +3701,31 @@ struct MsSmem {
     uint32_t work;
 };
 
-// BFS relaxation of one edge for a whole mask: true when v's next mask was empty.
-__device__ __forceinline__ bool ms_reach(const MsArgs &m, uint32_t v, unsigned long long f,
-                                         unsigned long long vis) {
-    const unsigned long long nb = f & ~vis;
-    if (!nb) return false;
-    return atomicOr(&m.next[v], nb) == 0ull;
-}
-
-__device__ __forceinline__ void mark_touched(const MsArgs &m, bool first, uint32_t v) {
-    if (first) atomicOr(&m.touched[v >> 5], 1u << (v & 31));
+// BFS relaxation of one edge for a whole mask f; now is the earlier load of v's
+// masks. The atomics are fire-and-forget: a thread that saw an empty next mask
+// marks v as touched (two may), one that saw it set leaves that to whoever set it,
+// and sources already there cost nothing.
+__device__ __forceinline__ void ms_reach(const MsArgs &m, uint32_t v, unsigned long long f, ulonglong2 now) {
+    const unsigned long long nb = f & ~(now.x | now.y);
+    if (!nb) return;
+    atomicOr(&m.masks[v].y, nb);
+    if (!now.y) atomicOr(&m.touched[v >> 5], 1u << (v & 31));
 }
 
 #ifndef ASC_MS_UNROLL
 #define ASC_MS_UNROLL 4
 #endif
 // Edges per thread per pass in the batched BFS expansion (all loads first).
+// Regions walked in id order go by merge items with visited and next masks in one
+// 16-byte load and atomics only for sources not yet there: 64 sources on RMAT
+// scale 21, 3.52 -> 2.4 ms (tiles of 256 vertices and an atomic with a returned
+// value per edge and new source before).
 // 64-source batch, RMAT scale 22 / 24: 5.45 / 18.27 ms at 4 (32 registers, 8
 // CTAs per SM), 5.58 / 18.46 at 6 (40, 6 CTAs), 5.78 / 18.96 at 8 (48, 5 CTAs).
 constexpr int kMsUnroll = ASC_MS_UNROLL;
+#ifndef ASC_MS_BFS_BLOCKS
+#define ASC_MS_BFS_BLOCKS 6
+#endif
 
 template <int WORDS>
 __device__ void ms_vertices(const MsArgs &m, const RegionArgs &a, bool act, uint32_t u, MsSmem &sm) {
@@ -3712,7 +3750,8 @@ __device__ void ms_vertices(const MsArgs &m, const RegionArgs &a, bool act, uint
     const uint32_t nact = __syncthreads_count(act);
     for (uint32_t base = 0; base < total; base += kMsUnroll * kBlock) {
         uint32_t v[kMsUnroll];
-        unsigned long long fk[kMsUnroll], vis[kMsUnroll];
+        unsigned long long fk[kMsUnroll];
+        ulonglong2 now[kMsUnroll];
 #pragma unroll
         for (int k = 0; k < kMsUnroll; k++) {
             const uint32_t e = base + k * kBlock + threadIdx.x;
@@ -3735,9 +3774,9 @@ __device__ void ms_vertices(const MsArgs &m, const RegionArgs &a, bool act, uint
             }
         }
 #pragma unroll
-        for (int k = 0; k < kMsUnroll; k++) vis[k] = fk[k] ? m.visit[v[k]] : ~0ull;
+        for (int k = 0; k < kMsUnroll; k++) now[k] = fk[k] ? m.masks[v[k]] : make_ulonglong2(0, 0);
 #pragma unroll
-        for (int k = 0; k < kMsUnroll; k++) mark_touched(m, ms_reach(m, v[k], fk[k], vis[k]), v[k]);
+        for (int k = 0; k < kMsUnroll; k++) ms_reach(m, v[k], fk[k], now[k]);
     }
     if (threadIdx.x == 0) {
         atomicAdd(&a.stats[a.region], (unsigned long long)total);
@@ -3757,7 +3796,7 @@ __device__ void ms_segment(const MsArgs &m, const RegionArgs &a, uint64_t item) 
     const unsigned long long f = m.front[u];
     for (uint32_t base = 0; base < n; base += kMsUnroll * kBlock) {
         uint32_t v[kMsUnroll];
-        unsigned long long vis[kMsUnroll];
+        ulonglong2 now[kMsUnroll];
         bool ok[kMsUnroll];
 #pragma unroll
         for (int k = 0; k < kMsUnroll; k++) {
@@ -3771,9 +3810,9 @@ __device__ void ms_segment(const MsArgs &m, const RegionArgs &a, uint64_t item) 
             }
         }
 #pragma unroll
-        for (int k = 0; k < kMsUnroll; k++) vis[k] = ok[k] ? m.visit[v[k]] : ~0ull;
+        for (int k = 0; k < kMsUnroll; k++) now[k] = ok[k] ? m.masks[v[k]] : make_ulonglong2(0, 0);
 #pragma unroll
-        for (int k = 0; k < kMsUnroll; k++) mark_touched(m, ok[k] && ms_reach(m, v[k], f, vis[k]), v[k]);
+        for (int k = 0; k < kMsUnroll; k++) ms_reach(m, v[k], ok[k] ? f : 0ull, now[k]);
     }
     if (threadIdx.x == 0) {
         atomicAdd(&a.stats[a.region], (unsigned long long)n);
@@ -3781,34 +3820,88 @@ __device__ void ms_segment(const MsArgs &m, const RegionArgs &a, uint64_t item) 
     }
 }
 
+// A merge item of a region that is walked in id order.
+template <int WORDS>
+__device__ void ms_merge_item(const MsArgs &m, const RegionArgs &a, uint32_t it,
+                              ItemSmem<WORDS, unsigned long long> &sm, uint32_t *counts) {
+    uint32_t ne, bit0;
+    unsigned long long *value;
+    if (!stage_merge_item(a, it, sm, [&](uint32_t u) { return m.front[u]; }, &counts[a.region], &counts[2 + a.region],
+                          ne, bit0, value))
+        return;
+    const uint32_t eb = WORDS == 2 ? 64 : WORDS == 1 ? 32 : a.ebits;
+    const uint32_t mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    const uint32_t x0 = threadIdx.x * kVt;
+    uint32_t act, st;
+    unsigned long long f;
+    if (merge_item_edges(sm, value, ne, x0, act, st, f)) {
+#pragma unroll
+        for (int k0 = 0; k0 < kVt; k0 += kMsUnroll) {
+            uint32_t v[kMsUnroll];
+            unsigned long long fk[kMsUnroll];
+            ulonglong2 now[kMsUnroll];
+#pragma unroll
+            for (int k = 0; k < kMsUnroll; k++) {
+                v[k] = 0;
+                fk[k] = 0;
+                if ((act >> (k0 + k)) & 1u) {
+                    if (k0 + k > 0 && ((st >> (k0 + k)) & 1u)) f = value[sm.row_at[x0 + k0 + k]];
+                    const uint32_t at = bit0 + (x0 + k0 + k) * eb;
+                    v[k] = (WORDS == kBitsLayout ? staged_word(sm.pool, at, mask) : sm.pool[at >> 5]) >> a.wbits;
+                    fk[k] = f;
+                    if (ASC_BAD(v[k] >= m.V, 5, v[k])) {
+                        v[k] = 0;
+                        fk[k] = 0;
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kMsUnroll; k++) now[k] = fk[k] ? m.masks[v[k]] : make_ulonglong2(0, 0);
+#pragma unroll
+            for (int k = 0; k < kMsUnroll; k++) ms_reach(m, v[k], fk[k], now[k]);
+        }
+    }
+    __syncthreads();
+}
+
+template <int WORDS>
+union MsExpandSmem {
+    MsSmem tile;
+    ItemSmem<WORDS, unsigned long long> item;
+};
+
 template <int WORDS>
 __device__ __forceinline__ void ms_item(const MsArgs &m, const RegionArgs &a, uint32_t w, uint32_t n_in,
-                                        uint32_t nseg, bool bitmap, MsSmem &sm) {
+                                        uint32_t nseg, bool bitmap, MsExpandSmem<WORDS> &sm, uint32_t *counts) {
     if (w < nseg) {
         ms_segment<WORDS>(m, a, a.seg_in[w]);
+    } else if (bitmap && a.items) {
+        ms_merge_item<WORDS>(m, a, a.item_begin + w, sm.item, counts);
     } else if (!bitmap) {
         const uint32_t i = (w - nseg) * kBlock + threadIdx.x;
         const bool act = i < n_in;
-        ms_vertices<WORDS>(m, a, act, act ? a.q_in[i] : 0, sm);
+        ms_vertices<WORDS>(m, a, act, act ? a.q_in[i] : 0, sm.tile);
     } else {
         const uint32_t u = (a.dense_begin & ~31u) + (w - nseg) * kBlock + threadIdx.x;
         const bool act = (region_word(a, u & ~31u) >> (u & 31)) & 1u;
-        if (__syncthreads_or(act)) ms_vertices<WORDS>(m, a, act, u, sm);
+        if (__syncthreads_or(act)) ms_vertices<WORDS>(m, a, act, u, sm.tile);
     }
 }
 
 template <int WORDS>
-__global__ void __launch_bounds__(kBlock) ms_bfs_expand_kernel(MsArgs m) {
-    __shared__ MsSmem sm;
+__global__ void __launch_bounds__(kBlock, ASC_MS_BFS_BLOCKS) ms_bfs_expand_kernel(MsArgs m) {
+    __shared__ MsExpandSmem<WORDS> sm;
+    __shared__ uint32_t s_work, counts[4];  // edges, vertices of merge items per region
+    if (threadIdx.x < 4) counts[threadIdx.x] = 0;
     uint32_t n0, s0, i0, n1, s1, i1;
     bool m0, m1;
     region_items_bits(m.r0, n0, s0, i0, m0);
     region_items_bits(m.r1, n1, s1, i1, m1);
     const uint32_t mm = min(i0, i1), total = i0 + i1;
     for (;;) {
-        if (threadIdx.x == 0) sm.work = atomicAdd(m.work, 1u);
+        if (threadIdx.x == 0) s_work = atomicAdd(m.work, 1u);
         __syncthreads();
-        const uint32_t w = sm.work;
+        const uint32_t w = s_work;
         __syncthreads();
         if (w >= total) break;
         bool od;
@@ -3820,9 +3913,11 @@ __global__ void __launch_bounds__(kBlock) ms_bfs_expand_kernel(MsArgs m) {
             od = i1 > i0;
             local = mm + (w - 2 * mm);
         }
-        if (od) ms_item<WORDS>(m, m.r1, local, n1, s1, m1, sm);
-        else ms_item<WORDS>(m, m.r0, local, n0, s0, m0, sm);
+        if (od) ms_item<WORDS>(m, m.r1, local, n1, s1, m1, sm, counts);
+        else ms_item<WORDS>(m, m.r0, local, n0, s0, m0, sm, counts);
     }
+    if (threadIdx.x < 4 && counts[threadIdx.x])
+        atomicAdd(&m.r0.stats[threadIdx.x], (unsigned long long)counts[threadIdx.x]);
 }
 
 // Batched SSSP expansion: one CTA per work item (a tile of frontier vertices,
@@ -3940,7 +4035,7 @@ __device__ __forceinline__ void ms_sssp_lane_quads(const MsArgs &m, uint32_t u, 
         }
     }
     if (imp) {
-        atomicOr(&m.next[v], imp);
+        atomicOr(&m.masks[v].y, imp);
         atomicOr(&m.touched[v >> 5], 1u << (v & 31));
     }
 }
@@ -4007,7 +4102,7 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
             }
         }
         if (imp) {
-            atomicOr(&m.next[v], imp);
+            atomicOr(&m.masks[v].y, imp);
             atomicOr(&m.touched[v >> 5], 1u << (v & 31));
         }
     }
@@ -4078,7 +4173,7 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
 #pragma unroll
             for (int d = G / 2; d > 0; d >>= 1) im |= __shfl_xor_sync(kFull, im, d);
             if (l == 0 && j < nd && im) {
-                atomicOr(&m.next[vk[k]], im);
+                atomicOr(&m.masks[vk[k]].y, im);
                 atomicOr(&m.touched[vk[k] >> 5], 1u << (vk[k] & 31));
             }
         }
@@ -4168,6 +4263,11 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_MIN_BLOCKS) ms_sssp_expand_kern
     }
 }
 
+#ifndef ASC_MS_APPLY_WORDS
+#define ASC_MS_APPLY_WORDS 4
+#endif
+constexpr uint32_t kApplyWords = ASC_MS_APPLY_WORDS;
+
 // Apply pass over the touched bitmap: the new sources of a touched vertex
 // become its frontier mask, BFS levels are written into the
 // sources' planes, and the vertex's bit goes into the next frontier bitmap
@@ -4176,7 +4276,7 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_MIN_BLOCKS) ms_sssp_expand_kern
 template <bool BFS>
 __global__ void ms_apply_kernel(MsArgs m, uint32_t **planes, const int32_t *lvl_off, uint32_t it,
                                 unsigned long long *alive, uint32_t nwords) {
-    // a warp takes 32 touched-bitmap words at a time and walks the non-empty
+    // a warp takes kApplyWords touched-bitmap words at a time and walks the non-empty
     // ones, lane = vertex: the level stores of one source go to 32 consecutive
     // entries of its plane (one coalesced store per source present in the word)
     const RegionArgs &a = m.r0;
@@ -4184,9 +4284,9 @@ __global__ void ms_apply_kernel(MsArgs m, uint32_t **planes, const int32_t *lvl_
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     unsigned long long any = 0;
     uint32_t n0 = 0, n1 = 0;
-    for (uint64_t g0 = (uint64_t)warp * 32; g0 < nwords; g0 += (uint64_t)nwarps * 32) {
+    for (uint64_t g0 = (uint64_t)warp * kApplyWords; g0 < nwords; g0 += (uint64_t)nwarps * kApplyWords) {
         const uint64_t gw = g0 + lane;
-        const uint32_t tw = gw < nwords ? m.touched[gw] : 0u;
+        const uint32_t tw = lane < kApplyWords && gw < nwords ? m.touched[gw] : 0u;
         unsigned nz = __ballot_sync(kFull, tw != 0);
         while (nz) {
             const int j = __ffs(nz) - 1;
@@ -4196,11 +4296,13 @@ __global__ void ms_apply_kernel(MsArgs m, uint32_t **planes, const int32_t *lvl_
             const uint32_t v = 32 * w + lane;
             unsigned long long nb = 0;
             if ((word >> lane) & 1u) {
-                nb = m.next[v];
-                m.next[v] = 0;
                 if (BFS) {
-                    nb &= ~m.visit[v];
-                    m.visit[v] |= nb;
+                    const ulonglong2 now = m.masks[v];
+                    nb = now.y & ~now.x;
+                    m.masks[v] = make_ulonglong2(now.x | nb, 0);
+                } else {
+                    nb = m.masks[v].y;
+                    m.masks[v].y = 0;
                 }
                 m.front[v] = nb;
                 any |= nb;
@@ -4247,7 +4349,7 @@ struct Admit {
 // Resets the per-slot state of newly admitted slots: BFS clears their bits in
 // every visited mask and fills their level planes, SSSP resets their distance
 // columns.
-__global__ void cb_clear_kernel(unsigned long long *visit, uint32_t *dist, uint32_t stride, uint32_t **planes,
+__global__ void cb_clear_kernel(ulonglong2 *masks, uint32_t *dist, uint32_t stride, uint32_t **planes,
                                 unsigned long long newmask, uint32_t V, uint32_t fill, uint32_t sssp) {
     if (sssp) {
         // stride / 4 lanes per distance row (16 for 64 sources): lane l owns
@@ -4274,7 +4376,7 @@ __global__ void cb_clear_kernel(unsigned long long *visit, uint32_t *dist, uint3
     }
     for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
         unsigned long long t = newmask;
-        visit[v] &= ~newmask;
+        masks[v].x &= ~newmask;
         while (t) {
             const int s = __ffsll((long long)t) - 1;
             t &= t - 1;
@@ -4306,7 +4408,7 @@ __global__ void cb_admit_kernel(Admit ad, MsArgs m, RegionArgs cur, uint32_t **p
     const unsigned long long bit = 1ull << s;
     if (sssp) m.dist[(uint64_t)v * stride + s] = 1;
     else {
-        atomicOr(&m.visit[v], bit);
+        atomicOr(&m.masks[v].x, bit);
         planes[s][v] = 1;
     }
     atomicOr(&m.front[v], bit);
@@ -4333,11 +4435,27 @@ __global__ void cb_gather_column_kernel(const uint32_t *dist, uint32_t stride, u
         out[v] = dist[(uint64_t)v * stride + s];
 }
 
+// Columns 8 * group .. + 7 of the distance rows whose bits are set in cols, as
+// rows of V values each: a thread reads a vertex's 32 bytes (one sector), and
+// each column's stores are consecutive.
+__global__ void cb_gather_columns_kernel(const uint32_t *dist, uint32_t stride, uint32_t group, uint32_t cols,
+                                         uint32_t *out, uint32_t V) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(dist + (uint64_t)v * stride + 8 * group);
+        const uint4 a = p[0], b = p[1];
+        const uint32_t x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if ((cols >> k) & 1u) out[(uint64_t)k * V + v] = x[k];
+    }
+}
+
 }  // namespace
 
 uint64_t batch_state_bytes(asc_graph *g, bool sssp, uint32_t stride) {
     const uint64_t V = g->V;
     uint64_t b = 24 * V + 4 * (V / 32 + 2) + 16 * V + 4 * 4 * (V / 32 + 2) + 8 * (g->E / 256 + 1024) + 4096;
+    if (!sssp) b += items_bytes(V, g->E);
     if (sssp) b += 4ull * V * stride + 4 * V;
     return b;
 }
@@ -4394,11 +4512,19 @@ void batch_destroy(BatchEngine *b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     free_ws_buffers(&b->ws);
-    for (void *p : {(void *)b->visit, (void *)b->front, (void *)b->next, (void *)b->touched, (void *)b->dist,
+    for (void *p : {(void *)b->masks, (void *)b->front, (void *)b->touched, (void *)b->dist,
                     (void *)b->d_plane, (void *)b->d_lvl_off, (void *)b->staging})
         if (p) cudaFree(p);
     for (auto p : b->plane)
         if (p) cudaFree(p);
+    for (int i = 0; i < 2; i++) {
+        if (b->out_stream[i]) {
+            cudaStreamSynchronize(b->out_stream[i]);
+            cudaStreamDestroy(b->out_stream[i]);
+        }
+        if (b->out_rows[i]) cudaFree(b->out_rows[i]);
+    }
+    if (b->out_ready) cudaEventDestroy(b->out_ready);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }
@@ -4421,9 +4547,8 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
         cudaError_t e = cudaMalloc(p, n ? n : 16);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
     };
-    al((void **)&b->visit, 8 * V);
+    al((void **)&b->masks, 16 * V);
     al((void **)&b->front, 8 * V);
-    al((void **)&b->next, 8 * V);
     al((void **)&b->touched, 4 * (V / 32 + 2));
     al((void **)&b->d_plane, 8 * 64);
     al((void **)&b->d_lvl_off, 4 * 64);
@@ -4435,15 +4560,15 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
         cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) st = cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
+    if (st == ASC_OK && !sssp) st = ensure_items(g, &b->ws, b->stream);
     // empty start state: no frontier, zero masks
     if (st == ASC_OK) {
         cudaError_t e = cudaMemsetAsync(b->ws.ctl, 0, 4 * CTL_WORDS, b->stream);
         for (int i = 0; i < 2 && e == cudaSuccess; i++)
             e = cudaMemsetAsync(b->ws.bitmap[i], 0, 4 * (V / 32 + 2), b->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->touched, 0, 4 * (V / 32 + 2), b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->visit, 0, 8 * V, b->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(b->masks, 0, 16 * V, b->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->front, 0, 8 * V, b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->next, 0, 8 * V, b->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(b->d_plane, 0, 8 * 64, b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "batch init", __FILE__, __LINE__);
@@ -4494,9 +4619,8 @@ asc_status batch_launch(BatchEngine *b) {
     const int p = b->parity, po = 1 - p;
     MsArgs m;
     memset(&m, 0, sizeof(m));
-    m.visit = b->visit;
     m.front = b->front;
-    m.next = b->next;
+    m.masks = b->masks;
     m.touched = b->touched;
     m.dist = b->dist;
     m.V = V;
@@ -4512,7 +4636,7 @@ asc_status batch_launch(BatchEngine *b) {
             b->lvl_off[ad.slot[i]] = 2 - (int32_t)(b->it + 1);  // found in the next iteration: level 2
         }
         ASC_CUDA(cudaMemcpyAsync(b->d_lvl_off, b->lvl_off, 4 * 64, cudaMemcpyHostToDevice, s));
-        cb_clear_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>(b->visit, b->dist, b->stride, b->d_plane, newmask, V, V + 1,
+        cb_clear_kernel<<<fill_grid(ws, V), kBlock, 0, s>>>(b->masks, b->dist, b->stride, b->d_plane, newmask, V, V + 1,
                                                              b->sssp ? 1 : 0);
         RegionArgs cur = base_args(g, ws, 1 - p);  // the lists/bitmap/counts of parity p (this iteration's input)
         cb_admit_reset_kernel<<<1, 64, 0, s>>>(ad, b->front, ws->bitmap[p]);
@@ -4527,7 +4651,11 @@ asc_status batch_launch(BatchEngine *b) {
     m.r0 = region_args(g, ws, p, 0, false);
     m.r1 = region_args(g, ws, p, 1, false);
     m.work = m.r0.cnt_out + 4;
-    const uint32_t grid = (uint32_t)(ws->num_sms * ws->tune.ctas_per_sm);
+    if (!b->sssp) {
+        attach_items(ws, m.r0);
+        attach_items(ws, m.r1);
+    }
+    const uint32_t grid = (uint32_t)(ws->num_sms * (b->sssp ? ws->tune.ctas_per_sm : ASC_MS_BFS_BLOCKS));
     b->it++;
     if (b->sssp && b->stride == 16) ms_sssp_expand_kernel<16><<<grid, kBlock, 0, s>>>(m);
     else if (b->sssp && b->stride == 32) ms_sssp_expand_kernel<32><<<grid, kBlock, 0, s>>>(m);
@@ -4535,9 +4663,9 @@ asc_status batch_launch(BatchEngine *b) {
     else if (g->edge_words == 2) ms_bfs_expand_kernel<2><<<grid, kBlock, 0, s>>>(m);
     else if (g->ebits < 32) ms_bfs_expand_kernel<kBitsLayout><<<grid, kBlock, 0, s>>>(m);
     else ms_bfs_expand_kernel<1><<<grid, kBlock, 0, s>>>(m);
-    if (b->sssp) ms_apply_kernel<false><<<fill_grid(ws, nwords), kBlock, 0, s>>>(m, b->d_plane, b->d_lvl_off, b->it,
+    if (b->sssp) ms_apply_kernel<false><<<fill_grid(ws, 32ull * nwords / kApplyWords), kBlock, 0, s>>>(m, b->d_plane, b->d_lvl_off, b->it,
                                                                                alive, nwords);
-    else ms_apply_kernel<true><<<fill_grid(ws, nwords), kBlock, 0, s>>>(m, b->d_plane, b->d_lvl_off, b->it, alive,
+    else ms_apply_kernel<true><<<fill_grid(ws, 32ull * nwords / kApplyWords), kBlock, 0, s>>>(m, b->d_plane, b->d_lvl_off, b->it, alive,
                                                                         nwords);
     build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(m.r0, ws->bitmap[po], nwords);
     ASC_CUDA(cudaGetLastError());
@@ -4573,6 +4701,46 @@ asc_status batch_fetch(BatchEngine *b, uint32_t slot, void *out, bool device_out
     return ASC_OK;
 }
 
+// Starts copying the rows of the finished slots to out (row i of a slot i) on the
+// engine's output streams, after what its own stream holds so far: their values
+// are final, and later iterations leave them alone. Groups of 8 slots alternate
+// between the streams, so the gather of one overlaps the copy of another.
+asc_status batch_copy_rows(BatchEngine *b, uint64_t slots, uint32_t *out, bool device_out) {
+    const uint64_t V = b->g->V;
+    const cudaMemcpyKind kind = device_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    if (!b->out_ready) ASC_CUDA(cudaEventCreateWithFlags(&b->out_ready, cudaEventDisableTiming));
+    ASC_CUDA(cudaEventRecord(b->out_ready, b->stream));
+    for (uint32_t group = 0; group < 8; group++) {
+        uint32_t cols = (uint32_t)(slots >> (8 * group)) & 0xffu;
+        if (!cols) continue;
+        const int i = group & 1;
+        if (!b->out_stream[i]) ASC_CUDA(cudaStreamCreateWithFlags(&b->out_stream[i], cudaStreamNonBlocking));
+        if (b->sssp && !b->out_rows[i]) ASC_CUDA(cudaMalloc((void **)&b->out_rows[i], 32 * V));
+        cudaStream_t s = b->out_stream[i];
+        ASC_CUDA(cudaStreamWaitEvent(s, b->out_ready, 0));
+        if (b->sssp) {
+            cb_gather_columns_kernel<<<fill_grid(&b->ws, V), kBlock, 0, s>>>(b->dist, b->stride, group, cols,
+                                                                              b->out_rows[i], (uint32_t)V);
+            ASC_CUDA(cudaGetLastError());
+        }
+        while (cols) {
+            const uint32_t first = __builtin_ctz(cols);
+            const uint32_t run = b->sssp ? __builtin_ctz(~(cols >> first)) : 1;  // gathered rows are consecutive
+            const uint32_t slot = 8 * group + first;
+            ASC_CUDA(cudaMemcpyAsync(out + slot * V, b->sssp ? b->out_rows[i] + first * V : b->plane[slot],
+                                     4 * V * run, kind, s));
+            cols &= ~(((1u << run) - 1u) << first);
+        }
+    }
+    return ASC_OK;
+}
+
+asc_status batch_finish_rows(BatchEngine *b) {
+    for (auto s : b->out_stream)
+        if (s) ASC_CUDA(cudaStreamSynchronize(s));
+    return ASC_OK;
+}
+
 // asc_run_batch: all n sources fill slots 0..n-1 of the graph's own batch
 // engine (kept for later batches), then iterations run until every source is
 // done; each finished slot's values are copied to row i of out.
@@ -4590,38 +4758,32 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
     for (uint32_t i = 0; i < n; i++) ASC_TRY(batch_admit(b, i, sources[i]));
     const uint32_t it0 = b->it;
     const int64_t cap = p.max_iterations > 0 ? p.max_iterations : (int64_t)4 * V + 64;
-    uint64_t done = 0;
     const bool want = out && !(p.flags & ASC_RUN_NO_OUTPUT);
-    double copy_ms = 0;
+    std::chrono::steady_clock::time_point done;  // the last iteration's end, on the host
     while (b->active) {
         if ((int64_t)(b->it - it0) >= cap) {
             // drop the unfinished slots so the engine is reusable
             b->active = 0;
+            ASC_TRY(batch_finish_rows(b));
             return fail(ASC_ERR_TIMEOUT, "batch has no fixpoint after %u iterations", b->it - it0);
         }
-        ASC_TRY(batch_launch(b));
+        asc_status rc = batch_launch(b);
         uint64_t fin = 0;
-        ASC_TRY(batch_collect(b, &fin));
-        done |= fin;
-        if (want) {
-            cudaEvent_t e0 = ws->ev[2], e1 = ws->ev[3];
-            ASC_CUDA(cudaEventRecord(e0, s));
-            while (fin) {
-                const uint32_t slot = __builtin_ctzll(fin);
-                fin &= fin - 1;
-                ASC_TRY(batch_fetch(b, slot, (uint32_t *)out + (uint64_t)slot * V,
-                                    (p.flags & ASC_RUN_DEVICE_OUT) != 0));
-            }
-            ASC_CUDA(cudaEventRecord(e1, s));
-            ASC_CUDA(cudaEventSynchronize(e1));
-            float ms = 0;
-            ASC_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            copy_ms += ms;
+        if (rc == ASC_OK) rc = batch_collect(b, &fin);
+        ASC_CUDA(cudaEventRecord(ws->ev[1], s));
+        done = std::chrono::steady_clock::now();
+        if (rc == ASC_OK && want && fin)
+            rc = batch_copy_rows(b, fin, (uint32_t *)out, (p.flags & ASC_RUN_DEVICE_OUT) != 0);
+        if (rc != ASC_OK) {
+            batch_finish_rows(b);  // no copy into the caller's buffer outlives the call
+            return rc;
         }
     }
-    ASC_CUDA(cudaEventRecord(ws->ev[1], s));
     ASC_CUDA(cudaMemcpyAsync(b->ws.h_ctl + CTL_STATS, b->ws.ctl + CTL_STATS, 8 * 6, cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
+    ASC_TRY(batch_finish_rows(b));
+    const double copy_ms =
+        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - done).count();
     if (st) {
         memset(st, 0, sizeof(*st));
         const unsigned long long *hs = (const unsigned long long *)(b->ws.h_ctl + CTL_STATS);
@@ -4633,7 +4795,7 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
         st->ondemand_vertices = hs[3];
         float ms = 0;
         ASC_CUDA(cudaEventElapsedTime(&ms, ws->ev[0], ws->ev[1]));
-        st->ms_total = ms - copy_ms;
+        st->ms_total = ms;
         st->ms_copyout = copy_ms;
         st->kernel_launches = (uint32_t)(4 * (b->it - it0) + 3);
     }
