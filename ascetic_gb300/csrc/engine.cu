@@ -843,19 +843,65 @@ constexpr int kBuWords = ASC_BU_WORDS;
 #endif
 constexpr int kBuMinBlocks = ASC_BU_MIN_BLOCKS;
 
+// Vertices whose first in-edge is no parent wait in a queue per warp until 32 of
+// them scan their further in-edges together (in_ptr, then host memory): such a
+// vertex costs a chain of three dependent reads, and a word of 32 vertices holds
+// only a few.
 struct BuSmem {
-    unsigned long long scanned, examined;
+    uint32_t queue[kWarps][32 + 32 * kBuWords];
 };
 
-__device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nwords, BuSmem &bs, uint32_t *s_next) {
-    if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
-    if (threadIdx.x == 0) bs.scanned = bs.examined = 0;
+// The further in-edges of up to 32 queued vertices (lanes below n). Returns
+// whether this lane's was found.
+__device__ __forceinline__ bool bottom_up_scan(const RegionArgs &a, const uint32_t *queue, uint32_t n, uint32_t nv,
+                                               uint32_t &v, uint32_t &scanned) {
+    const uint32_t lane = threadIdx.x & 31;
+    bool found = false;
+    v = 0;
+    if (lane < n) {
+        v = queue[lane];
+        uint32_t i = a.in_ptr[v];
+        const uint32_t e = a.in_ptr[v + 1];
+        if (a.in_heads && i < e) i++;  // the head was the first
+        for (; i < e && !found; i += kBuUnroll) {
+            uint32_t u[kBuUnroll];
+            bool in[kBuUnroll];
+#pragma unroll
+            for (int q = 0; q < kBuUnroll; q++) {
+                u[q] = i + q < e ? edge_word(a.in_edges, (uint64_t)i + q, a.in_ebits) : 0xffffffffu;
+                if (u[q] != 0xffffffffu && ASC_BAD(u[q] >= a.V, 17, u[q])) u[q] = 0xffffffffu;
+            }
+#pragma unroll
+            for (int q = 0; q < kBuUnroll; q++)
+                in[q] = u[q] != 0xffffffffu && ((a.bitmap_in[u[q] >> 5] >> (u[q] & 31)) & 1u);
+            // edges read count up to the parent
+#pragma unroll
+            for (int q = 0; q < kBuUnroll; q++)
+                if (!found && i + q < e) {
+                    scanned++;
+                    found = in[q];
+                }
+        }
+        if (found) {
+            a.val[v] = nv;
+            atomicOr(&a.visited[v >> 5], 1u << (v & 31));
+            atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+        }
+    }
+    return found;
+}
+
+// nv: the value of a vertex found in this step (every frontier vertex holds
+// nv - 1: the loop is level-synchronous).
+__device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nwords, uint32_t nv, BuSmem &bs,
+                                                uint32_t *s_next) {
+    if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = gridDim.x * (kBlock / 32);
-    unsigned long long scanned = 0, examined = 0;
-    for (uint32_t w0 = kBuWords * (blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5)); w0 < nwords;
-         w0 += kBuWords * warps) {
+    const uint32_t warps = gridDim.x * kWarps;
+    uint32_t *queue = bs.queue[threadIdx.x >> 5];
+    uint32_t waiting = 0, scanned = 0, examined = 0, n0 = 0, n1 = 0;
+    for (uint32_t w0 = kBuWords * (blockIdx.x * kWarps + (threadIdx.x >> 5)); w0 < nwords; w0 += kBuWords * warps) {
         // vertices without in-edges can never be reached: about half of an
         // RMAT graph, nearly all of its unreachable vertices
         uint32_t vis[kBuWords], done[kBuWords];
@@ -885,78 +931,63 @@ __device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nw
             if (done[k] == 0xffffffffu) continue;  // the whole warp: nothing to look for in this word
             const uint32_t w = w0 + k, v = 32 * w + lane;
             examined += todo[k];
-            uint32_t parent = hit[k] ? head[k] : 0xffffffffu;
-            uint32_t h = 0, e = 0;
-            if (todo[k] && !hit[k]) {
-                h = a.in_ptr[v];
-                e = a.in_ptr[v + 1];
-                if (a.in_heads && h < e) h++;  // the head was in-edge h
+            const unsigned found = __ballot_sync(kFull, hit[k]);
+            if (hit[k]) {
+                a.val[v] = nv;
+                n0 += v < a.S;
+                n1 += v >= a.S;
             }
-            if (parent == 0xffffffffu) {
-                for (uint32_t i = h; i < e; i += kBuUnroll) {
-                    uint32_t u[kBuUnroll];
-                    bool in[kBuUnroll];
-#pragma unroll
-                    for (int q = 0; q < kBuUnroll; q++) {
-                        u[q] = i + q < e ? edge_word(a.in_edges, (uint64_t)i + q, a.in_ebits) : 0xffffffffu;
-                        if (u[q] != 0xffffffffu && ASC_BAD(u[q] >= a.V, 17, u[q])) u[q] = 0xffffffffu;
-                    }
-#pragma unroll
-                    for (int q = 0; q < kBuUnroll; q++)
-                        in[q] = u[q] != 0xffffffffu && ((a.bitmap_in[u[q] >> 5] >> (u[q] & 31)) & 1u);
-                    int at = -1;
-#pragma unroll
-                    for (int q = kBuUnroll - 1; q >= 0; q--)
-                        if (in[q]) at = q;
-                    if (at >= 0) {
-                        parent = u[at];
-                        scanned += (i - h) + (uint32_t)at + 1;
-                        break;
-                    }
-                }
-                if (parent == 0xffffffffu) scanned += e - h;
-            }
-            const bool won = parent != 0xffffffffu;
-            const unsigned found = __ballot_sync(kFull, won);
-            // every frontier vertex holds the same value (the step is level-
-            // synchronous): one lane reads its parent's, the warp shares it
-            uint32_t nv = 0;
-            if (found) {
-                const int leader = __ffs(found) - 1;
-                if ((int)lane == leader) nv = a.val[parent] + 1;
-                nv = __shfl_sync(kFull, nv, leader);
-            }
-            if (won) a.val[v] = nv;
             if (lane == 0 && found) {
                 a.visited[w] = vis[k] | found;
                 a.bitmap[w] = found;
             }
-            count_next(a, won, v, s_next);
+            const bool miss = todo[k] && !hit[k];
+            const unsigned missed = __ballot_sync(kFull, miss);
+            if (miss) queue[waiting + __popc(missed & ((1u << lane) - 1u))] = v;
+            waiting += __popc(missed);
+        }
+        __syncwarp();  // the queue, and this word's bits before later ones are added
+        while (waiting >= 32) {
+            waiting -= 32;
+            uint32_t v;
+            const bool found = bottom_up_scan(a, queue + waiting, 32, nv, v, scanned);
+            n0 += found && v < a.S;
+            n1 += found && v >= a.S;
+            __syncwarp();
         }
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        scanned += __shfl_down_sync(kFull, scanned, d);
-        examined += __shfl_down_sync(kFull, examined, d);
+    if (waiting) {
+        uint32_t v;
+        const bool found = bottom_up_scan(a, queue, waiting, nv, v, scanned);
+        n0 += found && v < a.S;
+        n1 += found && v >= a.S;
     }
-    if (lane == 0 && scanned) atomicAdd(&bs.scanned, scanned);
-    if (lane == 0 && examined) atomicAdd(&bs.examined, examined);
+    n0 = __reduce_add_sync(kFull, n0);
+    n1 = __reduce_add_sync(kFull, n1);
+    scanned = __reduce_add_sync(kFull, scanned);
+    examined = __reduce_add_sync(kFull, examined);
+    if (lane == 0) {
+        if (n0) atomicAdd(&s_next[0], n0);
+        if (n1) atomicAdd(&s_next[1], n1);
+        if (scanned) atomicAdd(&s_next[2], scanned);
+        if (examined) atomicAdd(&s_next[3], examined);
+    }
     flush_next(a, s_next);
-    if (threadIdx.x == 0 && bs.examined)
-        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_VERTS - CTL_STATS) / 2), bs.examined);
+    if (threadIdx.x == 0 && s_next[3])
+        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_VERTS - CTL_STATS) / 2), (unsigned long long)s_next[3]);
     // in-edges are read in place from host memory (resident only on a graph
     // without a cap): the run's on-demand edges and its bottom-up edges
-    if (threadIdx.x == 0 && bs.scanned) {
-        atomicAdd(&a.stats[a.in_resident ? 0 : 1], bs.scanned);
-        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_EDGES - CTL_STATS) / 2), bs.scanned);
+    if (threadIdx.x == 0 && s_next[2]) {
+        atomicAdd(&a.stats[a.in_resident ? 0 : 1], (unsigned long long)s_next[2]);
+        atomicAdd((unsigned long long *)(a.stats + (CTL_BU_EDGES - CTL_STATS) / 2), (unsigned long long)s_next[2]);
     }
 }
 
-__global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionArgs a, uint32_t nwords) {
+__global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionArgs a, uint32_t nwords, uint32_t nv) {
     if (!bottom_up_step(a)) return;
-    __shared__ uint32_t s_next[2];
+    __shared__ uint32_t s_next[kNextWords];
     __shared__ BuSmem bs;
-    bottom_up_words(a, nwords, bs, s_next);
+    bottom_up_words(a, nwords, nv, bs, s_next);
 }
 
 // Gather-and-copy comparison engine: expands on-demand edges that host
@@ -1434,9 +1465,15 @@ enum LoopNext { kLoopGo, kLoopEnd, kLoopStuck };
 
 // One iteration from the frontier that x reads; y's arguments write that
 // frontier's lists (the other parity).
+template <int WORDS>
+union LoopSmem {
+    ExpandSmem<WORDS> expand;
+    BuSmem bottom_up;
+};
+
 template <int ALG, int WORDS>
 __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const FusedArgs &x, const FusedArgs &y,
-                                                   LoopState &st, ExpandSmem<WORDS> &sm, BuSmem &bs, uint32_t *s_next) {
+                                                   LoopState &st, LoopSmem<WORDS> &sm, uint32_t *s_next) {
     const RegionArgs &a = x.r0;
     volatile const uint32_t *cin = a.cnt_in;
     if (ALG == kCC && l.first_label && !st.promotions && (!(cin[6] | cin[7]) || st.it >= l.first_cap)) {
@@ -1490,8 +1527,8 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
         return kLoopEnd;
     }
     st.it++;
-    if (ALG == kBFS && bottom_up_step(a)) bottom_up_words(a, l.nwords, bs, s_next);
-    else expand_regions<ALG, WORDS>(x, st.thresh, sm, s_next);
+    if (ALG == kBFS && bottom_up_step(a)) bottom_up_words(a, l.nwords, st.it + 1, sm.bottom_up, s_next);
+    else expand_regions<ALG, WORDS>(x, st.thresh, sm.expand, s_next);
     if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
     build_frontier(a, a.bitmap, l.nwords, a.cnt_out[6], a.cnt_out[7]);
     // the input frontier's bitmap and counts are the next output's
@@ -1503,8 +1540,7 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
 
 template <int ALG, int WORDS>
 __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const __grid_constant__ LoopArgs l) {
-    __shared__ ExpandSmem<WORDS> sm;
-    __shared__ BuSmem bs;
+    __shared__ LoopSmem<WORDS> sm;
     __shared__ uint32_t s_next[kNextWords];
     LoopState st;
     st.thresh = l.thresh;
@@ -1515,8 +1551,8 @@ __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const
         if (!grid_barrier(l.ctl, st.target)) return;
     }
     for (;;) {
-        LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, bs, s_next);
-        if (n == kLoopGo) n = loop_iteration<ALG, WORDS>(l, l.x1, l.x0, st, sm, bs, s_next);
+        LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, s_next);
+        if (n == kLoopGo) n = loop_iteration<ALG, WORDS>(l, l.x1, l.x0, st, sm, s_next);
         if (n == kLoopStuck) return;
         if (n == kLoopEnd) break;
     }
@@ -3286,7 +3322,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             RegionArgs a = args_of(parity, 0);
             ASC_TRY(pt.begin(2));
             pt.record(s);
-            bottom_up_kernel<<<bu_grid(ws, nwords), kBlock, 0, s>>>(a, nwords);
+            bottom_up_kernel<<<bu_grid(ws, nwords), kBlock, 0, s>>>(a, nwords, iters + 1);
             pt.record(s);
             launches++;
         } else if (pt.on) {
@@ -3312,7 +3348,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             fused(s, x, grid_for(ws, items));
             launches++;
             if (algo == ASC_BFS && x.r0.in_ptr) {
-                bottom_up_kernel<<<bu_grid(ws, nwords), kBlock, 0, s>>>(x.r0, nwords);
+                bottom_up_kernel<<<bu_grid(ws, nwords), kBlock, 0, s>>>(x.r0, nwords, iters + 1);
                 launches++;
             }
         }
@@ -3994,6 +4030,33 @@ __device__ __forceinline__ void ms_sssp_load_edge(const RegionArgs &a, uint64_t 
     }
 }
 
+// Lowers *p to nd when cur, loaded earlier, is larger, and then sets bit in imp:
+// a compare and two predicated instructions. Fire-and-forget: a value lowered
+// further meanwhile is marked all the same, which costs at most one more
+// relaxation. Callers need not test which of a row's sources are active: an
+// inactive source's value at u has not changed since it relaxed this edge, so it
+// does not improve v (715 M warp instructions with those tests and a branch per
+// source on 16.8 M edges of 64 sources, 60% of the issue slots; bound by them).
+__device__ __forceinline__ void relax_min(uint32_t *p, uint32_t nd, uint32_t cur, uint32_t &imp, uint32_t bit) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.lt.u32 q, %2, %3;\n\t"
+        "@q red.relaxed.gpu.global.min.u32 [%1], %2;\n\t"
+        "@q or.b32 %0, %0, %4;\n\t}"
+        : "+r"(imp)
+        : "l"(p), "r"(nd), "r"(cur), "r"(bit)
+        : "memory");
+}
+
+// Marks v as reached for the sources in imp: 32-bit halves, as every atomic of
+// the batched SSSP on these masks.
+__device__ __forceinline__ void ms_sssp_mark(const MsArgs &m, uint32_t v, unsigned long long imp) {
+    uint32_t *next = reinterpret_cast<uint32_t *>(&m.masks[v].y);
+    if ((uint32_t)imp) atomicOr(next, (uint32_t)imp);
+    if ((uint32_t)(imp >> 32)) atomicOr(next + 1, (uint32_t)(imp >> 32));
+    atomicOr(&m.touched[v >> 5], 1u << (v & 31));
+}
+
 // Relaxes one edge (u -> v, weight w) for the sources in f, lane-per-edge:
 // the lane reads the two distance rows a 16-byte quad (four sources) at a
 // time, only the quads with an active source, kMsQuads quads in flight.
@@ -4023,21 +4086,16 @@ __device__ __forceinline__ void ms_sssp_lane_quads(const MsArgs &m, uint32_t u, 
 #pragma unroll
         for (int k = 0; k < kMsQuads; k++) {
             if (qx[k] < 0) continue;
-            const uint32_t a4 = (uint32_t)(f >> (4 * qx[k])) & 0xfu;
             uint32_t *r = vrow + 4 * qx[k];
-            const uint32_t n0 = du[k].x + w, n1 = du[k].y + w, n2 = du[k].z + w, n3 = du[k].w + w;
             uint32_t bits = 0;
-            if ((a4 & 1u) && n0 < cur[k].x) { atomicMin(r + 0, n0); bits |= 1u; }
-            if ((a4 & 2u) && n1 < cur[k].y) { atomicMin(r + 1, n1); bits |= 2u; }
-            if ((a4 & 4u) && n2 < cur[k].z) { atomicMin(r + 2, n2); bits |= 4u; }
-            if ((a4 & 8u) && n3 < cur[k].w) { atomicMin(r + 3, n3); bits |= 8u; }
+            relax_min(r + 0, du[k].x + w, cur[k].x, bits, 1u);
+            relax_min(r + 1, du[k].y + w, cur[k].y, bits, 2u);
+            relax_min(r + 2, du[k].z + w, cur[k].z, bits, 4u);
+            relax_min(r + 3, du[k].w + w, cur[k].w, bits, 8u);
             imp |= (unsigned long long)bits << (4 * qx[k]);
         }
     }
-    if (imp) {
-        atomicOr(&m.masks[v].y, imp);
-        atomicOr(&m.touched[v >> 5], 1u << (v & 31));
-    }
+    if (imp) ms_sssp_mark(m, v, imp);
 }
 
 // One warp relaxes 32 consecutive edges of the tile's flattened edge range
@@ -4101,10 +4159,7 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
                 }
             }
         }
-        if (imp) {
-            atomicOr(&m.masks[v].y, imp);
-            atomicOr(&m.touched[v >> 5], 1u << (v & 31));
-        }
+        if (imp) ms_sssp_mark(m, v, imp);
     }
     if (ok && mid) ms_sssp_lane_quads<R>(m, sm.vid[o], v, w, f);
     const uint32_t dm = __ballot_sync(kFull, ok && dense);
@@ -4158,22 +4213,19 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
                 uint32_t *row = m.dist + (uint64_t)vk[k] * R + S * l;
 #pragma unroll
                 for (int q = 0; q < Q; q++) {
-                    const uint32_t n0 = du[k][q].x + wk[k], n1 = du[k][q].y + wk[k];
-                    const uint32_t n2 = du[k][q].z + wk[k], n3 = du[k][q].w + wk[k];
-                    const uint32_t a4 = act[k] >> (4 * q);
-                    uint32_t *r = row + 4 * q;
-                    if ((a4 & 1u) && n0 < cur[k][q].x) { atomicMin(r + 0, n0); imp |= 1u << (4 * q); }
-                    if ((a4 & 2u) && n1 < cur[k][q].y) { atomicMin(r + 1, n1); imp |= 2u << (4 * q); }
-                    if ((a4 & 4u) && n2 < cur[k][q].z) { atomicMin(r + 2, n2); imp |= 4u << (4 * q); }
-                    if ((a4 & 8u) && n3 < cur[k][q].w) { atomicMin(r + 3, n3); imp |= 8u << (4 * q); }
+                    relax_min(row + 4 * q + 0, du[k][q].x + wk[k], cur[k][q].x, imp, 1u << (4 * q));
+                    relax_min(row + 4 * q + 1, du[k][q].y + wk[k], cur[k][q].y, imp, 2u << (4 * q));
+                    relax_min(row + 4 * q + 2, du[k][q].z + wk[k], cur[k][q].z, imp, 4u << (4 * q));
+                    relax_min(row + 4 * q + 3, du[k][q].w + wk[k], cur[k][q].w, imp, 8u << (4 * q));
                 }
             }
-            // the group's improved sources as one 64-bit mask
-            unsigned long long im = (unsigned long long)imp << (S * l);
+            // the improved sources of the H lanes that share a 32-bit half
+            constexpr int H = 32 / S < G ? 32 / S : G;
+            uint32_t im = imp << (S * (l % H));
 #pragma unroll
-            for (int d = G / 2; d > 0; d >>= 1) im |= __shfl_xor_sync(kFull, im, d);
-            if (l == 0 && j < nd && im) {
-                atomicOr(&m.masks[vk[k]].y, im);
+            for (int d = H / 2; d > 0; d >>= 1) im |= __shfl_xor_sync(kFull, im, d);
+            if (l % H == 0 && j < nd && im) {
+                atomicOr(reinterpret_cast<uint32_t *>(&m.masks[vk[k]].y) + l / H, im);
                 atomicOr(&m.touched[vk[k] >> 5], 1u << (vk[k] & 31));
             }
         }
@@ -4610,6 +4662,12 @@ uint32_t batch_slots(const BatchEngine *b) { return b->sssp ? b->stride : 64u; }
 
 // Applies the queued admissions and launches one iteration on the batch's
 // stream, ending with the readback of its counts (nothing waits here).
+namespace {
+// The sources still alive, to page-locked memory: a copy would queue behind the
+// rows that asc_run_batch copies out meanwhile.
+__global__ void report_alive_kernel(const unsigned long long *alive, unsigned long long *report) { *report = *alive; }
+}  // namespace
+
 asc_status batch_launch(BatchEngine *b) {
     asc_graph *g = b->g;
     Workspace *ws = &b->ws;
@@ -4669,7 +4727,8 @@ asc_status batch_launch(BatchEngine *b) {
                                                                         nwords);
     build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(m.r0, ws->bitmap[po], nwords);
     ASC_CUDA(cudaGetLastError());
-    ASC_CUDA(cudaMemcpyAsync(ws->h_ctl + CTL_ALIVE, alive, 8, cudaMemcpyDeviceToHost, s));
+    report_alive_kernel<<<1, 1, 0, s>>>(alive, (unsigned long long *)(ws->h_ctl + CTL_ALIVE));
+    ASC_CUDA(cudaGetLastError());
     b->parity = po;
     return ASC_OK;
 }
