@@ -846,7 +846,7 @@ constexpr int kBuMinBlocks = ASC_BU_MIN_BLOCKS;
 // Vertices whose first in-edge is no parent wait in a queue per warp until 32 of
 // them scan their further in-edges together (in_ptr, then host memory): such a
 // vertex costs a chain of three dependent reads, and a word of 32 vertices holds
-// only a few.
+// only a few (BFS on RMAT scale 24: 651 us a word at a time, 575 queued).
 struct BuSmem {
     uint32_t queue[kWarps][32 + 32 * kBuWords];
 };
@@ -3088,27 +3088,321 @@ asc_status ensure_gather_buffers(asc_graph *g) {
 // graph's first BFS. The in-edges stay in pinned host memory, read in place,
 // unless the graph has no cap (every out-edge resident): then they are
 // resident too.
+// ------------------------------------------- in-edges of a CSR graph -------
+//
+// Built on the device on the graph's first BFS: in-degrees counted over the merge
+// items, scanned to offsets, then one pass over all edges for every run of lists
+// that fits a queue of the workspace (V entries; nothing else is allocated on the
+// device), which scatters the run's sources, moves the best candidate of each list
+// to its front and packs the run into page-locked memory. On host threads this
+// took 4.0 s for the 268 M edges of RMAT scale 24.
+//
+// The first in-edge of a list is the source with the most out-edges: the one most
+// likely to be in a large frontier. Of the 7% of vertices whose smallest-id source
+// was no parent in the large step of a BFS on RMAT scale 21, 24,200 went on to read
+// host memory; with this choice 3,744 do.
+namespace {
+
+struct InEdgeArgs {
+    const uint2 *items;
+    PrSlice sl[2];
+    const uint32_t *ptr;
+    uint32_t *cnt;           // in-degrees, then cursors
+    uint32_t *raw;           // the run's sources by list
+    uint32_t V, ebits, wbits;
+    uint32_t lo, hi, base;   // the run: lists [lo, hi), the first starts at base
+};
+
+template <bool COUNT>
+__global__ void __launch_bounds__(kBlock, 6) in_edges_kernel(InEdgeArgs p) {
+    __shared__ PrItemSmem<float> sm;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = p.sl[0].n + p.sl[1].n;
+    const uint32_t eb = p.ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    uint32_t *marks = sm.marks[0];
+    for (uint32_t w = blockIdx.x; w < total; w += gridDim.x) {
+        bool od;
+        const uint32_t it = pr_slice_item(p.sl, w, od);
+        const uint2 a = p.items[it], b = p.items[it + 1];
+        const uint32_t r0 = a.x, e0 = a.y, nr = b.x - a.x, ne = b.y - a.y;
+        uint32_t nq;
+        if (threadIdx.x < kItem / 32) marks[threadIdx.x] = 0;
+        const uint32_t bit0 = stage_words(p.sl[od].edges, p.sl[od].edge_words, e0, ne, eb, sm.pool, nq);
+        __syncthreads();
+        if (!COUNT) {
+            pr_mark_rows<float>(p.ptr, r0, e0, nr, sm, marks);
+            __syncthreads();
+        }
+        const uint32_t x0 = threadIdx.x * kVt, xw = x0 - lane * kVt;
+        if (xw < ne) {
+            uint32_t ends = 0, open = 0, row = 0;
+            if (!COUNT) {
+                ends = (marks[x0 >> 5] >> (x0 & 31)) & ((1u << kVt) - 1u);
+                const unsigned ended = __ballot_sync(kFull, ends != 0);
+                const uint32_t first = ends ? sm.row_at[x0 + __ffs((int)ends) - 1] : nr;
+                const unsigned above = lane < 31 ? ended & (0xffffffffu << (lane + 1)) : 0u;
+                const uint32_t from_lane = __shfl_sync(kFull, first, above ? __ffs((int)above) - 1 : lane);
+                const uint32_t after = pr_next_row(marks, sm.row_at, xw + 32 * kVt, nr);
+                open = above ? from_lane : after;
+                row = ends ? first : open;
+            }
+#pragma unroll
+            for (int k = 0; k < kVt; k++) {
+                if (x0 + k < ne) {
+                    const uint32_t v = staged_word(sm.pool, bit0 + (x0 + k) * eb, mask) >> p.wbits;
+                    if (!ASC_BAD(v >= p.V, 24, v)) {
+                        if (COUNT) atomicAdd(&p.cnt[v], 1u);
+                        else if (v >= p.lo && v < p.hi) p.raw[atomicAdd(&p.cnt[v], 1u) - p.base] = r0 + row;
+                    }
+                }
+                if (!COUNT && ((ends >> k) & 1u)) {
+                    const uint32_t rest = ends >> k >> 1;
+                    row = rest ? (uint32_t)sm.row_at[x0 + k + __ffs((int)rest)] : open;
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Exclusive scan of cnt[V] in blocks of kItem: block sums, their scan, the
+// offsets (also left in cnt as the scatter's cursors).
+__global__ void scan_sums_kernel(const uint32_t *cnt, uint32_t V, uint32_t *sums) {
+    __shared__ uint32_t warp[kWarps + 1];
+    uint32_t x = 0, total;
+    for (int k = 0; k < kVt; k++) {
+        const uint64_t v = (uint64_t)blockIdx.x * kItem + k * kBlock + threadIdx.x;
+        if (v < V) x += cnt[v];
+    }
+    block_excl_scan(x, total, warp);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void scan_block_sums_kernel(uint32_t *sums, uint32_t n) {
+    __shared__ uint32_t warp[kWarps + 1];
+    uint32_t run = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += kBlock) {
+        const uint32_t i = i0 + threadIdx.x, x = i < n ? sums[i] : 0;
+        uint32_t total;
+        const uint32_t before = block_excl_scan(x, total, warp);
+        if (i < n) sums[i] = run + before;
+        run += total;
+        __syncthreads();
+    }
+}
+
+__global__ void scan_offsets_kernel(uint32_t *cnt, uint32_t V, const uint32_t *sums, uint32_t E, uint32_t *in_ptr,
+                                    uint32_t *in_none) {
+    __shared__ uint32_t warp[kWarps + 1];
+    const uint64_t v0 = (uint64_t)blockIdx.x * kItem + threadIdx.x * kVt;
+    uint32_t c[kVt], x = 0, total;
+#pragma unroll
+    for (int k = 0; k < kVt; k++) {
+        c[k] = v0 + k < V ? cnt[v0 + k] : 0;
+        x += c[k];
+    }
+    uint32_t run = sums[blockIdx.x] + block_excl_scan(x, total, warp);
+    uint32_t none = 0;
+#pragma unroll
+    for (int k = 0; k < kVt; k++) {
+        if (v0 + k < V) in_ptr[v0 + k] = cnt[v0 + k] = run;
+        if (v0 + k >= V || !c[k]) none |= 1u << k;
+        run += c[k];
+    }
+    // four threads' bytes are a word of the bitmap of vertices without in-edges
+    // (bits past V set: nothing to look for there)
+    none <<= 8 * (threadIdx.x & 3);
+    none |= __shfl_xor_sync(kFull, none, 1);
+    none |= __shfl_xor_sync(kFull, none, 2);
+    if ((threadIdx.x & 3) == 0 && v0 / 32 < V / 32 + 2) in_none[v0 / 32] = none;
+    if (blockIdx.x == 0 && threadIdx.x == 0) in_ptr[V] = E;
+}
+
+// A warp per list of the run: the source with the most out-edges among its first
+// kHeadSample goes to the front, and to heads[v] (a vertex without in-edges: itself).
+constexpr uint32_t kHeadSample = 4096;
+__global__ void in_heads_kernel(InEdgeArgs p, const uint32_t *in_ptr, uint32_t *heads) {
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * kWarps;
+    for (uint64_t v = (uint64_t)p.lo + blockIdx.x * kWarps + (threadIdx.x >> 5); v < p.hi; v += warps) {
+        const uint32_t b = in_ptr[v] - p.base, n = in_ptr[v + 1] - in_ptr[v];
+        unsigned long long best = 0;  // out-degree, then the smaller id
+        uint32_t at = 0;
+        for (uint32_t i = lane; i < min(n, kHeadSample); i += 32) {
+            const uint32_t u = p.raw[b + i];
+            const unsigned long long key = ((unsigned long long)(p.ptr[u + 1] - p.ptr[u]) << 32) | (0xffffffffu - u);
+            if (key > best) {
+                best = key;
+                at = i;
+            }
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            const unsigned long long k2 = __shfl_xor_sync(kFull, best, d);
+            const uint32_t a2 = __shfl_xor_sync(kFull, at, d);
+            if (k2 > best || (k2 == best && a2 < at)) {
+                best = k2;
+                at = a2;
+            }
+        }
+        if (lane == 0) {
+            if (n) {
+                const uint32_t u = p.raw[b + at];
+                p.raw[b + at] = p.raw[b];
+                p.raw[b] = u;
+                heads[v] = u;
+            } else {
+                heads[v] = (uint32_t)v;
+            }
+        }
+    }
+}
+
+// Packs src[0, n) (words first .. first + n - 1 of a stream of eb bits each) into
+// out. The last word, when words of a later call share it, goes to *carry_out,
+// and the first takes what an earlier call left in *carry_in.
+__global__ void pack_stream_kernel(const uint32_t *src, uint64_t first, uint64_t n, uint32_t eb, uint32_t *out,
+                                   const uint32_t *carry_in, uint32_t *carry_out, bool last) {
+    const uint64_t bit_lo = first * eb, bit_hi = (first + n) * eb;
+    const uint64_t w_lo = bit_lo >> 5, w_hi = (bit_hi + 31) >> 5;
+    for (uint64_t w = w_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < w_hi;
+         w += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t b0 = 32 * w;
+        uint32_t x = w == w_lo && (bit_lo & 31) ? *carry_in : 0u;
+        for (uint64_t i = max(first, b0 / eb); i < first + n && i * eb < b0 + 32; i++) {
+            const uint32_t y = src[i - first];
+            x |= i * eb >= b0 ? y << (i * eb - b0) : y >> (b0 - i * eb);
+        }
+        if (w == w_hi - 1 && (bit_hi & 31) && !last) *carry_out = x;
+        else out[w] = x;
+    }
+}
+
+// *done false (and nothing kept) where a list is longer than a queue or the runs
+// would be many: the host builds those.
+asc_status in_edges_on_device(asc_graph *g, bool *done) {
+    Workspace *ws = g->ws;
+    cudaStream_t s = g->stream;
+    const uint64_t V = g->V, E = g->E;
+    constexpr uint64_t kMaxRuns = 64;
+    *done = false;
+    if (!E || E / V >= kMaxRuns) return ASC_OK;
+    ASC_TRY(ensure_items(g));
+    InEdgeArgs p;
+    memset(&p, 0, sizeof(p));
+    p.items = ws->items;
+    p.sl[0] = pr_slice(g, 0);
+    p.sl[1] = pr_slice(g, 1);
+    p.ptr = g->d_ptr;
+    p.cnt = ws->val;
+    p.raw = ws->queue[0];
+    p.V = (uint32_t)V;
+    p.ebits = g->edge_words == 2 ? 64 : g->ebits;
+    p.wbits = g->wbits;
+    const uint32_t blocks = (uint32_t)((V + 63 + kItem) / kItem), grid = item_grid(ws, ws->n_items, 6);
+    uint32_t *heads = ws->queue[1], *carry = ws->ctl + CTL_BARRIER + 1;
+    ASC_CUDA(cudaMemsetAsync(p.cnt, 0, 4 * V, s));
+    ASC_CUDA(cudaMemsetAsync(carry, 0, 8, s));
+    in_edges_kernel<true><<<grid, kBlock, 0, s>>>(p);
+    // the block sums fit a queue: V / kItem + 2 words; graphs too small for that go to the host
+    if (blocks > V) return ASC_OK;
+    scan_sums_kernel<<<blocks, kBlock, 0, s>>>(p.cnt, p.V, heads);
+    scan_block_sums_kernel<<<1, kBlock, 0, s>>>(heads, blocks);
+    scan_offsets_kernel<<<blocks, kBlock, 0, s>>>(p.cnt, p.V, heads, (uint32_t)E, ws->in_ptr, ws->in_none);
+    ASC_CUDA(cudaGetLastError());
+    std::vector<uint32_t> in_ptr(V + 1);
+    ASC_CUDA(cudaMemcpyAsync(in_ptr.data(), ws->in_ptr, 4 * (V + 1), cudaMemcpyDeviceToHost, s));
+    ASC_CUDA(cudaStreamSynchronize(s));
+    std::vector<uint32_t> cuts(1, 0);  // runs of lists of at most V entries
+    while (cuts.back() < V) {
+        const uint32_t lo = cuts.back();
+        const uint32_t hi = (uint32_t)(std::upper_bound(in_ptr.begin() + lo, in_ptr.end(), in_ptr[lo] + V,
+                                                        [](uint64_t x, uint32_t y) { return x < y; }) -
+                                       in_ptr.begin()) - 1;
+        if (hi <= lo || cuts.size() > 2 * kMaxRuns) return ASC_OK;
+        cuts.push_back(hi);
+    }
+    const uint32_t bits = g->in_ebits;
+    const uint64_t words = bits == 32 ? E : (E * bits + 31) / 32 + 1;
+    uint32_t *packed = nullptr;
+    if (cudaHostAlloc((void **)&packed, 4 * words, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(ASC_ERR_NOMEM, "cudaHostAlloc of %llu bytes failed", (unsigned long long)(4 * words));
+    }
+    void *dp = nullptr;
+    cudaError_t e = cudaHostGetDevicePointer(&dp, packed, 0);
+    const uint32_t fill = fill_grid(ws, ~0ull >> 32);
+    for (size_t k = 0; e == cudaSuccess && k + 1 < cuts.size(); k++) {
+        p.lo = cuts[k];
+        p.hi = cuts[k + 1];
+        p.base = in_ptr[p.lo];
+        const uint64_t n = in_ptr[p.hi] - p.base;
+        const bool last = k + 2 == cuts.size();
+        in_edges_kernel<false><<<grid, kBlock, 0, s>>>(p);
+        in_heads_kernel<<<fill, kBlock, 0, s>>>(p, ws->in_ptr, heads);
+        if (n) pack_stream_kernel<<<fill, kBlock, 0, s>>>(p.raw, p.base, n, bits, (uint32_t *)dp, carry + (k & 1),
+                                                           carry + (1 - (k & 1)), last);
+        else e = cudaMemcpyAsync(carry + (1 - (k & 1)), carry + (k & 1), 4, cudaMemcpyDeviceToDevice, s);
+        if (e == cudaSuccess) e = cudaGetLastError();
+    }
+    if (e == cudaSuccess && g->d_in_heads && !g->in_heads_ready) {
+        e = cudaMemsetAsync(g->d_in_heads, 0, 4 * g->in_head_words, s);
+        pack_stream_kernel<<<fill, kBlock, 0, s>>>(heads, 0, V, bits, g->d_in_heads, carry, carry, true);
+        if (e == cudaSuccess) e = cudaGetLastError();
+    }
+    uint32_t *none = new uint32_t[V / 32 + 2];
+    if (e == cudaSuccess) e = cudaMemcpyAsync(none, ws->in_none, 4 * (V / 32 + 2), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        cudaFreeHost(packed);
+        delete[] none;
+        return cuda_fail(e, "in-edges", __FILE__, __LINE__);
+    }
+    if (bits < 32) packed[words - 1] = 0;  // the padding word
+    g->h_in_ptr = new uint32_t[V + 1];
+    memcpy(g->h_in_ptr, in_ptr.data(), 4 * (V + 1));
+    g->h_in_none = none;
+    g->h_in_edges = packed;
+    g->d_host_in_edges = (const uint32_t *)dp;
+    if (g->d_in_heads) g->in_heads_ready = true;
+    *done = true;
+    return ASC_OK;
+}
+
+}  // namespace
+
 asc_status ensure_in_ptr(asc_graph *g) {
     Workspace *ws = g->ws;
     if (ws->in_ptr) return ASC_OK;
-    ASC_TRY(build_in_edges(g));
+    const uint64_t nw = g->V / 32 + 2;
     ASC_CUDA(cudaMalloc(&ws->in_ptr, 4 * (g->V + 1)));
-    ASC_CUDA(cudaMemcpy(ws->in_ptr, g->h_in_ptr, 4 * (g->V + 1), cudaMemcpyHostToDevice));
     ws->device_bytes += 4 * (g->V + 1);
-    {
-        // one bit per vertex without in-edges (bits past V set: nothing to look
-        // for there), built once per graph: a server that frees the state of an
-        // idle graph uploads it again
-        const uint64_t nw = g->V / 32 + 2;
-        if (!g->h_in_none) {
+    ASC_CUDA(cudaMalloc(&ws->in_none, 4 * nw));
+    ws->device_bytes += 4 * nw;
+    bool on_device = false;
+    asc_status st = g->h_in_edges ? ASC_OK : in_edges_on_device(g, &on_device);
+    if (st == ASC_OK && !on_device) {
+        if (!g->h_in_edges) st = build_in_edges(g);
+        if (st == ASC_OK && !g->h_in_none) {
             uint32_t *none = new uint32_t[nw]();
             for (uint64_t v = 0; v < 32 * nw; v++)
                 if (v >= g->V || g->h_in_ptr[v + 1] == g->h_in_ptr[v]) none[v >> 5] |= 1u << (v & 31);
             g->h_in_none = none;
         }
-        ASC_CUDA(cudaMalloc(&ws->in_none, 4 * nw));
-        ASC_CUDA(cudaMemcpy(ws->in_none, g->h_in_none, 4 * nw, cudaMemcpyHostToDevice));
-        ws->device_bytes += 4 * nw;
+        // the graph's host copies: a server that freed the state of an idle graph uploads them again
+        auto up = [&](void *to, const void *from, size_t n) {
+            if (st != ASC_OK) return;
+            const cudaError_t e = cudaMemcpy(to, from, n, cudaMemcpyHostToDevice);
+            if (e != cudaSuccess) st = cuda_fail(e, "in-edge offsets", __FILE__, __LINE__);
+        };
+        up(ws->in_ptr, g->h_in_ptr, 4 * (g->V + 1));
+        up(ws->in_none, g->h_in_none, 4 * nw);
+    }
+    if (st != ASC_OK) {  // in_ptr marks the state as complete
+        cudaFree(ws->in_ptr);
+        cudaFree(ws->in_none);
+        ws->in_ptr = ws->in_none = nullptr;
+        ws->device_bytes -= 4 * (g->V + 1) + 4 * nw;
+        return st;
     }
     if (g->static_edges >= g->E) {
         const uint64_t words = g->in_ebits == 32 ? std::max<uint64_t>(1, g->E) : (g->E * g->in_ebits + 31) / 32 + 1;

@@ -706,7 +706,14 @@ asc_status build_in_edges(asc_graph *g) {
         }
     });
     parallel_for(V, host_threads(E), [&](unsigned, uint64_t b, uint64_t e) {
-        for (uint64_t v = b; v < e; v++) std::sort(raw.begin() + in_ptr[v], raw.begin() + in_ptr[v + 1]);
+        // sorted by source id, but for the first: the source with the most out-edges
+        for (uint64_t v = b; v < e; v++) {
+            const auto lo = raw.begin() + in_ptr[v], hi = raw.begin() + in_ptr[v + 1];
+            std::sort(lo, hi);
+            const auto deg = [&](uint32_t u) { return g->h_ptr[u + 1] - g->h_ptr[u]; };
+            const auto best = std::max_element(lo, hi, [&](uint32_t x, uint32_t y) { return deg(x) < deg(y); });
+            if (best != hi) std::rotate(lo, best, best + 1);
+        }
     });
     const uint32_t bits = g->in_ebits;  // chosen with the split (bits(V - 1), or 32 without packing)
     uint32_t *packed = nullptr;

@@ -75,3 +75,29 @@ def test_iteration_cap():
                 g.run(algo, 0, params=A.make_params(max_iterations=V // 2))
             assert e.value.status == A.ERR_TIMEOUT
             assert np.array_equal(g.run(algo, 0)[0], got)
+
+
+@pytest.mark.parametrize("V,ef", [(64, 3), (2045, 5), (2048, 16), (3001, 1), (5000, 40), (70001, 12)])
+@pytest.mark.parametrize("frac", [1.0, 0.3, 0.0])
+def test_in_edges(V, ef, frac):
+    """In-edges built on the device (in several runs of lists, V entries each) and,
+    where a list is longer than V or the degree above 64, on the host: bottom-up
+    steps from the first iteration on give the oracle's levels."""
+    rng = np.random.RandomState(V)
+    for hub in (False, True):
+        src = rng.randint(0, V, V * ef)
+        dst = np.minimum(rng.randint(0, V, V * ef), rng.randint(0, V, V * ef))
+        if hub:  # one in-list longer than V
+            dst[: 2 * V] = 7
+        order = np.argsort(src, kind="stable")
+        ptr = np.zeros(V + 1, np.uint64)
+        ptr[1:] = np.cumsum(np.bincount(src, minlength=V))
+        col = dst[order].astype(np.uint32)
+        for edges in (col, np.stack([col, rng.randint(1, 64, len(col)).astype(np.uint32)], 1)):
+            with A.Graph.from_csr(ptr, edges, budget=A.make_budget(frac=frac, fragment_edges=64)) as g:
+                g.set_tuning(bu_div=0x7fffffff)  # every step bottom-up
+                for s in (int(src[0]), V - 1):
+                    got, st = g.run("bfs", s)
+                    assert np.array_equal(got, oracle.bfs(ptr, col, s)), (hub, s)
+                    host, _ = g.run("bfs", s, params=A.make_params(flags=A.RUN_HOST_LOOP))
+                    assert np.array_equal(got, host)
