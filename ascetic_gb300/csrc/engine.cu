@@ -461,13 +461,13 @@ __device__ __forceinline__ uint32_t region_word(const RegionArgs &a, uint32_t u0
     return word;
 }
 
-// One tile of frontier vertices, one per thread: kBlock consecutive entries
+// One tile of frontier vertices, one per thread: per consecutive entries
 // of the region's list, or (bitmap) kBlock consecutive vertex ids walked
 // through the frontier bitmap (tiles start 32-aligned; a tile with no active
 // vertex costs one bitmap read per warp).
 template <int ALG, int WORDS>
-__device__ __forceinline__ void expand_tile(const RegionArgs &a, uint32_t tile, uint32_t n_in, bool bitmap, Smem &sm,
-                                            uint32_t *s_next, uint32_t thresh) {
+__device__ __forceinline__ void expand_tile(const RegionArgs &a, uint32_t tile, uint32_t n_in, bool bitmap,
+                                            uint32_t per, Smem &sm, uint32_t *s_next, uint32_t thresh) {
     bool act;
     uint32_t u;
     if (bitmap) {
@@ -475,8 +475,8 @@ __device__ __forceinline__ void expand_tile(const RegionArgs &a, uint32_t tile, 
         act = (region_word(a, u & ~31u) >> (u & 31)) & 1u;
         if (!__syncthreads_or(act)) return;
     } else {
-        const uint32_t i = tile * kBlock + threadIdx.x;
-        act = i < n_in;
+        const uint32_t i = tile * per + threadIdx.x;
+        act = threadIdx.x < per && i < n_in;
         u = act ? a.q_in[i] : 0;
     }
     expand_vertices<ALG, WORDS>(a, act, u, sm, s_next, thresh);
@@ -523,17 +523,25 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 // region whose frontier holds more than 1/dense_div of its vertices is walked
 // in id order through its bitmap (its list was not built), kBlock ids per
 // item, so the lists of neighbouring active vertices are read as one
-// contiguous run; otherwise through its list, kBlock entries per item. With
-// merge items, the id-order walk runs over those alone.
+// contiguous run; otherwise through its list, per entries per item: as few as
+// give every CTA of the grid one, at least kMinTile, since the lists of a tile
+// are walked by one CTA (the third iteration of a BFS on RMAT scale 16 took 93
+// us with its 800 vertices and 118,000 edges in four tiles of 256). With merge
+// items, the id-order walk runs over those alone.
+#ifndef ASC_MIN_TILE
+#define ASC_MIN_TILE 8
+#endif
+constexpr uint32_t kMinTile = ASC_MIN_TILE;
 __device__ __forceinline__ void region_items_bits(const RegionArgs &a, uint32_t &n_in, uint32_t &nseg,
-                                                  uint32_t &items, bool &bitmap) {
+                                                  uint32_t &items, bool &bitmap, uint32_t &per) {
     const uint32_t range = a.dense_end - a.dense_begin;
     const uint32_t bits = a.cnt_in[6 + a.region];
     nseg = a.cnt_in[2 + a.region];
     bitmap = a.bitmap_in && a.dense_div && bits > range / a.dense_div;
     n_in = bitmap ? 0 : a.cnt_in[a.region];
     const uint32_t nvert = bitmap ? a.dense_end - (a.dense_begin & ~31u) : n_in;
-    items = nseg + (nvert + kBlock - 1) / kBlock;
+    per = bitmap ? kBlock : min((uint32_t)kBlock, max(kMinTile, (n_in + gridDim.x - 1) / gridDim.x));
+    items = nseg + (nvert + per - 1) / per;
     if (bitmap && a.items) {
         nseg = 0;
         items = a.item_n;
@@ -718,10 +726,11 @@ constexpr int kNextWords = 6;
 
 template <int ALG, int WORDS>
 __device__ __forceinline__ void expand_item(const RegionArgs &a, uint32_t w, uint32_t n_in, uint32_t nseg,
-                                            bool bitmap, ExpandSmem<WORDS> &sm, uint32_t *s_next, uint32_t thresh) {
+                                            bool bitmap, uint32_t per, ExpandSmem<WORDS> &sm, uint32_t *s_next,
+                                            uint32_t thresh) {
     if (w < nseg) expand_segment<ALG, WORDS>(a, a.seg_in[w], s_next, thresh);
     else if (bitmap && a.items) expand_merge_item<ALG, WORDS>(a, a.item_begin + w, sm.item, s_next, thresh);
-    else expand_tile<ALG, WORDS>(a, w - nseg, n_in, bitmap, sm.tile, s_next, thresh);
+    else expand_tile<ALG, WORDS>(a, w - nseg, n_in, bitmap, per, sm.tile, s_next, thresh);
 }
 
 __device__ __forceinline__ void flush_next(const RegionArgs &a, uint32_t *s_next) {
@@ -747,7 +756,8 @@ __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_kernel(R
     if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     uint32_t n_in, nseg, total;
     bool bitmap;
-    region_items_bits(a, n_in, nseg, total, bitmap);
+    uint32_t per;
+    region_items_bits(a, n_in, nseg, total, bitmap, per);
     const uint32_t thresh = ALG == kSSSP && a.far_bits ? *a.thresh : 0u;
     for (;;) {
         if (threadIdx.x == 0) s_work = atomicAdd(a.work, 1u);
@@ -755,7 +765,7 @@ __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_kernel(R
         const uint32_t w = s_work;
         __syncthreads();
         if (w >= total) break;
-        expand_item<ALG, WORDS>(a, w, n_in, nseg, bitmap, sm, s_next, thresh);
+        expand_item<ALG, WORDS>(a, w, n_in, nseg, bitmap, per, sm, s_next, thresh);
     }
     flush_expansion(a, s_next);
 }
@@ -775,10 +785,10 @@ template <int ALG, int WORDS>
 __device__ __forceinline__ void expand_regions(const FusedArgs &x, uint32_t thresh, ExpandSmem<WORDS> &sm,
                                                uint32_t *s_next) {
     __shared__ uint32_t s_work;
-    uint32_t n0, s0, i0, n1, s1, i1;
+    uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(x.r0, n0, s0, i0, m0);
-    region_items_bits(x.r1, n1, s1, i1, m1);
+    region_items_bits(x.r0, n0, s0, i0, m0, t0);
+    region_items_bits(x.r1, n1, s1, i1, m1, t1);
     const uint32_t m = min(i0, i1), total = i0 + i1;
     if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     __syncthreads();
@@ -793,8 +803,8 @@ __device__ __forceinline__ void expand_regions(const FusedArgs &x, uint32_t thre
             local = m + (w - 2 * m);
         }
         if (threadIdx.x == 0) s_work = gridDim.x + atomicAdd(x.work, 1u);
-        if (od) expand_item<ALG, WORDS>(x.r1, local, n1, s1, m1, sm, s_next, thresh);
-        else expand_item<ALG, WORDS>(x.r0, local, n0, s0, m0, sm, s_next, thresh);
+        if (od) expand_item<ALG, WORDS>(x.r1, local, n1, s1, m1, t1, sm, s_next, thresh);
+        else expand_item<ALG, WORDS>(x.r0, local, n0, s0, m0, t0, sm, s_next, thresh);
         __syncthreads();
         w = s_work;
         __syncthreads();
@@ -1307,11 +1317,16 @@ struct LoopArgs {
     uint32_t thresh;        // near-far: the first threshold
     uint32_t delta;         // near-far: step of the next one beyond the smallest far value
     uint32_t count_reached;
+    uint32_t *values;       // host: small results too (null: the caller copies them)
     uint32_t first_label;   // connected components: src's label is spread first, the rest follow
     uint32_t first_cap;     // after at most this many iterations
 };
 
 constexpr uint32_t kFirstLabelIterations = 32;
+// Results of at most this many values come back with the report and are copied
+// from there on the host: the copy engine's latency is longer (BFS on 1,001
+// vertices: 11 to 14 us of 80).
+constexpr uint64_t kReportedValues = 16384;
 
 // Polls of a grid barrier (a read of L2 and a short sleep each) before it gives
 // up: tens of seconds, far above any phase.
@@ -1561,6 +1576,9 @@ __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const
         if (ALG == kBFS) reached_bits(l.x0.r0.visited, l.x0.r0.ptr, l.x0.r0.V, l.nwords, out);
         else reached_values(l.x0.r0.val, l.x0.r0.ptr, l.x0.r0.V, out);
     }
+    if (l.values)
+        for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < l.x0.r0.V; v += gridDim.x * blockDim.x)
+            l.values[v] = l.x0.r0.val[v];
     if (!grid_barrier(l.ctl, st.target)) return;
     if (blockIdx.x == 0 && threadIdx.x < CTL_WORDS)
         l.report[threadIdx.x] = threadIdx.x == CTL_ITERS ? st.it : ((volatile uint32_t *)l.ctl)[threadIdx.x];
@@ -1784,7 +1802,7 @@ __device__ void pr_segment(const PrArgs &p, uint64_t item, PrSmem &sm) {
 }
 
 __device__ __forceinline__ void pr_list_item(const PrArgs &p, uint32_t w, uint32_t n_in, uint32_t nseg, bool bitmap,
-                                             PrSmem &sm, uint32_t *s_next) {
+                                             uint32_t per, PrSmem &sm, uint32_t *s_next) {
     const RegionArgs &a = p.r;
     if (w < nseg) {
         pr_segment(p, a.seg_in[w], sm);
@@ -1793,8 +1811,9 @@ __device__ __forceinline__ void pr_list_item(const PrArgs &p, uint32_t w, uint32
         const bool valid = (region_word(a, u & ~31u) >> (u & 31)) & 1u;
         if (__syncthreads_or(valid)) pr_vertices(p, valid, u, sm, s_next);
     } else {
-        const uint32_t i = (w - nseg) * kBlock + threadIdx.x;
-        pr_vertices(p, i < n_in, i < n_in ? a.q_in[i] : 0u, sm, s_next);
+        const uint32_t i = (w - nseg) * per + threadIdx.x;
+        const bool valid = threadIdx.x < per && i < n_in;
+        pr_vertices(p, valid, valid ? a.q_in[i] : 0u, sm, s_next);
     }
 }
 
@@ -1807,10 +1826,10 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_lists_kerne
     __shared__ PrSmem sm;
     __shared__ uint32_t s_next[2];
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
-    uint32_t n0, s0, i0, n1, s1, i1;
+    uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool b0, b1;
-    region_items_bits(p0.r, n0, s0, i0, b0);
-    region_items_bits(p1.r, n1, s1, i1, b1);
+    region_items_bits(p0.r, n0, s0, i0, b0, t0);
+    region_items_bits(p1.r, n1, s1, i1, b1, t1);
     if (!(regions & 1u)) i0 = 0;
     if (!(regions & 2u)) i1 = 0;
     const uint32_t m = min(i0, i1), total = i0 + i1;
@@ -1830,8 +1849,8 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_lists_kerne
             od = i1 > i0;
             local = m + (w - 2 * m);
         }
-        if (od) pr_list_item(p1, local, n1, s1, b1, sm, s_next);
-        else pr_list_item(p0, local, n0, s0, b0, sm, s_next);
+        if (od) pr_list_item(p1, local, n1, s1, b1, t1, sm, s_next);
+        else pr_list_item(p0, local, n0, s0, b0, t0, sm, s_next);
     }
     flush_next(p0.r, s_next);
 }
@@ -2290,11 +2309,13 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         hit = cache.end() - 1;
         asc_graph::LongLists &ll = *hit;
         ll.bits.assign(V / 32 + 2, 0);
-        for (uint64_t v = 0; v < V; v++) {
-            uint32_t d = g->h_ptr[v + 1] - g->h_ptr[v];
-            if (d > t.huge_degree) {
-                uint64_t ns = (d + t.segment_edges - 1) / t.segment_edges;
-                (v < S ? ll.seg_static : ll.seg_ondemand) += ns;
+        const uint32_t *ptr = g->h_ptr;
+        const uint32_t huge = t.huge_degree;
+        for (uint64_t v = 0, b = ptr[0]; v < V; v++) {
+            const uint64_t e = ptr[v + 1], d = e - b;
+            b = e;
+            if (d > huge) {
+                (v < S ? ll.seg_static : ll.seg_ondemand) += (d + t.segment_edges - 1) / t.segment_edges;
                 ll.bits[v >> 5] |= 1u << (v & 31);
             }
         }
@@ -2324,7 +2345,8 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         ASC_TRY(dalloc((void **)&ws->segs[i], 8 * (cs + co)));
     }
     ASC_TRY(dalloc((void **)&ws->ctl, 4 * CTL_WORDS));
-    ASC_CUDA(cudaHostAlloc((void **)&ws->h_ctl, 4 * CTL_WORDS, cudaHostAllocDefault));
+    ASC_CUDA(cudaHostAlloc((void **)&ws->h_ctl, 4 * (CTL_WORDS + std::min<uint64_t>(V, kReportedValues)),
+                           cudaHostAllocDefault));
     for (auto &e : ws->ev) ASC_CUDA(cudaEventCreate(&e));
     ws->device_bytes = bytes;
     return ASC_OK;
@@ -3469,6 +3491,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     const uint32_t first =
         first_label ? (uint32_t)(std::upper_bound(g->h_ptr, g->h_ptr + V + 1, 0u) - g->h_ptr) - 1 : source;
     bool rest_waits = first_label && !device_loop;  // the other labels have not started
+    const bool want = out && !(p.flags & ASC_RUN_NO_OUTPUT);
+    const bool values_reported = device_loop && want && !(p.flags & ASC_RUN_DEVICE_OUT) && V <= kReportedValues;
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
     ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
     if (device_loop) {
@@ -3495,6 +3519,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         const TraverseFn fn = pick_traverse(algo, edge_layout(g));
         uint32_t grid;
         ASC_TRY(loop_grid(g, algo, fn, &grid));
+        if (values_reported) l.values = ws->h_ctl + CTL_WORDS;
         ws->h_ctl[CTL_TIMEOUT] = 2;  // stays when a barrier ran out of time and nothing is reported
         void *args[] = {&l};
         ASC_CUDA(cudaLaunchCooperativeKernel((const void *)fn, dim3(grid), dim3(kBlock), args, 0, s));
@@ -3532,7 +3557,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         const uint32_t range = region == 0 ? g->static_vertices : V - g->static_vertices;
         const bool bitmap_mode = div && cnt[6 + region] > range / div;
         if (bitmap_mode && !part) return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
-        return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + kBlock - 1) / kBlock;
+        const uint32_t per = bitmap_mode ? (uint32_t)kBlock : kMinTile;
+        return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + per - 1) / per;
     };
     while ((cnt[6] | cnt[7]) || rest_waits) {
         if (rest_waits && (!(cnt[6] | cnt[7]) || iters >= (int)kFirstLabelIterations)) {
@@ -3674,7 +3700,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     }
     ASC_CUDA(cudaEventRecord(ws->ev[1], s));
     ASC_CUDA(cudaGetLastError());
-    if (out && !(p.flags & ASC_RUN_NO_OUTPUT)) {
+    if (want && !values_reported) {
         ASC_CUDA(cudaMemcpyAsync(out, ws->val, 4ull * V,
                                  (p.flags & ASC_RUN_DEVICE_OUT) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                  s));
@@ -3686,6 +3712,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         if (ws->h_ctl[CTL_TIMEOUT] == 2) return fail(ASC_ERR_TIMEOUT, "a grid barrier ran out of time");
         iters = (int)ws->h_ctl[CTL_ITERS];
         if (ws->h_ctl[CTL_TIMEOUT]) return fail(ASC_ERR_TIMEOUT, "no fixpoint after %d iterations", iters);
+        if (values_reported) memcpy(out, ws->h_ctl + CTL_WORDS, 4ull * V);
     }
     if (st) {
         memset(st, 0, sizeof(*st));
@@ -4202,14 +4229,15 @@ union MsExpandSmem {
 
 template <int WORDS>
 __device__ __forceinline__ void ms_item(const MsArgs &m, const RegionArgs &a, uint32_t w, uint32_t n_in,
-                                        uint32_t nseg, bool bitmap, MsExpandSmem<WORDS> &sm, uint32_t *counts) {
+                                        uint32_t nseg, bool bitmap, uint32_t per, MsExpandSmem<WORDS> &sm,
+                                        uint32_t *counts) {
     if (w < nseg) {
         ms_segment<WORDS>(m, a, a.seg_in[w]);
     } else if (bitmap && a.items) {
         ms_merge_item<WORDS>(m, a, a.item_begin + w, sm.item, counts);
     } else if (!bitmap) {
-        const uint32_t i = (w - nseg) * kBlock + threadIdx.x;
-        const bool act = i < n_in;
+        const uint32_t i = (w - nseg) * per + threadIdx.x;
+        const bool act = threadIdx.x < per && i < n_in;
         ms_vertices<WORDS>(m, a, act, act ? a.q_in[i] : 0, sm.tile);
     } else {
         const uint32_t u = (a.dense_begin & ~31u) + (w - nseg) * kBlock + threadIdx.x;
@@ -4223,10 +4251,10 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_BFS_BLOCKS) ms_bfs_expand_kerne
     __shared__ MsExpandSmem<WORDS> sm;
     __shared__ uint32_t s_work, counts[4];  // edges, vertices of merge items per region
     if (threadIdx.x < 4) counts[threadIdx.x] = 0;
-    uint32_t n0, s0, i0, n1, s1, i1;
+    uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(m.r0, n0, s0, i0, m0);
-    region_items_bits(m.r1, n1, s1, i1, m1);
+    region_items_bits(m.r0, n0, s0, i0, m0, t0);
+    region_items_bits(m.r1, n1, s1, i1, m1, t1);
     const uint32_t mm = min(i0, i1), total = i0 + i1;
     for (;;) {
         if (threadIdx.x == 0) s_work = atomicAdd(m.work, 1u);
@@ -4243,8 +4271,8 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_BFS_BLOCKS) ms_bfs_expand_kerne
             od = i1 > i0;
             local = mm + (w - 2 * mm);
         }
-        if (od) ms_item<WORDS>(m, m.r1, local, n1, s1, m1, sm, counts);
-        else ms_item<WORDS>(m, m.r0, local, n0, s0, m0, sm, counts);
+        if (od) ms_item<WORDS>(m, m.r1, local, n1, s1, m1, t1, sm, counts);
+        else ms_item<WORDS>(m, m.r0, local, n0, s0, m0, t0, sm, counts);
     }
     if (threadIdx.x < 4 && counts[threadIdx.x])
         atomicAdd(&m.r0.stats[threadIdx.x], (unsigned long long)counts[threadIdx.x]);
@@ -4533,7 +4561,7 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
 // has loads in flight.
 template <int R>
 __device__ void ms_sssp_item(const MsArgs &m, const RegionArgs &a, uint32_t w, uint32_t n_in, uint32_t nseg,
-                             MsSsspSmem &sm) {
+                             uint32_t per, MsSsspSmem &sm) {
     bool act = false;
     uint32_t u = 0, start = 0, deg = 0;
     unsigned long long f = 0;
@@ -4551,8 +4579,8 @@ __device__ void ms_sssp_item(const MsArgs &m, const RegionArgs &a, uint32_t w, u
             f = m.front[u];
         }
     } else {
-        const uint32_t i = (w - nseg) * kBlock + threadIdx.x;
-        if (i < n_in && !ASC_BAD(a.q_in[i] >= m.V, 7, a.q_in[i])) {
+        const uint32_t i = (w - nseg) * per + threadIdx.x;
+        if (threadIdx.x < per && i < n_in && !ASC_BAD(a.q_in[i] >= m.V, 7, a.q_in[i])) {
             u = a.q_in[i];
             start = a.ptr[u];
             deg = a.ptr[u + 1] - start;
@@ -4584,10 +4612,10 @@ template <int R>
 __global__ void __launch_bounds__(kBlock, ASC_MS_MIN_BLOCKS) ms_sssp_expand_kernel(MsArgs m) {
     static_assert(ms_row_ok(R), "rows of 16, 32 or 64 sources");
     __shared__ MsSsspSmem sm;
-    uint32_t n0, s0, i0, n1, s1, i1;
+    uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(m.r0, n0, s0, i0, m0);
-    region_items_bits(m.r1, n1, s1, i1, m1);
+    region_items_bits(m.r0, n0, s0, i0, m0, t0);
+    region_items_bits(m.r1, n1, s1, i1, m1, t1);
     const uint32_t mm = min(i0, i1), total = i0 + i1;
     for (;;) {
         if (threadIdx.x == 0) sm.work = atomicAdd(m.work, 1u);
@@ -4604,8 +4632,8 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_MIN_BLOCKS) ms_sssp_expand_kern
             od = i1 > i0;
             local = mm + (w - 2 * mm);
         }
-        if (od) ms_sssp_item<R>(m, m.r1, local, n1, s1, sm);
-        else ms_sssp_item<R>(m, m.r0, local, n0, s0, sm);
+        if (od) ms_sssp_item<R>(m, m.r1, local, n1, s1, t1, sm);
+        else ms_sssp_item<R>(m, m.r0, local, n0, s0, t0, sm);
     }
 }
 
