@@ -2647,12 +2647,12 @@ TraverseFn pick_traverse(asc_algo algo, int layout) {
 }
 
 #ifndef ASC_LOOP_EDGES
-#define ASC_LOOP_EDGES 4096
+#define ASC_LOOP_EDGES 8192
 #endif
 // CTAs of the persistent loop: all that stay resident, or one per
-// ASC_LOOP_EDGES edges of a small graph (fewer arrivals per barrier): a two-
-// iteration BFS on 1 M edges took 63 / 58 / 33 / 29 / 28 us at 512 / 1024 / 2048 /
-// 4096 / 8192.
+// ASC_LOOP_EDGES edges of a small graph, since a barrier costs by its arrivals: BFS
+// on 65,536 / 200,000 vertices of degree 8 took 116 / 149 us at 1024, 99 / 144 at
+// 2048, 93 / 104 at 4096, 93 / 89 at 8192.
 asc_status loop_grid(asc_graph *g, asc_algo algo, TraverseFn fn, uint32_t *grid) {
     Workspace *ws = g->ws;
     int &per_sm = ws->loop_per_sm[algo];
