@@ -33,6 +33,8 @@
 
 #include <algorithm>
 #include <chrono>
+#include <memory>
+#include <new>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -2309,15 +2311,41 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         hit = cache.end() - 1;
         asc_graph::LongLists &ll = *hit;
         ll.bits.assign(V / 32 + 2, 0);
+        // on host threads, 2^20 vertices each or more (whole bitmap words)
         const uint32_t *ptr = g->h_ptr;
-        const uint32_t huge = t.huge_degree;
-        for (uint64_t v = 0, b = ptr[0]; v < V; v++) {
-            const uint64_t e = ptr[v + 1], d = e - b;
-            b = e;
-            if (d > huge) {
-                (v < S ? ll.seg_static : ll.seg_ondemand) += (d + t.segment_edges - 1) / t.segment_edges;
-                ll.bits[v >> 5] |= 1u << (v & 31);
+        const uint32_t huge = t.huge_degree, seg = t.segment_edges;
+        const uint64_t words = (V + 31) / 32;
+        const uint64_t nt = std::max<uint64_t>(
+            1, std::min<uint64_t>(std::max(1u, std::thread::hardware_concurrency()), words >> 15));
+        std::vector<uint64_t> sums(2 * nt, 0);
+        auto scan = [&](uint64_t k) {
+            uint64_t n0 = 0, n1 = 0;
+            for (uint64_t w = words * k / nt; w < words * (k + 1) / nt; w++) {
+                uint32_t bits = 0;
+                for (uint64_t v = 32 * w; v < std::min(V, 32 * w + 32); v++) {
+                    const uint32_t d = ptr[v + 1] - ptr[v];
+                    if (d <= huge) continue;
+                    bits |= 1u << (v & 31);
+                    (v < S ? n0 : n1) += ((uint64_t)d + seg - 1) / seg;
+                }
+                ll.bits[w] = bits;
             }
+            sums[2 * k] = n0;
+            sums[2 * k + 1] = n1;
+        };
+        std::vector<std::thread> threads;
+        for (uint64_t k = 1; k < nt; k++) {
+            try {
+                threads.emplace_back(scan, k);
+            } catch (...) {  // no thread to be had
+                scan(k);
+            }
+        }
+        scan(0);
+        for (auto &th : threads) th.join();
+        for (uint64_t k = 0; k < nt; k++) {
+            ll.seg_static += sums[2 * k];
+            ll.seg_ondemand += sums[2 * k + 1];
         }
         ll.huge_degree = t.huge_degree;
         ll.segment_edges = t.segment_edges;
@@ -3331,17 +3359,20 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
     scan_block_sums_kernel<<<1, kBlock, 0, s>>>(heads, blocks);
     scan_offsets_kernel<<<blocks, kBlock, 0, s>>>(p.cnt, p.V, heads, (uint32_t)E, ws->in_ptr, ws->in_none);
     ASC_CUDA(cudaGetLastError());
-    std::vector<uint32_t> in_ptr(V + 1);
-    ASC_CUDA(cudaMemcpyAsync(in_ptr.data(), ws->in_ptr, 4 * (V + 1), cudaMemcpyDeviceToHost, s));
+    std::unique_ptr<uint32_t[]> h_ptr(new (std::nothrow) uint32_t[V + 1]);
+    std::unique_ptr<uint32_t[]> none(new (std::nothrow) uint32_t[V / 32 + 2]);
+    if (!h_ptr || !none) return fail(ASC_ERR_NOMEM, "in-edge offsets: %llu vertices", (unsigned long long)V);
+    const uint32_t *in_ptr = h_ptr.get();
+    ASC_CUDA(cudaMemcpyAsync(h_ptr.get(), ws->in_ptr, 4 * (V + 1), cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
-    std::vector<uint32_t> cuts(1, 0);  // runs of lists of at most V entries
-    while (cuts.back() < V) {
-        const uint32_t lo = cuts.back();
-        const uint32_t hi = (uint32_t)(std::upper_bound(in_ptr.begin() + lo, in_ptr.end(), in_ptr[lo] + V,
+    uint32_t cuts[2 * kMaxRuns + 1] = {0}, runs = 0;  // runs of lists of at most V entries
+    while (cuts[runs] < V) {
+        const uint32_t lo = cuts[runs];
+        const uint32_t hi = (uint32_t)(std::upper_bound(in_ptr + lo, in_ptr + V + 1, in_ptr[lo] + V,
                                                         [](uint64_t x, uint32_t y) { return x < y; }) -
-                                       in_ptr.begin()) - 1;
-        if (hi <= lo || cuts.size() > 2 * kMaxRuns) return ASC_OK;
-        cuts.push_back(hi);
+                                       in_ptr) - 1;
+        if (hi <= lo || runs == 2 * kMaxRuns) return ASC_OK;
+        cuts[++runs] = hi;
     }
     const uint32_t bits = g->in_ebits;
     const uint64_t words = bits == 32 ? E : (E * bits + 31) / 32 + 1;
@@ -3353,12 +3384,12 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
     void *dp = nullptr;
     cudaError_t e = cudaHostGetDevicePointer(&dp, packed, 0);
     const uint32_t fill = fill_grid(ws, ~0ull >> 32);
-    for (size_t k = 0; e == cudaSuccess && k + 1 < cuts.size(); k++) {
+    for (uint32_t k = 0; e == cudaSuccess && k < runs; k++) {
         p.lo = cuts[k];
         p.hi = cuts[k + 1];
         p.base = in_ptr[p.lo];
         const uint64_t n = in_ptr[p.hi] - p.base;
-        const bool last = k + 2 == cuts.size();
+        const bool last = k + 1 == runs;
         in_edges_kernel<false><<<grid, kBlock, 0, s>>>(p);
         in_heads_kernel<<<fill, kBlock, 0, s>>>(p, ws->in_ptr, heads);
         if (n) pack_stream_kernel<<<fill, kBlock, 0, s>>>(p.raw, p.base, n, bits, (uint32_t *)dp, carry + (k & 1),
@@ -3371,18 +3402,15 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
         pack_stream_kernel<<<fill, kBlock, 0, s>>>(heads, 0, V, bits, g->d_in_heads, carry, carry, true);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
-    uint32_t *none = new uint32_t[V / 32 + 2];
-    if (e == cudaSuccess) e = cudaMemcpyAsync(none, ws->in_none, 4 * (V / 32 + 2), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(none.get(), ws->in_none, 4 * (V / 32 + 2), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaFreeHost(packed);
-        delete[] none;
         return cuda_fail(e, "in-edges", __FILE__, __LINE__);
     }
     if (bits < 32) packed[words - 1] = 0;  // the padding word
-    g->h_in_ptr = new uint32_t[V + 1];
-    memcpy(g->h_in_ptr, in_ptr.data(), 4 * (V + 1));
-    g->h_in_none = none;
+    g->h_in_ptr = h_ptr.release();
+    g->h_in_none = none.release();
     g->h_in_edges = packed;
     g->d_host_in_edges = (const uint32_t *)dp;
     if (g->d_in_heads) g->in_heads_ready = true;
