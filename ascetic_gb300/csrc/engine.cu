@@ -5920,7 +5920,8 @@ extern "C" asc_status asc_bfs_device_noalloc(uint64_t V, uint64_t E, const uint3
         a.seg_out = segs[po];
         a.work = a.cnt_out + 4;
         const bool dense = cnt[6] > V32 / a.dense_div;
-        const uint64_t items = (uint64_t)cnt[2] + ((dense ? V32 : cnt[0]) + kBlock - 1) / kBlock;
+        const uint32_t per = dense ? (uint32_t)kBlock : kMinTile;
+        const uint64_t items = (uint64_t)cnt[2] + ((dense ? V32 : cnt[0]) + per - 1) / per;
         const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)sms * 4));
         expand_kernel<kBFS, 1><<<grid, kBlock, 0, s>>>(a);
         build_frontier_kernel<<<fill, kBlock, 0, s>>>(a, bitmap[po], nwords);

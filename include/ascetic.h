@@ -144,7 +144,7 @@ enum {
     ASC_RUN_PHASE_TIMING = 1u << 2, /* time static and on-demand kernels separately (CUDA events);
                                        implies a host-driven iteration loop */
     ASC_RUN_HOST_LOOP = 1u << 3,    /* drive iterations from the host (one readback per iteration)
-                                       instead of the CUDA-graph loop */
+                                       instead of in one cooperative launch */
     ASC_RUN_FRAGMENT_COUNTS = 1u << 4, /* BFS/SSSP/CC: add the edges this run reads to per-fragment
                                           counters (4096 edges a fragment; read them with
                                           asc_graph_fragment_counts); implies ASC_RUN_HOST_LOOP */
@@ -274,7 +274,7 @@ typedef struct asc_tuning {
                         distance + delta (0: plain frontier relaxation) */
     uint32_t bu_div; /* BFS on a CSR graph: an iteration whose frontier holds more than V / bu_div
                         vertices steps bottom-up, every unreached vertex scanning its in-edges for a
-                        frontier parent (in-edges built once on the host, read in place; the device
+                        frontier parent (in-edges built once, held by the host, read in place; the device
                         holds their V + 1 offsets). Same levels. 0: top-down only. Default 64. */
     double ms;
 } asc_tuning;
