@@ -101,3 +101,39 @@ def test_in_edges(V, ef, frac):
                     assert np.array_equal(got, oracle.bfs(ptr, col, s)), (hub, s)
                     host, _ = g.run("bfs", s, params=A.make_params(flags=A.RUN_HOST_LOOP))
                     assert np.array_equal(got, host)
+
+
+def test_concurrent_graphs():
+    """Threads with a graph each: their persistent loops fill the GPU one after the other."""
+    import threading
+
+    sizes = [(65536, 16), (1001, 8), (200000, 8), (65536, 16)]
+    graphs, expect, failed = [], [], []
+    for k, (V, ef) in enumerate(sizes):
+        rng = np.random.RandomState(k)
+        src = np.sort((V * rng.rand(V * ef) ** 2).astype(np.int64))
+        col = (V * rng.rand(V * ef) ** 2).astype(np.uint32)
+        ptr = np.zeros(V + 1, np.uint64)
+        ptr[1:] = np.cumsum(np.bincount(src, minlength=V))
+        w = np.stack([col, rng.randint(1, 64, len(col)).astype(np.uint32)], 1)
+        graphs.append(A.Graph.from_csr(ptr, w, budget=A.make_budget(frac=0.3)))
+        expect.append({"bfs": oracle.bfs(ptr, col, 0), "sssp": oracle.sssp(ptr, w, 0), "cc": oracle.cc(ptr, col)})
+
+    def work(k):
+        try:
+            for i in range(20):
+                algo = ("bfs", "sssp", "cc")[(i + k) % 3]
+                got, _ = graphs[k].run(algo, 0)
+                if not np.array_equal(got, expect[k][algo]):
+                    failed.append((k, i, algo, "values"))
+        except Exception as e:  # reported below: a thread's exception fails no test by itself
+            failed.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g in graphs:
+        g.close()
+    assert not failed, failed
