@@ -3520,7 +3520,12 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         first_label ? (uint32_t)(std::upper_bound(g->h_ptr, g->h_ptr + V + 1, 0u) - g->h_ptr) - 1 : source;
     bool rest_waits = first_label && !device_loop;  // the other labels have not started
     const bool want = out && !(p.flags & ASC_RUN_NO_OUTPUT);
-    const bool values_reported = device_loop && want && !(p.flags & ASC_RUN_DEVICE_OUT) && V <= kReportedValues;
+    bool values_reported = device_loop && want && !(p.flags & ASC_RUN_DEVICE_OUT) && V <= kReportedValues;
+    if (values_reported) {  // only what the host can write to; the copy below answers for the rest
+        cudaPointerAttributes attr;
+        if (cudaPointerGetAttributes(&attr, out) != cudaSuccess) cudaGetLastError();
+        else if (attr.type == cudaMemoryTypeDevice) values_reported = false;
+    }
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
     ASC_CUDA(cudaMemsetAsync(ws->ctl, 0, 4 * CTL_WORDS, s));
     if (device_loop) {
