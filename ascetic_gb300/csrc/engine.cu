@@ -5018,9 +5018,18 @@ uint32_t batch_slots(const BatchEngine *b) { return b->sssp ? b->stride : 64u; }
 // Applies the queued admissions and launches one iteration on the batch's
 // stream, ending with the readback of its counts (nothing waits here).
 namespace {
-// The sources still alive, to page-locked memory: a copy would queue behind the
-// rows that asc_run_batch copies out meanwhile.
-__global__ void report_alive_kernel(const unsigned long long *alive, unsigned long long *report) { *report = *alive; }
+// Ends a batch iteration: reports the sources still alive to page-locked memory (a
+// copy would queue behind the rows that asc_run_batch copies out meanwhile) and
+// clears what the next iteration writes, the counts and bitmap that this one read.
+__global__ void batch_end_kernel(unsigned long long *alive, unsigned long long *report, uint32_t *cnt,
+                                 uint32_t *bitmap, uint32_t nwords) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *report = *alive;
+        *alive = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) cnt[threadIdx.x] = 0;
+    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nwords; w += gridDim.x * blockDim.x) bitmap[w] = 0;
+}
 }  // namespace
 
 asc_status batch_launch(BatchEngine *b) {
@@ -5058,9 +5067,6 @@ asc_status batch_launch(BatchEngine *b) {
         b->pend_n = 0;
     }
     unsigned long long *alive = (unsigned long long *)(ws->ctl + CTL_ALIVE);
-    ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_BLOCK * po, 0, 4 * CTL_BLOCK, s));
-    ASC_CUDA(cudaMemsetAsync(alive, 0, 8, s));
-    ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
     m.r0 = region_args(g, ws, p, 0, false);
     m.r1 = region_args(g, ws, p, 1, false);
     m.work = m.r0.cnt_out + 4;
@@ -5082,7 +5088,8 @@ asc_status batch_launch(BatchEngine *b) {
                                                                         nwords);
     build_frontier_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(m.r0, ws->bitmap[po], nwords);
     ASC_CUDA(cudaGetLastError());
-    report_alive_kernel<<<1, 1, 0, s>>>(alive, (unsigned long long *)(ws->h_ctl + CTL_ALIVE));
+    batch_end_kernel<<<fill_grid(ws, nwords), kBlock, 0, s>>>(alive, (unsigned long long *)(ws->h_ctl + CTL_ALIVE),
+                                                               ws->ctl + CTL_BLOCK * p, ws->bitmap[p], nwords);
     ASC_CUDA(cudaGetLastError());
     b->parity = po;
     return ASC_OK;
