@@ -4936,6 +4936,21 @@ void batch_destroy(BatchEngine *b) {
     delete b;
 }
 
+// Empties a batch, on its stream: no source, no frontier (lists, bitmaps, counts,
+// front masks), no masks. A source dropped without this would leave its frontier to
+// whichever source takes its slot next.
+static asc_status batch_clear(BatchEngine *b) {
+    const uint64_t V = b->g->V;
+    b->active = 0;
+    b->pend_n = 0;
+    ASC_CUDA(cudaMemsetAsync(b->ws.ctl, 0, 4 * CTL_WORDS, b->stream));
+    for (auto q : {b->ws.bitmap[0], b->ws.bitmap[1], b->touched})
+        ASC_CUDA(cudaMemsetAsync(q, 0, 4 * (V / 32 + 2), b->stream));
+    ASC_CUDA(cudaMemsetAsync(b->masks, 0, 16 * V, b->stream));
+    ASC_CUDA(cudaMemsetAsync(b->front, 0, 8 * V, b->stream));
+    return ASC_OK;
+}
+
 asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **out) {
     BatchEngine *b = new BatchEngine();
     b->g = g;
@@ -4968,15 +4983,9 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
         if (e != cudaSuccess) st = cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
     if (st == ASC_OK && !sssp) st = ensure_items(g, &b->ws, b->stream);
-    // empty start state: no frontier, zero masks
+    if (st == ASC_OK) st = batch_clear(b);
     if (st == ASC_OK) {
-        cudaError_t e = cudaMemsetAsync(b->ws.ctl, 0, 4 * CTL_WORDS, b->stream);
-        for (int i = 0; i < 2 && e == cudaSuccess; i++)
-            e = cudaMemsetAsync(b->ws.bitmap[i], 0, 4 * (V / 32 + 2), b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->touched, 0, 4 * (V / 32 + 2), b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->masks, 0, 16 * V, b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->front, 0, 8 * V, b->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(b->d_plane, 0, 8 * 64, b->stream);
+        cudaError_t e = cudaMemsetAsync(b->d_plane, 0, 8 * 64, b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         if (e != cudaSuccess) st = cuda_fail(e, "batch init", __FILE__, __LINE__);
     }
@@ -5183,8 +5192,8 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
     std::chrono::steady_clock::time_point done;  // the last iteration's end, on the host
     while (b->active) {
         if ((int64_t)(b->it - it0) >= cap) {
-            // drop the unfinished slots so the engine is reusable
-            b->active = 0;
+            // drop the unfinished sources so the engine is reusable
+            ASC_TRY(batch_clear(b));
             ASC_TRY(batch_finish_rows(b));
             return fail(ASC_ERR_TIMEOUT, "batch has no fixpoint after %u iterations", b->it - it0);
         }

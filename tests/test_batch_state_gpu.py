@@ -1,0 +1,46 @@
+"""What a batch leaves behind for the next one on the same graph."""
+import numpy as np
+import pytest
+
+import ascetic_gb300 as A
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _random_csr(V, ef, seed):
+    rng = np.random.RandomState(seed)
+    src = np.sort(rng.randint(0, V, V * ef))
+    ptr = np.zeros(V + 1, np.uint64)
+    ptr[1:] = np.cumsum(np.bincount(src, minlength=V))
+    return ptr, rng.randint(0, V, V * ef).astype(np.uint32)
+
+
+@pytest.mark.parametrize("frac", [1.0, 0.25])
+@pytest.mark.parametrize("algo", ["bfs", "sssp"])
+def test_capped_batch_leaves_nothing(algo, frac):
+    """A batch stopped by its iteration cap drops its sources: the frontier they
+    had does not go on in the next batch, under the sources that take their slots
+    or beside them."""
+    V = 5003
+    ptr, col = _random_csr(V, 3, 5)
+    edges = col
+    if algo == "sssp":
+        edges = np.stack([col, np.random.RandomState(6).randint(1, 64, len(col)).astype(np.uint32)], 1)
+    ref = oracle.bfs if algo == "bfs" else oracle.sssp
+    old = np.arange(64) * 70 + 3
+    new = np.arange(64) * 71 + 9
+    cap = A.make_params(max_iterations=2)
+    with A.Graph.from_csr(ptr, edges, budget=A.make_budget(frac=frac)) as g:
+        for first, then in ((64, 2), (3, 3), (40, 64), (64, 1)):
+            with pytest.raises(A.AscError) as e:
+                g.run_batch(algo, old[:first], params=cap)
+            assert e.value.status == A.ERR_TIMEOUT
+            for _ in range(2):
+                got, st = g.run_batch(algo, new[:then])
+                for row, s in zip(got, new):
+                    assert np.array_equal(row, ref(ptr, edges, int(s))), (first, then, s)
+                if then == 1:  # one source: every vertex it reaches is expanded, and no other
+                    reached = got[0] < V + 1
+                    deg = np.diff(ptr.astype(np.int64))
+                    assert algo == "sssp" or st["edges_processed"] == deg[reached].sum()
