@@ -3612,6 +3612,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         const int po = 1 - parity;
         ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_BLOCK * po, 0, 4 * CTL_BLOCK, s));
         ASC_CUDA(cudaMemsetAsync(ws->bitmap[po], 0, 4 * (V / 32 + 2), s));
+        if (near_far(g, algo)) ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 4, s));
         if (gather) {
             // the on-demand list and segments go to the host first, so the host
             // gathers while the static region expands on the device
@@ -3680,7 +3681,6 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             launches++;
         } else if (pt.on) {
             // diagnostic: one launch per region, each timed on its own
-            if (near_far(g, algo)) ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 4, s));
             for (int region = 0; region < 2; region++) {
                 const uint64_t items = region_work(region);
                 if (!items) continue;
@@ -3697,7 +3697,6 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
             x.r0 = args_of(parity, 0);
             x.r1 = args_of(parity, 1);
             x.work = x.r0.cnt_out + 4;
-            if (near_far(g, algo)) ASC_CUDA(cudaMemsetAsync(ws->ctl + CTL_MINFAR, 0xff, 4, s));
             fused(s, x, grid_for(ws, items));
             launches++;
             if (algo == ASC_BFS && x.r0.in_ptr) {
