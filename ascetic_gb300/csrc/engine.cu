@@ -4387,10 +4387,13 @@ __device__ __forceinline__ void ms_sssp_load_edge(const RegionArgs &a, uint64_t 
 // Lowers *p to nd when cur, loaded earlier, is larger, and then sets bit in imp:
 // a compare and two predicated instructions. Fire-and-forget: a value lowered
 // further meanwhile is marked all the same, which costs at most one more
-// relaxation. Callers need not test which of a row's sources are active: an
-// inactive source's value at u has not changed since it relaxed this edge, so it
-// does not improve v (715 M warp instructions with those tests and a branch per
-// source on 16.8 M edges of 64 sources, 60% of the issue slots; bound by them).
+// relaxation. Callers need not test which of a row's sources are active at u (715 M
+// warp instructions with those tests and a branch per source on 16.8 M edges of 64
+// sources, 60% of the issue slots; bound by them): every column is one that no edge
+// improves, but for its source's active vertices. A source not active at u has not
+// changed there since it relaxed this edge; a finished one is at its fixpoint; a
+// column without a source holds V + 1 everywhere (batch_create, batch_clear), and
+// V + 1 plus a weight does not wrap (graphs whose weights could are refused).
 __device__ __forceinline__ void relax_min(uint32_t *p, uint32_t nd, uint32_t cur, uint32_t &imp, uint32_t bit) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -4937,8 +4940,10 @@ void batch_destroy(BatchEngine *b) {
 
 // Empties a batch, on its stream: no source, no frontier (lists, bitmaps, counts,
 // front masks), no masks. A source dropped without this would leave its frontier to
-// whichever source takes its slot next.
-static asc_status batch_clear(BatchEngine *b) {
+// whichever source takes its slot next. SSSP: the distance columns of the slots in
+// `columns` become those of a source that reaches nothing, since iterations relax
+// them along with the columns beside them (see relax_min).
+static asc_status batch_clear(BatchEngine *b, uint64_t columns) {
     const uint64_t V = b->g->V;
     b->active = 0;
     b->pend_n = 0;
@@ -4947,6 +4952,11 @@ static asc_status batch_clear(BatchEngine *b) {
         ASC_CUDA(cudaMemsetAsync(q, 0, 4 * (V / 32 + 2), b->stream));
     ASC_CUDA(cudaMemsetAsync(b->masks, 0, 16 * V, b->stream));
     ASC_CUDA(cudaMemsetAsync(b->front, 0, 8 * V, b->stream));
+    if (b->sssp && columns) {
+        cb_clear_kernel<<<fill_grid(&b->ws, V), kBlock, 0, b->stream>>>(b->masks, b->dist, b->stride, b->d_plane,
+                                                                        columns, (uint32_t)V, (uint32_t)V + 1, 1);
+        ASC_CUDA(cudaGetLastError());
+    }
     return ASC_OK;
 }
 
@@ -4982,7 +4992,7 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
         if (e != cudaSuccess) st = cuda_fail(e, "cudaStreamCreate", __FILE__, __LINE__);
     }
     if (st == ASC_OK && !sssp) st = ensure_items(g, &b->ws, b->stream);
-    if (st == ASC_OK) st = batch_clear(b);
+    if (st == ASC_OK) st = batch_clear(b, ~0ull);
     if (st == ASC_OK) {
         cudaError_t e = cudaMemsetAsync(b->d_plane, 0, 8 * 64, b->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -5192,7 +5202,7 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
     while (b->active) {
         if ((int64_t)(b->it - it0) >= cap) {
             // drop the unfinished sources so the engine is reusable
-            ASC_TRY(batch_clear(b));
+            ASC_TRY(batch_clear(b, b->active));
             ASC_TRY(batch_finish_rows(b));
             return fail(ASC_ERR_TIMEOUT, "batch has no fixpoint after %u iterations", b->it - it0);
         }

@@ -44,3 +44,32 @@ def test_capped_batch_leaves_nothing(algo, frac):
                     reached = got[0] < V + 1
                     deg = np.diff(ptr.astype(np.int64))
                     assert algo == "sssp" or st["edges_processed"] == deg[reached].sum()
+
+
+@pytest.mark.parametrize("n", [5, 7, 30, 63])
+def test_sssp_columns_without_a_source(n):
+    """Distance columns that hold no source take no part in a batch, whatever the
+    memory held before: with unit weights and every slot at one vertex, each
+    reached list is read once. Columns that a cap left unfinished likewise."""
+    torch = pytest.importorskip("torch")
+    V = 100003
+    ptr, col = _random_csr(V, 8, n)
+    edges = np.stack([col, np.ones_like(col)], 1)
+    exp = oracle.sssp(ptr, edges, 17)
+    reads = np.diff(ptr.astype(np.int64))[exp < V + 1].sum()
+    with A.Graph.from_csr(ptr, edges) as g:
+        g.run("sssp", 17)  # the single-source state is not what takes the memory below
+        # device memory full of small numbers, returned for the distance rows to take
+        dirty = [torch.randint(1, 2 * V, (64 * V,), dtype=torch.int32, device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        del dirty
+        torch.cuda.empty_cache()
+        for _ in range(2):
+            got, st = g.run_batch("sssp", [17] * n)
+            assert all(np.array_equal(row, exp) for row in got)
+            assert st["edges_processed"] == reads
+        with pytest.raises(A.AscError):
+            g.run_batch("sssp", np.arange(64) * 1500, params=A.make_params(max_iterations=2))
+        got, st = g.run_batch("sssp", [17] * n)
+        assert all(np.array_equal(row, exp) for row in got)
+        assert st["edges_processed"] == reads
