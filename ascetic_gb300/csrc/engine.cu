@@ -4938,6 +4938,18 @@ void batch_destroy(BatchEngine *b) {
     delete b;
 }
 
+// Device memory of a batch. Tests make one of a thread's allocations fail as if
+// memory had run out: the one after t_allocs_left more (negative: none).
+static thread_local int t_allocs_left = -1;
+static asc_status batch_alloc(void **p, uint64_t n) {
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (t_allocs_left != 0) e = cudaMalloc(p, n ? n : 16);
+    if (t_allocs_left >= 0) t_allocs_left--;
+    return e == cudaSuccess ? ASC_OK : cuda_fail(e, "cudaMalloc(batch)", __FILE__, __LINE__);
+}
+
+extern "C" void asc_test_fail_batch_alloc(int after) { t_allocs_left = after; }
+
 // Empties a batch, on its stream: no source, no frontier (lists, bitmaps, counts,
 // front masks), no masks. A source dropped without this would leave its frontier to
 // whichever source takes its slot next. SSSP: the distance columns of the slots in
@@ -4974,9 +4986,7 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
     if (sssp) b->ws.tune.dense_div = 0;  // the SSSP batch walks lists only
     const uint64_t V = g->V;
     auto al = [&](void **p, size_t n) {
-        if (st != ASC_OK) return;
-        cudaError_t e = cudaMalloc(p, n ? n : 16);
-        if (e != cudaSuccess) st = cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
+        if (st == ASC_OK) st = batch_alloc(p, n);
     };
     al((void **)&b->masks, 16 * V);
     al((void **)&b->front, 8 * V);
@@ -5012,7 +5022,7 @@ bool batch_has_plane(BatchEngine *b, uint32_t slot) { return b->sssp || b->plane
 // their level plane; it is allocated here on first use.
 asc_status batch_admit(BatchEngine *b, uint32_t slot, uint32_t source) {
     if (!b->sssp && !b->plane[slot]) {
-        ASC_CUDA(cudaMalloc(&b->plane[slot], 4ull * b->g->V));
+        ASC_TRY(batch_alloc((void **)&b->plane[slot], 4ull * b->g->V));
         ASC_CUDA(cudaMemcpyAsync(b->d_plane, b->plane, 8 * 64, cudaMemcpyHostToDevice, b->stream));
     }
     b->pend_slot[b->pend_n] = slot;
@@ -5174,22 +5184,21 @@ asc_status batch_copy_rows(BatchEngine *b, uint64_t slots, uint32_t *out, bool d
     return ASC_OK;
 }
 
-asc_status batch_finish_rows(BatchEngine *b) {
-    for (auto s : b->out_stream)
-        if (s) ASC_CUDA(cudaStreamSynchronize(s));
-    return ASC_OK;
+// Waits for the rows on their way out.
+cudaError_t batch_finish_rows(BatchEngine *b) {
+    cudaError_t first = cudaSuccess;
+    for (auto s : b->out_stream) {
+        const cudaError_t e = s ? cudaStreamSynchronize(s) : cudaSuccess;
+        if (first == cudaSuccess) first = e;
+    }
+    return first;
 }
 
-// asc_run_batch: all n sources fill slots 0..n-1 of the graph's own batch
-// engine (kept for later batches), then iterations run until every source is
-// done; each finished slot's values are copied to row i of out.
-asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint32_t n, const asc_params &p,
-                     void *out, asc_stats *st) {
-    ASC_TRY(ensure_workspace(g));
+// run_batch on engine b. After ASC_ERR_TIMEOUT b is empty, after any other error
+// its state is undefined; rows may still be on their way out.
+static asc_status run_sources(asc_graph *g, BatchEngine *b, const uint32_t *sources, uint32_t n, const asc_params &p,
+                              void *out, asc_stats *st) {
     Workspace *ws = g->ws;
-    const int k = algo == ASC_SSSP ? 1 : 0;
-    if (!ws->batch[k]) ASC_TRY(batch_create(g, k == 1, 64, &ws->batch[k]));
-    BatchEngine *b = ws->batch[k];
     const uint32_t V = (uint32_t)g->V;
     cudaStream_t s = b->stream;
     ASC_CUDA(cudaMemsetAsync(b->ws.ctl + CTL_STATS, 0, 8 * 6, s));
@@ -5203,24 +5212,18 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
         if ((int64_t)(b->it - it0) >= cap) {
             // drop the unfinished sources so the engine is reusable
             ASC_TRY(batch_clear(b, b->active));
-            ASC_TRY(batch_finish_rows(b));
             return fail(ASC_ERR_TIMEOUT, "batch has no fixpoint after %u iterations", b->it - it0);
         }
-        asc_status rc = batch_launch(b);
         uint64_t fin = 0;
-        if (rc == ASC_OK) rc = batch_collect(b, &fin);
+        ASC_TRY(batch_launch(b));
+        ASC_TRY(batch_collect(b, &fin));
         ASC_CUDA(cudaEventRecord(ws->ev[1], s));
         done = std::chrono::steady_clock::now();
-        if (rc == ASC_OK && want && fin)
-            rc = batch_copy_rows(b, fin, (uint32_t *)out, (p.flags & ASC_RUN_DEVICE_OUT) != 0);
-        if (rc != ASC_OK) {
-            batch_finish_rows(b);  // no copy into the caller's buffer outlives the call
-            return rc;
-        }
+        if (want && fin) ASC_TRY(batch_copy_rows(b, fin, (uint32_t *)out, (p.flags & ASC_RUN_DEVICE_OUT) != 0));
     }
     ASC_CUDA(cudaMemcpyAsync(b->ws.h_ctl + CTL_STATS, b->ws.ctl + CTL_STATS, 8 * 6, cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
-    ASC_TRY(batch_finish_rows(b));
+    ASC_CUDA(batch_finish_rows(b));
     const double copy_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - done).count();
     if (st) {
@@ -5239,6 +5242,27 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
         st->kernel_launches = (uint32_t)(4 * (b->it - it0) + 3);
     }
     return ASC_OK;
+}
+
+// asc_run_batch: all n sources fill slots 0..n-1 of the graph's own batch
+// engine (kept for later batches), then iterations run until every source is
+// done; each finished slot's values are copied to row i of out. An engine that a
+// call left in the middle is not used again: its sources would go on in the next
+// call, and their rows are not that call's.
+asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint32_t n, const asc_params &p,
+                     void *out, asc_stats *st) {
+    ASC_TRY(ensure_workspace(g));
+    const int k = algo == ASC_SSSP ? 1 : 0;
+    BatchEngine *&b = g->ws->batch[k];
+    if (!b) ASC_TRY(batch_create(g, k == 1, 64, &b));
+    const asc_status rc = run_sources(g, b, sources, n, p, out, st);
+    if (rc == ASC_OK) return rc;
+    batch_finish_rows(b);  // no copy into the caller's buffer outlives the call
+    if (rc != ASC_ERR_TIMEOUT) {
+        batch_destroy(b);
+        b = nullptr;
+    }
+    return rc;
 }
 
 // ------------------------------------------------- PageRank over CSR graphs --

@@ -1,4 +1,6 @@
 """What a batch leaves behind for the next one on the same graph."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -73,3 +75,37 @@ def test_sssp_columns_without_a_source(n):
         got, st = g.run_batch("sssp", [17] * n)
         assert all(np.array_equal(row, exp) for row in got)
         assert st["edges_processed"] == reads
+
+
+@pytest.mark.parametrize("algo", ["bfs", "sssp"])
+def test_batch_after_a_failed_one(algo):
+    """A batch that ran out of device memory, at its start or on the way, fails with
+    a status; the next one starts anew, and writes the rows of its own sources only."""
+    V = 5003
+    ptr, col = _random_csr(V, 6, 8)
+    edges = col
+    if algo == "sssp":
+        edges = np.stack([col, np.random.RandomState(6).randint(1, 64, len(col)).astype(np.uint32)], 1)
+    ref = oracle.bfs if algo == "bfs" else oracle.sssp
+    fail_after = A.lib().asc_test_fail_batch_alloc
+    fail_after.argtypes, fail_after.restype = [ctypes.c_int], None
+    src = np.arange(64) * 70 + 3
+    failed = 0
+    for after in list(range(0, 10)) + [40, 60, 68]:
+        with A.Graph.from_csr(ptr, edges, budget=A.make_budget(frac=0.25)) as g:
+            for _ in range(3):
+                fail_after(after)
+                try:
+                    got, _ = g.run_batch(algo, src)
+                    assert all(np.array_equal(got[i], ref(ptr, edges, int(src[i]))) for i in (0, 63))
+                except A.AscError as e:
+                    assert e.status == A.ERR_BUDGET, e
+                    failed += 1
+                finally:
+                    fail_after(-1)
+            buf = np.full((6, V), 0xdeadbeef, np.uint32)
+            g.run_batch(algo, src[5:7], out=buf[2:4])
+            assert np.array_equal(buf[2], ref(ptr, edges, int(src[5]))), after
+            assert np.array_equal(buf[3], ref(ptr, edges, int(src[6]))), after
+            assert (buf[:2] == 0xdeadbeef).all() and (buf[4:] == 0xdeadbeef).all(), after
+    assert failed >= 5
