@@ -172,6 +172,7 @@ void free_workspace(asc_graph *g);
 // continuous multi-source batches (engine.cu)
 uint64_t batch_state_bytes(asc_graph *g, bool sssp, uint32_t stride);
 uint64_t batch_plane_bytes(asc_graph *g);
+uint64_t batch_bytes(const asc_graph *g);
 asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **out);
 void batch_destroy(BatchEngine *b);
 bool batch_has_plane(BatchEngine *b, uint32_t slot);

@@ -4056,7 +4056,8 @@ struct BatchEngine {
     int32_t lvl_off[64] = {0};
     uint32_t *staging = nullptr;      // SSSP column gather [V]
     // asc_run_batch copies finished rows out while later iterations run: two
-    // streams, each with 8 gathered SSSP columns, made on first use
+    // streams, each with 8 gathered SSSP columns (null: memory was short), made
+    // before the first iteration
     cudaStream_t out_stream[2] = {nullptr, nullptr};
     uint32_t *out_rows[2] = {nullptr, nullptr};
     cudaEvent_t out_ready = nullptr;  // the iteration that finished the rows
@@ -4064,6 +4065,7 @@ struct BatchEngine {
     int parity = 0;
     uint32_t it = 0;                  // iterations run so far
     uint64_t active = 0;              // slots in use
+    uint64_t device_bytes = 0;        // beside ws
     uint32_t pend_n = 0, pend_slot[64], pend_src[64];
 };
 
@@ -4941,10 +4943,11 @@ void batch_destroy(BatchEngine *b) {
 // Device memory of a batch. Tests make one of a thread's allocations fail as if
 // memory had run out: the one after t_allocs_left more (negative: none).
 static thread_local int t_allocs_left = -1;
-static asc_status batch_alloc(void **p, uint64_t n) {
+static asc_status batch_alloc(BatchEngine *b, void **p, uint64_t n) {
     cudaError_t e = cudaErrorMemoryAllocation;
     if (t_allocs_left != 0) e = cudaMalloc(p, n ? n : 16);
     if (t_allocs_left >= 0) t_allocs_left--;
+    if (e == cudaSuccess) b->device_bytes += n;
     return e == cudaSuccess ? ASC_OK : cuda_fail(e, "cudaMalloc(batch)", __FILE__, __LINE__);
 }
 
@@ -4986,7 +4989,7 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
     if (sssp) b->ws.tune.dense_div = 0;  // the SSSP batch walks lists only
     const uint64_t V = g->V;
     auto al = [&](void **p, size_t n) {
-        if (st == ASC_OK) st = batch_alloc(p, n);
+        if (st == ASC_OK) st = batch_alloc(b, p, n);
     };
     al((void **)&b->masks, 16 * V);
     al((void **)&b->front, 8 * V);
@@ -5022,7 +5025,7 @@ bool batch_has_plane(BatchEngine *b, uint32_t slot) { return b->sssp || b->plane
 // their level plane; it is allocated here on first use.
 asc_status batch_admit(BatchEngine *b, uint32_t slot, uint32_t source) {
     if (!b->sssp && !b->plane[slot]) {
-        ASC_TRY(batch_alloc((void **)&b->plane[slot], 4ull * b->g->V));
+        ASC_TRY(batch_alloc(b, (void **)&b->plane[slot], 4ull * b->g->V));
         ASC_CUDA(cudaMemcpyAsync(b->d_plane, b->plane, 8 * 64, cudaMemcpyHostToDevice, b->stream));
     }
     b->pend_slot[b->pend_n] = slot;
@@ -5150,23 +5153,51 @@ asc_status batch_fetch(BatchEngine *b, uint32_t slot, void *out, bool device_out
     return ASC_OK;
 }
 
+// Makes what copies rows out, before any source runs: nothing of it can fail in
+// the middle. Buffers of 64 bytes per vertex that do not fit are done without.
+asc_status batch_prepare_rows(BatchEngine *b) {
+    if (!b->out_ready) ASC_CUDA(cudaEventCreateWithFlags(&b->out_ready, cudaEventDisableTiming));
+    for (auto &s : b->out_stream)
+        if (!s) ASC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    if (!b->sssp || b->out_rows[1]) return ASC_OK;
+    asc_status st = ASC_OK;
+    for (auto &q : b->out_rows)
+        if (st == ASC_OK) st = batch_alloc(b, (void **)&q, 32ull * b->g->V);
+    if (st == ASC_OK) return ASC_OK;
+    if (b->out_rows[0]) {
+        ASC_CUDA(cudaFree(b->out_rows[0]));
+        b->out_rows[0] = nullptr;
+        b->device_bytes -= 32ull * b->g->V;
+    }
+    return st == ASC_ERR_BUDGET ? ASC_OK : st;
+}
+
 // Starts copying the rows of the finished slots to out (row i of a slot i) on the
 // engine's output streams, after what its own stream holds so far: their values
 // are final, and later iterations leave them alone. Groups of 8 slots alternate
-// between the streams, so the gather of one overlaps the copy of another.
+// between the streams, so the gather of one overlaps the copy of another. Without
+// buffers for that, SSSP columns go one at a time through the single column's.
 asc_status batch_copy_rows(BatchEngine *b, uint64_t slots, uint32_t *out, bool device_out) {
     const uint64_t V = b->g->V;
     const cudaMemcpyKind kind = device_out ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (!b->out_ready) ASC_CUDA(cudaEventCreateWithFlags(&b->out_ready, cudaEventDisableTiming));
     ASC_CUDA(cudaEventRecord(b->out_ready, b->stream));
+    for (auto s : b->out_stream) ASC_CUDA(cudaStreamWaitEvent(s, b->out_ready, 0));
+    if (b->sssp && !b->out_rows[1]) {
+        cudaStream_t s = b->out_stream[0];
+        for (; slots; slots &= slots - 1) {
+            const uint32_t slot = __builtin_ctzll(slots);
+            cb_gather_column_kernel<<<fill_grid(&b->ws, V), kBlock, 0, s>>>(b->dist, b->stride, slot, b->staging,
+                                                                            (uint32_t)V);
+            ASC_CUDA(cudaGetLastError());
+            ASC_CUDA(cudaMemcpyAsync(out + slot * V, b->staging, 4 * V, kind, s));
+        }
+        return ASC_OK;
+    }
     for (uint32_t group = 0; group < 8; group++) {
         uint32_t cols = (uint32_t)(slots >> (8 * group)) & 0xffu;
         if (!cols) continue;
         const int i = group & 1;
-        if (!b->out_stream[i]) ASC_CUDA(cudaStreamCreateWithFlags(&b->out_stream[i], cudaStreamNonBlocking));
-        if (b->sssp && !b->out_rows[i]) ASC_CUDA(cudaMalloc((void **)&b->out_rows[i], 32 * V));
         cudaStream_t s = b->out_stream[i];
-        ASC_CUDA(cudaStreamWaitEvent(s, b->out_ready, 0));
         if (b->sssp) {
             cb_gather_columns_kernel<<<fill_grid(&b->ws, V), kBlock, 0, s>>>(b->dist, b->stride, group, cols,
                                                                               b->out_rows[i], (uint32_t)V);
@@ -5203,10 +5234,11 @@ static asc_status run_sources(asc_graph *g, BatchEngine *b, const uint32_t *sour
     cudaStream_t s = b->stream;
     ASC_CUDA(cudaMemsetAsync(b->ws.ctl + CTL_STATS, 0, 8 * 6, s));
     ASC_CUDA(cudaEventRecord(ws->ev[0], s));
+    const bool want = out && !(p.flags & ASC_RUN_NO_OUTPUT);
+    if (want) ASC_TRY(batch_prepare_rows(b));
     for (uint32_t i = 0; i < n; i++) ASC_TRY(batch_admit(b, i, sources[i]));
     const uint32_t it0 = b->it;
     const int64_t cap = p.max_iterations > 0 ? p.max_iterations : (int64_t)4 * V + 64;
-    const bool want = out && !(p.flags & ASC_RUN_NO_OUTPUT);
     std::chrono::steady_clock::time_point done;  // the last iteration's end, on the host
     while (b->active) {
         if ((int64_t)(b->it - it0) >= cap) {
@@ -5263,6 +5295,15 @@ asc_status run_batch(asc_graph *g, asc_algo algo, const uint32_t *sources, uint3
         b = nullptr;
     }
     return rc;
+}
+
+// Device bytes of the graph's own batch engines.
+uint64_t batch_bytes(const asc_graph *g) {
+    uint64_t n = 0;
+    if (g->ws)
+        for (auto b : g->ws->batch)
+            if (b) n += b->device_bytes + b->ws.device_bytes;
+    return n;
 }
 
 // ------------------------------------------------- PageRank over CSR graphs --

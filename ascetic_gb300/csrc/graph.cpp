@@ -970,7 +970,7 @@ asc_status asc_graph_info_get(const asc_graph *g, asc_graph_info *info) {
     info->in_head_bytes = 4 * g->in_head_words;
     info->device_edge_bytes = (g->static_edges ? 4ull * edge_store_words(g, g->static_edges) : 0) +
                               info->staging_bytes + info->in_head_bytes;
-    info->device_vertex_bytes = g->device_vertex_bytes + (g->ws ? g->ws->device_bytes : 0);
+    info->device_vertex_bytes = g->device_vertex_bytes + (g->ws ? g->ws->device_bytes : 0) + batch_bytes(g);
     info->host_pinned_bytes = 4ull * edge_store_words(g, g->E);
     info->max_degree = g->max_degree;
     info->max_weight = g->max_weight;

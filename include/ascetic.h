@@ -107,7 +107,8 @@ typedef struct asc_graph_info {
     uint64_t static_edges;        /* edges in the device-resident prefix */
     uint64_t static_vertices;     /* vertices [0, static_vertices) have every edge in the prefix */
     uint64_t device_edge_bytes;   /* static region bytes (what the budget caps) */
-    uint64_t device_vertex_bytes; /* offsets and per-run vertex state (outside the cap) */
+    uint64_t device_vertex_bytes; /* offsets, per-run vertex state and, once asc_run_batch was called,
+                                     its batches' state (outside the cap) */
     uint64_t host_pinned_bytes;   /* pinned host copy of the edge array (on-demand source) */
     uint32_t max_degree;
     uint32_t max_weight;          /* 0 for unweighted graphs */

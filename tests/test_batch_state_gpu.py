@@ -109,3 +109,29 @@ def test_batch_after_a_failed_one(algo):
             assert np.array_equal(buf[3], ref(ptr, edges, int(src[6]))), after
             assert (buf[:2] == 0xdeadbeef).all() and (buf[4:] == 0xdeadbeef).all(), after
     assert failed >= 5
+
+
+@pytest.mark.parametrize("after", [7, 8])
+def test_sssp_rows_without_copy_buffers(after):
+    """Where the buffers that several columns leave through do not fit, columns leave
+    one at a time: the batch still succeeds. The state's bytes are reported."""
+    V = 3001
+    ptr, col = _random_csr(V, 6, 8)
+    edges = np.stack([col, np.random.RandomState(6).randint(1, 64, len(col)).astype(np.uint32)], 1)
+    src = np.arange(64) * 40 + 3
+    fail_after = A.lib().asc_test_fail_batch_alloc
+    fail_after.argtypes, fail_after.restype = [ctypes.c_int], None
+    with A.Graph.from_csr(ptr, edges) as g:
+        exp = np.stack([g.run("sssp", int(s))[0] for s in src])
+        before = g.refresh_info().device_vertex_bytes
+        fail_after(after)  # the state is seven allocations
+        try:
+            got, _ = g.run_batch("sssp", src)
+        finally:
+            fail_after(-1)
+        assert np.array_equal(got, exp)
+        short = g.refresh_info().device_vertex_bytes
+        assert short - before >= (256 + 28) * V
+        got, _ = g.run_batch("sssp", src)
+        assert np.array_equal(got, exp)
+        assert g.refresh_info().device_vertex_bytes - short == 64 * V
