@@ -156,8 +156,8 @@ struct RegionArgs {
 // region bit counts of the previous step, upper bounds) holds more than
 // V / bu_div vertices. The top-down and bottom-up kernels of an iteration both
 // evaluate it from the same counts and exactly one of them does the work.
-__device__ __forceinline__ bool bottom_up_step(const RegionArgs &a) {
-    return a.in_ptr && a.bu_div && ((uint64_t)a.cnt_in[6] + a.cnt_in[7]) * a.bu_div > a.V;
+__device__ __forceinline__ bool bottom_up_step(const RegionArgs &a, const uint32_t *cnt) {
+    return a.in_ptr && a.bu_div && ((uint64_t)cnt[6] + cnt[7]) * a.bu_div > a.V;
 }
 
 // Adds the n edges read from [b, b + n) to their 4096-edge fragments' counters.
@@ -534,13 +534,14 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 #define ASC_MIN_TILE 8
 #endif
 constexpr uint32_t kMinTile = ASC_MIN_TILE;
-__device__ __forceinline__ void region_items_bits(const RegionArgs &a, uint32_t &n_in, uint32_t &nseg,
-                                                  uint32_t &items, bool &bitmap, uint32_t &per) {
+// cnt: the frontier's counts (a.cnt_in or a copy).
+__device__ __forceinline__ void region_items_bits(const RegionArgs &a, const uint32_t *cnt, uint32_t &n_in,
+                                                  uint32_t &nseg, uint32_t &items, bool &bitmap, uint32_t &per) {
     const uint32_t range = a.dense_end - a.dense_begin;
-    const uint32_t bits = a.cnt_in[6 + a.region];
-    nseg = a.cnt_in[2 + a.region];
+    const uint32_t bits = cnt[6 + a.region];
+    nseg = cnt[2 + a.region];
     bitmap = a.bitmap_in && a.dense_div && bits > range / a.dense_div;
-    n_in = bitmap ? 0 : a.cnt_in[a.region];
+    n_in = bitmap ? 0 : cnt[a.region];
     const uint32_t nvert = bitmap ? a.dense_end - (a.dense_begin & ~31u) : n_in;
     per = bitmap ? kBlock : min((uint32_t)kBlock, max(kMinTile, (n_in + gridDim.x - 1) / gridDim.x));
     items = nseg + (nvert + per - 1) / per;
@@ -752,14 +753,14 @@ __device__ __forceinline__ void flush_expansion(const RegionArgs &a, uint32_t *s
 
 template <int ALG, int WORDS>
 __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_kernel(RegionArgs a) {
-    if (ALG == kBFS && bottom_up_step(a)) return;
+    if (ALG == kBFS && bottom_up_step(a, a.cnt_in)) return;
     __shared__ ExpandSmem<WORDS> sm;
     __shared__ uint32_t s_next[kNextWords], s_work;
     if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     uint32_t n_in, nseg, total;
     bool bitmap;
     uint32_t per;
-    region_items_bits(a, n_in, nseg, total, bitmap, per);
+    region_items_bits(a, a.cnt_in, n_in, nseg, total, bitmap, per);
     const uint32_t thresh = ALG == kSSSP && a.far_bits ? *a.thresh : 0u;
     for (;;) {
         if (threadIdx.x == 0) s_work = atomicAdd(a.work, 1u);
@@ -782,15 +783,15 @@ struct FusedArgs {
 };
 
 // A CTA's first item is its own number; later ones come from the cursor, which
-// starts behind them.
+// starts behind them. cnt: the frontier's counts.
 template <int ALG, int WORDS>
-__device__ __forceinline__ void expand_regions(const FusedArgs &x, uint32_t thresh, ExpandSmem<WORDS> &sm,
-                                               uint32_t *s_next) {
+__device__ __forceinline__ void expand_regions(const FusedArgs &x, const uint32_t *cnt, uint32_t thresh,
+                                               ExpandSmem<WORDS> &sm, uint32_t *s_next) {
     __shared__ uint32_t s_work;
     uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(x.r0, n0, s0, i0, m0, t0);
-    region_items_bits(x.r1, n1, s1, i1, m1, t1);
+    region_items_bits(x.r0, cnt, n0, s0, i0, m0, t0);
+    region_items_bits(x.r1, cnt, n1, s1, i1, m1, t1);
     const uint32_t m = min(i0, i1), total = i0 + i1;
     if (threadIdx.x < kNextWords) s_next[threadIdx.x] = 0;
     __syncthreads();
@@ -816,10 +817,10 @@ __device__ __forceinline__ void expand_regions(const FusedArgs &x, uint32_t thre
 
 template <int ALG, int WORDS>
 __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_kernel(FusedArgs x) {
-    if (ALG == kBFS && bottom_up_step(x.r0)) return;
+    if (ALG == kBFS && bottom_up_step(x.r0, x.r0.cnt_in)) return;
     __shared__ ExpandSmem<WORDS> sm;
     __shared__ uint32_t s_next[kNextWords];
-    expand_regions<ALG, WORDS>(x, ALG == kSSSP && x.r0.far_bits ? *x.r0.thresh : 0u, sm, s_next);
+    expand_regions<ALG, WORDS>(x, x.r0.cnt_in, ALG == kSSSP && x.r0.far_bits ? *x.r0.thresh : 0u, sm, s_next);
 }
 
 // Bottom-up BFS step (direction-optimizing BFS): every vertex not yet reached
@@ -996,7 +997,7 @@ __device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nw
 }
 
 __global__ void __launch_bounds__(kBlock, kBuMinBlocks) bottom_up_kernel(RegionArgs a, uint32_t nwords, uint32_t nv) {
-    if (!bottom_up_step(a)) return;
+    if (!bottom_up_step(a, a.cnt_in)) return;
     __shared__ uint32_t s_next[kNextWords];
     __shared__ BuSmem bs;
     bottom_up_words(a, nwords, nv, bs, s_next);
@@ -1335,8 +1336,13 @@ constexpr uint64_t kReportedValues = 16384;
 constexpr uint32_t kBarrierPolls = 1u << 25;
 
 // Barrier over the grid: arrivals count up from zero for the whole launch.
-// False when the other CTAs did not arrive in time.
-__device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target) {
+// False when the other CTAs did not arrive in time. Where counts is given, the
+// CTL_BLOCK words there (16-byte aligned) are read once for the CTA into s_counts:
+// with every warp of 912 CTAs reading them for itself, those reads of one line cost
+// more than the barrier (an iteration of a BFS that reaches 700 vertices at a time
+// on a grid graph of a million: 18 us, 13.5 so).
+__device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target, const uint32_t *counts = nullptr,
+                                             uint32_t *s_counts = nullptr) {
     __shared__ uint32_t s_ok;
     __syncthreads();
     target += gridDim.x;
@@ -1353,6 +1359,12 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target) {
         s_ok = (int32_t)(now - target) >= 0;
         if (!s_ok) atomicExch(ctl + CTL_TIMEOUT, 2u);
         __threadfence();
+        if (counts) {
+            const uint4 a = __ldcg(reinterpret_cast<const uint4 *>(counts));
+            const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(counts) + 1);
+            reinterpret_cast<uint4 *>(s_counts)[0] = a;
+            reinterpret_cast<uint4 *>(s_counts)[1] = b;
+        }
     }
     __syncthreads();
     return s_ok != 0;
@@ -1480,19 +1492,20 @@ struct LoopState {
 
 enum LoopNext { kLoopGo, kLoopEnd, kLoopStuck };
 
-// One iteration from the frontier that x reads; y's arguments write that
-// frontier's lists (the other parity).
 template <int WORDS>
 union LoopSmem {
     ExpandSmem<WORDS> expand;
     BuSmem bottom_up;
 };
 
+// One iteration from the frontier that x reads; y's arguments write that
+// frontier's lists (the other parity). cin: shared, its counts; the next one's
+// when the iteration ends.
 template <int ALG, int WORDS>
 __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const FusedArgs &x, const FusedArgs &y,
-                                                   LoopState &st, LoopSmem<WORDS> &sm, uint32_t *s_next) {
+                                                   LoopState &st, LoopSmem<WORDS> &sm, uint32_t *s_next,
+                                                   uint32_t *cin) {
     const RegionArgs &a = x.r0;
-    volatile const uint32_t *cin = a.cnt_in;
     if (ALG == kCC && l.first_label && !st.promotions && (!(cin[6] | cin[7]) || st.it >= l.first_cap)) {
         // the frontier of the remaining labels, in place of an empty one or beside
         // what the first label still has to reach
@@ -1500,15 +1513,14 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
         if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;  // every thread has read the counts
         if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
         seed_unlabelled(a, y.r0.bitmap, l.src, l.ctl + CTL_PROMOTED);
-        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
-        volatile const uint32_t *moved = l.ctl + CTL_PROMOTED;
-        const uint32_t n0 = moved[0], n1 = moved[1];
+        if (!grid_barrier(l.ctl, st.target, l.ctl + CTL_PROMOTED, cin)) return kLoopStuck;
+        const uint32_t n0 = cin[0], n1 = cin[1];
         build_frontier(y.r0, y.r0.bitmap, l.nwords, n0, n1);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             y.r0.cnt_out[6] = n0;
             y.r0.cnt_out[7] = n1;
         }
-        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+        if (!grid_barrier(l.ctl, st.target, a.cnt_in, cin)) return kLoopStuck;
     }
     if (!(cin[6] | cin[7])) {
         if (ALG != kSSSP || !a.far_bits) return kLoopEnd;
@@ -1537,39 +1549,40 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
             y.r0.cnt_out[6] = n0;
             y.r0.cnt_out[7] = n1;
         }
-        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+        if (!grid_barrier(l.ctl, st.target, a.cnt_in, cin)) return kLoopStuck;
     }
     if (st.it >= l.cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) l.ctl[CTL_TIMEOUT] = 1;
         return kLoopEnd;
     }
     st.it++;
-    if (ALG == kBFS && bottom_up_step(a)) bottom_up_words(a, l.nwords, st.it + 1, sm.bottom_up, s_next);
-    else expand_regions<ALG, WORDS>(x, st.thresh, sm.expand, s_next);
-    if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
-    build_frontier(a, a.bitmap, l.nwords, a.cnt_out[6], a.cnt_out[7]);
+    if (ALG == kBFS && bottom_up_step(a, cin)) bottom_up_words(a, l.nwords, st.it + 1, sm.bottom_up, s_next);
+    else expand_regions<ALG, WORDS>(x, cin, st.thresh, sm.expand, s_next);
+    if (!grid_barrier(l.ctl, st.target, a.cnt_out, cin)) return kLoopStuck;
+    build_frontier(a, a.bitmap, l.nwords, cin[6], cin[7]);
     // the input frontier's bitmap and counts are the next output's
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < l.nwords; w += gridDim.x * blockDim.x)
         y.r0.bitmap[w] = 0;
     if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
-    return grid_barrier(l.ctl, st.target) ? kLoopGo : kLoopStuck;
+    return grid_barrier(l.ctl, st.target, a.cnt_out, cin) ? kLoopGo : kLoopStuck;
 }
 
 template <int ALG, int WORDS>
 __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const __grid_constant__ LoopArgs l) {
     __shared__ LoopSmem<WORDS> sm;
     __shared__ uint32_t s_next[kNextWords];
+    __shared__ alignas(16) uint32_t cin[CTL_BLOCK];
     LoopState st;
     st.thresh = l.thresh;
     loop_setup<ALG>(l);
-    if (!grid_barrier(l.ctl, st.target)) return;
+    if (!grid_barrier(l.ctl, st.target, l.x0.r0.cnt_in, cin)) return;
     if (l.all) {
-        build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords, l.x1.r0.cnt_out[6], l.x1.r0.cnt_out[7]);
-        if (!grid_barrier(l.ctl, st.target)) return;
+        build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords, cin[6], cin[7]);
+        if (!grid_barrier(l.ctl, st.target, l.x0.r0.cnt_in, cin)) return;
     }
     for (;;) {
-        LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, s_next);
-        if (n == kLoopGo) n = loop_iteration<ALG, WORDS>(l, l.x1, l.x0, st, sm, s_next);
+        LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, s_next, cin);
+        if (n == kLoopGo) n = loop_iteration<ALG, WORDS>(l, l.x1, l.x0, st, sm, s_next, cin);
         if (n == kLoopStuck) return;
         if (n == kLoopEnd) break;
     }
@@ -1830,8 +1843,8 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_MIN_BLOCKS) pr_pull_lists_kerne
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
     uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool b0, b1;
-    region_items_bits(p0.r, n0, s0, i0, b0, t0);
-    region_items_bits(p1.r, n1, s1, i1, b1, t1);
+    region_items_bits(p0.r, p0.r.cnt_in, n0, s0, i0, b0, t0);
+    region_items_bits(p1.r, p1.r.cnt_in, n1, s1, i1, b1, t1);
     if (!(regions & 1u)) i0 = 0;
     if (!(regions & 2u)) i1 = 0;
     const uint32_t m = min(i0, i1), total = i0 + i1;
@@ -4287,8 +4300,8 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_BFS_BLOCKS) ms_bfs_expand_kerne
     if (threadIdx.x < 4) counts[threadIdx.x] = 0;
     uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(m.r0, n0, s0, i0, m0, t0);
-    region_items_bits(m.r1, n1, s1, i1, m1, t1);
+    region_items_bits(m.r0, m.r0.cnt_in, n0, s0, i0, m0, t0);
+    region_items_bits(m.r1, m.r1.cnt_in, n1, s1, i1, m1, t1);
     const uint32_t mm = min(i0, i1), total = i0 + i1;
     for (;;) {
         if (threadIdx.x == 0) s_work = atomicAdd(m.work, 1u);
@@ -4651,8 +4664,8 @@ __global__ void __launch_bounds__(kBlock, ASC_MS_MIN_BLOCKS) ms_sssp_expand_kern
     __shared__ MsSsspSmem sm;
     uint32_t n0, s0, i0, t0, n1, s1, i1, t1;
     bool m0, m1;
-    region_items_bits(m.r0, n0, s0, i0, m0, t0);
-    region_items_bits(m.r1, n1, s1, i1, m1, t1);
+    region_items_bits(m.r0, m.r0.cnt_in, n0, s0, i0, m0, t0);
+    region_items_bits(m.r1, m.r1.cnt_in, n1, s1, i1, m1, t1);
     const uint32_t mm = min(i0, i1), total = i0 + i1;
     for (;;) {
         if (threadIdx.x == 0) sm.work = atomicAdd(m.work, 1u);
