@@ -2690,16 +2690,27 @@ TraverseFn pick_traverse(asc_algo algo, int layout) {
 #ifndef ASC_LOOP_EDGES
 #define ASC_LOOP_EDGES 8192
 #endif
-// CTAs of the persistent loop: all that stay resident, or one per
-// ASC_LOOP_EDGES edges of a small graph, since a barrier costs by its arrivals: BFS
-// on 65,536 / 200,000 vertices of degree 8 took 116 / 149 us at 1024, 99 / 144 at
-// 2048, 93 / 104 at 4096, 93 / 89 at 8192.
+// CTAs of the persistent loop: all that stay resident, or on a small graph one per
+// ASC_LOOP_EDGES edges and vertices, since a barrier costs by its arrivals. Connected
+// components read most lists in many iterations: one per 2048. SSSP without thresholds
+// does on some graphs: one per 2048 up to 256 CTAs. us at one per 1024 / 2048 / 4096 /
+// 8192:
+//   BFS   grid of 300 x 300   4826 / 4336 / 4204 / 4201   RMAT scale 16   110 / 88 / 86 / 78
+//   SSSP  grid of 300 x 300   5246 / 4899 / 6206 / 8738   RMAT scale 16   196 / 172 / 172 / 191
+//   CC    grid of 300 x 300   7655 / 7234 / 9179 / 13805  RMAT scale 16   159 / 139 / 147 / 163
+//   CC    path of 4000       38899 / 38902 / 50757 / 61712
+// and on 131,072 rings of 8 at 2048 / 4096 / 8192 (912, 768, 384 CTAs): SSSP 131 / 119 /
+// 108, CC 193 / 192 / 228 (every vertex at once).
 asc_status loop_grid(asc_graph *g, asc_algo algo, TraverseFn fn, uint32_t *grid) {
     Workspace *ws = g->ws;
     int &per_sm = ws->loop_per_sm[algo];
     if (!per_sm) ASC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0));
     const uint64_t resident = (uint64_t)ws->num_sms * std::max(1, std::min(per_sm, (int)ws->tune.ctas_per_sm));
-    *grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(resident, (g->E + g->V) / ASC_LOOP_EDGES + 1));
+    const uint64_t n = g->E + g->V;
+    uint64_t ctas = n / ASC_LOOP_EDGES + 1;
+    if (algo == ASC_CC) ctas = n / 2048 + 1;
+    else if (algo == ASC_SSSP && !near_far(g, algo)) ctas = std::max(ctas, std::min<uint64_t>(256, n / 2048 + 1));
+    *grid = (uint32_t)std::min(resident, ctas);
     return ASC_OK;
 }
 
