@@ -68,6 +68,7 @@ struct Workspace {
     size_t pr_elem = 0;
     uint2 *items = nullptr;          // first (row, edge) of each merge item
     uint32_t n_items_static = 0, n_items = 0;
+    uint32_t item_div = 0;           // items while more than 1 / item_div of a region is active
     unsigned long long *pr_hot = nullptr;  // scatter passes: most frequent destinations
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> phase_events;
@@ -129,6 +130,7 @@ struct asc_graph {
         uint32_t huge_degree = 0, segment_edges = 0;
         std::vector<uint32_t> bits;  // one bit per vertex, set for the long lists (V/32+2 words)
         uint64_t seg_static = 0, seg_ondemand = 0;  // segments of the static / on-demand long lists
+        bool even = false;          // equal numbers of vertices have nearly equal numbers of edges
     };
     std::vector<LongLists> long_lists;
     std::mutex long_lists_mu;

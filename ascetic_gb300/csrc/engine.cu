@@ -150,6 +150,7 @@ struct RegionArgs {
     const uint2 *items;
     uint32_t item_begin, item_n;
     uint64_t edge_words;
+    uint32_t item_div;            // by items while more than 1 / item_div of the region is active
 };
 
 // True when this BFS iteration steps bottom-up: its input frontier (the
@@ -237,6 +238,21 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t &total,
     __syncthreads();
     total = s_warp[kWarps];
     return s_warp[w] + incl - x;
+}
+
+// Whether a region walked in id order goes by merge items or by tiles. Items hold
+// equal work whatever the degrees; one with few active rows costs nearly as much to
+// set up as a full one, a tile only its active edges, but a tile of kBlock vertices
+// holds more edges than an item where degrees are high. So where the tiles of a graph
+// are even (see kEvenTiles), items are for frontiers of over a quarter of the region
+// at 8 edges per vertex and above, of over a sixteenth from 3 on, and for every dense
+// frontier below. us, items for every dense frontier / above 1/16 / 1/8 / 1/4 / 1/2:
+//   uniform random, 6 M vertices of 16: SSSP 6265 / 5715 / 5185 / 4808 / 4691
+//   2 M of 8: SSSP 1468 / 1417 / 1384 / 1377 / 1375; of 4: 1067 / 1075 / 1077 / 1128 / 1151
+//   of 2: 1073 / 1141 / 1205 / 1316 / 1313; grid of 1000 x 1000: 30420 / 29239 / 28998 /
+//   28982 / 28986; RMAT scale 20 (uneven): CC 331 / 388 / 392 / 390 / 416
+__device__ __forceinline__ bool by_items(const RegionArgs &a, uint32_t bits, uint32_t range) {
+    return a.items && (uint64_t)bits * a.item_div > range;
 }
 
 // Merge items: a region's rows (each counted at its end) and edges in their
@@ -534,7 +550,7 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 #define ASC_MIN_TILE 8
 #endif
 constexpr uint32_t kMinTile = ASC_MIN_TILE;
-// cnt: the frontier's counts (a.cnt_in or a copy).
+// cnt: the frontier's counts (a.cnt_in or a copy). per is 0 for merge items.
 __device__ __forceinline__ void region_items_bits(const RegionArgs &a, const uint32_t *cnt, uint32_t &n_in,
                                                   uint32_t &nseg, uint32_t &items, bool &bitmap, uint32_t &per) {
     const uint32_t range = a.dense_end - a.dense_begin;
@@ -545,8 +561,8 @@ __device__ __forceinline__ void region_items_bits(const RegionArgs &a, const uin
     const uint32_t nvert = bitmap ? a.dense_end - (a.dense_begin & ~31u) : n_in;
     per = bitmap ? kBlock : min((uint32_t)kBlock, max(kMinTile, (n_in + gridDim.x - 1) / gridDim.x));
     items = nseg + (nvert + per - 1) / per;
-    if (bitmap && a.items) {
-        nseg = 0;
+    if (bitmap && by_items(a, bits, range)) {
+        per = nseg = 0;
         items = a.item_n;
     }
 }
@@ -732,7 +748,7 @@ __device__ __forceinline__ void expand_item(const RegionArgs &a, uint32_t w, uin
                                             bool bitmap, uint32_t per, ExpandSmem<WORDS> &sm, uint32_t *s_next,
                                             uint32_t thresh) {
     if (w < nseg) expand_segment<ALG, WORDS>(a, a.seg_in[w], s_next, thresh);
-    else if (bitmap && a.items) expand_merge_item<ALG, WORDS>(a, a.item_begin + w, sm.item, s_next, thresh);
+    else if (!per) expand_merge_item<ALG, WORDS>(a, a.item_begin + w, sm.item, s_next, thresh);
     else expand_tile<ALG, WORDS>(a, w - nseg, n_in, bitmap, per, sm.tile, s_next, thresh);
 }
 
@@ -1079,8 +1095,8 @@ __device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32
         else smask = (1u << (a.S - v0)) - 1u;
         // long lists: one thread per vertex appends its segments (rare); merge
         // items need none
-        if (a.items && !list0) hw &= ~smask;
-        if (a.items && !list1) hw &= smask;
+        if (!list0 && by_items(a, bits0, range0)) hw &= ~smask;
+        if (!list1 && by_items(a, bits1, range1)) hw &= smask;
         while (hw) {
             const int b = __ffs(hw) - 1;
             hw &= hw - 1;
@@ -2296,6 +2312,11 @@ __global__ void pr_rank_to_float_kernel(const double *rank, float *out, uint32_t
 
 // --------------------------------------------------------------- host -------
 
+// A graph's tiles are even when none of kBlock vertices holds more than kEvenTiles
+// times the mean edges (uniform random graphs, grids, rings: at most 1.2 times; RMAT
+// scale 10: 2.3 times, 16: 29, 22: 350).
+constexpr uint64_t kEvenTiles = 2;
+
 // Sizes and allocates the frontier machinery of one run for graph g, with
 // the graph's tuning or (graph_tuning false) the default thresholds.
 asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true) {
@@ -2360,6 +2381,10 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
             ll.seg_static += sums[2 * k];
             ll.seg_ondemand += sums[2 * k + 1];
         }
+        uint64_t most = 0;
+        for (uint64_t v = 0; v < V; v += kBlock)
+            most = std::max<uint64_t>(most, ptr[std::min<uint64_t>(V, v + kBlock)] - ptr[v]);
+        ll.even = most * V <= kEvenTiles * g->E * std::min<uint64_t>(kBlock, V);
         ll.huge_degree = t.huge_degree;
         ll.segment_edges = t.segment_edges;
     }
@@ -2368,6 +2393,7 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
     const uint64_t cs = ll.seg_static, co = ll.seg_ondemand;
     ws->segcap_static = cs;
     ws->segcap_ondemand = co;
+    ws->item_div = ll.even && g->E >= 8 * V ? 4 : ll.even && g->E >= 3 * V ? 16 : 0xffffffffu;
     uint64_t bytes = 0;
     auto dalloc = [&](void **p, size_t n) -> asc_status {
         n = n ? n : 16;
@@ -2559,6 +2585,7 @@ bool near_far(asc_graph *g, asc_algo algo) { return algo == ASC_SSSP && g->ws->t
 
 void attach_items(const Workspace *ws, RegionArgs &a) {
     a.items = ws->items;
+    a.item_div = ws->item_div;
     a.item_begin = a.region == 0 ? 0 : ws->n_items_static;
     a.item_n = a.region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
 }
@@ -3613,7 +3640,8 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     auto region_work = [&](int region) -> uint64_t {
         const uint32_t range = region == 0 ? g->static_vertices : V - g->static_vertices;
         const bool bitmap_mode = div && cnt[6 + region] > range / div;
-        if (bitmap_mode && !part) return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
+        if (bitmap_mode && !part && (uint64_t)cnt[6 + region] * ws->item_div > range)
+            return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
         const uint32_t per = bitmap_mode ? (uint32_t)kBlock : kMinTile;
         return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + per - 1) / per;
     };
@@ -4291,7 +4319,7 @@ __device__ __forceinline__ void ms_item(const MsArgs &m, const RegionArgs &a, ui
                                         uint32_t *counts) {
     if (w < nseg) {
         ms_segment<WORDS>(m, a, a.seg_in[w]);
-    } else if (bitmap && a.items) {
+    } else if (!per) {
         ms_merge_item<WORDS>(m, a, a.item_begin + w, sm.item, counts);
     } else if (!bitmap) {
         const uint32_t i = (w - nseg) * per + threadIdx.x;
