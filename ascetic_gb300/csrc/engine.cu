@@ -1342,6 +1342,14 @@ struct LoopArgs {
 };
 
 constexpr uint32_t kFirstLabelIterations = 32;
+// A first label that reaches fewer than this many vertices in its second iteration
+// follows a thread (a path, a ring, the corner of a grid): the rest joins then. 131,072
+// rings of 8 vertices: 5 iterations from every vertex at once 193 us, after the first
+// label's own 5 265, after 2 of them 222.
+constexpr uint32_t kFirstLabelLeast = 4;
+__host__ __device__ __forceinline__ bool rest_joins(uint32_t it, uint64_t frontier, uint32_t first_cap) {
+    return !frontier || it >= first_cap || (it == 2 && frontier < kFirstLabelLeast);
+}
 // Results of at most this many values come back with the report and are copied
 // from there on the host: the copy engine's latency is longer (BFS on 1,001
 // vertices: 11 to 14 us of 80).
@@ -1522,7 +1530,8 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
                                                    LoopState &st, LoopSmem<WORDS> &sm, uint32_t *s_next,
                                                    uint32_t *cin) {
     const RegionArgs &a = x.r0;
-    if (ALG == kCC && l.first_label && !st.promotions && (!(cin[6] | cin[7]) || st.it >= l.first_cap)) {
+    if (ALG == kCC && l.first_label && !st.promotions &&
+        rest_joins(st.it, (uint64_t)cin[6] + cin[7], l.first_cap)) {
         // the frontier of the remaining labels, in place of an empty one or beside
         // what the first label still has to reach
         st.promotions = 1;
@@ -3646,7 +3655,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + per - 1) / per;
     };
     while ((cnt[6] | cnt[7]) || rest_waits) {
-        if (rest_waits && (!(cnt[6] | cnt[7]) || iters >= (int)kFirstLabelIterations)) {
+        if (rest_waits && rest_joins((uint32_t)iters, (uint64_t)cnt[6] + cnt[7], kFirstLabelIterations)) {
             rest_waits = false;
             RegionArgs a = args_of(1 - parity, 0);  // writes this parity's lists
             ASC_CUDA(cudaMemsetAsync(a.cnt_out, 0, 4 * CTL_BLOCK, s));
