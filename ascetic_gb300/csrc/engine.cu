@@ -150,6 +150,7 @@ struct RegionArgs {
     const uint2 *items;
     uint32_t item_begin, item_n;
     uint64_t edge_words;
+    uint64_t in_words;            // words that may be read at in_edges
     uint32_t item_div;            // by items while more than 1 / item_div of the region is active
 };
 
@@ -863,58 +864,91 @@ constexpr int kBuUnroll = ASC_BU_UNROLL;
 #endif
 constexpr int kBuWords = ASC_BU_WORDS;
 // CTAs per SM the bottom-up kernel is compiled for; its grid is one wave of
-// them. RMAT scale 24, 25% budget: 352.4 GTEPS at 8 (32 registers), 336.4 at 6
-// (40), 303.8 at 4 (48); with 2 in-edges per scan step instead of 4, 351.0; with
-// 2 words per pass, 335.6 (all at 6 except the first). At 8, 2 in-edges per scan
-// step measured 330.6 against 343.5 for 4.
+// them: at 8 it would spill (6 M vertices of 16 random neighbours, 25% resident,
+// host-driven loop: 2.93 ms at 8, 2.73 at 6; RMAT scale 22: 0.652 and 0.655).
 #ifndef ASC_BU_MIN_BLOCKS
-#define ASC_BU_MIN_BLOCKS 8
+#define ASC_BU_MIN_BLOCKS 6
 #endif
 constexpr int kBuMinBlocks = ASC_BU_MIN_BLOCKS;
 
-// Vertices whose first in-edge is no parent wait in a queue per warp until 32 of
-// them scan their further in-edges together (in_ptr, then host memory): such a
-// vertex costs a chain of three dependent reads, and a word of 32 vertices holds
-// only a few (BFS on RMAT scale 24: 651 us a word at a time, 575 queued).
+// Vertices whose first in-edge is no parent scan the others: a chain of three
+// dependent reads (in_ptr, then host memory). A word of 32 vertices with kBuDirect of
+// them or more scans at once, as one run of lists; fewer wait in a queue per warp
+// until 32 scan together (BFS on RMAT scale 24: 651 us a word at a time, 575 queued).
+constexpr uint32_t kBuDirect = 24;
 struct BuSmem {
-    uint32_t queue[kWarps][32 + 32 * kBuWords];
+    uint32_t queue[kWarps][32 + (kBuDirect - 1) * kBuWords];
+    uint32_t open[kWarps][kBuWords];  // of a word that scans at once: its vertices
 };
 
-// The further in-edges of up to 32 queued vertices (lanes below n). Returns
-// whether this lane's was found.
-__device__ __forceinline__ bool bottom_up_scan(const RegionArgs &a, const uint32_t *queue, uint32_t n, uint32_t nv,
-                                               uint32_t &v, uint32_t &scanned) {
-    const uint32_t lane = threadIdx.x & 31;
-    bool found = false;
-    v = 0;
-    if (lane < n) {
-        v = queue[lane];
-        uint32_t i = a.in_ptr[v];
-        const uint32_t e = a.in_ptr[v + 1];
+// Whether an in-edge of v after its first comes from the frontier, in the lanes that
+// want to know. Lists in host memory are read 16 aligned bytes at a time: word by
+// word, their sectors came over the link again and again, as often as the L1 had lost
+// them meanwhile (2 M vertices of 16 random neighbours, 25% resident: 10.0 M sectors
+// for 62 MB of lists, BFS 2.85 ms; 1.68 so). Resident lists come from L2, where that
+// costs little and the fewer instructions count (500,009 vertices of a rewired ring,
+// host-driven loop: 1.75 ms a word at a time, 1.91 by 16 bytes).
+__device__ __forceinline__ bool bottom_up_scan(const RegionArgs &a, bool want, uint32_t v, uint32_t &scanned) {
+    const uint32_t eb = a.in_ebits, mask = eb >= 32 ? 0xffffffffu : (1u << eb) - 1u;
+    uint32_t i = 0, e = 0;
+    if (want) {
+        i = a.in_ptr[v];
+        e = a.in_ptr[v + 1];
         if (a.in_heads && i < e) i++;  // the head was the first
+    }
+    bool found = false;
+    if (a.in_resident) {
         for (; i < e && !found; i += kBuUnroll) {
             uint32_t u[kBuUnroll];
             bool in[kBuUnroll];
 #pragma unroll
-            for (int q = 0; q < kBuUnroll; q++) {
-                u[q] = i + q < e ? edge_word(a.in_edges, (uint64_t)i + q, a.in_ebits) : 0xffffffffu;
-                if (u[q] != 0xffffffffu && ASC_BAD(u[q] >= a.V, 17, u[q])) u[q] = 0xffffffffu;
+            for (int k = 0; k < kBuUnroll; k++) {
+                u[k] = i + k < e ? edge_word(a.in_edges, (uint64_t)i + k, eb) : 0xffffffffu;
+                if (u[k] != 0xffffffffu && ASC_BAD(u[k] >= a.V, 17, u[k])) u[k] = 0xffffffffu;
             }
 #pragma unroll
-            for (int q = 0; q < kBuUnroll; q++)
-                in[q] = u[q] != 0xffffffffu && ((a.bitmap_in[u[q] >> 5] >> (u[q] & 31)) & 1u);
+            for (int k = 0; k < kBuUnroll; k++)
+                in[k] = u[k] != 0xffffffffu && ((a.bitmap_in[u[k] >> 5] >> (u[k] & 31)) & 1u);
             // edges read count up to the parent
 #pragma unroll
-            for (int q = 0; q < kBuUnroll; q++)
-                if (!found && i + q < e) {
+            for (int k = 0; k < kBuUnroll; k++)
+                if (!found && i + k < e) {
                     scanned++;
-                    found = in[q];
+                    found = in[k];
                 }
         }
-        if (found) {
-            a.val[v] = nv;
-            atomicOr(&a.visited[v >> 5], 1u << (v & 31));
-            atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+        return found;
+    }
+    while (i < e && !found) {
+        const uint64_t bit = (uint64_t)i * eb, w = (bit >> 5) & ~3ull;
+        const uint4 q = load_words16(a.in_edges, a.in_words, w);
+        // the last edge that begins in these words may end in the next one
+        const uint32_t q4 = (uint64_t)e * eb > 32 * (w + 4) ? __ldg(a.in_edges + w + 4) : 0u;
+        for (uint32_t at = (uint32_t)(bit - 32 * w); at < 128 && i < e && !found;) {
+            uint32_t u[kBuUnroll], n = 0;
+            bool in[kBuUnroll];
+#pragma unroll
+            for (int k = 0; k < kBuUnroll; k++) {
+                const uint32_t x = at >> 5;
+                const uint32_t lo = x == 0 ? q.x : x == 1 ? q.y : x == 2 ? q.z : q.w;
+                const uint32_t hi = x == 0 ? q.y : x == 1 ? q.z : x == 2 ? q.w : q4;
+                const bool begins = at < 128 && i + k < e;
+                n += begins;
+                u[k] = begins ? __funnelshift_r(lo, hi, at & 31u) & mask : 0xffffffffu;
+                if (u[k] != 0xffffffffu && ASC_BAD(u[k] >= a.V, 17, u[k])) u[k] = 0xffffffffu;
+                at += eb;
+            }
+#pragma unroll
+            for (int k = 0; k < kBuUnroll; k++)
+                in[k] = u[k] != 0xffffffffu && ((a.bitmap_in[u[k] >> 5] >> (u[k] & 31)) & 1u);
+            // edges read count up to the parent
+#pragma unroll
+            for (int k = 0; k < kBuUnroll; k++)
+                if (!found && u[k] != 0xffffffffu) {
+                    scanned++;
+                    found = in[k];
+                }
+            i += n;
         }
     }
     return found;
@@ -933,7 +967,7 @@ __device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nw
     for (uint32_t w0 = kBuWords * (blockIdx.x * kWarps + (threadIdx.x >> 5)); w0 < nwords; w0 += kBuWords * warps) {
         // vertices without in-edges can never be reached: about half of an
         // RMAT graph, nearly all of its unreachable vertices
-        uint32_t vis[kBuWords], done[kBuWords];
+        uint32_t vis[kBuWords], done[kBuWords], dense = 0;
 #pragma unroll
         for (int k = 0; k < kBuWords; k++) {
             const bool in = w0 + k < nwords;
@@ -972,24 +1006,48 @@ __device__ __forceinline__ void bottom_up_words(const RegionArgs &a, uint32_t nw
             }
             const bool miss = todo[k] && !hit[k];
             const unsigned missed = __ballot_sync(kFull, miss);
+            if (__popc(missed) >= kBuDirect) {
+                dense |= 1u << k;
+                if (lane == 0) bs.open[threadIdx.x >> 5][k] = missed;
+                continue;
+            }
             if (miss) queue[waiting + __popc(missed & ((1u << lane) - 1u))] = v;
             waiting += __popc(missed);
         }
-        __syncwarp();  // the queue, and this word's bits before later ones are added
-        while (waiting >= 32) {
-            waiting -= 32;
-            uint32_t v;
-            const bool found = bottom_up_scan(a, queue + waiting, 32, nv, v, scanned);
-            n0 += found && v < a.S;
-            n1 += found && v >= a.S;
+        __syncwarp();  // the queue, and these words' bits before later ones are added
+        const bool last = w0 + kBuWords * warps >= nwords;
+        while (dense || waiting >= 32 || (last && waiting)) {  // one scan for both: code is fetched too
+            uint32_t v, w = 0xffffffffu;
+            bool want;
+            if (dense) {
+                const int k = __ffs((int)dense) - 1;
+                dense &= dense - 1;
+                w = w0 + k;
+                v = 32 * w + lane;
+                want = (bs.open[threadIdx.x >> 5][k] >> lane) & 1u;
+            } else {
+                const uint32_t n = min(waiting, 32u);
+                waiting -= n;
+                want = lane < n;
+                v = want ? queue[waiting + lane] : 0u;
+            }
+            const bool found = bottom_up_scan(a, want, v, scanned);
+            const unsigned all = __ballot_sync(kFull, found);
+            if (found) {
+                a.val[v] = nv;
+                n0 += v < a.S;
+                n1 += v >= a.S;
+                if (w == 0xffffffffu) {
+                    atomicOr(&a.visited[v >> 5], 1u << (v & 31));
+                    atomicOr(&a.bitmap[v >> 5], 1u << (v & 31));
+                }
+            }
+            if (w != 0xffffffffu && lane == 0 && all) {
+                atomicOr(&a.visited[w], all);
+                atomicOr(&a.bitmap[w], all);
+            }
             __syncwarp();
         }
-    }
-    if (waiting) {
-        uint32_t v;
-        const bool found = bottom_up_scan(a, queue, waiting, nv, v, scanned);
-        n0 += found && v < a.S;
-        n1 += found && v >= a.S;
     }
     n0 = __reduce_add_sync(kFull, n0);
     n1 = __reduce_add_sync(kFull, n1);
@@ -2548,6 +2606,7 @@ RegionArgs base_args(asc_graph *g, Workspace *ws, int parity_in) {
         a.in_heads = g->in_heads_ready ? g->d_in_heads : nullptr;
         a.in_none = ws->in_none;
         a.in_ebits = g->in_ebits;
+        a.in_words = in_edge_words(g);
         a.bu_div = ws->tune.bu_div;
     }
     a.S = g->static_vertices;
@@ -3435,7 +3494,7 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
         cuts[++runs] = hi;
     }
     const uint32_t bits = g->in_ebits;
-    const uint64_t words = bits == 32 ? E : (E * bits + 31) / 32 + 1;
+    const uint64_t words = in_edge_words(g);
     uint32_t *packed = nullptr;
     if (cudaHostAlloc((void **)&packed, 4 * words, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
@@ -3515,7 +3574,7 @@ asc_status ensure_in_ptr(asc_graph *g) {
         return st;
     }
     if (g->static_edges >= g->E) {
-        const uint64_t words = g->in_ebits == 32 ? std::max<uint64_t>(1, g->E) : (g->E * g->in_ebits + 31) / 32 + 1;
+        const uint64_t words = in_edge_words(g);
         ASC_CUDA(cudaMalloc(&ws->in_edges, 4 * words));
         ASC_CUDA(cudaMemcpy(ws->in_edges, g->h_in_edges, 4 * words, cudaMemcpyHostToDevice));
         ws->device_bytes += 4 * words;
@@ -4975,7 +5034,7 @@ uint64_t workspace_bytes(asc_graph *g, bool pagerank) {
     // the in-edges themselves when every out-edge is resident)
     if (!g->is_csc && t.bu_div && (!g->ws || !g->ws->in_ptr)) {
         b += 4 * (V + 1) + 4 * (V / 32 + 2);
-        if (g->static_edges >= E) b += 4 * (g->in_ebits == 32 ? std::max<uint64_t>(1, E) : (E * g->in_ebits + 31) / 32 + 1);
+        if (g->static_edges >= E) b += 4 * in_edge_words(g);
     }
     return b;
 }
