@@ -2418,11 +2418,13 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         const uint64_t words = (V + 31) / 32;
         const uint64_t nt = std::max<uint64_t>(
             1, std::min<uint64_t>(std::max(1u, std::thread::hardware_concurrency()), words >> 15));
-        std::vector<uint64_t> sums(2 * nt, 0);
+        std::vector<uint64_t> sums(3 * nt, 0);
         auto scan = [&](uint64_t k) {
             uint64_t n0 = 0, n1 = 0;
+            uint32_t tile = 0;
             for (uint64_t w = words * k / nt; w < words * (k + 1) / nt; w++) {
                 uint32_t bits = 0;
+                if (w % (kBlock / 32) == 0) tile = std::max(tile, ptr[std::min(V, 32 * w + kBlock)] - ptr[32 * w]);
                 for (uint64_t v = 32 * w; v < std::min(V, 32 * w + 32); v++) {
                     const uint32_t d = ptr[v + 1] - ptr[v];
                     if (d <= huge) continue;
@@ -2431,8 +2433,9 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
                 }
                 ll.bits[w] = bits;
             }
-            sums[2 * k] = n0;
-            sums[2 * k + 1] = n1;
+            sums[3 * k] = n0;
+            sums[3 * k + 1] = n1;
+            sums[3 * k + 2] = tile;
         };
         std::vector<std::thread> threads;
         for (uint64_t k = 1; k < nt; k++) {
@@ -2444,13 +2447,12 @@ asc_status alloc_workspace(asc_graph *g, Workspace *ws, bool graph_tuning = true
         }
         scan(0);
         for (auto &th : threads) th.join();
+        uint64_t most = 0;  // edges of the fullest tile
         for (uint64_t k = 0; k < nt; k++) {
-            ll.seg_static += sums[2 * k];
-            ll.seg_ondemand += sums[2 * k + 1];
+            ll.seg_static += sums[3 * k];
+            ll.seg_ondemand += sums[3 * k + 1];
+            most = std::max(most, sums[3 * k + 2]);
         }
-        uint64_t most = 0;
-        for (uint64_t v = 0; v < V; v += kBlock)
-            most = std::max<uint64_t>(most, ptr[std::min<uint64_t>(V, v + kBlock)] - ptr[v]);
         ll.even = most * V <= kEvenTiles * g->E * std::min<uint64_t>(kBlock, V);
         ll.huge_degree = t.huge_degree;
         ll.segment_edges = t.segment_edges;
