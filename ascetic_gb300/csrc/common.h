@@ -164,7 +164,7 @@ inline uint64_t edge_store_bytes(const asc_graph *g, uint64_t n) {
     if (g->edge_words == 2) return 8 * n;
     return (n * g->ebits + 7) / 8;
 }
-// u32 words of the in-edges of a CSR graph, likewise
+// u32 words of the in-edges of a CSR graph, likewise (the arrays are rounded up to 16 bytes)
 inline uint64_t in_edge_words(const asc_graph *g) {
     if (g->in_ebits == 32) return g->E ? g->E : 1;
     return (g->E * g->in_ebits + 31) / 32 + 1;

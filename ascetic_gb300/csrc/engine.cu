@@ -136,6 +136,7 @@ struct RegionArgs {
     uint32_t dense_div;
     uint32_t wbits;               // > 0: u32 edges packed as (dst << wbits) | weight
     uint32_t ebits;               // bits per stored edge word: 32, or a bit stream of ebits per edge
+    uint32_t item_div;            // by items while more than 1 / item_div of the region is active
     unsigned long long *frag;     // non-null: add edges read per 4096-edge fragment
     // bottom-up BFS steps (null in_ptr: top-down only)
     const uint32_t *in_ptr;       // in-edge offsets (device)
@@ -150,8 +151,6 @@ struct RegionArgs {
     const uint2 *items;
     uint32_t item_begin, item_n;
     uint64_t edge_words;
-    uint64_t in_words;            // words that may be read at in_edges
-    uint32_t item_div;            // by items while more than 1 / item_div of the region is active
 };
 
 // True when this BFS iteration steps bottom-up: its input frontier (the
@@ -921,7 +920,7 @@ __device__ __forceinline__ bool bottom_up_scan(const RegionArgs &a, bool want, u
     }
     while (i < e && !found) {
         const uint64_t bit = (uint64_t)i * eb, w = (bit >> 5) & ~3ull;
-        const uint4 q = load_words16(a.in_edges, a.in_words, w);
+        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(a.in_edges + w));  // the array ends on 16 bytes
         // the last edge that begins in these words may end in the next one
         const uint32_t q4 = (uint64_t)e * eb > 32 * (w + 4) ? __ldg(a.in_edges + w + 4) : 0u;
         for (uint32_t at = (uint32_t)(bit - 32 * w); at < 128 && i < e && !found;) {
@@ -2608,7 +2607,6 @@ RegionArgs base_args(asc_graph *g, Workspace *ws, int parity_in) {
         a.in_heads = g->in_heads_ready ? g->d_in_heads : nullptr;
         a.in_none = ws->in_none;
         a.in_ebits = g->in_ebits;
-        a.in_words = in_edge_words(g);
         a.bu_div = ws->tune.bu_div;
     }
     a.S = g->static_vertices;
@@ -3498,7 +3496,7 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
     const uint32_t bits = g->in_ebits;
     const uint64_t words = in_edge_words(g);
     uint32_t *packed = nullptr;
-    if (cudaHostAlloc((void **)&packed, 4 * words, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&packed, 4 * ((words + 3) & ~3ull), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
         return fail(ASC_ERR_NOMEM, "cudaHostAlloc of %llu bytes failed", (unsigned long long)(4 * words));
     }
@@ -3577,7 +3575,7 @@ asc_status ensure_in_ptr(asc_graph *g) {
     }
     if (g->static_edges >= g->E) {
         const uint64_t words = in_edge_words(g);
-        ASC_CUDA(cudaMalloc(&ws->in_edges, 4 * words));
+        ASC_CUDA(cudaMalloc(&ws->in_edges, 4 * ((words + 3) & ~3ull)));
         ASC_CUDA(cudaMemcpy(ws->in_edges, g->h_in_edges, 4 * words, cudaMemcpyHostToDevice));
         ws->device_bytes += 4 * words;
     }
@@ -3854,12 +3852,13 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     }
     ASC_CUDA(cudaEventRecord(ws->ev[1], s));
     ASC_CUDA(cudaGetLastError());
-    if (want && !values_reported) {
+    const bool copies = want && !values_reported;
+    if (copies) {
         ASC_CUDA(cudaMemcpyAsync(out, ws->val, 4ull * V,
                                  (p.flags & ASC_RUN_DEVICE_OUT) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                                  s));
+        ASC_CUDA(cudaEventRecord(ws->ev[2], s));
     }
-    ASC_CUDA(cudaEventRecord(ws->ev[2], s));
     if (!device_loop) ASC_CUDA(cudaMemcpyAsync(ws->h_ctl, ws->ctl, 4 * CTL_WORDS, cudaMemcpyDeviceToHost, s));
     ASC_CUDA(cudaStreamSynchronize(s));
     if (device_loop) {
@@ -3899,8 +3898,10 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         float ms = 0;
         ASC_CUDA(cudaEventElapsedTime(&ms, ws->ev[0], ws->ev[1]));
         st->ms_total = ms;
-        ASC_CUDA(cudaEventElapsedTime(&ms, ws->ev[1], ws->ev[2]));
-        st->ms_copyout = ms;
+        if (copies) {
+            ASC_CUDA(cudaEventElapsedTime(&ms, ws->ev[1], ws->ev[2]));
+            st->ms_copyout = ms;
+        }
         st->ms_static = phase_ms[0];
         st->ms_ondemand = phase_ms[1];
         st->ms_bottom_up = phase_ms[2];

@@ -422,7 +422,7 @@ static asc_status narrow_edges(asc_graph *g) {
 static asc_status pack_stream(const uint32_t *src, uint64_t n, uint32_t bits, uint32_t **out) {
     const uint64_t words = bits == 32 ? (n ? n : 1) : (n * bits + 31) / 32 + 1;
     uint32_t *packed = nullptr;
-    ASC_TRY(pinned_alloc((void **)&packed, sizeof(uint32_t) * words));
+    ASC_TRY(pinned_alloc((void **)&packed, sizeof(uint32_t) * ((words + 3) & ~3ull)));  // read 16 bytes at a time
     if (bits == 32) {
         parallel_for(n, host_threads(n), [&](unsigned, uint64_t b, uint64_t e) {
             memcpy(packed + b, src + b, sizeof(uint32_t) * (e - b));
