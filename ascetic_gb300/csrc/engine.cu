@@ -1396,6 +1396,7 @@ struct LoopArgs {
     uint32_t *values;       // host: small results too (null: the caller copies them)
     uint32_t first_label;   // connected components: src's label is spread first, the rest follow
     uint32_t first_cap;     // after at most this many iterations
+    uint32_t polls;         // of a grid barrier before it gives up
 };
 
 constexpr uint32_t kFirstLabelIterations = 32;
@@ -1415,6 +1416,7 @@ constexpr uint64_t kReportedValues = 16384;
 // Polls of a grid barrier (a read of L2 and a short sleep each) before it gives
 // up: tens of seconds, far above any phase.
 constexpr uint32_t kBarrierPolls = 1u << 25;
+thread_local uint32_t t_barrier_polls = kBarrierPolls;  // tests make a thread's runs give up sooner
 
 // Barrier over the grid: arrivals count up from zero for the whole launch.
 // False when the other CTAs did not arrive in time. Where counts is given, the
@@ -1422,8 +1424,9 @@ constexpr uint32_t kBarrierPolls = 1u << 25;
 // with every warp of 912 CTAs reading them for itself, those reads of one line cost
 // more than the barrier (an iteration of a BFS that reaches 700 vertices at a time
 // on a grid graph of a million: 18 us, 13.5 so).
-__device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target, const uint32_t *counts = nullptr,
+__device__ __forceinline__ bool grid_barrier(const LoopArgs &l, uint32_t &target, const uint32_t *counts = nullptr,
                                              uint32_t *s_counts = nullptr) {
+    uint32_t *ctl = l.ctl;
     __shared__ uint32_t s_ok;
     __syncthreads();
     target += gridDim.x;
@@ -1434,7 +1437,7 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *ctl, uint32_t &target, co
         for (;;) {
             // relaxed: an acquire would empty the L1 that the SM's other CTAs still work in
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(ctl + CTL_BARRIER) : "memory");
-            if ((int32_t)(now - target) >= 0 || ++polls > kBarrierPolls) break;
+            if ((int32_t)(now - target) >= 0 || ++polls > l.polls) break;
             if (polls > 16) __nanosleep(64);
         }
         s_ok = (int32_t)(now - target) >= 0;
@@ -1592,17 +1595,17 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
         // the frontier of the remaining labels, in place of an empty one or beside
         // what the first label still has to reach
         st.promotions = 1;
-        if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;  // every thread has read the counts
+        if (!grid_barrier(l, st.target)) return kLoopStuck;  // every thread has read the counts
         if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
         seed_unlabelled(a, y.r0.bitmap, l.src, l.ctl + CTL_PROMOTED);
-        if (!grid_barrier(l.ctl, st.target, l.ctl + CTL_PROMOTED, cin)) return kLoopStuck;
+        if (!grid_barrier(l, st.target, l.ctl + CTL_PROMOTED, cin)) return kLoopStuck;
         const uint32_t n0 = cin[0], n1 = cin[1];
         build_frontier(y.r0, y.r0.bitmap, l.nwords, n0, n1);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             y.r0.cnt_out[6] = n0;
             y.r0.cnt_out[7] = n1;
         }
-        if (!grid_barrier(l.ctl, st.target, a.cnt_in, cin)) return kLoopStuck;
+        if (!grid_barrier(l, st.target, a.cnt_in, cin)) return kLoopStuck;
     }
     if (!(cin[6] | cin[7])) {
         if (ALG != kSSSP || !a.far_bits) return kLoopEnd;
@@ -1617,7 +1620,7 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
                 l.ctl[CTL_PROMOTED + 2 * clear] = l.ctl[CTL_PROMOTED + 2 * clear + 1] = 0;
             }
             promote_far(a, y.r0.bitmap, l.ctl + CTL_PROMOTED + 2 * k, l.nwords, st.thresh, l.ctl + CTL_MINFAR + k);
-            if (!grid_barrier(l.ctl, st.target)) return kLoopStuck;
+            if (!grid_barrier(l, st.target)) return kLoopStuck;
             volatile const uint32_t *moved = l.ctl + CTL_PROMOTED + 2 * k;
             n0 = moved[0];
             n1 = moved[1];
@@ -1631,7 +1634,7 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
             y.r0.cnt_out[6] = n0;
             y.r0.cnt_out[7] = n1;
         }
-        if (!grid_barrier(l.ctl, st.target, a.cnt_in, cin)) return kLoopStuck;
+        if (!grid_barrier(l, st.target, a.cnt_in, cin)) return kLoopStuck;
     }
     if (st.it >= l.cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) l.ctl[CTL_TIMEOUT] = 1;
@@ -1640,13 +1643,13 @@ __device__ __forceinline__ LoopNext loop_iteration(const LoopArgs &l, const Fuse
     st.it++;
     if (ALG == kBFS && bottom_up_step(a, cin)) bottom_up_words(a, l.nwords, st.it + 1, sm.bottom_up, s_next);
     else expand_regions<ALG, WORDS>(x, cin, st.thresh, sm.expand, s_next);
-    if (!grid_barrier(l.ctl, st.target, a.cnt_out, cin)) return kLoopStuck;
+    if (!grid_barrier(l, st.target, a.cnt_out, cin)) return kLoopStuck;
     build_frontier(a, a.bitmap, l.nwords, cin[6], cin[7]);
     // the input frontier's bitmap and counts are the next output's
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < l.nwords; w += gridDim.x * blockDim.x)
         y.r0.bitmap[w] = 0;
     if (blockIdx.x == 0 && threadIdx.x < CTL_BLOCK) y.r0.cnt_out[threadIdx.x] = 0;
-    return grid_barrier(l.ctl, st.target, a.cnt_out, cin) ? kLoopGo : kLoopStuck;
+    return grid_barrier(l, st.target, a.cnt_out, cin) ? kLoopGo : kLoopStuck;
 }
 
 template <int ALG, int WORDS>
@@ -1657,10 +1660,10 @@ __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const
     LoopState st;
     st.thresh = l.thresh;
     loop_setup<ALG>(l);
-    if (!grid_barrier(l.ctl, st.target, l.x0.r0.cnt_in, cin)) return;
+    if (!grid_barrier(l, st.target, l.x0.r0.cnt_in, cin)) return;
     if (l.all) {
         build_frontier(l.x1.r0, l.x1.r0.bitmap, l.nwords, cin[6], cin[7]);
-        if (!grid_barrier(l.ctl, st.target, l.x0.r0.cnt_in, cin)) return;
+        if (!grid_barrier(l, st.target, l.x0.r0.cnt_in, cin)) return;
     }
     for (;;) {
         LoopNext n = loop_iteration<ALG, WORDS>(l, l.x0, l.x1, st, sm, s_next, cin);
@@ -1676,7 +1679,7 @@ __global__ void __launch_bounds__(kBlock, ASC_TRAV_BLOCKS) traverse_kernel(const
     if (l.values)
         for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < l.x0.r0.V; v += gridDim.x * blockDim.x)
             l.values[v] = l.x0.r0.val[v];
-    if (!grid_barrier(l.ctl, st.target)) return;
+    if (!grid_barrier(l, st.target)) return;
     if (blockIdx.x == 0 && threadIdx.x < CTL_WORDS)
         l.report[threadIdx.x] = threadIdx.x == CTL_ITERS ? st.it : ((volatile uint32_t *)l.ctl)[threadIdx.x];
 }
@@ -3663,6 +3666,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
         l.all = all && !first_label ? 1 : 0;
         l.first_label = first_label ? 1 : 0;
         l.first_cap = kFirstLabelIterations;
+        l.polls = t_barrier_polls;
         l.cap = (uint32_t)std::min<int64_t>(cap, 0x7fffffff);
         l.thresh = 1 + ws->tune.delta;
         l.delta = ws->tune.delta;
@@ -5075,6 +5079,7 @@ static asc_status batch_alloc(BatchEngine *b, void **p, uint64_t n) {
 }
 
 extern "C" void asc_test_fail_batch_alloc(int after) { t_allocs_left = after; }
+extern "C" void asc_test_barrier_polls(uint32_t polls) { t_barrier_polls = polls; }
 
 // Empties a batch, on its stream: no source, no frontier (lists, bitmaps, counts,
 // front masks), no masks. A source dropped without this would leave its frontier to
