@@ -21,11 +21,12 @@
 //    prKernel_Opt (gpu_kernels.cuh:533-594).
 //
 // Load balance: each expansion launch is a persistent grid pulling work items
-// from an atomic cursor. A work item is either a tile of 256 frontier vertices
-// (the CTA scans their degrees and walks the tile's concatenated edge range,
-// so consecutive threads read consecutive column indices) or one segment of a
-// vertex whose degree exceeds the huge-degree threshold (a CTA-wide stride
-// over up to segment_edges edges of that list).
+// from an atomic cursor. A work item of a sparse frontier is a tile of up to 256
+// list entries (the CTA scans their degrees and walks the tile's concatenated edge
+// range, so consecutive threads read consecutive column indices) or one segment of
+// a vertex whose degree exceeds the huge-degree threshold (a CTA-wide stride over up
+// to segment_edges edges of that list). A dense one is walked in id order, by merge
+// items of 2048 rows plus edges or by tiles of 256 vertices (by_items).
 #include <cooperative_groups.h>
 #include <math.h>
 #include <stdio.h>
@@ -52,10 +53,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // 8 x 256 threads fill an SM, 32 registers each. Measured on RMAT scale 24 with
 // bit-packed edges: 65.6 GTEPS at 8, 64.5 at 6, 57.3 at 4 (64 registers, half
 // the warps: the loads over the host link want every warp the SM can hold).
-// The same for the PageRank pull/scatter kernels (8: FP32 standard PageRank on
-// RMAT scale 23 in 181 ms against 195 at the compiler's choice of 40 registers).
-// The batched SSSP kernel takes 5 (48 registers; at 6 or 8 it spills more than
-// a few bytes); the batched BFS kernels are left to the compiler (32 registers).
+// The same for the list-driven PageRank pull. The batched SSSP kernel takes 5 (48
+// registers; at 6 or 8 it spills more than a few bytes). Kernels that hold a merge
+// item in shared memory name their own: 6 (ASC_TRAV_BLOCKS, ASC_PR_ITEM_BLOCKS,
+// ASC_MS_BFS_BLOCKS; 40 registers) or 4 (ASC_PR_SCATTER_BLOCKS).
 #ifndef ASC_PR_MIN_BLOCKS
 #define ASC_PR_MIN_BLOCKS 8
 #endif
@@ -544,8 +545,8 @@ __device__ void expand_segment(const RegionArgs &a, uint64_t item, uint32_t *s_n
 // contiguous run; otherwise through its list, per entries per item: as few as
 // give every CTA of the grid one, at least kMinTile, since the lists of a tile
 // are walked by one CTA (the third iteration of a BFS on RMAT scale 16 took 93
-// us with its 800 vertices and 118,000 edges in four tiles of 256). With merge
-// items, the id-order walk runs over those alone.
+// us with its 800 vertices and 118,000 edges in four tiles of 256). An id-order walk
+// by merge items (by_items) has no other items.
 #ifndef ASC_MIN_TILE
 #define ASC_MIN_TILE 8
 #endif
@@ -840,16 +841,17 @@ __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_ke
 }
 
 // Bottom-up BFS step (direction-optimizing BFS): every vertex not yet reached
-// scans its in-edges, in source-id order, for a parent in this iteration's
-// frontier and stops at the first one; a vertex found takes the parent's value
+// scans its in-edges, from the one whose source has the most out-edges on, for a
+// parent in this iteration's frontier and stops at the first one; a vertex found takes the parent's value
 // + 1 (the level-synchronous top-down step gives every unreached vertex with a
 // frontier in-neighbour the same value, so levels are identical) and joins the
 // next frontier. When the frontier is a large part of the graph, most unreached
 // vertices find a parent among their first in-edges, so the step reads far
 // fewer edge bytes over the host link than expanding the frontier's out-lists.
-// One warp per 32-vertex bitmap word, lane = vertex: the warp writes the
-// word's reached and next-frontier bits whole. In-edges are read in place from
-// pinned host memory, kBuUnroll per lane before any frontier probe.
+// A warp takes bitmap words of 32 vertices, lane = vertex, and writes the bits of
+// those whose first in-edge is a parent; bits of vertices found later are added.
+// Further in-edges are read in place from pinned host memory (device memory on a
+// graph without a cap), kBuUnroll per lane before any frontier probe.
 #ifndef ASC_BU_UNROLL
 #define ASC_BU_UNROLL 4
 #endif
@@ -3256,10 +3258,6 @@ asc_status ensure_gather_buffers(asc_graph *g) {
     return ASC_OK;
 }
 
-// In-edge offsets on the device for bottom-up BFS steps, built on the
-// graph's first BFS. The in-edges stay in pinned host memory, read in place,
-// unless the graph has no cap (every out-edge resident): then they are
-// resident too.
 // ------------------------------------------- in-edges of a CSR graph -------
 //
 // Built on the device on the graph's first BFS: in-degrees counted over the merge
@@ -3269,10 +3267,13 @@ asc_status ensure_gather_buffers(asc_graph *g) {
 // to its front and packs the run into page-locked memory. On host threads this
 // took 4.0 s for the 268 M edges of RMAT scale 24.
 //
-// The first in-edge of a list is the source with the most out-edges: the one most
-// likely to be in a large frontier. Of the 7% of vertices whose smallest-id source
-// was no parent in the large step of a BFS on RMAT scale 21, 24,200 went on to read
-// host memory; with this choice 3,744 do.
+// The first in-edge of a list is the source with the most out-edges among the first
+// kHeadSample that arrived: the one most likely to be in a large frontier. Of the 7% of
+// vertices whose smallest-id source was no parent in the large step of a BFS on RMAT
+// scale 21, 24,200 went on to read host memory; with this choice 3,744 do. The others
+// follow in the order in which the scatter's atomics came, which differs from one build
+// to the next (host-built lists are sorted): the levels do not depend on it, the number
+// of in-edges that a step reads does.
 namespace {
 
 struct InEdgeArgs {
@@ -3542,6 +3543,10 @@ asc_status in_edges_on_device(asc_graph *g, bool *done) {
 
 }  // namespace
 
+// In-edge offsets on the device for bottom-up BFS steps, built on the
+// graph's first BFS. The in-edges stay in pinned host memory, read in place,
+// unless the graph has no cap (every out-edge resident): then they are
+// resident too.
 asc_status ensure_in_ptr(asc_graph *g) {
     Workspace *ws = g->ws;
     if (ws->in_ptr) return ASC_OK;
@@ -4238,9 +4243,11 @@ __device__ __forceinline__ void ms_reach(const MsArgs &m, uint32_t v, unsigned l
 // 16-byte load and atomics only for sources not yet there: 64 sources on RMAT
 // scale 21, 3.52 -> 2.4 ms (tiles of 256 vertices and an atomic with a returned
 // value per edge and new source before).
-// 64-source batch, RMAT scale 22 / 24: 5.45 / 18.27 ms at 4 (32 registers, 8
-// CTAs per SM), 5.58 / 18.46 at 6 (40, 6 CTAs), 5.78 / 18.96 at 8 (48, 5 CTAs).
+// With tiles alone, 8 CTAs per SM: 64-source batch, RMAT scale 22 / 24, 5.45 / 18.27
+// ms at 4 edges, 5.58 / 18.46 at 6, 5.78 / 18.96 at 8.
 constexpr int kMsUnroll = ASC_MS_UNROLL;
+// CTAs per SM (40 registers at 6): 64 sources on RMAT scale 21, 5.33 / 5.28 / 5.51 ms
+// at 5 / 6 / 7, the copy of the rows included.
 #ifndef ASC_MS_BFS_BLOCKS
 #define ASC_MS_BFS_BLOCKS 6
 #endif

@@ -667,10 +667,11 @@ asc_status rmat_build(uint32_t scale, uint32_t ef, uint64_t seed, double a, doub
 namespace asc {
 
 // In-edges of a CSR graph for bottom-up BFS steps: a counting sort of the
-// out-edges by destination (host threads), each in-list sorted by source id,
-// stored as a bit stream of bits(V - 1) per edge in pinned memory that the
-// device reads in place. Built once per graph, on its first BFS that may step
-// bottom-up.
+// out-edges by destination (host threads), each in-list sorted by source id but for
+// the source with the most out-edges, which comes first, stored as a bit stream of
+// bits(V - 1) per edge in pinned memory that the device reads in place. Built once per
+// graph, on its first BFS that may step bottom-up, where the device does not build them
+// (a list longer than V, an average degree of 64 and above).
 asc_status build_in_edges(asc_graph *g) {
     if (g->h_in_edges || g->is_csc) return ASC_OK;
     const uint64_t V = g->V, E = g->E;

@@ -228,8 +228,7 @@ def pr_study(args):
             res[name] = (r.astype(np.float64), st)
         # host-link rate of the on-demand pull: 8 FP32 passes with the static and
         # on-demand regions in separate launches timed apart; the on-demand
-        # launch reads every in-edge of the on-demand vertices (tiles of short
-        # lists and the segments of long ones) over the host link
+        # launch reads every in-edge of the on-demand vertices over the host link
         prm = A.make_params(pr_mode=A.PR_STD, precision=A.F32, max_iterations=8,
                             flags=A.RUN_PHASE_TIMING | A.RUN_NO_OUTPUT)
         _, st = g.run("pr", params=prm)
@@ -237,7 +236,7 @@ def pr_study(args):
         gbs = pull_bytes / (st["ms_ondemand"] * 1e-3) / 1e9 if st["ms_ondemand"] else 0.0
         peak = getattr(args, "link_gbs", 0.0) or 0.0
         out["ondemand_pull_link"] = {
-            "kernel": "pr_pull_kernel<float> on-demand region (phase-timed passes)", "bound": "host-link",
+            "kernel": "pr_pull_items_kernel<float> on-demand region (phase-timed passes)", "bound": "host-link",
             "passes": st["iterations"], "bytes_per_pass": int(pull_bytes / max(1, st["iterations"])),
             "ms_per_pass": round(st["ms_ondemand"] / max(1, st["iterations"]), 3),
             "achieved": round(gbs, 1), "peak": round(peak, 1), "unit": "GB/s",
@@ -312,8 +311,7 @@ def pagerank_leg(args):
             res[name] = (r.astype(np.float64), st)
         # host-link rate of the on-demand pull: 8 FP32 passes with the static and
         # on-demand regions in separate launches timed apart; the on-demand
-        # launch reads every in-edge of the on-demand vertices (tiles of short
-        # lists and the segments of long ones) over the host link
+        # launch reads every in-edge of the on-demand vertices over the host link
         prm = A.make_params(pr_mode=A.PR_STD, precision=A.F32, max_iterations=8,
                             flags=A.RUN_PHASE_TIMING | A.RUN_NO_OUTPUT)
         _, st = g.run("pr", params=prm)
@@ -321,7 +319,7 @@ def pagerank_leg(args):
         gbs = pull_bytes / (st["ms_ondemand"] * 1e-3) / 1e9 if st["ms_ondemand"] else 0.0
         peak = getattr(args, "link_gbs", 0.0) or 0.0
         out["ondemand_pull_link"] = {
-            "kernel": "pr_pull_kernel<float> on-demand region (phase-timed passes)", "bound": "host-link",
+            "kernel": "pr_pull_items_kernel<float> on-demand region (phase-timed passes)", "bound": "host-link",
             "passes": st["iterations"], "bytes_per_pass": int(pull_bytes / max(1, st["iterations"])),
             "ms_per_pass": round(st["ms_ondemand"] / max(1, st["iterations"]), 3),
             "achieved": round(gbs, 1), "peak": round(peak, 1), "unit": "GB/s",
@@ -440,7 +438,7 @@ def serve_leg(args):
             wall = time.perf_counter() - t_start
         return st, kept, wall
 
-    # warm-up (graph loops, batch state) then saturating load
+    # warm-up (single-query and batch state) then saturating load
     run(A.SERVE_BATCHED, n=min(40, len(plan)))
     run(A.SERVE_FIFO, n=min(8, len(plan)))
     log("serving warm-up done")
@@ -999,9 +997,11 @@ def main():
            "value_pageable_result": round(pg_edges / pg_s / 1e9, 4),
            "note": "h2d = on-demand edge bytes read over the host link per BFS plus the source id"}
 
-    # phase split and roofline of the kernels: top-down expansion of the
-    # static and of the on-demand region, and the bottom-up steps, each timed
-    # with CUDA events on the engine's stream in phase-timed runs of the same
+    # phase split and roofline of the kernels: the timed steps run as one
+    # launch (traverse_kernel), whose phases cannot be timed from outside; so
+    # top-down expansion of the static and of the on-demand region, and the
+    # bottom-up steps, are launched apart (the same device code) and timed with
+    # CUDA events on the engine's stream in phase-timed runs of the same
     # sources (same levels, same step directions)
     ms_s = ms_o = ms_b = 0.0
     ed_s = ed_o = ed_b = vs = vo = vx_b = 0
@@ -1043,14 +1043,16 @@ def main():
                                   "cudaMemcpyAsync, best of 3 (sm_zero_copy_read_peak: the SMs reading the same "
                                   "buffer in place with 16-byte loads, best of 3)",
                    "sm_zero_copy_read_peak": round(smread_gbs, 1)}
-    roof_static = {"kernel": "expand_fused_kernel<BFS> static region (top-down)", "bound": "hbm",
+    roof_static = {"kernel": "top-down expansion of traverse_kernel<BFS>, static region, launched apart (expand_kernel)",
+                   "bound": "hbm",
                    "achieved": round(hbm_gbs, 1), "peak": hbm_peak, "unit": "GB/s",
                    "frac": round(hbm_gbs / hbm_peak, 4),
                    "traffic": (traffic.get("static") or {}).get("dram_bytes_per_launch"),
                    "traffic_source": "profiles/traffic.json (ncu, DRAM read+write bytes per launch)",
                    "peak_source": "MEASURED_PEAKS.json hbm_gbs (measured)",
                    "ms_share": round(ms_s / ms_all, 3) if ms_all else None}
-    roof_link = dict({"kernel": "expand_fused_kernel<BFS> on-demand region (top-down)", "bound": "host-link",
+    roof_link = dict({"kernel": "top-down expansion of traverse_kernel<BFS>, on-demand region, launched apart "
+                                "(expand_kernel)", "bound": "host-link",
                       "achieved": round(link_gbs, 1), "peak": round(dma_gbs, 1), "unit": "GB/s",
                       "frac": round(link_gbs / dma_gbs, 4) if dma_gbs else None,
                       "traffic": (traffic.get("ondemand") or {}).get("dram_bytes_per_launch"),
@@ -1058,7 +1060,7 @@ def main():
                       "traffic_source": "profiles/traffic.json (ncu: DRAM read+write and host-link sector bytes "
                                         "per on-demand launch)",
                       "ms_share": round(ms_o / ms_all, 3) if ms_all else None}, **link_common)
-    roof_bu = {"kernel": "bottom_up_kernel (BFS bottom-up steps)", "bound": "hbm",
+    roof_bu = {"kernel": "bottom-up steps of traverse_kernel<BFS>, launched apart (bottom_up_kernel)", "bound": "hbm",
                "achieved": round(bu_gbs, 1), "peak": hbm_peak, "unit": "GB/s",
                "frac": round(bu_gbs / hbm_peak, 4),
                "traffic": (traffic.get("bottom_up") or {}).get("dram_bytes_per_launch"),
