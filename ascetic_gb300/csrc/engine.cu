@@ -247,13 +247,16 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t &total,
 // holds more edges than an item where degrees are high. So where the tiles of a graph
 // are even (see kEvenTiles), items are for frontiers of over a quarter of the region
 // at 8 edges per vertex and above, of over a sixteenth from 3 on, and for every dense
-// frontier below. us, items for every dense frontier / above 1/16 / 1/8 / 1/4 / 1/2:
+// frontier below. The on-demand region always goes by items, whose 16-byte reads keep
+// the link's runs long where active vertices lie together (CC of 1 M vertices linked
+// to 16 within 1,000 ids, 25% resident: 37.6 ms, by the rule 56.0). us, items for every
+// dense frontier / above 1/16 / 1/8 / 1/4 / 1/2:
 //   uniform random, 6 M vertices of 16: SSSP 6265 / 5715 / 5185 / 4808 / 4691
 //   2 M of 8: SSSP 1468 / 1417 / 1384 / 1377 / 1375; of 4: 1067 / 1075 / 1077 / 1128 / 1151
 //   of 2: 1073 / 1141 / 1205 / 1316 / 1313; grid of 1000 x 1000: 30420 / 29239 / 28998 /
 //   28982 / 28986; RMAT scale 20 (uneven): CC 331 / 388 / 392 / 390 / 416
-__device__ __forceinline__ bool by_items(const RegionArgs &a, uint32_t bits, uint32_t range) {
-    return a.items && (uint64_t)bits * a.item_div > range;
+__device__ __forceinline__ bool by_items(const RegionArgs &a, uint32_t region, uint32_t bits, uint32_t range) {
+    return a.items && (region || (uint64_t)bits * a.item_div > range);
 }
 
 // Merge items: a region's rows (each counted at its end) and edges in their
@@ -562,7 +565,7 @@ __device__ __forceinline__ void region_items_bits(const RegionArgs &a, const uin
     const uint32_t nvert = bitmap ? a.dense_end - (a.dense_begin & ~31u) : n_in;
     per = bitmap ? kBlock : min((uint32_t)kBlock, max(kMinTile, (n_in + gridDim.x - 1) / gridDim.x));
     items = nseg + (nvert + per - 1) / per;
-    if (bitmap && by_items(a, bits, range)) {
+    if (bitmap && by_items(a, a.region, bits, range)) {
         per = nseg = 0;
         items = a.item_n;
     }
@@ -1154,8 +1157,8 @@ __device__ __forceinline__ void build_frontier(const RegionArgs &a, const uint32
         else smask = (1u << (a.S - v0)) - 1u;
         // long lists: one thread per vertex appends its segments (rare); merge
         // items need none
-        if (!list0 && by_items(a, bits0, range0)) hw &= ~smask;
-        if (!list1 && by_items(a, bits1, range1)) hw &= smask;
+        if (!list0 && by_items(a, 0, bits0, range0)) hw &= ~smask;
+        if (!list1 && by_items(a, 1, bits1, range1)) hw &= smask;
         while (hw) {
             const int b = __ffs(hw) - 1;
             hw &= hw - 1;
@@ -3717,7 +3720,7 @@ asc_status run_traversal_impl(asc_graph *g, asc_algo algo, uint32_t source, cons
     auto region_work = [&](int region) -> uint64_t {
         const uint32_t range = region == 0 ? g->static_vertices : V - g->static_vertices;
         const bool bitmap_mode = div && cnt[6 + region] > range / div;
-        if (bitmap_mode && !part && (uint64_t)cnt[6 + region] * ws->item_div > range)
+        if (bitmap_mode && !part && (region || (uint64_t)cnt[6 + region] * ws->item_div > range))
             return region == 0 ? ws->n_items_static : ws->n_items - ws->n_items_static;
         const uint32_t per = bitmap_mode ? (uint32_t)kBlock : kMinTile;
         return (uint64_t)cnt[2 + region] + ((bitmap_mode ? range : cnt[region]) + per - 1) / per;
