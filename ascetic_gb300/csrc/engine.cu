@@ -4187,7 +4187,8 @@ struct BatchEngine {
     uint32_t stride = 64;             // SSSP distance row length (sources per row)
     Workspace ws;                     // own frontier lists, bitmaps, counters
     unsigned long long *front = nullptr;
-    ulonglong2 *masks = nullptr;      // per vertex: visited (BFS) and next masks, one 16-byte load
+    ulonglong2 *masks = nullptr;      // BFS, per vertex: visited and next masks, one 16-byte load
+    unsigned long long *next = nullptr;  // SSSP, per vertex: the next mask
     uint32_t *touched = nullptr;      // bitmap of vertices whose next mask went non-zero
     uint32_t *dist = nullptr;         // SSSP [V][stride]
     uint32_t *plane[64] = {nullptr};  // BFS per-slot level planes [V]
@@ -4216,8 +4217,9 @@ enum { CTL_ALIVE = 34 };  // u64 (words 34-35): OR of the new frontier masks of 
 struct MsArgs {
     RegionArgs r0, r1;            // frontier lists/segments/bitmaps of both regions (val unused)
     unsigned long long *front;    // sources for which v is in the current frontier
-    ulonglong2 *masks;            // per vertex: x sources that reached it (BFS), y those that reached it
+    ulonglong2 *masks;            // BFS, per vertex: x sources that reached it, y those that reached it
                                   // in this iteration (atomicOr)
+    unsigned long long *next;     // SSSP: the latter alone (8 bytes per vertex)
     uint32_t *touched;            // bitmap: v's next mask went non-zero this iteration
     uint32_t *work;
     uint32_t *dist;               // SSSP: [V][64]
@@ -4552,7 +4554,7 @@ __device__ __forceinline__ void relax_min(uint32_t *p, uint32_t nd, uint32_t cur
 // Marks v as reached for the sources in imp: 32-bit halves, as every atomic of
 // the batched SSSP on these masks.
 __device__ __forceinline__ void ms_sssp_mark(const MsArgs &m, uint32_t v, unsigned long long imp) {
-    uint32_t *next = reinterpret_cast<uint32_t *>(&m.masks[v].y);
+    uint32_t *next = reinterpret_cast<uint32_t *>(m.next + v);
     if ((uint32_t)imp) atomicOr(next, (uint32_t)imp);
     if ((uint32_t)(imp >> 32)) atomicOr(next + 1, (uint32_t)(imp >> 32));
     atomicOr(&m.touched[v >> 5], 1u << (v & 31));
@@ -4726,7 +4728,7 @@ __device__ __forceinline__ void ms_sssp_chunk(const MsArgs &m, const RegionArgs 
 #pragma unroll
             for (int d = H / 2; d > 0; d >>= 1) im |= __shfl_xor_sync(kFull, im, d);
             if (l % H == 0 && j < nd && im) {
-                atomicOr(reinterpret_cast<uint32_t *>(&m.masks[vk[k]].y) + l / H, im);
+                atomicOr(reinterpret_cast<uint32_t *>(m.next + vk[k]) + l / H, im);
                 atomicOr(&m.touched[vk[k] >> 5], 1u << (vk[k] & 31));
             }
         }
@@ -4854,8 +4856,8 @@ __global__ void ms_apply_kernel(MsArgs m, uint32_t **planes, const int32_t *lvl_
                     nb = now.y & ~now.x;
                     m.masks[v] = make_ulonglong2(now.x | nb, 0);
                 } else {
-                    nb = m.masks[v].y;
-                    m.masks[v].y = 0;
+                    nb = m.next[v];
+                    m.next[v] = 0;
                 }
                 m.front[v] = nb;
                 any |= nb;
@@ -5007,7 +5009,7 @@ __global__ void cb_gather_columns_kernel(const uint32_t *dist, uint32_t stride, 
 
 uint64_t batch_state_bytes(asc_graph *g, bool sssp, uint32_t stride) {
     const uint64_t V = g->V;
-    uint64_t b = 24 * V + 4 * (V / 32 + 2) + 16 * V + 4 * 4 * (V / 32 + 2) + 8 * (g->E / 256 + 1024) + 4096;
+    uint64_t b = (sssp ? 16 : 24) * V + 4 * (V / 32 + 2) + 16 * V + 4 * 4 * (V / 32 + 2) + 8 * (g->E / 256 + 1024) + 4096;
     if (!sssp) b += items_bytes(V, g->E);
     if (sssp) b += 4ull * V * stride + 4 * V;
     return b;
@@ -5065,7 +5067,7 @@ void batch_destroy(BatchEngine *b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     free_ws_buffers(&b->ws);
-    for (void *p : {(void *)b->masks, (void *)b->front, (void *)b->touched, (void *)b->dist,
+    for (void *p : {(void *)b->masks, (void *)b->next, (void *)b->front, (void *)b->touched, (void *)b->dist,
                     (void *)b->d_plane, (void *)b->d_lvl_off, (void *)b->staging})
         if (p) cudaFree(p);
     for (auto p : b->plane)
@@ -5108,7 +5110,8 @@ static asc_status batch_clear(BatchEngine *b, uint64_t columns) {
     ASC_CUDA(cudaMemsetAsync(b->ws.ctl, 0, 4 * CTL_WORDS, b->stream));
     for (auto q : {b->ws.bitmap[0], b->ws.bitmap[1], b->touched})
         ASC_CUDA(cudaMemsetAsync(q, 0, 4 * (V / 32 + 2), b->stream));
-    ASC_CUDA(cudaMemsetAsync(b->masks, 0, 16 * V, b->stream));
+    if (b->sssp) ASC_CUDA(cudaMemsetAsync(b->next, 0, 8 * V, b->stream));
+    else ASC_CUDA(cudaMemsetAsync(b->masks, 0, 16 * V, b->stream));
     ASC_CUDA(cudaMemsetAsync(b->front, 0, 8 * V, b->stream));
     if (b->sssp && columns) {
         cb_clear_kernel<<<fill_grid(&b->ws, V), kBlock, 0, b->stream>>>(b->masks, b->dist, b->stride, b->d_plane,
@@ -5134,7 +5137,8 @@ asc_status batch_create(asc_graph *g, bool sssp, uint32_t stride, BatchEngine **
     auto al = [&](void **p, size_t n) {
         if (st == ASC_OK) st = batch_alloc(b, p, n);
     };
-    al((void **)&b->masks, 16 * V);
+    if (sssp) al((void **)&b->next, 8 * V);
+    else al((void **)&b->masks, 16 * V);
     al((void **)&b->front, 8 * V);
     al((void **)&b->touched, 4 * (V / 32 + 2));
     al((void **)&b->d_plane, 8 * 64);
@@ -5217,6 +5221,7 @@ asc_status batch_launch(BatchEngine *b) {
     memset(&m, 0, sizeof(m));
     m.front = b->front;
     m.masks = b->masks;
+    m.next = b->next;
     m.touched = b->touched;
     m.dist = b->dist;
     m.V = V;
