@@ -5588,24 +5588,42 @@ __global__ void __launch_bounds__(kBlock, ASC_PR_SCATTER_BLOCKS) pr_scatter_item
 #pragma unroll
             for (int k = 0; k < kVt; k++)
                 v[k] = x0 + k < ne ? staged_word(sm.pool, bit0 + (x0 + k) * eb, mask) >> p.wbits : 0u;
-            // consecutive edges to one destination (the leaves of a hub, duplicates) are
+            // Consecutive edges to one destination (the leaves of a hub, duplicates) are
             // one add: FP64 adds to one shared address go one after the other (1,000 hubs
-            // of 2,000 leaves: 28.1 ms an add per edge, 12.4 so)
-            Acc run = (Acc)0;
+            // of 2,000 leaves: 28.1 ms an add per edge, 12.1 so). A warp without any skips
+            // the comparisons, which cost 3 to 5% of an FP64 pass on other graphs.
+            bool same = false;
 #pragma unroll
-            for (int k = 0; k < kVt; k++) {
-                if (x0 + k < ne && !ASC_BAD(v[k] >= p.V, 18, v[k])) {
-                    run += c;
-                    if (k + 1 == kVt || x0 + k + 1 >= ne || v[k + 1 < kVt ? k + 1 : k] != v[k]) {
-                        const uint32_t h = pr_hot_slot(v[k]);
-                        if (hot.key[h] == v[k]) hot.add(h, run);
-                        else atomicAdd(&p.sum[v[k]], run);
-                        run = (Acc)0;
-                    }
+            for (int k = 1; k < kVt; k++) same = same || (v[k] == v[k - 1] && x0 + k < ne);
+            const bool runs = __any_sync(kFull, same);
+            auto add = [&](uint32_t to, Acc x) {
+                const uint32_t h = pr_hot_slot(to);
+                if (hot.key[h] == to) hot.add(h, x);
+                else atomicAdd(&p.sum[to], x);
+            };
+            auto next_row = [&](int k) {
+                if (!((ends >> k) & 1u)) return;
+                const uint32_t rest = ends >> k >> 1;
+                c = share[rest ? sm.row_at[x0 + k + __ffs((int)rest)] : open];
+            };
+            if (!runs) {
+#pragma unroll
+                for (int k = 0; k < kVt; k++) {
+                    if (x0 + k < ne && !ASC_BAD(v[k] >= p.V, 18, v[k])) add(v[k], c);
+                    next_row(k);
                 }
-                if ((ends >> k) & 1u) {
-                    const uint32_t rest = ends >> k >> 1;
-                    c = share[rest ? sm.row_at[x0 + k + __ffs((int)rest)] : open];
+            } else {
+                Acc run = (Acc)0;
+#pragma unroll
+                for (int k = 0; k < kVt; k++) {
+                    if (x0 + k < ne && !ASC_BAD(v[k] >= p.V, 18, v[k])) {
+                        run += c;
+                        if (k + 1 == kVt || x0 + k + 1 >= ne || v[k + 1 < kVt ? k + 1 : k] != v[k]) {
+                            add(v[k], run);
+                            run = (Acc)0;
+                        }
+                    }
+                    next_row(k);
                 }
             }
         }
