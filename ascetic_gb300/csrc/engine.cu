@@ -845,10 +845,10 @@ __global__ void __launch_bounds__(kBlock, ASC_EXPAND_MIN_BLOCKS) expand_fused_ke
 
 // Bottom-up BFS step (direction-optimizing BFS): every vertex not yet reached
 // scans its in-edges, from the one whose source has the most out-edges on, for a
-// parent in this iteration's frontier and stops at the first one; a vertex found takes the parent's value
-// + 1 (the level-synchronous top-down step gives every unreached vertex with a
-// frontier in-neighbour the same value, so levels are identical) and joins the
-// next frontier. When the frontier is a large part of the graph, most unreached
+// parent in this iteration's frontier and stops at the first one; a vertex found
+// takes the parent's value + 1 (the level-synchronous top-down step gives every
+// unreached vertex with a frontier in-neighbour the same value, so levels are
+// identical) and joins the next frontier. When the frontier is a large part of the graph, most unreached
 // vertices find a parent among their first in-edges, so the step reads far
 // fewer edge bytes over the host link than expanding the frontier's out-lists.
 // A warp takes bitmap words of 32 vertices, lane = vertex, and writes the bits of
